@@ -272,6 +272,12 @@ OCTEX_B200_EXPORT cuvsError_t octexB200Attach(cuvsResources_t res, const octexB2
                                               cuvsOctexLoadParams_t params, int32_t rank,
                                               int32_t world, cuvsOctexIndex_t index);
 
+/* octexB200Search, returning when the results are in their arrays (searches with device memory are
+ * otherwise only queued on the stream of `res`) and reporting what octexB200CheckLast would. */
+OCTEX_B200_EXPORT cuvsError_t octexB200SearchWait(cuvsResources_t res, cuvsOctexSearchParams_t params,
+                                                  cuvsOctexIndex_t index, const float* queries,
+                                                  int64_t n_queries, int64_t dim, int64_t* neighbors,
+                                                  float* distances, int64_t k, int32_t on_device);
 /* detail::resident_search (cpp/src/neighbors/octex/search.cu:983-997): search again the queries of
  * the previous call, which are still on the GPU, and leave the results there. The timing protocol
  * of the reference's benchmark uses it (cpp/bench/octex_bench.cu:223-253). */

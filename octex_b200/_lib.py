@@ -89,7 +89,7 @@ SYMBOLS = (
     "cuvsOctexIndexGetDim", "cuvsOctexIndexGetCopies", "cuvsOctexIndexGetNumDevices",
     "cuvsOctexIndexGetDevices", "cuvsOctexIndexGetDeviceBytes", "cuvsOctexBuild", "cuvsOctexLoad",
     "cuvsOctexSearch", "octexB200Search", "octexB200LoadRank", "octexB200Attach",
-    "octexB200SearchResident", "octexB200ProfileBatch", "octexB200SetDebug", "octexB200Fetch",
+    "octexB200SearchWait", "octexB200SearchResident", "octexB200ProfileBatch", "octexB200SetDebug", "octexB200Fetch",
     "octexB200CellCodes", "octexB200QueryCodesStatic", "octexB200SetProjection",
     "octexB200CommUniqueId", "octexB200CommInit", "octexB200CommDisconnect", "octexB200CheckLast",
     "octexB200MemoryReport", "octexB200Build", "octexB200ExactNeighbors", "octexB200SetTable", "octexB200SearchedTable",
@@ -108,6 +108,9 @@ def lib():
         L = C.CDLL(LIB_PATH)
         L.cuvsGetLastErrorText.restype = C.c_char_p
         L.cuvsSetLastErrorText.restype = None
+        # the call of every search takes plain Python numbers: no argument objects to build
+        L.octexB200SearchWait.argtypes = [C.c_size_t, C.POINTER(SearchParams), C.POINTER(IndexHandle), C.c_void_p,
+                                          C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32]
         _lib = L
     return _lib
 

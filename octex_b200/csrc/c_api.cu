@@ -89,7 +89,7 @@ auto as_index(cuvsOctexIndex const& index) -> octex_b200::index*
   return reinterpret_cast<octex_b200::index*>(index.addr);
 }
 
-/// Report (once) a kernel of the last batches that gave up; the stream of the index is idle.
+/// Wait for the last batches and report (once) a kernel of theirs that gave up.
 void check_last(octex_b200::detail::index_impl& ix)
 {
   std::vector<std::shared_ptr<octex_b200::detail::plan>> plans;
@@ -98,8 +98,14 @@ void check_last(octex_b200::detail::index_impl& ix)
     for (auto const& kv : ix.plans)
       plans.push_back(kv.second);
   }
-  for (auto const& pl : plans)
+  for (auto const& pl : plans) {
+    if (pl == nullptr) continue;
+    {
+      std::lock_guard<std::mutex> lock(pl->mu);
+      if (pl->used) OCTEX_CUDA_TRY(cudaEventSynchronize(pl->done_ev));
+    }
     octex_b200::detail::check_tc(*pl);
+  }
 }
 
 template <typename T>
@@ -464,6 +470,20 @@ cuvsError_t octexB200Search(cuvsResources_t res, cuvsOctexSearchParams_t params,
   });
 }
 
+cuvsError_t octexB200SearchWait(cuvsResources_t res, cuvsOctexSearchParams_t params,
+                                cuvsOctexIndex_t index, const float* queries, int64_t n_queries,
+                                int64_t dim, int64_t* neighbors, float* distances, int64_t k,
+                                int32_t on_device)
+{
+  return translate([=] {
+    OCTEX_EXPECTS(params != nullptr && index != nullptr, "octex: a search argument is NULL");
+    OCTEX_EXPECTS(n_queries == 0 || (queries != nullptr && neighbors != nullptr && distances != nullptr),
+                  "octex: a search array is NULL");
+    octex_b200::detail::search_impl(as_res(res), to_cpp(*params), *as_index(*index), queries,
+                                    n_queries, dim, neighbors, distances, k, on_device == 0, false, true);
+  });
+}
+
 cuvsError_t octexB200SearchResident(cuvsResources_t res, cuvsOctexSearchParams_t params,
                                     cuvsOctexIndex_t index, int64_t n_queries, int64_t k)
 {
@@ -511,7 +531,7 @@ cuvsError_t octexB200MemoryReport(cuvsOctexIndex_t index, int64_t* bytes)
     auto const& p = ix.part;
     auto dev = [](octex_b200::dbuf const& b) { return b.host ? int64_t{0} : static_cast<int64_t>(b.size); };
     bytes[0] = p.device;
-    bytes[1] = dev(p.lists) + dev(p.base) + dev(p.cell_table) + dev(p.cell_off) + dev(p.cell_mask) + dev(p.level_on);
+    bytes[1] = dev(p.lists) + dev(p.base) + dev(p.cell_table) + dev(p.cell_keys) + dev(p.cell_levels);
     bytes[2] = dev(p.sketch) + dev(p.sketch_norm);
     bytes[3] = dev(p.table);
     bytes[4] = dev(p.vectors);
@@ -520,7 +540,7 @@ cuvsError_t octexB200MemoryReport(cuvsOctexIndex_t index, int64_t* bytes)
     bytes[6] = 0;
     std::lock_guard<std::mutex> lock(ix.mu);
     for (auto const& kv : ix.plans)
-      bytes[6] += kv.second->buffer_bytes;
+      if (kv.second != nullptr) bytes[6] += kv.second->buffer_bytes;
   });
 }
 
@@ -621,13 +641,16 @@ cuvsError_t octexB200Fetch(cuvsOctexIndex_t index, const char* name, void* dst, 
     else if (n == "phase_rows") b = &pl->phase2;
     OCTEX_EXPECTS(b != nullptr, "octex: unknown array name \"" + n + "\"");
     OCTEX_EXPECTS(b->ptr != nullptr, "octex: \"" + n + "\" is not kept (see octexB200SetDebug)");
-    if (bytes != nullptr) *bytes = static_cast<int64_t>(b->size);
+    // the rows of the last batch; every one of these arrays has a row per query
+    const size_t size = b->size / static_cast<size_t>(std::max(pl->cap, 1)) * static_cast<size_t>(rows_used(*pl));
+    if (bytes != nullptr) *bytes = static_cast<int64_t>(size);
     if (dst == nullptr) return;
-    OCTEX_EXPECTS(capacity >= static_cast<int64_t>(b->size), "octex: the destination is too small");
+    OCTEX_EXPECTS(capacity >= static_cast<int64_t>(size), "octex: the destination is too small");
     std::lock_guard<std::mutex> lock(pl->mu);
     OCTEX_CUDA_TRY(cudaSetDevice(pl->device));
+    if (pl->used) OCTEX_CUDA_TRY(cudaEventSynchronize(pl->done_ev));
     OCTEX_CUDA_TRY(cudaStreamSynchronize(ix.part.stream));
-    OCTEX_CUDA_TRY(cudaMemcpy(dst, b->ptr, b->size, cudaMemcpyDeviceToHost));
+    OCTEX_CUDA_TRY(cudaMemcpy(dst, b->ptr, size, cudaMemcpyDeviceToHost));
   });
 }
 

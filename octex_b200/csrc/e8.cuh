@@ -220,4 +220,131 @@ __device__ __forceinline__ long long cell_code_tame(const float (&y)[8 * B], flo
   return finish_code(h);
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same code again with half the instructions of block_code_tame (117 against 248), for the
+// kernel that decodes every query. Rounding v to r leaves e = v - r (exact); the other coset leaves
+// 1/2 - |e| in every coordinate. With A = sum |e|, m = max |e|, n = min |e| the squared errors of the
+// two cosets after their parity repairs differ by
+//     D = A - 2 + (odd ? 1 - 2 m : 0) - (odd' ? 2 n : 0)
+// so the nearer coset is known before either is worked out, and only the one taken is repaired. D is
+// good to 4e-6 (eight additions of terms up to 1/2, and the 2^-25 by which v - 1/2 may be rounded), and
+// the two sums that block_code_tame compares, of at most eight squares up to 1, to 1e-6 each: where
+// |D| < 2e-5 the block is `doubtful` and goes to block_code_tame. The rest is exact: both parities come
+// from the low bits of the rounded values, and the coset taken is rounded and repaired by the same
+// operations on the same values as in nearest_d8_tame. Two coordinates at a time share an instruction
+// (the packed fp32 arithmetic of sm_100, each half rounded as on its own).
+
+struct f32_pair {
+  unsigned long long v;
+};
+__device__ __forceinline__ f32_pair pack2(float lo, float hi)
+{
+  f32_pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ void unpack2(f32_pair p, float& lo, float& hi)
+{
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v));
+}
+__device__ __forceinline__ f32_pair add2(f32_pair a, f32_pair b)
+{
+  f32_pair d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ f32_pair mul2(f32_pair a, f32_pair b)
+{
+  f32_pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ f32_pair fma2(f32_pair a, f32_pair b, f32_pair c)
+{
+  f32_pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+__device__ __forceinline__ float max3_abs(float a, float b, float c)
+{
+  return fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c));
+}
+__device__ __forceinline__ float min3_abs(float a, float b, float c)
+{
+  return fminf(fminf(fabsf(a), fabsf(b)), fabsf(c));
+}
+
+/// Block code of the four pairs y scaled by inv; primes: the eight cell primes in shared memory.
+__device__ __forceinline__ unsigned long long block_code_fast(const f32_pair (&y)[4], float inv,
+                                                              const unsigned long long* primes, bool& doubtful)
+{
+  const f32_pair up = pack2(kRintMagic, kRintMagic), down = pack2(-kRintMagic, -kRintMagic);
+  const f32_pair minus1 = pack2(-1.f, -1.f), less_half = pack2(-0.5f, -0.5f), scale = pack2(inv, inv);
+  f32_pair v[4];
+  float e[8], M[8], H[8];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[i]             = mul2(y[i], scale);
+    const f32_pair b = add2(v[i], up);
+    const f32_pair d = fma2(add2(b, down), minus1, v[i]);
+    const f32_pair h = add2(add2(v[i], less_half), up);
+    unpack2(b, M[2 * i], M[2 * i + 1]);
+    unpack2(d, e[2 * i], e[2 * i + 1]);
+    unpack2(h, H[2 * i], H[2 * i + 1]);
+  }
+  unsigned odd_i = 0, odd_h = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    odd_i ^= __float_as_uint(M[i]);
+    odd_h ^= __float_as_uint(H[i]);
+  }
+  const float A = ((fabsf(e[0]) + fabsf(e[1])) + (fabsf(e[2]) + fabsf(e[3]))) +
+                  ((fabsf(e[4]) + fabsf(e[5])) + (fabsf(e[6]) + fabsf(e[7])));
+  const float m = fmaxf(max3_abs(e[0], e[1], e[2]), fmaxf(max3_abs(e[3], e[4], e[5]), fmaxf(fabsf(e[6]), fabsf(e[7]))));
+  const float n = fminf(min3_abs(e[0], e[1], e[2]), fminf(min3_abs(e[3], e[4], e[5]), fminf(fabsf(e[6]), fabsf(e[7]))));
+  float D = A - 2.f;
+  if (odd_i & 1u) D += fmaf(-2.f, m, 1.f);
+  if (odd_h & 1u) D = fmaf(-2.f, n, D);
+  doubtful         = fabsf(D) < 2e-5f;
+  const bool halves = D > 0.f;
+  const bool odd    = ((halves ? odd_h : odd_i) & 1u) != 0;
+  // the coset taken, from its own rounding on
+  const f32_pair off = halves ? less_half : pack2(0.f, 0.f);
+  float c[8];
+  unsigned long long sum = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const f32_pair w = add2(v[i], off);
+    const f32_pair b = add2(w, up);
+    const f32_pair d = fma2(add2(b, down), minus1, w);
+    unpack2(d, c[2 * i], c[2 * i + 1]);
+    float lo, hi;
+    unpack2(b, lo, hi);
+    sum += static_cast<unsigned long long>(__float_as_uint(lo)) * cell_prime(2 * i);
+    sum += static_cast<unsigned long long>(__float_as_uint(hi)) * cell_prime(2 * i + 1);
+  }
+  // the worst rounded coordinate, the first of equal ones: a tree in which the left side stays unless
+  // the right one is strictly larger
+  int at[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+    at[i] = i;
+#pragma unroll
+  for (int s = 1; s < 8; s <<= 1)
+#pragma unroll
+    for (int i = 0; i < 8; i += 2 * s) {
+      const bool right = fabsf(c[i + s]) > fabsf(c[i]);
+      c[i]             = right ? c[i + s] : c[i];
+      at[i]            = right ? at[i + s] : at[i];
+    }
+  const unsigned long long prime = primes[at[0]];
+  unsigned long long step        = c[0] >= 0.f ? prime : 0ULL - prime;
+  step                           = odd ? step : 0ULL;
+  constexpr unsigned long long all = cell_prime(0) + cell_prime(1) + cell_prime(2) + cell_prime(3) + cell_prime(4) +
+                                     cell_prime(5) + cell_prime(6) + cell_prime(7);
+  // twice the coordinates: 2 (bits - 0x4B400000), plus 1 in the half coset
+  const unsigned long long constant = halves ? all - 2 * 0x4B400000ULL * all : 0ULL - 2 * 0x4B400000ULL * all;
+  return 2 * (sum + step) + constant;
+}
+
 }  // namespace octex_b200

@@ -3,10 +3,11 @@
 // Layout (the reference's is in cpp/src/neighbors/octex/detail/index_impl.hpp:115-177 of
 // hpdic/octex; differences are marked *):
 //   lists   i32 [Cg, stride]     cell rows of list_len ids, nearest to the cell centre first
-// * cell_table {i64 key, i32 row, pad} [sum of the (copy, level) table sizes]: the cells of every
-//                                (copy, level) in an open-addressing table at most half full (slot =
-//                                low bits of the code, linear probing), with cell_off i64 [Cg, L]
-//                                (first slot) and cell_mask i32 [Cg, L] (slots - 1). Built at placement
+// * cell_table {i32 tag, i32 row} [sum of the (copy, level) table sizes]: the cells of every
+//                                (copy, level) in an open-addressing table at most a quarter full
+//                                (buckets of four slots by the low bits of the code, linear probing from
+//                                there; tag = high half of the code), cell_keys i64 [cells] the whole
+//                                codes in list order, cell_levels [Cg, L] where both begin. Built at placement
 //                                from the directory's keys i64 [C, L, mmax] and the cell counts in its
 //                                offsets i32 [C, L, T + 1]; the reference keeps those two arrays on the
 //                                GPU and walks a bucket of keys per lookup
@@ -17,7 +18,6 @@
 //   shift   f16 [Cg * 8b]        inv_f f32 [L]     mean f32 [dim]
 //   basis   f32 [dim, S]         scale f32 [S]     sketch i8 [n, S]
 //   vectors f16 [n, dim]         table i32 [n, table_len]
-// * level_on u8 [Cg, L]          1 when the level of the copy holds at least one cell
 // * sketch_norm f32 [n]          sum_k (code_k scale_k)^2 of every sketch row, computed at placement
 //                                (the row's constant in the integer form of the sketch distance)
 #pragma once
@@ -65,8 +65,8 @@ struct device_part {
   int64_t stride = 0;
   int64_t mmax   = 0;
   int ldu        = 0;
-  dbuf lists, base, ut, shift, inv_f, mean, basis, scale, sketch, vectors, table, level_on;
-  dbuf cell_table, cell_off, cell_mask;  // open-addressing table of the cells of every (copy, level)
+  dbuf lists, base, ut, shift, inv_f, mean, basis, scale, sketch, vectors, table;
+  dbuf cell_table, cell_keys, cell_levels;  // open-addressing table of the cells of every (copy, level)
   dbuf sketch_norm;                      // f32 [n]: sum_k (code_k scale_k)^2 of every sketch row
   dealt_rows table_rows, sketch_rows, vector_rows;
   cudaStream_t stream = nullptr;
@@ -104,6 +104,10 @@ struct index_impl {
   std::mutex mu;  // guards plans
   std::map<std::string, std::shared_ptr<plan>> plans;
   debug_options debug;
+  // recorded on the caller's stream at the start of a search that runs on the index's own streams
+  std::mutex start_mu;
+  cudaEvent_t start_ev = nullptr;
+  int start_dev        = -1;  // device it was created on
   std::unique_ptr<communicator> comm;  // set when world > 1 (octexB200CommInit)
   ~index_impl();
 };

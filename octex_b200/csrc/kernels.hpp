@@ -49,63 +49,90 @@ void project_ordered(const __half* qh, int ldq, const __half* ut, int ldu, const
 void decode_codes(const __half* Y, int64_t pairs, int C, int blocks, int L, const float* inv_f,
                   const unsigned char* level_on, long long* codes, cudaStream_t s);
 
-/// Tensor-core projection with the decode in its epilogue (project_tc.cu): TMA tensor maps of the
-/// two operands, made once per plan.
+/// The sketch-space queries of a batch, computed by extra blocks of the projection's launch:
+/// qs [m, S] = (q - mean) @ basis in fp32 (one fused multiply-add per dimension, in dimension
+/// order); keep [m, D] (may be null) receives a copy of the queries.
+struct sketch_job {
+  const float* q     = nullptr;  // [m, D], device-readable
+  const float* mean  = nullptr;
+  const float* basis = nullptr;
+  int m = 0, D = 0, S = 0;
+  float* qs   = nullptr;
+  float* keep = nullptr;
+};
+
+/// Tensor-core projection with the decode in its epilogue (project_tc.cu): TMA tensor map of the
+/// projections, made once per plan.
 struct project_tc_plan {
-  alignas(64) unsigned char map_a[128];  // fp16 queries [m, ldu]
   alignas(64) unsigned char map_b[128];  // fp16 projections [copies * 32, ldu]
-  int m = 0, copies = 0, ldu = 0;
+  int copies = 0, ldu = 0, sms = 1;
 };
 /// The cell lookup done inside the projection's epilogue (table == nullptr: not done there; the
-/// codes are written out for the separate kernel instead). Needs level_on.
+/// codes are written out for the separate kernel instead).
 struct cell_slot;
+/// The cells of a (copy, level): first slot of its table, its first code in the array of codes, slots
+/// - 1 (-1: the level has no cell), first list row of the level inside the copy.
+struct cell_level {
+  long long off;
+  long long keys;
+  int mask;
+  int base;
+};
 struct tc_lookup {
-  const cell_slot* table = nullptr;
-  const long long* toff  = nullptr;
-  const int* tmask       = nullptr;
-  const int* base        = nullptr;
+  const cell_slot* table   = nullptr;
+  const long long* keys    = nullptr;  // codes of the cells, per level in list order
+  const cell_level* levels = nullptr;  // [copies, L]
   int list_len = 0, lr = 0;
   int2* seg        = nullptr;  // [m, copies]
   long long* stats = nullptr;  // [m, 8] += (levels tried, slots examined), may be null
 };
 /// True when the tensor-core kernel covers this index shape (4 blocks per copy).
 bool project_tc_supported(int blocks, int ldu);
-void project_tc_setup(project_tc_plan& p, const __half* qh, int m, const __half* ut, int copies, int ldu);
-/// codes [m, copies, L] (and Yout [m, copies * 32] fp16 when not null) from the operands of the
-/// plan. *error (device-visible int) becomes non-zero when a wait inside the kernel ran out.
-/// finest = the smallest spacing (host copy): coordinates small against it take the short decode.
-/// With look.table set, the lookup of the cells happens in the same kernel: seg is written, codes
-/// is not.
-void project_decode_tc(const project_tc_plan& p, int L, const __half* shift, const float* inv_f,
-                       float finest, const unsigned char* level_on, long long* codes, __half* Yout,
+void project_tc_setup(project_tc_plan& p, const __half* ut, int copies, int ldu, int sms);
+/// The job's sketch-space queries, and seg of every (query, copy), or with look.table null the codes
+/// [m, copies, L] (and Yout [m, copies * 32] fp16 when not null). *error (device-visible int)
+/// becomes non-zero when a wait inside the kernel ran out. finest = the smallest spacing (host
+/// copy): coordinates small against it take the short decode.
+void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, const __half* shift, const float* inv_f,
+                       float finest, long long* codes, __half* Yout,
                        const tc_lookup& look, int* error, cudaStream_t s);
+/// The same step for indexes of another number of blocks per copy (project_ord.cu): projection in
+/// dimension order (the order of project_ordered), decode and lookup in one kernel.
+void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
+                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, cudaStream_t s);
 
 /// codes [n] = cell code of each row of y [n, 8*blocks] float32 scaled by inv_f.
 void cell_codes_f32(const float* y, int64_t n, int blocks, float inv_f, long long* codes,
                     cudaStream_t s);
 
-/// One slot of the cell table of a (copy, level): the 64-bit code of a cell and the row of its list
-/// among the level's cells (-1: empty slot). 16 bytes: a lookup reads one 32-byte sector, where the
-/// reference's bucket array plus key array (detail/search_kernels.cuh:100-126) costs two dependent
-/// ones.
+/// One slot of the cell table of a (copy, level): the high half of a cell's 64-bit code and the row of
+/// its list among the level's cells (-1: empty slot). Four slots are a bucket of 32 bytes, one memory
+/// sector, and at no more than a quarter full nearly every lookup ends in its first bucket: one random
+/// sector, where the reference's bucket array plus key array (detail/search_kernels.cuh:100-126) costs
+/// two dependent ones. The low half of a code has chosen the bucket; a hit is confirmed against the
+/// whole code (cell_level::keys), which a lookup reads once, when it has found its level.
 struct cell_slot {
-  long long key;
+  int tag;
   int row;
-  int pad;
 };
+__host__ __device__ inline int cell_tag(long long code) { return static_cast<int>(code >> 32); }
+/// Home slot of a code in a table of mask + 1 slots: the first of a bucket of four, from which the
+/// probing is linear.
+__host__ __device__ inline unsigned cell_home(long long code, unsigned mask)
+{
+  return static_cast<unsigned>(code) & mask & ~3u;
+}
 
 /// Fill the open-addressing tables of CL (copy, level) pairs from their key arrays: pair cl holds
-/// ncells[cl] codes keys[cl * mmax + p], p = row of the cell; its table is table + toff[cl],
-/// tmask[cl] + 1 slots (a power of two, at least twice the cells), home slot = low bits of the code.
-/// The table must be filled with 0xff bytes before (row -1 everywhere).
-void build_cell_tables(const long long* keys, int64_t mmax, const int* ncells, const long long* toff,
-                       const int* tmask, int CL, cell_slot* table, cudaStream_t s);
+/// ncells[cl] codes keys[cl * mmax + p], p = row of the cell; its level is levels[cl]. The table must
+/// be filled with 0xff bytes before (row -1 everywhere); packed receives the codes at
+/// levels[cl].keys.
+void build_cell_tables(const long long* keys, int64_t mmax, const int* ncells, const cell_level* levels, int CL,
+                       cell_slot* table, long long* packed, cudaStream_t s);
 
 /// seg [m, C] = (first list entry, entries read) of the finest level whose cell holds a list,
 /// (0, 0) when none does. stats (may be null) [m, 2] += (levels tried, table slots examined).
-void probe(const long long* codes, int m, int C, int L, const cell_slot* table, const long long* toff,
-           const int* tmask, const int* base, const unsigned char* level_on, int list_len, int lr,
-           int2* seg, long long* stats, cudaStream_t s);
+void probe(const long long* codes, int m, int C, int L, const tc_lookup& look, cudaStream_t s);
 
 /// norm [rows] = sum_k (code_k * scale_k)^2 of each row of codes [rows, S] as fp32 (one fused
 /// multiply-add per code, in code order): the part of the sketch distance that depends on the row
@@ -163,8 +190,13 @@ struct round_args {
   int hash_twelfths = 16;  // slots per 12 gathered entries (host: as sparse as shared memory allows)
   int keep_sketch = 0;  // the sketch and its row constants fit the L2 cache with room to spare: load them
                         // with an evict-last policy, the large arrays with evict-first (host decides)
-  int threads = kRoundThreads;  // threads per query block: 128, 256 or 512 (host: the smallest
+  int threads = kRoundThreads;  // threads per query block in a large batch: 128 to 1024 (host: the smallest
                                 // that still fills a multiprocessor with the blocks that fit it)
+  int sms = 1;                  // multiprocessors of the GPU
+  // the results of the search, when this round is its last: the first k kept entries [m, k]
+  long long* out_i = nullptr;
+  float* out_d     = nullptr;
+  int k            = 0;
   int nmax = 0;       // capacity of the candidate / distance arrays
   int P = 0;          // keys sorted by the merge (power of two >= KO)
   int* cand_global = nullptr;    // [m, nmax] when the candidates do not fit shared memory

@@ -22,6 +22,7 @@ namespace detail {
 index_impl::~index_impl()
 {
   plans.clear();
+  if (start_ev != nullptr) cudaEventDestroy(start_ev);
 }
 
 namespace {
@@ -223,15 +224,16 @@ void place(index_impl& ix, source_arrays const& src)
 
   // The cells of every (copy, level). The directory holds them as CSR bucket bounds over sorted
   // keys (offsets [C, L, T + 1], keys [C, L, mmax]: build.cu:215-349 of the reference); the kernels
-  // here look them up in one open-addressing table per (copy, level), slot = (key, row of the
-  // cell), at most half full, built on the GPU from the keys. The last CSR bound of a level is its
+  // here look them up in one open-addressing table per (copy, level), slot = (half of the key, row of
+  // the cell), at most a quarter full, built on the GPU from the keys. The last CSR bound of a level is its
   // cell count; the bucket bounds themselves never go to the GPU.
   {
     const int CL = Cg * L;
-    std::vector<int> ncells(CL), mask(CL);
-    std::vector<long long> off(CL);
-    std::vector<unsigned char> on(static_cast<size_t>(CL));
-    long long slots = 0;
+    std::vector<int> ncells(CL);
+    std::vector<int32_t> first(CL);
+    st.fetch(first.data(), p.base.ptr, sizeof(int32_t) * CL);
+    std::vector<kernels::cell_level> levels(CL);
+    long long slots = 0, cells = 0;
     for (int c = 0; c < Cg; c++)
       for (int j = 0; j < L; j++) {
         int32_t last = 0;
@@ -239,20 +241,17 @@ void place(index_impl& ix, source_arrays const& src)
         OCTEX_EXPECTS(last >= 0 && last <= p.mmax, "octex: a level's cell count exceeds its key array");
         const int k = c * L + j;
         ncells[k]   = last;
-        on[k]       = last > 0;
-        int cap     = 4;
-        while (cap < 2 * last)
+        int64_t cap = 4;
+        while (cap < 4 * int64_t{last})
           cap <<= 1;
-        mask[k] = cap - 1;
-        off[k]  = slots;
+        OCTEX_EXPECTS(cap <= int64_t{1} << 31, "octex: too many cells in a level");
+        levels[k] = {slots, cells, last > 0 ? static_cast<int>(cap - 1) : -1, first[k]};
         slots += cap;
+        cells += last;
       }
-    own(p.level_on, on.size());
-    st.copy(p.level_on.ptr, on.data(), on.size());
-    own(p.cell_off, sizeof(long long) * CL);
-    st.copy(p.cell_off.ptr, off.data(), p.cell_off.size);
-    own(p.cell_mask, sizeof(int) * CL);
-    st.copy(p.cell_mask.ptr, mask.data(), p.cell_mask.size);
+    own(p.cell_levels, sizeof(kernels::cell_level) * CL);
+    st.copy(p.cell_levels.ptr, levels.data(), p.cell_levels.size);
+    own(p.cell_keys, sizeof(long long) * static_cast<size_t>(std::max<long long>(cells, 1)));
     own(p.cell_table, sizeof(kernels::cell_slot) * static_cast<size_t>(slots));
     OCTEX_CUDA_TRY(cudaMemsetAsync(p.cell_table.ptr, 0xff, p.cell_table.size, p.stream));
     // the keys of this process's copies on the GPU for the duration of the build
@@ -261,8 +260,8 @@ void place(index_impl& ix, source_arrays const& src)
     put(keys, a.keys, static_cast<size_t>(L) * p.mmax * sizeof(int64_t));
     p.bytes = before;  // not kept
     st.copy(counts.ptr, ncells.data(), counts.size);
-    kernels::build_cell_tables(keys.as<long long>(), p.mmax, counts.as<int>(), p.cell_off.as<long long>(),
-                               p.cell_mask.as<int>(), CL, p.cell_table.as<kernels::cell_slot>(), p.stream);
+    kernels::build_cell_tables(keys.as<long long>(), p.mmax, counts.as<int>(), p.cell_levels.as<kernels::cell_level>(), CL,
+                               p.cell_table.as<kernels::cell_slot>(), p.cell_keys.as<long long>(), p.stream);
     OCTEX_CUDA_TRY(cudaStreamSynchronize(p.stream));
   }
 

@@ -9,7 +9,7 @@
 
 #include "kernels.hpp"
 
-#include "e8.cuh"
+#include "prep_common.cuh"
 
 #include <cfloat>
 #include <cmath>
@@ -205,125 +205,77 @@ __global__ void decode_codes_kernel(const __half* __restrict__ Y,
   }
 }
 
-// Cell code of rows of 8 * B float32 coordinates at one scale (the device function on its own,
-// for checks against other implementations of the decode).
+// Cell code of rows of 8 * B float32 coordinates at one scale (the decode of the search kernels on
+// its own, for checks against other implementations of it).
 template <int B>
 __global__ void cell_codes_f32_kernel(const float* __restrict__ y, int64_t n, float inv_f,
                                       long long* __restrict__ codes)
 {
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  float v[8 * B];
-  // rows small against the spacing take the short decode, as in the projection's epilogue
-  const float tame_y = inv_f > 0.f ? 0.99f * kTameLimit / inv_f : 0.f;
-  bool wild          = false;
+  constexpr int kG = kGroup<B>;
+  __shared__ unsigned long long primes[8];
+  fill_primes(primes);
+  __syncthreads();
+  const int sub   = threadIdx.x % kG;
+  const int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kG;
+  group_decoder<B> dec(sub, primes);
+  const float* own = y + (t < n ? t : n - 1) * 8 * B + sub * 8 * group_decoder<B>::kOwn;
 #pragma unroll
-  for (int i = 0; i < 8 * B; i++) {
-    v[i] = y[t * 8 * B + i];
-    wild = wild || !(fabsf(v[i]) < tame_y);
-  }
-  codes[t] = wild ? cell_code<B>(v, inv_f) : cell_code_tame<B>(v, inv_f);
+  for (int i = 0; i < 4 * group_decoder<B>::kOwn; i++)
+    dec.y[i] = pack2(own[2 * i], own[2 * i + 1]);
+  dec.settle(inv_f > 0.f ? 0.99f * kTameLimit / inv_f : 0.f);
+  const long long code = dec.code(inv_f);
+  if (t < n && sub == 0) codes[t] = code;
 }
 
 // ---- cell lookup -----------------------------------------------------------------------------
 
-// The cells of a (copy, level) in an open-addressing table (slot = low bits of the 64-bit code,
-// linear probing): what the reference keeps as a bucket-bound array plus a key array
-// (search_kernels.cuh:100-126), re-laid so that a lookup costs one random 32-byte sector instead of
-// two dependent ones. Built once when the index is placed.
+// The cells of a (copy, level) in an open-addressing table (cell_slot): what the reference keeps as a
+// bucket-bound array plus a key array (search_kernels.cuh:100-126), re-laid so that a lookup costs one
+// random 32-byte sector instead of two dependent ones. Built once when the index is placed.
 __global__ void fill_cell_tables_kernel(const long long* __restrict__ keys,
                                         int64_t mmax,
                                         const int* __restrict__ ncells,
-                                        const long long* __restrict__ toff,
-                                        const int* __restrict__ tmask,
-                                        cell_slot* __restrict__ table)
+                                        const cell_level* __restrict__ levels,
+                                        cell_slot* __restrict__ table,
+                                        long long* __restrict__ packed)
 {
   const int cl = blockIdx.y;
   const int p  = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= ncells[cl]) return;
-  const long long key = keys[static_cast<int64_t>(cl) * mmax + p];
-  const unsigned mask = static_cast<unsigned>(tmask[cl]);
-  cell_slot* mine     = table + toff[cl];
-  unsigned s          = static_cast<unsigned>(key) & mask;
+  const long long key  = keys[static_cast<int64_t>(cl) * mmax + p];
+  const cell_level lv  = levels[cl];
+  packed[lv.keys + p]  = key;
+  const unsigned mask  = static_cast<unsigned>(lv.mask);
+  cell_slot* mine      = table + lv.off;
+  unsigned s           = cell_home(key, mask);
   for (unsigned probe = 0; probe <= mask; probe++) {
     if (atomicCAS(&mine[s].row, -1, p) == -1) {
-      mine[s].key = key;  // nobody reads the table before this kernel is over
+      mine[s].tag = cell_tag(key);  // nobody reads the table before this kernel is over
       return;
     }
     s = (s + 1) & mask;
   }
 }
 
-// search_kernels.cuh:100-126: the finest level whose cell holds a list. One thread per
-// (query, copy). The codes of all levels are already there, so the home slot of every level is
-// fetched at once (one 16-byte load each): one memory round trip for the common case instead of
-// two per level tried. The answer is that of the level-by-level walk.
-constexpr int kProbeLevels = 8;  // levels handled in one sweep; more are walked in further sweeps
-__global__ void probe_kernel(const long long* __restrict__ codes,
-                             int64_t pairs,
-                             int C,
-                             int L,
-                             const cell_slot* __restrict__ table,
-                             const long long* __restrict__ toff,
-                             const int* __restrict__ tmask,
-                             const int* __restrict__ base,
-                             const unsigned char* __restrict__ level_on,
-                             int list_len,
-                             int lr,
-                             int2* __restrict__ seg,
-                             long long* __restrict__ stats)
+// search_kernels.cuh:100-126: the finest level whose cell holds a list, from codes of all levels kept
+// for inspection. One thread per (query, copy).
+__global__ void probe_kernel(const long long* codes, int64_t pairs, int C, int L, const tc_lookup look)
 {
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= pairs) return;
   const int c = static_cast<int>(t % C);
-  int2 sg     = make_int2(0, 0);
-  long long tried = 0, scanned = 0;
-  bool found = false;
-  for (int j0 = 0; j0 < L && !found; j0 += kProbeLevels) {
-    long long h[kProbeLevels];
-    int4 first[kProbeLevels];  // the home slot: (key low, key high, row, pad)
-    bool on[kProbeLevels];
-#pragma unroll
-    for (int u = 0; u < kProbeLevels; u++) {
-      const int j = j0 + u;
-      on[u]       = j < L && (level_on == nullptr || level_on[c * L + j]);
-      h[u]        = 0;
-      first[u]    = make_int4(0, 0, -1, 0);
-      if (on[u]) {
-        const int cl = c * L + j;
-        h[u]         = codes[t * L + j];
-        first[u]     = __ldg(reinterpret_cast<const int4*>(table + toff[cl] +
-                                                       (static_cast<unsigned>(h[u]) & static_cast<unsigned>(tmask[cl]))));
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kProbeLevels; u++) {
-      if (found || !on[u]) continue;
-      tried++;
-      const int cl        = c * L + j0 + u;
-      const unsigned mask = static_cast<unsigned>(tmask[cl]);
-      const cell_slot* tb = table + toff[cl];
-      unsigned s          = static_cast<unsigned>(h[u]) & mask;
-      int4 e              = first[u];
-      for (unsigned probe = 0; probe <= mask; probe++) {
-        scanned++;
-        if (e.z < 0) break;  // an empty slot ends the run: the cell does not exist
-        const long long key = (static_cast<long long>(e.y) << 32) | static_cast<unsigned>(e.x);
-        if (key == h[u]) {
-          sg    = make_int2((base[cl] + e.z) * list_len, lr);
-          found = true;
-          break;
-        }
-        s = (s + 1) & mask;
-        e = __ldg(reinterpret_cast<const int4*>(tb + s));
-      }
-    }
+  int tried = 0, first = -1;
+  for (int j = 0; j < L && first < 0; j++) {
+    const cell_level lv = look.levels[c * L + j];
+    if (lv.mask < 0) continue;
+    tried++;
+    first = lookup_settle(look, lv, codes[t * L + j], kNotSure);
   }
-  seg[t] = sg;
-  if (stats != nullptr) {
+  look.seg[t] = first >= 0 ? make_int2(first, look.lr) : make_int2(0, 0);
+  if (look.stats != nullptr) {
     const int64_t q = t / C;
-    atomicAdd(reinterpret_cast<unsigned long long*>(stats + q * 8), static_cast<unsigned long long>(tried));
-    atomicAdd(reinterpret_cast<unsigned long long*>(stats + q * 8 + 1), static_cast<unsigned long long>(scanned));
+    atomicAdd(reinterpret_cast<unsigned long long*>(look.stats + q * 8), static_cast<unsigned long long>(tried));
+    atomicAdd(reinterpret_cast<unsigned long long*>(look.stats + q * 8 + 1), static_cast<unsigned long long>(4 * tried));
   }
 }
 
@@ -422,35 +374,32 @@ void cell_codes_f32(const float* y, int64_t n, int blocks, float inv_f, long lon
                     cudaStream_t s)
 {
   if (n <= 0) return;
-  const unsigned g = blocks_for(n, 128);
+  auto launch = [&](auto kernel, int lanes) { kernel<<<blocks_for(n * lanes, 128), 128, 0, s>>>(y, n, inv_f, codes); };
   switch (blocks) {
-    case 1: cell_codes_f32_kernel<1><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
-    case 2: cell_codes_f32_kernel<2><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
-    case 3: cell_codes_f32_kernel<3><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
-    case 4: cell_codes_f32_kernel<4><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
-    case 5: cell_codes_f32_kernel<5><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
-    case 6: cell_codes_f32_kernel<6><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
-    case 8: cell_codes_f32_kernel<8><<<g, 128, 0, s>>>(y, n, inv_f, codes); break;
+    case 1: launch(cell_codes_f32_kernel<1>, kGroup<1>); break;
+    case 2: launch(cell_codes_f32_kernel<2>, kGroup<2>); break;
+    case 3: launch(cell_codes_f32_kernel<3>, kGroup<3>); break;
+    case 4: launch(cell_codes_f32_kernel<4>, kGroup<4>); break;
+    case 5: launch(cell_codes_f32_kernel<5>, kGroup<5>); break;
+    case 6: launch(cell_codes_f32_kernel<6>, kGroup<6>); break;
+    case 8: launch(cell_codes_f32_kernel<8>, kGroup<8>); break;
     default: break;
   }
 }
 
-void build_cell_tables(const long long* keys, int64_t mmax, const int* ncells, const long long* toff,
-                       const int* tmask, int CL, cell_slot* table, cudaStream_t s)
+void build_cell_tables(const long long* keys, int64_t mmax, const int* ncells, const cell_level* levels, int CL,
+                       cell_slot* table, long long* packed, cudaStream_t s)
 {
   if (CL <= 0 || mmax <= 0) return;
   dim3 grid(blocks_for(mmax, 256), static_cast<unsigned>(CL));
-  fill_cell_tables_kernel<<<grid, 256, 0, s>>>(keys, mmax, ncells, toff, tmask, table);
+  fill_cell_tables_kernel<<<grid, 256, 0, s>>>(keys, mmax, ncells, levels, table, packed);
 }
 
-void probe(const long long* codes, int m, int C, int L, const cell_slot* table, const long long* toff,
-           const int* tmask, const int* base, const unsigned char* level_on, int list_len, int lr,
-           int2* seg, long long* stats, cudaStream_t s)
+void probe(const long long* codes, int m, int C, int L, const tc_lookup& look, cudaStream_t s)
 {
   const int64_t pairs = static_cast<int64_t>(m) * C;
   if (pairs <= 0) return;
-  probe_kernel<<<blocks_for(pairs, 256), 256, 0, s>>>(codes, pairs, C, L, table, toff, tmask, base, level_on,
-                                                      list_len, lr, seg, stats);
+  probe_kernel<<<blocks_for(pairs, 256), 256, 0, s>>>(codes, pairs, C, L, look);
 }
 
 void sketch_row_norms(const signed char* codes, const float* scale, int64_t rows, int S, float* norm,

@@ -14,6 +14,8 @@
 
 #include "kernels.hpp"
 
+#include "prep_common.cuh"
+
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -59,7 +61,7 @@ struct round_layout {
     st     = take(a.nseg);
     len    = take(a.nseg);
     hist   = take(256);
-    wsum   = take(20);
+    wsum   = take(36);  // one word per warp of at most 32, and the total
     ctrl   = take(8);
     kid    = take(a.KO);
     kd     = take(a.KO);
@@ -729,7 +731,7 @@ __device__ __forceinline__ void exact_distances(const int* sid, int ns, const __
 /// cannot make it and is dropped at once; what remains is sorted directly when it is short, or the
 /// KO smallest are cut out by radix passes first. kid / kd: the kept list as it was (shared
 /// memory), null when it starts empty. pool holds KO + ns keys, sorted holds 2 * P (P a power of
-/// two >= KO).
+/// two >= KO). oi / od (k > 0): the first k entries go there too, the results of a last round.
 __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
                                                 unsigned long long* sorted,
                                                 int P,
@@ -742,7 +744,10 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
                                                 const float* sdv,
                                                 int ns,
                                                 unsigned* hist,
-                                                int* ctrl)
+                                                int* ctrl,
+                                                long long* oi = nullptr,
+                                                float* od = nullptr,
+                                                int k = 0)
 {
   const bool fresh = kid == nullptr;
   if (threadIdx.x == 0) ctrl[6] = 0;
@@ -812,20 +817,27 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
   }
   __syncthreads();
   for (int i = threadIdx.x; i < KO; i += blockDim.x) {
-    const unsigned long long k = i < cnt ? sorted[i] : kNoKey;
-    pb[i] = k == kNoKey ? -1 : static_cast<long long>(static_cast<unsigned>(k & 0xffffffffULL));
-    pd[i] = k == kNoKey ? INFINITY : __uint_as_float(static_cast<unsigned>(k >> 32));
+    const unsigned long long key = i < cnt ? sorted[i] : kNoKey;
+    const long long id = key == kNoKey ? -1 : static_cast<long long>(static_cast<unsigned>(key & 0xffffffffULL));
+    const float d      = key == kNoKey ? INFINITY : __uint_as_float(static_cast<unsigned>(key >> 32));
+    pb[i] = id;
+    pd[i] = d;
+    if (i < k) {
+      oi[i] = id;
+      od[i] = d;
+    }
   }
 }
 
-
 // kThreads: 128 with eight blocks per multiprocessor when a block's shared memory allows that; a
-// round whose hash set is too large for eight blocks runs 256 or 512 threads per block instead, so
-// that the blocks that do fit still bring 32 warps to a multiprocessor.
+// round whose hash set is too large for eight blocks runs 256, 512 or 1024 threads per block instead,
+// so that the blocks that do fit still bring 32 warps to a multiprocessor, and so does a batch with
+// too few queries to fill the multiprocessors with small blocks (round_threads).
 template <bool kRows, bool kDealt, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const round_args a)
 {
   extern __shared__ __align__(16) int smem[];
+  let_next_kernel_start();
   const round_layout lay(a);
   const int q = blockIdx.x;
   int* table  = smem + lay.table;
@@ -855,6 +867,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // that ranks by sketch distance: there the distances of all rounds meet in one kept list, where
   // an id found twice must bring the same key both times.
   const bool int_form = !kRows && !a.sketch_rank;
+  wait_for_previous_kernel();
   if (int_form) {
     if (warp == 0) sketch_query_setup(a.qs + static_cast<int64_t>(q) * S, a.scale, S, w16, kq);
   } else {
@@ -1183,7 +1196,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
     exact_distances<kDealt>(sid, ns, a.vectors, a.vector_map, a.D, fq, sdv);
     tick(5);
   }
-  merge_into_kept(pool, sorted, a.P, pb, pd, a.KO, fresh ? nullptr : kid, kd, sid, sdv, ns, hist, ctrl);
+  merge_into_kept(pool, sorted, a.P, pb, pd, a.KO, fresh ? nullptr : kid, kd, sid, sdv, ns, hist, ctrl,
+                  a.out_i == nullptr ? nullptr : a.out_i + static_cast<int64_t>(q) * a.k,
+                  a.out_i == nullptr ? nullptr : a.out_d + static_cast<int64_t>(q) * a.k,
+                  a.out_i == nullptr ? 0 : a.k);
   __syncthreads();
   tick(6);
   if (a.stats != nullptr && threadIdx.x == 0) {
@@ -1225,6 +1241,7 @@ __global__ void __launch_bounds__(kRoundThreads) final_rerank_kernel(const long 
   int* ctrl                  = wsum + 16;
   const int q                = blockIdx.x;
   const long long* ps        = si + static_cast<int64_t>(q) * KO;
+  wait_for_previous_kernel();
   for (int i = threadIdx.x; i < D; i += blockDim.x)
     fq[(D & 7) ? i : query_slot(i)] = Q[static_cast<int64_t>(q) * D + i];
   // the kept list is packed (valid entries first), so the valid ones among the first R are a prefix
@@ -1304,20 +1321,55 @@ __global__ void merge_kept_kernel(const long long* __restrict__ src_i,
 size_t round_smem_bytes(const round_args& a) { return sizeof(int) * round_layout(a).words; }
 
 namespace {
+
+/// Launch that may begin while the kernel before it in the stream is finishing; the kernel waits for
+/// it where it first needs its results (wait_for_previous_kernel).
+/// Only where it matters, in batches that leave multiprocessors idle: the first blocks of a kernel
+/// that starts under the last of another find the L1 cache split for the other's shared memory, and no
+/// block that follows on the multiprocessor gets it back (10 000 queries: 1 131 us a batch against 990).
+template <typename... P, typename... A>
+void launch_overlapped(bool early, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
+                       A&&... args)
+{
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim          = dim3(grid);
+  cfg.blockDim         = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream           = s;
+  cudaLaunchAttribute at{};
+  at.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+  cfg.attrs                                     = &at;
+  cfg.numAttrs                                  = 1;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+/// Threads per query block. A multiprocessor runs 1024 threads of this kernel whatever the block size
+/// (64 registers each): a.threads makes the most of the blocks its shared memory holds. A batch of
+/// fewer blocks than the multiprocessors can hold at once is a matter of latency: its blocks get as
+/// many threads as still run side by side (one query, 1 M rows: 25 us a round with 128 threads).
+int round_threads(const round_args& a)
+{
+  int threads = a.threads;
+  while (threads < 1024 && static_cast<int64_t>(a.m) * threads * 2 <= int64_t{1024} * a.sms)
+    threads *= 2;
+  return threads;
+}
+
 template <bool kRows, bool kDealt, int kThreads>
 void launch_round(const round_args& a, cudaStream_t s)
 {
-  round_kernel<kRows, kDealt, kThreads><<<a.m, kThreads, round_smem_bytes(a), s>>>(a);
+  launch_overlapped(a.m <= a.sms, round_kernel<kRows, kDealt, kThreads>, static_cast<unsigned>(a.m), kThreads, round_smem_bytes(a), s, a);
 }
 template <bool kRows, bool kDealt>
 void launch_round(const round_args& a, cudaStream_t s)
 {
-  if (a.threads >= 512)
-    launch_round<kRows, kDealt, 512>(a, s);
-  else if (a.threads >= 256)
-    launch_round<kRows, kDealt, 256>(a, s);
-  else
-    launch_round<kRows, kDealt, 128>(a, s);
+  switch (round_threads(a)) {
+    case 1024: launch_round<kRows, kDealt, 1024>(a, s); break;
+    case 512: launch_round<kRows, kDealt, 512>(a, s); break;
+    case 256: launch_round<kRows, kDealt, 256>(a, s); break;
+    default: launch_round<kRows, kDealt, 128>(a, s); break;
+  }
 }
 template <bool kRows, bool kDealt>
 void allow_smem(int b)
@@ -1325,6 +1377,7 @@ void allow_smem(int b)
   cudaFuncSetAttribute(round_kernel<kRows, kDealt, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
   cudaFuncSetAttribute(round_kernel<kRows, kDealt, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
   cudaFuncSetAttribute(round_kernel<kRows, kDealt, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
 }
 bool dealt(const round_args& a)
 {
@@ -1369,8 +1422,8 @@ void final_rerank(const long long* si, int KO, int R, const __half* vectors, row
     P <<= 1;
   const size_t words = 2 * static_cast<size_t>((k + R + 1) & ~1) + 2 * static_cast<size_t>(std::max(2 * P, 64)) +
                        2 * static_cast<size_t>((R + 3) & ~3) + ((D + 63) & ~63) + 256 + 16 + 8;
-  final_rerank_kernel<<<m, kRoundThreads, sizeof(int) * words, s>>>(si, KO, R, vectors, vector_map, D, Q,
-                                                                    k, P, bi, bd, stats);
+  launch_overlapped(m <= 128, final_rerank_kernel, static_cast<unsigned>(m), kRoundThreads, sizeof(int) * words, s, si, KO, R,
+                    vectors, vector_map, D, Q, k, P, bi, bd, stats);
 }
 
 void merge_kept(const long long* src_i, const float* src_d, int nsrc, int64_t src_stride, int KO,

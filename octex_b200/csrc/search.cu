@@ -2,9 +2,11 @@
 //
 // Answers cpp/src/neighbors/octex/search.cu of hpdic/octex (make_plan :619-794, get_plan :796-814,
 // search_impl :816-961, the two search overloads :1020-1064) for one process per GPU. Parameter
-// limits and error texts are the reference's. A batch is: copy the queries in, pad a partial batch
-// with copies of its first row, replay the graph (centre + sketch-space query, projection, cell
-// codes, cell lookup, first round, waves, best k), copy the results out.
+// limits and error texts are the reference's. A batch is two kernels and one per wave: projection
+// with cell lookup and sketch-space queries, first round, waves, the last of which writes the
+// results. Queries and results in device memory are used where they are, on the caller's stream, and
+// every kernel is launched for the queries there are: no copies, no padding. A batch that stays in the
+// plan's buffers (resident searches, several processes) is replayed as one CUDA graph.
 
 #include "search_impl.hpp"
 
@@ -94,7 +96,8 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, int pick_entr
   // fewer than eight blocks fit its shared memory, the blocks get more threads to make up for it
   const size_t per_block = kernels::round_smem_bytes(r) + 1024;
   const int fit          = static_cast<int>(std::max<size_t>((size_t{228} << 10) / per_block, 1));
-  r.threads              = fit >= 8 ? 128 : fit >= 4 ? 256 : 512;
+  r.threads              = fit >= 8 ? 128 : fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
+  OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, device));
   {
     // the sketch stays in the L2 cache when it and its constants take at most 60 % of it
     int l2 = 0;
@@ -110,9 +113,9 @@ plan::~plan()
   int cur = 0;
   cudaGetDevice(&cur);
   cudaSetDevice(device);
+  if (used) cudaEventSynchronize(done_ev);  // its kernels may be running on a caller's stream
   if (graph != nullptr) cudaGraphExecDestroy(graph);
   if (done_ev != nullptr) cudaEventDestroy(done_ev);
-  if (start_ev != nullptr) cudaEventDestroy(start_ev);
   if (tc_error_host != nullptr) cudaFreeHost(tc_error_host);
   cudaSetDevice(cur);
 }
@@ -130,10 +133,44 @@ void check_tc(plan const& pl)
               "the results of that batch are not valid");
 }
 
-/// Launch every kernel of a batch on s (captured into the graph, or run directly).
-void run_batch(index_impl const& ix, plan& pl, cudaStream_t s, std::vector<cudaEvent_t>* marks)
+/// Where a batch's queries are and its results go (device-accessible memory).
+struct batch_io {
+  const float* q;
+  long long* ids;
+  float* dist;
+};
+
+/// The plan's own buffers.
+auto own_io(plan const& pl) -> batch_io { return {pl.qbuf.as<float>(), pl.bi, pl.bd}; }
+
+/// What is queued on s from here on comes after the plan's last batch, whose buffers it uses.
+void follow_last_batch(plan& pl, cudaStream_t s)
 {
-  // marks (profiling only): one event before the first kernel and one after every kernel
+  if (!pl.used) return;
+  unsigned long long id = 0;
+  OCTEX_CUDA_TRY(cudaStreamGetId(s, &id));
+  if (id == pl.last_stream) return;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  OCTEX_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+  // a graph the caller is capturing is ordered by whoever launches it
+  if (cap == cudaStreamCaptureStatusNone) OCTEX_CUDA_TRY(cudaStreamWaitEvent(s, pl.done_ev, 0));
+}
+
+/// The plan's last batch is what s holds now.
+void mark_last_batch(plan& pl, cudaStream_t s)
+{
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  OCTEX_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return;
+  OCTEX_CUDA_TRY(cudaEventRecord(pl.done_ev, s));
+  OCTEX_CUDA_TRY(cudaStreamGetId(s, &pl.last_stream));
+  pl.used = true;
+}
+
+/// Launch every kernel of a batch of pl.m queries on s (captured into the graph, or run directly).
+void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t s, std::vector<cudaEvent_t>* marks)
+{
+  // marks (profiling only): one event before the first kernel and one after every step
   auto mark = [&] {
     if (marks == nullptr) return;
     cudaEvent_t e = nullptr;
@@ -152,48 +189,73 @@ void run_batch(index_impl const& ix, plan& pl, cudaStream_t s, std::vector<cudaE
     OCTEX_CUDA_TRY(cudaMemsetAsync(pl.phase2.ptr, 0, pl.phase2.size, s));
   }
   mark();
-  kernels::center_sketch(pl.qbuf.as<float>(), p.mean.as<float>(), p.basis.as<float>(), pl.m1, D, sw,
-                         pl.qh.as<__half>(), p.ldu, pl.qs.as<float>(), s);
-  mark();
-  const unsigned char* levels = pl.dbg.taps ? nullptr : p.level_on.as<unsigned char>();
+  float finest   = ix.spacings[0];
+  for (float f : ix.spacings)
+    finest = std::min(finest, f);
+  kernels::sketch_job job;
+  job.q = io.q, job.mean = p.mean.as<float>(), job.basis = p.basis.as<float>();
+  job.m = pl.m1, job.D = D, job.S = sw;
+  job.qs   = pl.qs.as<float>();
+  job.keep = io.q == pl.qbuf.as<float>() ? nullptr : pl.qbuf.as<float>();
+  kernels::tc_lookup look;
+  look.table    = p.cell_table.as<kernels::cell_slot>();
+  look.keys     = p.cell_keys.as<long long>();
+  look.levels   = p.cell_levels.as<kernels::cell_level>();
+  look.list_len = ix.list_len;
+  look.lr       = pl.lr;
+  look.seg      = pl.seg.as<int2>();
+  look.stats    = pl.stats.as<long long>();
   // without inspection the cells are looked up where their codes are computed: no codes array, no
   // lookup kernel
-  const bool fused_lookup = pl.use_tc && !pl.dbg.taps;
-  if (pl.use_tc) {
-    // tensor cores; the projected coordinates stay in TMEM unless they are asked for
-    float finest = ix.spacings[0];
-    for (float f : ix.spacings)
-      finest = std::min(finest, f);
-    kernels::tc_lookup look;
-    if (fused_lookup) {
-      look.table    = p.cell_table.as<kernels::cell_slot>();
-      look.toff     = p.cell_off.as<long long>();
-      look.tmask    = p.cell_mask.as<int>();
-      look.base     = p.base.as<int>();
-      look.list_len = ix.list_len;
-      look.lr       = pl.lr;
-      look.seg      = pl.seg.as<int2>();
-      look.stats    = pl.stats.as<long long>();
-    }
-    kernels::project_decode_tc(pl.tc, L, p.shift.as<__half>(), p.inv_f.as<float>(), finest, levels,
-                               pl.codes.as<long long>(), pl.dbg.taps ? pl.Y.as<__half>() : nullptr, look,
-                               pl.tc_error_dev, s);
+  if (!pl.dbg.taps && pl.use_tc) {
+    mark();
+    kernels::project_decode_tc(pl.tc, job, L, p.shift.as<__half>(), p.inv_f.as<float>(), finest, nullptr, nullptr,
+                               look, pl.tc_error_dev, s);
+    mark();
+    mark();
+  } else if (!pl.dbg.taps) {
+    mark();
+    kernels::project_lookup_ordered(job, ix.blocks, p.ut.as<__half>(), p.ldu, p.copies, L, p.shift.as<__half>(),
+                                    p.inv_f.as<float>(), finest, look, s);
+    mark();
     mark();
   } else {
-    kernels::project_ordered(pl.qh.as<__half>(), p.ldu, p.ut.as<__half>(), p.ldu,
-                             p.shift.as<__half>(), pl.m1, wdt, D, pl.Y.as<__half>(), s);
+    // everything is written out: codes of every level, coordinates, then the lookup on its own
+    if (job.keep != nullptr)
+      OCTEX_CUDA_TRY(cudaMemcpyAsync(job.keep, io.q, sizeof(float) * pl.m1 * D, cudaMemcpyDefault, s));
+    if (pl.use_tc) {
+      mark();
+      job.keep = nullptr;
+      kernels::project_decode_tc(pl.tc, job, L, p.shift.as<__half>(), p.inv_f.as<float>(), finest,
+                                 pl.codes.as<long long>(), pl.Y.as<__half>(), kernels::tc_lookup{}, pl.tc_error_dev, s);
+      mark();
+    } else {
+      kernels::center_sketch(pl.qbuf.as<float>(), job.mean, job.basis, pl.m1, D, sw, pl.qh.as<__half>(), p.ldu, job.qs, s);
+      mark();
+      kernels::project_ordered(pl.qh.as<__half>(), p.ldu, p.ut.as<__half>(), p.ldu, p.shift.as<__half>(), pl.m1, wdt, D,
+                               pl.Y.as<__half>(), s);
+      mark();
+      kernels::decode_codes(pl.Y.as<__half>(), int64_t{pl.m1} * p.copies, p.copies, ix.blocks, L, p.inv_f.as<float>(),
+                            nullptr, pl.codes.as<long long>(), s);
+    }
     mark();
-    kernels::decode_codes(pl.Y.as<__half>(), int64_t{pl.m1} * p.copies, p.copies, ix.blocks, L,
-                          p.inv_f.as<float>(), levels, pl.codes.as<long long>(), s);
+    kernels::probe(pl.codes.as<long long>(), pl.m1, p.copies, L, look, s);
   }
   mark();
-  if (!fused_lookup)
-    kernels::probe(pl.codes.as<long long>(), pl.m1, p.copies, L, p.cell_table.as<kernels::cell_slot>(),
-                   p.cell_off.as<long long>(), p.cell_mask.as<int>(), p.base.as<int>(),
-                   p.level_on.as<unsigned char>(), ix.list_len, pl.lr, pl.seg.as<int2>(),
-                   pl.stats.as<long long>(), s);
-  mark();
-  kernels::round_lists(pl.r1, s);
+  // the last round writes the results unless a kernel of its own makes them
+  const bool reranks_at_end = pl.sp.sketch_rank && pl.FR > 0;
+  const bool last_is_lists  = pl.sp.waves == 0 && !pl.shard;
+  auto with_results         = [&](kernels::round_args r, bool last) {
+    if (last && !reranks_at_end) {
+      r.out_i = io.ids;
+      r.out_d = io.dist;
+      r.k     = pl.k;
+    }
+    return r;
+  };
+  pl.r1.m = pl.m1;
+  pl.r2.m = pl.mw;
+  kernels::round_lists(with_results(pl.r1, last_is_lists), s);
   mark();
   if (pl.shard) {
     // Every process ran the first round of all m rows over its own copies. Row block [lo_r, hi_r)
@@ -233,17 +295,16 @@ void run_batch(index_impl const& ix, plan& pl, cudaStream_t s, std::vector<cudaE
   }
   const float* Qw = pl.qbuf.as<float>() + static_cast<size_t>(pl.lo - pl.q1) * D;
   for (int wv = 0; wv < pl.sp.waves; wv++) {
-    kernels::round_args r = pl.r2;
+    kernels::round_args r = with_results(pl.r2, wv == pl.sp.waves - 1);
     r.done_off            = wv * pl.sp.starts;
     kernels::round_rows(r, s);
     mark();
   }
-  if (pl.sp.sketch_rank && pl.FR > 0) {
-    kernels::final_rerank(pl.wsi, pl.KO, pl.FR, p.vectors.as<__half>(), pl.r1.vector_map, D, Qw, pl.k,
-                          pl.mw, pl.bi, pl.bd, pl.stats.as<long long>(), s);
-  } else {
-    kernels::take_k(pl.wsi, pl.wsd, pl.KO, pl.k, pl.mw, pl.bi, pl.bd, s);
-  }
+  if (reranks_at_end)
+    kernels::final_rerank(pl.wsi, pl.KO, pl.FR, p.vectors.as<__half>(), pl.r1.vector_map, D, Qw, pl.k, pl.mw, io.ids,
+                          io.dist, pl.stats.as<long long>(), s);
+  else if (pl.sp.waves == 0 && pl.shard)
+    kernels::take_k(pl.wsi, pl.wsd, pl.KO, pl.k, pl.mw, io.ids, io.dist, s);
   mark();
   if (pl.world > 1) {
     // every process gets the results of all slices (blocks of mwmax rows, the last rows of a
@@ -252,6 +313,46 @@ void run_batch(index_impl const& ix, plan& pl, cudaStream_t s, std::vector<cudaE
     mark();
   }
   OCTEX_CUDA_TRY(cudaPeekAtLastError());
+}
+
+/// The slices of a batch of m queries (search.cu:666-676 of the reference).
+void set_rows(plan& pl, int m)
+{
+  pl.m  = m;
+  pl.lo = static_cast<int>(int64_t{m} * pl.rank / pl.world);
+  pl.hi = static_cast<int>(int64_t{m} * (pl.rank + 1) / pl.world);
+  pl.mw = pl.hi - pl.lo;
+  pl.q1 = pl.shard ? 0 : pl.lo;
+  pl.m1 = pl.shard ? m : pl.mw;
+}
+
+/// The batch in the plan's own buffers as one graph.
+void capture_batch(index_impl const& ix, plan& pl, cudaStream_t s)
+{
+  // one eager run first (module loading), then the capture (search.cu:754-786); with several processes
+  // the NCCL exchanges between the kernels are captured too (every process replays its graph in the
+  // same order, as it would launch the calls)
+  run_batch(ix, pl, own_io(pl), s, nullptr);
+  OCTEX_CUDA_TRY(cudaStreamSynchronize(s));
+  check_tc(pl);
+  if (pl.graph != nullptr) {
+    cudaGraphExecDestroy(pl.graph);
+    pl.graph = nullptr;
+  }
+  cudaGraph_t graph = nullptr;
+  OCTEX_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  try {
+    run_batch(ix, pl, own_io(pl), s, nullptr);
+  } catch (...) {
+    cudaStreamEndCapture(s, &graph);
+    if (graph != nullptr) cudaGraphDestroy(graph);
+    throw;
+  }
+  OCTEX_CUDA_TRY(cudaStreamEndCapture(s, &graph));
+  const cudaError_t made = cudaGraphInstantiate(&pl.graph, graph, 0);
+  cudaGraphDestroy(graph);
+  OCTEX_CUDA_TRY(made);
+  pl.graph_m = pl.m;
 }
 
 auto profile_batch(resources const& res, search_params const& sp, index const& idx, int64_t nq,
@@ -269,7 +370,9 @@ auto profile_batch(resources const& res, search_params const& sp, index const& i
   std::vector<cudaEvent_t> marks;
   std::vector<float> ms;
   try {
-    run_batch(ix, *pl, ix.part.stream, &marks);
+    set_rows(*pl, static_cast<int>(nq));
+    follow_last_batch(*pl, ix.part.stream);
+    run_batch(ix, *pl, own_io(*pl), ix.part.stream, &marks);
     OCTEX_CUDA_TRY(cudaStreamSynchronize(ix.part.stream));
     for (size_t i = 1; i < marks.size(); i++) {
       float t = 0.f;
@@ -288,6 +391,7 @@ auto profile_batch(resources const& res, search_params const& sp, index const& i
   return ms;
 }
 
+/// A plan for batches of up to m queries (of exactly m, when several processes share the index).
 auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_options dbg)
   -> std::shared_ptr<plan>
 {
@@ -296,7 +400,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   auto& p   = ix.part;
   pl.sp     = sp;
   pl.dbg    = dbg;
-  pl.m      = m;
+  pl.cap    = m;
   pl.k      = k;
   pl.KO     = std::max(sp.starts, k);
   pl.lr     = std::min(sp.read, ix.list_len);
@@ -337,29 +441,29 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
                 "octex: an index shared by several processes needs its communicator first "
                 "(octexB200CommInit)");
   OCTEX_EXPECTS(!pl.shard || ix.world * pl.KO <= 4096, "octex: devices * max(starts, k) <= 4096");
-  pl.lo    = static_cast<int>(int64_t{m} * ix.rank / ix.world);
-  pl.hi    = static_cast<int>(int64_t{m} * (ix.rank + 1) / ix.world);
-  pl.mw    = pl.hi - pl.lo;
   pl.mwmax = (m + ix.world - 1) / ix.world;
-  pl.q1    = pl.shard ? 0 : pl.lo;
-  pl.m1    = pl.shard ? m : pl.mw;
+  set_rows(pl, m);
 
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
   const int m1  = std::max(pl.m1, 1);
   const int wdt = 8 * ix.blocks * p.copies;
   pl.qbuf  = alloc<float>(pl, p.device, int64_t{m1} * D, 0);
-  pl.qh    = alloc<__half>(pl, p.device, int64_t{m1} * p.ldu);
   pl.qs    = alloc<float>(pl, p.device, int64_t{m1} * sw);
   pl.use_tc = !dbg.ordered_projection && kernels::project_tc_supported(ix.blocks, p.ldu);
-  if (!pl.use_tc || dbg.taps) pl.Y = alloc<__half>(pl, p.device, int64_t{m1} * wdt);
+  if (dbg.taps) {
+    pl.qh    = alloc<__half>(pl, p.device, int64_t{m1} * p.ldu);
+    pl.Y     = alloc<__half>(pl, p.device, int64_t{m1} * wdt);
+    pl.codes = alloc<long long>(pl, p.device, int64_t{m1} * p.copies * L);
+  }
   // the word a kernel sets when one of its bounded waits (on an mbarrier) ran out
   OCTEX_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&pl.tc_error_host), sizeof(int), cudaHostAllocMapped));
   *pl.tc_error_host = 0;
   OCTEX_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&pl.tc_error_dev), pl.tc_error_host, 0));
   if (pl.use_tc) {
-    kernels::project_tc_setup(pl.tc, pl.qh.as<__half>(), m1, p.ut.as<__half>(), p.copies, p.ldu);
+    int sms = 0;
+    OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device));
+    kernels::project_tc_setup(pl.tc, p.ut.as<__half>(), p.copies, p.ldu, sms);
   }
-  pl.codes = alloc<long long>(pl, p.device, int64_t{m1} * p.copies * L);
   pl.seg   = alloc<int2>(pl, p.device, int64_t{m1} * p.copies);
   pl.si    = alloc<long long>(pl, p.device, int64_t{m1} * pl.KO, 0xff);
   pl.sd    = alloc<float>(pl, p.device, int64_t{m1} * pl.KO);
@@ -470,33 +574,18 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   }
   kernels::round_allow_smem(pl.smem_max);
 
-  // one eager run (module loading), then the capture (search.cu:754-786)
-  OCTEX_CUDA_TRY(cudaDeviceSynchronize());
-  run_batch(ix, pl, p.stream, nullptr);
-  OCTEX_CUDA_TRY(cudaStreamSynchronize(p.stream));
-  check_tc(pl);
   OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.done_ev, cudaEventDisableTiming));
-  // one graph per batch; with several processes the NCCL exchanges between the kernels are captured
-  // into it too (every process replays its graph in the same order, as it would launch the calls)
-  cudaGraph_t graph = nullptr;
-  OCTEX_CUDA_TRY(cudaStreamBeginCapture(p.stream, cudaStreamCaptureModeThreadLocal));
-  try {
-    run_batch(ix, pl, p.stream, nullptr);
-  } catch (...) {
-    cudaStreamEndCapture(p.stream, &graph);
-    if (graph != nullptr) cudaGraphDestroy(graph);
-    throw;
-  }
-  OCTEX_CUDA_TRY(cudaStreamEndCapture(p.stream, &graph));
-  OCTEX_CUDA_TRY(cudaGraphInstantiate(&pl.graph, graph, 0));
-  OCTEX_CUDA_TRY(cudaGraphDestroy(graph));
+  OCTEX_CUDA_TRY(cudaDeviceSynchronize());  // the buffers are filled on the default stream
+  if (ix.world > 1) capture_batch(ix, pl, p.stream);
   return plp;
 }
 
 auto get_plan(index_impl& ix, search_params const& sp, int m, int k, int lane) -> std::shared_ptr<plan>
 {
   const debug_options dbg = ix_debug(ix);
-  std::string key = std::to_string(m) + "/" + std::to_string(k) + "/" + std::to_string(sp.read) +
+  // One process: a plan serves every batch it has room for. Several: their slices and exchanges
+  // depend on the number of queries.
+  std::string key = std::to_string(ix.world > 1 ? m : 0) + "/" + std::to_string(k) + "/" + std::to_string(sp.read) +
                     "/" + std::to_string(sp.starts) + "/" + std::to_string(sp.waves) + "/" +
                     std::to_string(sp.rerank) + "/" + std::to_string(sp.wave_rerank) + "/" +
                     std::to_string(sp.sketch_rank) + "/" + std::to_string(sp.final_rerank) + "/" +
@@ -505,18 +594,155 @@ auto get_plan(index_impl& ix, search_params const& sp, int m, int k, int lane) -
   std::lock_guard<std::mutex> lock(ix.mu);
   // one cached configuration: the previous buffers and graphs go before the new ones come
   // (search.cu:807-812); a configuration has one plan per lane (see search_impl)
-  if (ix.plans.find(key) == ix.plans.end()) {
-    ix.plans.clear();
-    ix.plans[key] = make_plan(ix, sp, m, k, dbg);
+  if (ix.plans.find(key) == ix.plans.end()) ix.plans.clear();
+  const std::string name = lane == 0 ? key : key + "#" + std::to_string(lane);
+  auto& pl               = ix.plans[name];
+  if (pl == nullptr || pl->cap < m) {
+    pl.reset();
+    try {
+      pl = make_plan(ix, sp, m, k, dbg);
+    } catch (...) {
+      ix.plans.erase(name);
+      throw;
+    }
   }
-  if (lane == 0) return ix.plans[key];
-  const std::string other = key + "#" + std::to_string(lane);
-  auto it = ix.plans.find(other);
-  if (it != ix.plans.end()) return it->second;
-  auto pl          = make_plan(ix, sp, m, k, dbg);
-  ix.plans[other]  = pl;
   return pl;
 }
+
+namespace {
+
+/// True when a kernel of this GPU and the copy engines reach p directly (page-locked or device memory).
+auto device_reaches(const void* p) -> bool
+{
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type != cudaMemoryTypeUnregistered;
+}
+
+/// Page-locked staging of at least `bytes`, kept with the plan.
+void* staging(dbuf& b, int device, size_t bytes)
+{
+  if (b.size < bytes) b = dbuf::pinned(device, bytes);
+  return b.ptr;
+}
+
+/// A search by one process with queries and results in the memory of its GPU: every batch runs on
+/// the caller's stream from the caller's arrays and into them.
+auto search_device(index_impl& ix, search_params const& sp, cudaStream_t caller, const float* queries, int64_t nq,
+                   int64_t* neighbors, float* distances, int64_t k) -> std::shared_ptr<plan>
+{
+  // equal batches rather than full ones and a rest
+  const int64_t most = std::max(sp.batch, 1), batches = (nq + most - 1) / most;
+  const int m        = static_cast<int>((nq + batches - 1) / batches);
+  auto pl            = get_plan(ix, sp, m, static_cast<int>(k));
+  std::lock_guard<std::mutex> lock(pl->mu);
+  // a search with device outputs returns before its kernels ran; had one of them given up, the
+  // word is still set and this is the first host code to see it
+  check_tc(*pl);
+  follow_last_batch(*pl, caller);
+  for (int64_t b0 = 0; b0 < nq; b0 += m) {
+    set_rows(*pl, static_cast<int>(std::min<int64_t>(m, nq - b0)));
+    run_batch(ix, *pl, {queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k},
+              caller, nullptr);
+  }
+  mark_last_batch(*pl, caller);
+  return pl;
+}
+
+/// A search by one process with queries and results in host memory (or in another GPU's): the copies
+/// are queued around the kernels. Several batches alternate between two lanes, each a plan on a stream
+/// of its own: the copies of one batch run under the kernels of the other. Page-locked arrays are
+/// copied from and to directly; ordinary ones pass through page-locked staging of the plan.
+void search_copied(index_impl& ix, search_params const& sp, cudaStream_t caller, int cur, const float* queries,
+                   int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
+{
+  auto& p            = ix.part;
+  const int D        = static_cast<int>(ix.dim);
+  const int64_t most = std::max(sp.batch, 1), batches = (nq + most - 1) / most;
+  const int m        = static_cast<int>((nq + batches - 1) / batches);
+  const debug_options dbg = ix_debug(ix);
+  // one lane when there is one batch and when the plan keeps observations
+  const int lanes = batches > 1 && !dbg.stats && !dbg.taps ? 2 : 1;
+  std::shared_ptr<plan> lane[2];
+  for (int l = 0; l < lanes; l++)
+    lane[l] = get_plan(ix, sp, m, static_cast<int>(k), l);
+  std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
+  if (lanes > 1) lock1 = std::unique_lock<std::mutex>(lane[1]->mu);
+  cudaStream_t stream[2] = {p.stream, p.second};
+  for (int l = 0; l < lanes; l++) {
+    check_tc(*lane[l]);
+    follow_last_batch(*lane[l], stream[l]);
+  }
+  const bool stage_in  = host_out && !device_reaches(queries);
+  const bool stage_out = host_out && !(device_reaches(neighbors) && device_reaches(distances));
+  struct pending {
+    int64_t b0 = 0;
+    int n      = 0;
+  } out[2];
+  // results of the last batch of a lane from its staging to the caller's arrays
+  auto deliver = [&](int l) {
+    if (out[l].n == 0) return;
+    OCTEX_CUDA_TRY(cudaStreamSynchronize(stream[l]));
+    plan& w          = *lane[l];
+    const size_t cnt = static_cast<size_t>(out[l].n) * k;
+    std::memcpy(neighbors + out[l].b0 * k, w.stage_out.ptr, cnt * sizeof(int64_t));
+    std::memcpy(distances + out[l].b0 * k, w.stage_out.as<char>() + sizeof(int64_t) * static_cast<size_t>(w.cap) * k,
+                cnt * sizeof(float));
+    out[l].n = 0;
+  };
+  int64_t batch = 0;
+  for (int64_t b0 = 0; b0 < nq; b0 += m, batch++) {
+    const int l    = static_cast<int>(batch % lanes);
+    plan& w        = *lane[l];
+    cudaStream_t s = stream[l];
+    const int n    = static_cast<int>(std::min<int64_t>(m, nq - b0));
+    const size_t bytes = sizeof(float) * static_cast<size_t>(n) * D;
+    if (stage_out) deliver(l);  // the lane's staging is free again, its queries too
+    const void* src = queries + b0 * D;
+    if (stage_in) {
+      if (!stage_out && batch >= lanes) OCTEX_CUDA_TRY(cudaStreamSynchronize(s));
+      void* pin = staging(w.stage_q, p.device, sizeof(float) * static_cast<size_t>(w.cap) * D);
+      std::memcpy(pin, src, bytes);
+      src = pin;
+    }
+    OCTEX_CUDA_TRY(cudaMemcpyAsync(w.qbuf.ptr, src, bytes, cudaMemcpyDefault, s));
+    set_rows(w, n);
+    batch_io io = own_io(w);
+    if (stage_out) {
+      // the last kernel writes through to host memory
+      auto* pin = static_cast<char*>(staging(w.stage_out, p.device, (sizeof(int64_t) + sizeof(float)) * static_cast<size_t>(w.cap) * k));
+      io.ids    = reinterpret_cast<long long*>(pin);
+      io.dist   = reinterpret_cast<float*>(pin + sizeof(int64_t) * static_cast<size_t>(w.cap) * k);
+    }
+    run_batch(ix, w, io, s, nullptr);
+    if (stage_out) {
+      out[l].b0 = b0;
+      out[l].n  = n;
+    } else {
+      OCTEX_CUDA_TRY(cudaMemcpyAsync(neighbors + b0 * k, w.bi, sizeof(int64_t) * n * k, cudaMemcpyDefault, s));
+      OCTEX_CUDA_TRY(cudaMemcpyAsync(distances + b0 * k, w.bd, sizeof(float) * n * k, cudaMemcpyDefault, s));
+    }
+  }
+  for (int l = 0; l < lanes; l++)
+    mark_last_batch(*lane[l], stream[l]);
+  if (host_out) {
+    if (stage_out && lanes > 1) deliver(static_cast<int>(batch % lanes));  // the older of the two first
+    for (int l = 0; l < lanes; l++) {
+      if (stage_out) deliver(l);
+      OCTEX_CUDA_TRY(cudaStreamSynchronize(stream[l]));
+      check_tc(*lane[l]);
+    }
+  } else {
+    OCTEX_CUDA_TRY(cudaSetDevice(cur));
+    for (int l = 0; l < lanes; l++)
+      OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->done_ev, 0));
+  }
+}
+
+}  // namespace
 
 void search_impl(resources const& res,
                  search_params const& sp,
@@ -528,7 +754,8 @@ void search_impl(resources const& res,
                  float* distances,
                  int64_t k,
                  bool host_out,
-                 bool resident)
+                 bool resident,
+                 bool wait)
 {
   auto& ix = idx.impl();
   OCTEX_EXPECTS(qdim == ix.dim, "octex: query dimension differs from the index");
@@ -537,50 +764,63 @@ void search_impl(resources const& res,
   int cur = 0;
   OCTEX_CUDA_TRY(cudaGetDevice(&cur));
   cudaStream_t caller = res.stream;
-  const int m         = static_cast<int>(std::min<int64_t>(std::max(sp.batch, 1), nq));
-  auto pl             = get_plan(ix, sp, m, static_cast<int>(k));
-  const int D = static_cast<int>(ix.dim);
-  auto& p     = ix.part;
-  // A call of several batches whose queries and results cross the bus alternates them between two
-  // lanes, each a plan (buffers and graph) on a stream of its own: the copies of one batch run
-  // under the kernels of the other. One lane when there is one batch, when the data is resident,
-  // when processes exchange inside the batch (their collectives are ordered on one stream), and
-  // when the plan keeps observations.
-  const bool two_lanes = !resident && pl->world == 1 && nq > m && !pl->dbg.stats && !pl->dbg.taps;
-  std::shared_ptr<plan> lane[2] = {pl, two_lanes ? get_plan(ix, sp, m, static_cast<int>(k), 1) : pl};
-  std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
-  if (two_lanes) lock1 = std::unique_lock<std::mutex>(lane[1]->mu);
-  if (two_lanes && p.second == nullptr) {
-    OCTEX_CUDA_TRY(cudaSetDevice(p.device));
-    OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&p.second, cudaStreamNonBlocking));
-    OCTEX_CUDA_TRY(cudaSetDevice(cur));
+  auto& p             = ix.part;
+  if (ix.world == 1 && !resident && !host_out && cur == p.device) {
+    auto pl = search_device(ix, sp, caller, queries, nq, neighbors, distances, k);
+    if (wait) {
+      OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
+      check_tc(*pl);
+    }
+    return;
   }
-  cudaStream_t stream[2] = {p.stream, two_lanes ? p.second : p.stream};
-  const int lanes        = two_lanes ? 2 : 1;
-  // a search with device outputs returns before its kernels ran; had one of them given up, the
-  // word is still set and this is the first host code to see it
-  for (int l = 0; l < lanes; l++)
-    check_tc(*lane[l]);
-
-  // the work of this call starts after what the caller queued on its stream (search.cu:841-848)
-  // an event of the plan (one search at a time uses it: pl->mu), on the device of the caller's
-  // stream, which is the current one
-  if (pl->start_ev == nullptr || pl->start_dev != cur) {
-    if (pl->start_ev != nullptr) cudaEventDestroy(pl->start_ev);
-    pl->start_ev = nullptr;
-    OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl->start_ev, cudaEventDisableTiming));
-    pl->start_dev = cur;
+  // the work of this call starts after what the caller queued on its stream (search.cu:841-848): an
+  // event of the index, on the device of the caller's stream, which is the current one
+  struct back_to {
+    int device;
+    ~back_to() { cudaSetDevice(device); }
+  } back{cur};
+  std::unique_lock<std::mutex> one_start(ix.start_mu);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  OCTEX_CUDA_TRY(cudaStreamIsCapturing(caller, &cap));
+  const bool busy = cap != cudaStreamCaptureStatusNone || cudaStreamQuery(caller) != cudaSuccess;
+  if (busy) {
+    cudaGetLastError();  // "not ready" is no failure
+    if (ix.start_ev == nullptr || ix.start_dev != cur) {
+      if (ix.start_ev != nullptr) cudaEventDestroy(ix.start_ev);
+      ix.start_ev = nullptr;
+      OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&ix.start_ev, cudaEventDisableTiming));
+      ix.start_dev = cur;
+    }
+    OCTEX_CUDA_TRY(cudaEventRecord(ix.start_ev, caller));
   }
-  cudaEvent_t start = pl->start_ev;
-  OCTEX_CUDA_TRY(cudaEventRecord(start, caller));
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
-  for (int l = 0; l < lanes; l++)
-    OCTEX_CUDA_TRY(cudaStreamWaitEvent(stream[l], start, 0));
-  int64_t batch = 0;
-  for (int64_t b0 = 0; b0 < nq; b0 += m, batch++) {
-    plan& w        = *lane[batch % lanes];
-    cudaStream_t s = stream[batch % lanes];
-    const int n    = static_cast<int>(std::min<int64_t>(m, nq - b0));
+  if (p.second == nullptr && ix.world == 1 && nq > sp.batch)
+    OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&p.second, cudaStreamNonBlocking));
+  if (busy) {
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.stream, ix.start_ev, 0));
+    if (p.second != nullptr) OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.second, ix.start_ev, 0));
+  }
+  one_start.unlock();
+  if (ix.world == 1 && !resident) {
+    search_copied(ix, sp, caller, cur, queries, nq, neighbors, distances, k, host_out);
+    if (wait && !host_out) OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
+    return;
+  }
+  // resident queries, or batches in which processes exchange: one lane, one graph per batch
+  const int m = static_cast<int>(std::min<int64_t>(std::max(sp.batch, 1), nq));
+  auto pl     = get_plan(ix, sp, m, static_cast<int>(k));
+  plan& w     = *pl;
+  const int D = static_cast<int>(ix.dim);
+  std::unique_lock<std::mutex> lock0(w.mu);
+  cudaStream_t s = p.stream;
+  check_tc(w);
+  follow_last_batch(w, s);
+  if (ix.world == 1) {
+    set_rows(w, m);
+    if (sp.use_graph && (w.graph == nullptr || w.graph_m != m)) capture_batch(ix, w, s);
+  }
+  for (int64_t b0 = 0; b0 < nq; b0 += m) {
+    const int n = static_cast<int>(std::min<int64_t>(m, nq - b0));
     if (!resident) {
       // rows [q1, q1 + m1) of the batch, the part beyond its end filled with copies of a row
       // (search.cu:870-883)
@@ -597,11 +837,8 @@ void search_impl(resources const& res,
     if (sp.use_graph && w.graph != nullptr)
       OCTEX_CUDA_TRY(cudaGraphLaunch(w.graph, s));
     else
-      run_batch(ix, w, s, nullptr);  // use_graph = false, or a batch with exchanges
-    if (!resident && w.world == 1) {
-      OCTEX_CUDA_TRY(cudaMemcpyAsync(neighbors + b0 * k, w.bi, sizeof(int64_t) * n * k, cudaMemcpyDefault, s));
-      OCTEX_CUDA_TRY(cudaMemcpyAsync(distances + b0 * k, w.bd, sizeof(float) * n * k, cudaMemcpyDefault, s));
-    } else if (!resident) {
+      run_batch(ix, w, own_io(w), s, nullptr);  // use_graph = false
+    if (!resident) {
       // the gathered results: block r holds the rows [lo_r, hi_r) of the batch
       for (int r = 0; r < w.world; r++) {
         const int lo_r = static_cast<int>(int64_t{m} * r / w.world);
@@ -616,15 +853,13 @@ void search_impl(resources const& res,
       }
     }
   }
-  for (int l = 0; l < lanes; l++)
-    OCTEX_CUDA_TRY(cudaEventRecord(lane[l]->done_ev, stream[l]));
+  mark_last_batch(w, s);
   OCTEX_CUDA_TRY(cudaSetDevice(cur));
-  for (int l = 0; l < lanes; l++)
-    OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->done_ev, 0));
-  if (host_out) OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
-  if (host_out)
-    for (int l = 0; l < lanes; l++)
-      check_tc(*lane[l]);
+  OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, w.done_ev, 0));
+  if (host_out || wait) {
+    OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
+    check_tc(w);
+  }
 }
 
 }  // namespace detail

@@ -14,7 +14,9 @@ struct plan {
   search_params sp;
   debug_options dbg;
   int device = 0;
-  int m = 0, k = 0, KO = 0, lr = 0, R1 = 0, R2 = 0, FR = 0;
+  // m: queries of the last batch (with several processes: of every batch); cap: the most a batch may
+  // have, what the buffers are sized for
+  int m = 0, cap = 0, k = 0, KO = 0, lr = 0, R1 = 0, R2 = 0, FR = 0;
   // Who answers what in a batch of m rows when `world` processes share the index
   // (search.cu:666-676 of the reference, per GPU there, per process here): the first round runs on
   // rows [q1, q1 + m1) — all m rows when the copies are sharded, the own slice otherwise — and the
@@ -42,11 +44,16 @@ struct plan {
   std::vector<dbuf> scratch_cand, scratch_dist;
   kernels::round_args r1, r2;
   size_t smem_max       = 0;
-  cudaGraphExec_t graph = nullptr;
-  cudaEvent_t done_ev   = nullptr;
-  cudaEvent_t start_ev  = nullptr;  // recorded on the caller's stream at the start of a search
-  int start_dev         = -1;       // device it was created on
+  cudaGraphExec_t graph = nullptr;  // of a batch of graph_m queries in the plan's own buffers
+  int graph_m           = 0;
+  cudaEvent_t done_ev   = nullptr;  // the end of the plan's last batch
+  // the stream done_ev was recorded on (cudaStreamGetId): a batch on another one waits for it first
+  unsigned long long last_stream = 0;
+  bool used                      = false;
   int64_t buffer_bytes  = 0;
+  // page-locked staging of calls with ordinary host memory, made when first needed: queries in,
+  // results out (the last kernel of the batch writes them there)
+  dbuf stage_q, stage_out;
   std::mutex mu;  // one search at a time per plan
   ~plan();
 };
@@ -63,7 +70,8 @@ void search_impl(resources const& res,
                  float* distances,
                  int64_t k,
                  bool host_out,
-                 bool resident);
+                 bool resident,
+                 bool wait = false);
 
 /// One batch of the queries already on the GPU, launched kernel by kernel with an event between
 /// them: milliseconds of center+sketch, projection, cell codes, lookup, first round, each wave,
@@ -75,6 +83,10 @@ auto profile_batch(resources const& res, search_params const& sp, index const& i
 /// report).
 void check_tc(plan const& pl);
 
+/// The plan of these parameters for batches of up to m queries.
 auto get_plan(index_impl& ix, search_params const& sp, int m, int k, int lane = 0) -> std::shared_ptr<plan>;
+
+/// Rows of the plan's buffers that hold something of the last batch, of `cap` allocated.
+inline auto rows_used(plan const& pl) -> int { return pl.world > 1 ? pl.cap : pl.m; }
 
 }  // namespace octex_b200::detail

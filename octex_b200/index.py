@@ -9,6 +9,7 @@ reference goes through a nanobind extension; this module calls the C interface o
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import json
 import os
 import shutil
@@ -43,6 +44,7 @@ def check_metric(metric):
             "distance (metric='sqeuclidean')")
 
 
+@functools.lru_cache(maxsize=None)
 def _torch():
     try:
         import torch
@@ -119,6 +121,14 @@ def search_params(**kw) -> _lib.SearchParams:
     return p
 
 
+@functools.lru_cache(maxsize=64)
+def _search_params_ref(read, starts, waves, rerank, wave_rerank, batch, sketch_rank, final_rerank):
+    """A pointer to the struct of these parameters, made once (the library only reads it)."""
+    p = search_params(read=read, starts=starts, waves=waves, rerank=rerank, wave_rerank=wave_rerank,
+                      batch=batch, sketch_rank=sketch_rank, final_rerank=final_rerank)
+    return C.pointer(p)
+
+
 def load_params(placement="shard", sketch="replicate", **kw):
     """(struct cuvsOctexLoadParams, keep-alive) from the reference's keyword arguments."""
     if placement not in PLACEMENTS:
@@ -156,6 +166,10 @@ class Index:
         self._keep = keep  # arrays borrowed by the library live as long as the index
         self._connected = False  # set by octex_b200.dist.connect
         self._res = {}  # cuvsResources per caller stream, made once
+
+    @functools.cached_property
+    def _dim(self):
+        return self.dim
 
     def _get(self, fn, ctype):
         v = ctype(0)
@@ -299,12 +313,16 @@ class Index:
                                wave_rerank=wave_rerank, batch=batch, sketch_rank=sketch_rank,
                                final_rerank=final_rerank, neighbors=neighbors, distances=distances)
             return back(D), back(I)
-        p = search_params(read=read, starts=starts, waves=waves, rerank=rerank,
-                          wave_rerank=wave_rerank, batch=batch, sketch_rank=sketch_rank,
-                          final_rerank=final_rerank)
+        try:
+            p = _search_params_ref(read, starts, waves, rerank, wave_rerank, batch, sketch_rank,
+                                   final_rerank)
+        except TypeError:  # an unhashable number (a 0-d array)
+            p = C.pointer(search_params(read=read, starts=starts, waves=waves, rerank=rerank,
+                                        wave_rerank=wave_rerank, batch=batch, sketch_rank=sketch_rank,
+                                        final_rerank=final_rerank))
         torch = _torch()
         if _is_torch(queries):
-            q = queries.detach()
+            q = queries.detach() if queries.requires_grad else queries
             if q.dtype != torch.float32:
                 raise TypeError("octex: queries must be float32")
             q = q.contiguous()
@@ -315,10 +333,10 @@ class Index:
             def usable(g, dt):
                 return (_is_torch(g) and g.dtype == dt and g.device == q.device
                         and g.is_contiguous() and tuple(g.shape) == (m, k))
-            I = neighbors if usable(neighbors, torch.int64) else \
-                torch.empty((m, k), dtype=torch.int64, device=q.device)
-            D = distances if usable(distances, torch.float32) else \
-                torch.empty((m, k), dtype=torch.float32, device=q.device)
+            I = neighbors if neighbors is not None and usable(neighbors, torch.int64) else \
+                q.new_empty((m, k), dtype=torch.int64)
+            D = distances if distances is not None and usable(distances, torch.float32) else \
+                q.new_empty((m, k))
             ptrs = (q.data_ptr(), I.data_ptr(), D.data_ptr())
             stream = torch.cuda.current_stream(q.device).cuda_stream if on_device else 0
         else:
@@ -332,22 +350,19 @@ class Index:
             def usable(g, dt):
                 return (isinstance(g, np.ndarray) and g.dtype == dt and g.flags.c_contiguous
                         and g.flags.writeable and g.shape == (m, k))
-            I = neighbors if usable(neighbors, np.int64) else np.empty((m, k), np.int64)
-            D = distances if usable(distances, np.float32) else np.empty((m, k), np.float32)
+            I = neighbors if neighbors is not None and usable(neighbors, np.int64) else np.empty((m, k), np.int64)
+            D = distances if distances is not None and usable(distances, np.float32) else np.empty((m, k), np.float32)
             ptrs = (q.ctypes.data, I.ctypes.data, D.ctypes.data)
             stream = 0
-        if d != self.dim:
-            raise ValueError(f"octex: queries have dimension {d}, the index {self.dim}")
+        if d != self._dim:
+            raise ValueError(f"octex: queries have dimension {d}, the index {self._dim}")
         for given in (neighbors, distances):
             if given is not None and tuple(given.shape) != (m, k):
                 raise ValueError(f"octex: output arrays must have shape {(m, k)}, not {tuple(given.shape)}")
-        res = self._resources(stream)
-        _lib.check(_lib.lib().octexB200Search(
-            res.h, C.byref(p), self._h, C.c_void_p(ptrs[0]), C.c_int64(m), C.c_int64(d),
-            C.c_void_p(ptrs[1]), C.c_void_p(ptrs[2]), C.c_int64(k), C.c_int32(1 if on_device else 0)))
-        if on_device:
-            res.sync()
-            _lib.check(_lib.lib().octexB200CheckLast(self._h))
+        rc = _lib.lib().octexB200SearchWait(self._resources(stream).h, p, self._h, ptrs[0], m, d, ptrs[1], ptrs[2],
+                                            k, 1 if on_device else 0)
+        if rc != _lib.CUVS_SUCCESS:
+            _lib.check(rc)
         if neighbors is not None and neighbors is not I:
             neighbors[...] = I if not _is_torch(neighbors) or _is_torch(I) else torch.as_tensor(I)
             I = neighbors

@@ -1,0 +1,98 @@
+"""The forms a kernel or a call takes by size, against each other and against the inspected run of the
+same search (coordinates and codes written out, separate lookup kernel), which test_gpu_parity.py
+compares with the CPU checker bit for bit.  Whatever the form, the answer is the same: ids and
+distances are compared for equality."""
+import numpy as np
+import pytest
+
+import octex_b200
+from conftest import small_params
+
+pytestmark = pytest.mark.gpu
+
+
+def make_index(dim, rows=4000, **kw):
+    from octex_b200 import build_index, synth
+    base = synth.plumbing(rows, dim, seed=0)
+    base_kw = dict(pca_dims=min(64, dim), list_len=16, min_cell=2, sketch_width=32, table_len=24)
+    base_kw.update(kw)
+    arrays, meta = build_index.build_arrays(base, small_params(**base_kw), device="cpu")
+    return octex_b200.attach(arrays, meta, borrow=False), meta
+
+
+def same(a, b):
+    return np.array_equal(a[1], b[1]) and np.array_equal(a[0].view(np.uint32), b[0].view(np.uint32))
+
+
+def inspected(idx, queries, k, **kw):
+    idx.set_debug(taps=True)
+    out = idx.search(queries, k, **kw)
+    seg = idx.fetch("seg", np.int32)
+    idx.set_debug()
+    return out, seg
+
+
+@pytest.mark.parametrize("blocks,dim", [(1, 48), (2, 100), (3, 96), (4, 98), (4, 64), (4, 200), (5, 64), (6, 130), (8, 64)])
+def test_projection_forms(blocks, dim):
+    """Lookup in the projection: a lane per block of coordinates with the levels side by side (few
+    queries), a lane group per (query, copy), a thread per (query, copy) in blocks that go through many
+    tiles (large batches, four blocks per copy; 64 dimensions fit the operand stages, 200 do not, and
+    rows of 98 floats do not start on 16-byte boundaries). An odd number of copies leaves the last tile
+    half empty."""
+    import torch
+    from octex_b200 import synth
+    idx, meta = make_index(dim, copies=7, blocks=blocks, pca_dims=min(64, dim))
+    kw = dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)
+    sizes = (1, 2, 12, 13, 64, 65, 129, 400) + ((9600,) if blocks == 4 else ())
+    queries = synth.plumbing(max(sizes), dim, seed=1)
+    queries[3, 5] = 3.0e6  # a coordinate for the general decode
+    for n in sizes:
+        want, seg = inspected(idx, queries[:n], 10, **kw)
+        got = idx.search(queries[:n], 10, **kw)
+        assert same(got, want), n
+        assert np.array_equal(idx.fetch("seg", np.int32), seg), n
+        # from rows in the middle of a device array, into new arrays
+        q = torch.as_tensor(np.concatenate([queries[-1:], queries[:n]]), device="cuda")[1:]
+        d, i = idx.search(q, 10, **kw)
+        assert same((d.cpu().numpy(), i.cpu().numpy()), want), n
+    idx.close()
+
+
+def test_batches_of_any_size_share_a_plan():
+    """A plan made for the largest batch serves smaller ones; searches on several streams and threads
+    use its buffers in turn."""
+    import threading
+    import torch
+    from octex_b200 import synth
+    idx, meta = make_index(64, copies=8, blocks=4)
+    kw = dict(read=8, starts=32, waves=2, rerank=64, wave_rerank=64)
+    queries = synth.plumbing(700, 64, seed=1)
+    want = idx.search(queries, 10, **kw)
+    sizes = (700, 1, 33, 300, 699, 2, 700)
+    for n in sizes:
+        assert same(idx.search(queries[:n], 10, **kw), (want[0][:n], want[1][:n])), n
+        assert idx.fetch("kept_ids", np.int64, (n, -1)).shape[1] == 32
+    assert same(idx.search(queries, 10, batch=131, **kw), want)
+    q = torch.as_tensor(queries, device="cuda")
+    failures = []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(40):
+                a = int(rng.integers(0, 600))
+                n = int(rng.integers(1, 700 - a))
+                if rng.random() < 0.3:
+                    d, i = idx.search(queries[a:a + n], 10, **kw)
+                else:
+                    d, i = (t.cpu().numpy() for t in idx.search(q[a:a + n], 10, **kw))
+                if not same((d, i), (want[0][a:a + n], want[1][a:a + n])):
+                    failures.append((seed, a, n))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
+    idx.close()
