@@ -542,14 +542,31 @@ __global__ void quantize_kernel(const float* __restrict__ v, const float* __rest
 
 // ---- exact neighbor table (build_table.cuh:60-142) ------------------------------------------------
 
+// |x_r|^2, one fused multiply-add per element in order. kVec: eight elements a load, for rows that all
+// start on 16-byte boundaries (200 001 x 128: the element-wise form is a chain of 2-byte loads).
+template <bool kVec>
 __global__ void row_norms_kernel(const __half* __restrict__ x, int64_t n, int D, float* __restrict__ norm)
 {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = 0.f;
-  for (int k = 0; k < D; k++) {
-    const float v = __half2float(x[i * D + k]);
-    acc           = __fmaf_rn(v, v, acc);
+  if constexpr (kVec) {
+    const uint4* row = reinterpret_cast<const uint4*>(x + i * D);
+#pragma unroll 4
+    for (int k = 0; k < D / 8; k++) {
+      const uint4 w        = __ldg(row + k);
+      const uint32_t h2[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h2[t]));
+        acc            = __fmaf_rn(v.y, v.y, __fmaf_rn(v.x, v.x, acc));
+      }
+    }
+  } else {
+    for (int k = 0; k < D; k++) {
+      const float v = __half2float(x[i * D + k]);
+      acc           = __fmaf_rn(v, v, acc);
+    }
   }
   norm[i] = acc;
 }
@@ -769,7 +786,8 @@ void exact_neighbors(const __half* x, int64_t n, int D, int K, int method, int32
   int dev = 0;
   OCTEX_CUDA_TRY(cudaGetDevice(&dev));
   dbuf norm(dev, sizeof(float) * n);
-  row_norms_kernel<<<grid_for(n, 128), 128, 0, s>>>(x, n, D, norm.as<float>());
+  const auto norms = D % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 ? row_norms_kernel<true> : row_norms_kernel<false>;
+  norms<<<grid_for(n, 128), 128, 0, s>>>(x, n, D, norm.as<float>());
   const bool covered = kernels::knn_tc_supported(n, D, K);
   OCTEX_EXPECTS(method != 1 || covered,
                 "octex: the tensor-core neighbor scan needs a dimension that is a multiple of 8 and K <= 120");

@@ -4,22 +4,24 @@
 //
 //   t[q, r] = |x_r|^2 - 2 x_q . x_r          squared distance up to the row's own constant |x_q|^2
 //
-// A block owns 128 query rows and walks over all rows in tiles of 128. Per tile the 128 x 128 dot
-// products are one tcgen05.mma chain (fp16 operands by TMA, 128-byte swizzle, fp32 accumulators in
-// TMEM); the accumulators are double buffered, so the tensor cores work on tile i + 1 while the
-// epilogue warps read tile i out of TMEM (tcgen05.ld, one query row per thread), add the row norms
-// and compare against the worst entry the row keeps. A row meets about K (1 + ln(n / K))
-// improvements in all, so after the first few tiles the epilogue is one fused multiply-add and a
-// fraction of a comparison per element. A thread only notes an improvement (value, row) in a
-// small buffer; after every 32 columns the warp empties the buffers of its 32 rows together: the
-// new entry replaces the worst of the row's list in shared memory and the lanes look for the new
-// worst with warp-wide maximum instructions. The lists are put in order once, at the end.
-// Nothing in the loop calls a function or touches the stack: with nearly all of the L1 given to
-// shared memory, a call's spills would go to the L2 cache and cost more than the tile.
+// A block owns one or two sets of 128 query rows and walks over all rows in tiles of 128. Per tile and
+// set the 128 x 128 dot products are one tcgen05.mma chain (fp16 operands by TMA, 128-byte swizzle,
+// fp32 accumulators in TMEM); the accumulators are double buffered, so the tensor cores work on tile
+// i + 1 while four epilogue warps per set read tile i out of TMEM (tcgen05.ld, one query row per
+// thread), add the row norms and compare against the worst entry the row keeps. The query rows stay in
+// shared memory for the whole scan when they fit (256 dimensions at most), so a tile of 128 rows is read
+// from the L2 cache once for 256 query rows.
+//
+// A row meets about K (1 + ln(n / K)) improvements in all. A thread only appends an improvement (value,
+// row) to a short buffer of its row in shared memory; when one of a warp's rows has no room for eight
+// more, the warp sorts that buffer (bitonic, a key per lane) and merges it into the row's K best, which
+// stand in order in the output arrays (L2 cache). So the bar a row compares with is up to a buffer old,
+// which costs a few more appends, and a merge serves 16 to 32 of them: the list upkeep is a few hundred
+// instructions per merge and K ln(n / K) / 25 merges per row. 200 001 x 128, K = 64: 133 ms with a list
+// update per improvement and a list per half of the tiles, 26 ms this way.
 //
 // Roles: warp 0 issues the TMA copies, warp 1 the MMAs (one lane each); the other warps are the
-// epilogue, in sets of four (one per quarter of the TMEM lanes). With two sets (short lists only:
-// each set keeps its own list per row, merged at the end) the tiles alternate between them.
+// epilogue, in sets of four (one per quarter of the TMEM lanes).
 // Every wait on an mbarrier is bounded; a wait that runs out raises a flag the other roles see, the
 // block waits for its copies in flight, frees its TMEM and returns with the error word set.
 
@@ -33,21 +35,35 @@ namespace octex_b200::kernels {
 
 namespace {
 
-constexpr int kTile       = 128;  // query rows per block = rows per tile = TMEM lanes
-constexpr int kKnnThreads = 320;  // at most: copy warp, MMA warp, two sets of four epilogue warps
-constexpr int kTmemCols   = 256;  // two accumulators of 128 fp32 columns
-constexpr uint32_t kStageBytes = 2 * kTile * kTileK * 2;  // A and B tile of a stage
+constexpr int kTile       = 128;  // query rows per set = rows per tile = TMEM lanes
+constexpr int kKnnThreads = 320;  // copy warp, MMA warp, two sets of four epilogue warps
+constexpr int kTmemCols   = 512;  // two accumulators of 128 fp32 columns per set
+constexpr int kMaxStages  = 6;
+constexpr uint32_t kPartBytes = kTile * kTileK * 2;  // 128 rows x 64 halves of an operand
 
 struct knn_ctl {
-  uint64_t full[4], empty[4];
+  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t queries;
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int failed;
   alignas(16) float nb[8][kTile];  // norms of the rows of the tile an epilogue warp works on
-  int state[2][kTile][2];          // per set and query row: entries kept at the end of the scan
 };
-constexpr int kCtlBytes = 8192;
-constexpr int kNoted    = 32;  // improvements a row can note between two visits of its warp (32 columns)
+constexpr int kCtlBytes = 4608;
+static_assert(sizeof(knn_ctl) <= kCtlBytes && kCtlBytes % 16 == 0, "control block");
+
+/// How a block's shared memory is used.
+struct knn_shape {
+  int stages;    // of 64 dimensions of a tile (and of the query rows, when those do not stay)
+  int room;      // noted improvements per row: 32 or 16
+  int resident;  // the query rows stay in shared memory
+  __host__ __device__ size_t stage_bytes() const { return (resident ? 1 : 3) * static_cast<size_t>(kPartBytes); }
+  __host__ __device__ size_t query_bytes(int nkb) const { return resident ? 2 * static_cast<size_t>(nkb) * kPartBytes : 0; }
+  size_t smem_bytes(int nkb) const
+  {
+    return 1024 + query_bytes(nkb) + stages * stage_bytes() + kCtlBytes + 2 * kTile * static_cast<size_t>(room + 1) * 8;
+  }
+};
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 {
@@ -77,32 +93,139 @@ __device__ __forceinline__ void tmem_ld_wait()
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+/// (a, b) * -2 + (x, y): two fused multiply-adds in one instruction.
+__device__ __forceinline__ void minus_twice(uint32_t a, uint32_t b, float x, float y, float& u, float& v)
+{
+  asm("{\n\t"
+      ".reg .b64 ab, xy, m2, r;\n\t"
+      "mov.b64 ab, {%2, %3};\n\t"
+      "mov.b64 xy, {%4, %5};\n\t"
+      "mov.b64 m2, {%6, %6};\n\t"
+      "fma.rn.f32x2 r, ab, m2, xy;\n\t"
+      "mov.b64 {%0, %1}, r;\n\t"
+      "}"
+      : "=f"(u), "=f"(v)
+      : "r"(a), "r"(b), "f"(x), "f"(y), "f"(-2.0f));
+}
 
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+/// Keys in the order of (value, row); no value is NaN or -0.
+__device__ __forceinline__ unsigned long long order_key(float v, int32_t id)
+{
+  const unsigned u = __float_as_uint(v);
+  return (static_cast<unsigned long long>(u ^ ((u & 0x80000000u) ? 0xffffffffu : 0x80000000u)) << 32) |
+         static_cast<unsigned>(id);
+}
+__device__ __forceinline__ float key_value(unsigned long long k)
+{
+  const unsigned u = static_cast<unsigned>(k >> 32);
+  return __uint_as_float(u ^ ((u & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+
+/// A step of a bitonic network between lanes `stride` apart; the lower lane takes the smaller key when up.
+__device__ __forceinline__ unsigned long long exchange(unsigned long long k, int stride, bool up)
+{
+  const unsigned long long other = __shfl_xor_sync(0xffffffffu, k, stride);
+  const bool smaller             = ((threadIdx.x & stride) == 0) == up;
+  return (k < other) == smaller ? k : other;
+}
+
+/// The warp's merge of `count` <= 32 noted entries into a row's list: `have` entries in order in
+/// vals / ids (slot i * 32 + lane belongs to the lane, so no ordering between lanes is needed in memory).
+/// Returns the K-th value, +inf while there are fewer. kRegs * 32 >= K.
+template <int kRegs>
+__device__ __forceinline__ float merge_noted(const float2* noted, int count, int have, int K, float* vals, int32_t* ids)
+{
+  const int lane = threadIdx.x & 31;
+  unsigned long long key[kRegs];
+#pragma unroll
+  for (int i = 0; i < kRegs; i++) {
+    const int at = i * 32 + lane;
+    key[i]       = ~0ULL;
+    if (at < have) key[i] = order_key(vals[at], ids[at]);
+  }
+  unsigned long long add = ~0ULL;
+  if (lane < count) {
+    const float2 e = noted[lane];
+    add            = order_key(e.x, __float_as_int(e.y));
+  }
+  // descending, so that lane j meets the list's entry j of the last 32: of two sorted sequences the
+  // smaller ones of opposite pairs are the smallest and form a bitonic sequence
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1)
+      add = exchange(add, stride, size < 32 && (lane & size) != 0);
+  key[kRegs - 1] = min(key[kRegs - 1], add);
+#pragma unroll
+  for (int half = kRegs / 2; half > 0; half >>= 1)
+#pragma unroll
+    for (int i = 0; i < kRegs; i++)
+      if ((i & half) == 0) {
+        const unsigned long long a = key[i], b = key[i + half];
+        key[i]        = min(a, b);
+        key[i + half] = max(a, b);
+      }
+#pragma unroll
+  for (int i = 0; i < kRegs; i++)
+#pragma unroll
+    for (int stride = 16; stride > 0; stride >>= 1)
+      key[i] = exchange(key[i], stride, true);
+  const int now = min(K, have + count);
+  float last    = INFINITY;
+#pragma unroll
+  for (int i = 0; i < kRegs; i++) {
+    const int at  = i * 32 + lane;
+    const float v = key_value(key[i]);
+    if (at < now) {
+      vals[at] = v;
+      ids[at]  = static_cast<int32_t>(key[i] & 0xffffffffu);
+    }
+    const float kth = __shfl_sync(0xffffffffu, v, (K - 1) & 31);
+    if (i == (K - 1) >> 5 && now == K) last = kth;
+  }
+  return last;
+}
+
+template <int kRegs>
 __global__ void __launch_bounds__(kKnnThreads, 1)
   knn_tc_kernel(const __grid_constant__ CUtensorMap map, const float* __restrict__ norm, int64_t n, int nkb,
-                int K, int stages, int64_t q_first, int64_t q_count, int32_t* __restrict__ best_id,
-                float* __restrict__ best_d, int* __restrict__ error)
+                int K, const knn_shape shape, int wide_blocks, int64_t q_first, int64_t q_count,
+                int32_t* best_id, float* best_d, int* __restrict__ error)
 {
   extern __shared__ unsigned char raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t{1023});
-  __half* tiles       = reinterpret_cast<__half*>(base);  // [stages][A 128 x 64 | B 128 x 64]
-  knn_ctl& ctl        = *reinterpret_cast<knn_ctl*>(base + static_cast<size_t>(stages) * kStageBytes);
-  float* lists        = reinterpret_cast<float*>(base + static_cast<size_t>(stages) * kStageBytes + kCtlBytes);
-  static_assert(sizeof(knn_ctl) <= kCtlBytes, "control block");
-  const int sets = (static_cast<int>(blockDim.x) - 64) / 128;  // sets of four epilogue warps: 1 or 2
+  // [set][64 dimensions][128 x 64] query rows that stay; [stages][tile | query rows of both sets]
+  __half* queries = reinterpret_cast<__half*>(base);
+  __half* tiles   = reinterpret_cast<__half*>(base + shape.query_bytes(nkb));
+  unsigned char* after = base + shape.query_bytes(nkb) + shape.stages * shape.stage_bytes();
+  knn_ctl& ctl    = *reinterpret_cast<knn_ctl*>(after);
+  float2* noted   = reinterpret_cast<float2*>(after + kCtlBytes);  // [set][row][room + 1]
+  constexpr int kPart = kPartBytes / 2;                            // halves
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q0     = q_first + static_cast<int64_t>(blockIdx.x) * kTile;
+  const bool wide      = static_cast<int>(blockIdx.x) < wide_blocks;
+  const int64_t q_end  = min(q_first + q_count, n);
+  const int64_t q0     = q_first + (static_cast<int64_t>(blockIdx.x) + min(static_cast<int>(blockIdx.x), wide_blocks)) * kTile;
+  const int sets       = wide && q0 + kTile < q_end ? 2 : 1;
   const int64_t ntiles = (n + kTile - 1) / kTile;
+  const int stages     = shape.stages;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 4; s++) {
+    for (int s = 0; s < stages; s++) {
       mbar_init(&ctl.full[s], 1);
       mbar_init(&ctl.empty[s], 1);
     }
+    mbar_init(&ctl.queries, 1);
     for (int b = 0; b < 2; b++) {
       mbar_init(&ctl.acc_full[b], 1);
-      mbar_init(&ctl.acc_empty[b], 4);  // one arrival per epilogue warp
+      mbar_init(&ctl.acc_empty[b], 4 * sets);  // one arrival per epilogue warp
     }
     ctl.failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -122,18 +245,26 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
   if (warp == 0) {
     // ---- copies ------------------------------------------------------------------------------
     if (lane == 0) {
-      bool ok    = true;
-      int64_t it = 0;
+      bool ok = true;
+      if (shape.resident) {
+        mbar_expect_tx(&ctl.queries, static_cast<uint32_t>(sets * nkb) * kPartBytes);
+        for (int set = 0; set < sets; set++)
+          for (int kb = 0; kb < nkb; kb++)
+            tma_load_2d(queries + (set * nkb + kb) * kPart, &map, kb * kTileK, static_cast<int>(q0) + set * kTile, &ctl.queries);
+      }
+      int s         = 0;
+      uint32_t turn = 0;
       for (int64_t t = 0; t < ntiles && ok; t++) {
-        for (int kb = 0; kb < nkb; kb++, it++) {
-          const int s       = static_cast<int>(it % stages);
-          const uint32_t ph = static_cast<uint32_t>(it / stages) & 1u;
-          if (it >= stages) ok = mbar_wait(&ctl.empty[s], ph ^ 1u, stop);
+        for (int kb = 0; kb < nkb; kb++) {
+          if (turn > 0) ok = mbar_wait(&ctl.empty[s], (turn & 1u) ^ 1u, stop);
           if (!ok) break;
-          __half* a = tiles + static_cast<size_t>(s) * (kStageBytes / 2);
-          mbar_expect_tx(&ctl.full[s], kStageBytes);
-          tma_load_2d(a, &map, kb * kTileK, static_cast<int>(q0), &ctl.full[s]);
-          tma_load_2d(a + kTile * kTileK, &map, kb * kTileK, static_cast<int>(t * kTile), &ctl.full[s]);
+          __half* b = tiles + s * (shape.stage_bytes() / 2);
+          mbar_expect_tx(&ctl.full[s], shape.resident ? kPartBytes : kPartBytes * (1 + sets));
+          tma_load_2d(b, &map, kb * kTileK, static_cast<int>(t * kTile), &ctl.full[s]);
+          if (!shape.resident)
+            for (int set = 0; set < sets; set++)
+              tma_load_2d(b + (1 + set) * kPart, &map, kb * kTileK, static_cast<int>(q0) + set * kTile, &ctl.full[s]);
+          if (++s == stages) s = 0, turn++;
         }
       }
       if (!ok && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 1);
@@ -143,137 +274,104 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
     if (lane == 0) {
       constexpr uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(kTile >> 3) << 17) |
                                  (static_cast<uint32_t>(kTile >> 4) << 24);
-      bool ok    = true;
-      int64_t it = 0;
+      bool ok       = !shape.resident || mbar_wait(&ctl.queries, 0, stop);
+      int s         = 0;
+      uint32_t turn = 0;
       for (int64_t t = 0; t < ntiles && ok; t++) {
         const int b      = static_cast<int>(t & 1);
         const uint32_t u = static_cast<uint32_t>(t >> 1);
         if (t >= 2) ok = mbar_wait(&ctl.acc_empty[b], (u & 1u) ^ 1u, stop);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = 0; kb < nkb; kb++, it++) {
-          const int s       = static_cast<int>(it % stages);
-          const uint32_t ph = static_cast<uint32_t>(it / stages) & 1u;
-          ok = mbar_wait(&ctl.full[s], ph, stop);
+        for (int kb = 0; kb < nkb; kb++) {
+          ok = mbar_wait(&ctl.full[s], turn & 1u, stop);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const __half* a   = tiles + static_cast<size_t>(s) * (kStageBytes / 2);
-          const uint64_t da = umma_desc(a), db = umma_desc(a + kTile * kTileK);
+          const __half* tile = tiles + s * (shape.stage_bytes() / 2);
+          const uint64_t db  = umma_desc(tile);
+          for (int set = 0; set < sets; set++) {
+            const uint64_t da = umma_desc(shape.resident ? queries + (set * nkb + kb) * kPart : tile + (1 + set) * kPart);
 #pragma unroll
-          for (int k = 0; k < kTileK / 16; k++)
-            umma_f16(tmem + static_cast<uint32_t>(b * kTile), da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < kTileK / 16; k++)
+              umma_f16(tmem + static_cast<uint32_t>((2 * b + set) * kTile), da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          }
           umma_commit(&ctl.empty[s]);  // arrives when the MMAs reading this stage are done
+          if (++s == stages) s = 0, turn++;
         }
         if (ok) umma_commit(&ctl.acc_full[b]);
       }
       if (!ok && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 2);
     }
-  } else {
-    // ---- epilogue: one query row per thread, the tiles dealt over the sets of four warps --------
-    const int quarter = warp & 3;  // the TMEM lanes this warp may read
-    const int e       = quarter * 32 + lane;
-    const int ew      = warp - 2;
-    const int set     = ew >> 2;
-    const int64_t row = q0 + e;
-    const bool live   = row < q_first + q_count && row < n;
-    // lists: values [set][row][K], then ids alike; noted improvements: values [set][slot][row], ids alike
-    float* values = lists;
-    int32_t* ids  = reinterpret_cast<int32_t*>(lists + static_cast<size_t>(sets) * kTile * K);
-    auto list_of  = [&](int of_set, int of_row) { return (static_cast<size_t>(of_set) * kTile + of_row) * K; };
-    float* noted_d   = reinterpret_cast<float*>(ids + static_cast<size_t>(sets) * kTile * K) + static_cast<size_t>(set) * kNoted * kTile + e;
-    int32_t* noted_i = reinterpret_cast<int32_t*>(lists + static_cast<size_t>(sets) * kTile * (2 * K + kNoted)) +
-                       static_cast<size_t>(set) * kNoted * kTile + e;
-    float* ld    = values + list_of(set, quarter * 32);  // the lists of the warp's 32 rows
-    int32_t* li  = ids + list_of(set, quarter * 32);
-    float kth    = live ? INFINITY : -INFINITY;  // what a row has to beat: the worst kept, once the list is full
-    int have     = live ? 0 : K;                  // entries the row's list holds
-    int worst    = 0;                             // slot of the worst one
-    int noted    = 0;                             // improvements noted since the warp last took them in
-    float* nb    = ctl.nb[ew];
-    // 32 columns of the tile: note what beats the row's bar, then the warp takes in what its lanes
-    // noted, a row at a time. The tile loop calls this from one place (a rolled loop over the four
-    // quarters of the columns): the loop has to stay small, its warp is alone on its scheduler and
-    // nothing hides an instruction fetch.
+  } else if (const int set = (warp - 2) >> 2; set < sets) {
+    // ---- epilogue: one query row per thread ----------------------------------------------------
+    const int quarter  = warp & 3;  // the TMEM lanes this warp may read
+    const int64_t wrow = q0 + set * kTile + quarter * 32;  // the warp's first query row
+    const int64_t row  = wrow + lane;
+    const bool live    = row < q_end;
+    const int room     = shape.room;
+    float2* rows_noted = noted + static_cast<size_t>(set * kTile + quarter * 32) * (room + 1);  // of the warp's 32 rows
+    float2* mine       = rows_noted + lane * (room + 1);  // an odd number of entries apart: no bank conflicts either way
+    int32_t* ids       = best_id + (wrow - q_first) * K;
+    float* vals        = best_d + (wrow - q_first) * K;
+    float kth          = live ? INFINITY : -INFINITY;  // what a row has to beat: its K-th best at the last merge
+    int have           = 0;                            // entries of the row in the output arrays
+    int count          = 0;                            // entries noted since
+    float* nb          = ctl.nb[warp - 2];
+    auto merge_rows = [&](unsigned which) {
+      while (which != 0) {
+        const int L = __ffs(which) - 1;
+        which &= which - 1;
+        const int c = __shfl_sync(0xffffffffu, count, L), h = __shfl_sync(0xffffffffu, have, L);
+        __syncwarp();
+        const float last = merge_noted<kRegs>(rows_noted + L * (room + 1), c, h, K, vals + static_cast<int64_t>(L) * K,
+                                              ids + static_cast<int64_t>(L) * K);
+        __syncwarp();
+        if (lane == L) {
+          kth   = last;
+          have  = min(K, h + c);
+          count = 0;
+        }
+      }
+    };
+    // 32 columns of the tile: the least of every eight is looked at first; where one of the warp's rows
+    // has an improvement among them, every thread appends its own. Once a row has no room for eight
+    // more, the full rows are merged and the scan goes on with the columns after.
     auto scan = [&](const uint32_t (&r)[32], int col, int64_t first) {
       float d[32];
 #pragma unroll
       for (int g = 0; g < 8; g++) {
         const float4 nn = *reinterpret_cast<const float4*>(nb + col + g * 4);
-        d[g * 4 + 0]    = fmaf(-2.f, __uint_as_float(r[g * 4 + 0]), nn.x);
-        d[g * 4 + 1]    = fmaf(-2.f, __uint_as_float(r[g * 4 + 1]), nn.y);
-        d[g * 4 + 2]    = fmaf(-2.f, __uint_as_float(r[g * 4 + 2]), nn.z);
-        d[g * 4 + 3]    = fmaf(-2.f, __uint_as_float(r[g * 4 + 3]), nn.w);
+        minus_twice(r[g * 4 + 0], r[g * 4 + 1], nn.x, nn.y, d[g * 4 + 0], d[g * 4 + 1]);
+        minus_twice(r[g * 4 + 2], r[g * 4 + 3], nn.z, nn.w, d[g * 4 + 2], d[g * 4 + 3]);
       }
-      float m[16];
-#pragma unroll
-      for (int i = 0; i < 16; i++)
-        m[i] = fminf(d[i], d[i + 16]);
-#pragma unroll
-      for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-        for (int i = 0; i < w; i++)
-          m[i] = fminf(m[i], m[i + w]);
-      const float least = m[0];
-      if (least < kth) {  // rare
+      if (first < wrow + 32 && first + 32 > wrow) {  // the rows themselves
 #pragma unroll
         for (int i = 0; i < 32; i++)
-          if (d[i] < kth) {
-            noted_d[noted * kTile] = d[i];
-            noted_i[noted * kTile] = static_cast<int32_t>(first + i);
-            noted++;  // at most 32 between two visits of the warp: kNoted slots
-          }
+          if (first + i == row) d[i] = INFINITY;
       }
-      unsigned has = __ballot_sync(0xffffffffu, noted > 0);
-      while (has != 0) {
-        const int L = __ffs(has) - 1;
-        has &= has - 1;
-        const int count = __shfl_sync(0xffffffffu, noted, L);
-        float beat      = __shfl_sync(0xffffffffu, kth, L);
-        int kept        = __shfl_sync(0xffffffffu, have, L);
-        int slot        = __shfl_sync(0xffffffffu, worst, L);
-        float* vd       = ld + static_cast<size_t>(L) * K;
-        int32_t* vi     = li + static_cast<size_t>(L) * K;
-        for (int j = 0; j < count; j++) {
-          const float dj   = noted_d[j * kTile + (L - lane)];  // row L's slot j: the same word for every lane
-          const int32_t id = noted_i[j * kTile + (L - lane)];
-          if (!(dj < beat) || id == q0 + quarter * 32 + L) continue;
-          // the new entry takes a free slot or the worst one's
-          const int at = kept < K ? kept : slot;
-          if (lane == 0) {
-            vd[at] = dj;
-            vi[at] = id;
+      float least[4];
+#pragma unroll
+      for (int g = 0; g < 4; g++)
+        least[g] = fminf(min3(min3(d[8 * g], d[8 * g + 1], d[8 * g + 2]), d[8 * g + 3], d[8 * g + 4]),
+                         min3(d[8 * g + 5], d[8 * g + 6], d[8 * g + 7]));
+      if (!__any_sync(0xffffffffu, fminf(min3(least[0], least[1], least[2]), least[3]) < kth)) return;
+      int from = 0;
+      for (;;) {
+        bool full = false;
+#pragma unroll
+        for (int g = 0; g < 4; g++)
+          if (!full && g >= from && __any_sync(0xffffffffu, least[g] < kth)) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              if (d[8 * g + i] < kth) {
+                mine[count] = make_float2(d[8 * g + i], __int_as_float(static_cast<int32_t>(first) + 8 * g + i));
+                count++;
+              }
+            full = __any_sync(0xffffffffu, count > room - 8);
+            from = g + 1;
           }
-          if (kept < K) kept++;
-          __syncwarp();
-          if (kept < K) continue;  // still filling: everything gets in
-          // the worst kept, the largest (value, id): rows arrive by ascending id, so of equal values
-          // the later row is the worse one and a row equal to the worst never gets in
-          unsigned bk = 0;
-          int32_t bi  = -1;
-          int bs      = 0;
-          for (int t = lane; t < K; t += 32) {
-            const unsigned u = __float_as_uint(vd[t]);
-            const unsigned k = (u & 0x80000000u) ? ~u : (u | 0x80000000u);  // same order as the floats
-            const int32_t i  = vi[t];
-            if (k > bk || (k == bk && i > bi)) {
-              bk = k;
-              bi = i;
-              bs = t;
-            }
-          }
-          const unsigned top  = __reduce_max_sync(0xffffffffu, bk);
-          const int32_t last  = __reduce_max_sync(0xffffffffu, bk == top ? bi : -1);
-          const unsigned owns = __ballot_sync(0xffffffffu, bk == top && bi == last);
-          slot                = __shfl_sync(0xffffffffu, bs, __ffs(owns) - 1);
-          beat                = __uint_as_float((top & 0x80000000u) ? (top & 0x7fffffffu) : ~top);
-          __syncwarp();
-        }
-        if (lane == L) {
-          kth   = beat;
-          have  = kept;
-          worst = slot;
-          noted = 0;
-        }
+        if (!full) break;
+        merge_rows(__ballot_sync(0xffffffffu, count > room - 8));
       }
     };
     // norms of the rows of a tile, four per lane; rows beyond the matrix never win
@@ -281,27 +379,26 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int64_t r = t * kTile + i * 32 + lane;
-        v[i]            = (t < ntiles && r < n) ? __ldg(norm + r) : INFINITY;
+        v[i]            = r < n ? __ldg(norm + r) : INFINITY;
       }
     };
     float ahead[4];
-    fetch_norms(set, ahead);
+    fetch_norms(0, ahead);
     bool ok = true;
-    for (int64_t t = set; t < ntiles; t += sets) {
+    for (int64_t t = 0; t < ntiles; t++) {
       const int b      = static_cast<int>(t & 1);
       const uint32_t u = static_cast<uint32_t>(t >> 1);
-      const int64_t r0 = t * kTile;
-      __syncwarp();  // every lane is done with the norms of the warp's previous tile
+      __syncwarp();  // every lane is done with the norms of the tile before
 #pragma unroll
       for (int i = 0; i < 4; i++)
         nb[i * 32 + lane] = ahead[i];
-      fetch_norms(t + sets, ahead);  // for the warp's next tile: in flight behind this one
+      fetch_norms(t + 1, ahead);  // in flight behind this tile
       __syncwarp();
       ok = mbar_wait(&ctl.acc_full[b], u & 1u, stop);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * kTile);
+      const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>((2 * b + set) * kTile);
 #pragma unroll 1
       for (int c = 0; c < 4; c++) {
         uint32_t r[32];
@@ -313,47 +410,19 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl.acc_empty[b]);
         }
-        scan(r, c * 32, r0 + c * 32);
+        scan(r, c * 32, t * kTile + c * 32);
       }
     }
-    ctl.state[set][e][0] = live ? have : 0;
     if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 3);
-    // the sets meet; the warps of the first one put the lists of their rows in order, a row at a
-    // time: an entry's place is the number of entries before it by (value, id)
-    asm volatile("bar.sync 1, %0;" ::"r"(sets * 128) : "memory");
-    if (set == 0 && *stop == 0) {
-      for (int L = 0; L < 32; L++) {
-        const int of_row  = quarter * 32 + L;
-        const int64_t qr  = q0 + of_row;
-        if (!(qr < q_first + q_count && qr < n)) continue;
-        const int have0   = ctl.state[0][of_row][0];
-        const int total   = have0 + (sets == 2 ? ctl.state[1][of_row][0] : 0);
-        const size_t at0  = list_of(0, of_row), at1 = list_of(sets - 1, of_row);
-        auto entry = [&](int j, float& v, int32_t& id) {
-          const size_t w = j < have0 ? at0 + j : at1 + (j - have0);
-          v  = values[w];
-          id = ids[w];
-        };
-        const float qn = __ldg(norm + qr);
-        int32_t* oi    = best_id + (qr - q_first) * K;
-        float* od      = best_d + (qr - q_first) * K;
-        for (int j = lane; j < total; j += 32) {
-          float v, w;
-          int32_t id, other;
-          entry(j, v, id);
-          int place = 0;
-          for (int t = 0; t < total; t++) {
-            entry(t, w, other);
-            place += (w < v || (w == v && other < id)) ? 1 : 0;
-          }
-          if (place < K) {
-            oi[place] = id;
-            od[place] = fmaxf(__fadd_rn(qn, v), 0.f);
-          }
-        }
-        for (int t = total + lane; t < K; t += 32) {
-          oi[t] = -1;
-          od[t] = INFINITY;
+    if (ok) {
+      merge_rows(__ballot_sync(0xffffffffu, count > 0));
+      for (int L = 0; L < 32 && wrow + L < q_end; L++) {
+        const int h    = __shfl_sync(0xffffffffu, have, L);
+        const float qn = __ldg(norm + wrow + L);
+        float* od      = vals + static_cast<int64_t>(L) * K;
+        for (int t = lane; t < K; t += 32) {
+          od[t] = t < h ? fmaxf(__fadd_rn(qn, od[t]), 0.f) : INFINITY;
+          if (t >= h) ids[static_cast<int64_t>(L) * K + t] = -1;
         }
       }
     }
@@ -371,20 +440,18 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
   }
 }
 
-size_t knn_smem_bytes(int K, int stages, int sets)
+/// Query rows that stay in shared memory with as many stages as fit behind them; buffers of half the
+/// length buy the third stage at 256 dimensions. Beyond that they come in again with every tile.
+knn_shape choose_shape(int nkb)
 {
-  return 1024 + static_cast<size_t>(stages) * kStageBytes + kCtlBytes + static_cast<size_t>(sets) * (K + kNoted) * kTile * 8;
-}
-
-/// Two sets of epilogue warps (each keeps a list per row, merged at the end) when their lists
-/// leave room for two stages of operands; else one set with as many stages as fit.
-void knn_shape(int K, int& stages, int& sets)
-{
-  for (sets = 2; sets >= 1; sets--)
-    for (stages = sets == 2 ? 3 : 4; stages >= 2; stages--)
-      if (knn_smem_bytes(K, stages, sets) <= 227 * 1024) return;
-  stages = 0;
-  sets   = 0;
+  constexpr size_t kLimit = 227 * 1024;
+  for (const knn_shape s : {knn_shape{kMaxStages, 32, 1}, knn_shape{kMaxStages, 16, 1}}) {
+    knn_shape fit = s;
+    while (fit.stages > 3 && fit.smem_bytes(nkb) > kLimit)
+      fit.stages--;
+    if (fit.smem_bytes(nkb) <= kLimit) return fit;
+  }
+  return knn_shape{3, 32, 0};
 }
 
 }  // namespace
@@ -392,9 +459,7 @@ void knn_shape(int K, int& stages, int& sets)
 bool knn_tc_supported(int64_t n, int D, int K)
 {
   // rows must start on 16-byte boundaries for the tensor map; ids are 32-bit
-  int stages = 0, sets = 0;
-  knn_shape(K, stages, sets);
-  return D % 8 == 0 && K >= 1 && stages >= 2 && n < (int64_t{1} << 31) - kTile;
+  return D % 8 == 0 && K >= 1 && K <= 122 && n < (int64_t{1} << 31) - 2 * kTile;
 }
 
 void knn_tc(const __half* x, const float* norm, int64_t n, int D, int K, int64_t q_first, int64_t q_count,
@@ -404,14 +469,23 @@ void knn_tc(const __half* x, const float* norm, int64_t n, int D, int K, int64_t
   if (!knn_tc_supported(n, D, K)) throw std::runtime_error("octex: shape not covered by the tensor-core neighbor scan");
   CUtensorMap map;
   make_map(&map, x, n, D, kTile);
-  int stages = 0, sets = 0;
-  knn_shape(K, stages, sets);
-  const size_t smem  = knn_smem_bytes(K, stages, sets);
-  cudaError_t status = cudaFuncSetAttribute(knn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const int nkb         = (D + kTileK - 1) / kTileK;
+  const knn_shape shape = choose_shape(nkb);
+  const size_t smem     = shape.smem_bytes(nkb);
+  const auto kernel     = K <= 32 ? knn_tc_kernel<1> : K <= 64 ? knn_tc_kernel<2> : knn_tc_kernel<4>;
+  cudaError_t status    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  int dev = 0, sms = 1;
+  if (status == cudaSuccess) status = cudaGetDevice(&dev);
+  if (status == cudaSuccess) status = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (status != cudaSuccess) throw std::runtime_error(std::string("octex: ") + cudaGetErrorString(status));
-  const int64_t blocks = (q_count + kTile - 1) / kTile;
-  knn_tc_kernel<<<static_cast<unsigned>(blocks), 64 + 128 * sets, smem, s>>>(map, norm, n, (D + kTileK - 1) / kTileK, K, stages,
-                                                                         q_first, q_count, best_id, best_d, error);
+  // A block per multiprocessor, 256 query rows each; what is left after the whole rounds goes out in
+  // blocks of 128 rows when those fit one more round, which then takes half the time.
+  const int64_t round  = int64_t{2} * kTile * sms;
+  const int64_t rest   = q_count % round;
+  const int64_t narrow = rest <= round / 2 ? (rest + kTile - 1) / kTile : 0;
+  const int64_t wide   = narrow > 0 || rest == 0 ? (q_count - rest) / (2 * kTile) : (q_count + 2 * kTile - 1) / (2 * kTile);
+  kernel<<<static_cast<unsigned>(wide + narrow), kKnnThreads, smem, s>>>(map, norm, n, nkb, K, shape, static_cast<int>(wide), q_first,
+                                                                         q_count, best_id, best_d, error);
 }
 
 }  // namespace octex_b200::kernels

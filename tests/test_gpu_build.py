@@ -218,6 +218,42 @@ def test_tensor_core_neighbor_scan(n, dim, k):
     assert same > 0.999, same
 
 
+@pytest.mark.parametrize("n,dim,k,order", [
+    (129, 8, 1, "random"), (257, 64, 32, "random"), (641, 72, 33, "falling"), (1000, 192, 65, "random"),
+    (999, 256, 64, "falling"), (900, 264, 122, "random"), (40, 128, 64, "random"), (3001, 128, 64, "ties"),
+    (19101, 16, 64, "falling"), (38001, 128, 10, "ties")])
+def test_tensor_core_scan_is_exact(n, dim, k, order):
+    """The tcgen05 scan on whole numbers, where every product and sum is exact: ids and distances as
+    float64 has them, equal distances by ascending id. Query rows that stay in shared memory with long
+    and short buffers (256 dimensions) and rows that do not (264); lists of one, two and four keys a
+    lane; fewer rows than the list is long; one set, two sets and both kinds of block (38001 rows on
+    148 multiprocessors); rows that come nearer with every id up to a row's own (each one an
+    improvement), and many equal rows."""
+    import torch
+    g = torch.Generator("cuda").manual_seed(n)
+    if order == "falling":  # a row i steps along, little else
+        x = torch.randint(0, 2, (n, dim), generator=g, device="cuda").float()
+        x[:, 0] = torch.arange(n, device="cuda") % 2048
+    else:
+        x = torch.randint(0, 3 if order == "ties" else 256, (n, dim), generator=g, device="cuda").float()
+        if order == "ties":
+            x = x[torch.randint(0, n // 3, (n,), generator=g, device="cuda")]
+    ids, d = octex_b200.exact_neighbors(x.half(), k, method="tensor")
+    kept = min(k, n - 1)
+    xd = x.double()
+    sq = (xd * xd).sum(1)
+    for q0 in range(0, n, 4096):
+        q1 = min(n, q0 + 4096)
+        full = sq[q0:q1, None] + sq[None, :] - 2 * (xd[q0:q1] @ xd.T)
+        # the id breaks ties: distances are whole numbers below 2^25, ids below 2^16
+        key = full * 65536 + torch.arange(n, device="cuda")
+        key[torch.arange(q1 - q0), torch.arange(q0, q1)] = float("inf")
+        want = key.topk(kept, dim=1, largest=False, sorted=True).values
+        assert torch.equal(ids[q0:q1, :kept].double(), want % 65536)
+        assert torch.equal(d[q0:q1, :kept].double(), (want / 65536).floor())
+    assert (ids[:, kept:] == -1).all() and torch.isinf(d[:, kept:]).all()
+
+
 def test_searched_table(built, oracle, tmp_path):
     """The table by the index's own search (octexB200SearchedTable; cuvsOctexBuild above
     exact_table_max), the way the reference checks its own (cpp/tests/test_build.cu, table quality):
