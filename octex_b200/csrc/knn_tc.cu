@@ -12,16 +12,23 @@
 // shared memory for the whole scan when they fit (256 dimensions at most), so a tile of 128 rows is read
 // from the L2 cache once for 256 query rows.
 //
-// A row meets about K (1 + ln(n / K)) improvements in all. A thread only appends an improvement (value,
-// row) to a short buffer of its row in shared memory; when one of a warp's rows has no room for eight
-// more, the warp sorts that buffer (bitonic, a key per lane) and merges it into the row's K best, which
-// stand in order in the output arrays (L2 cache). So the bar a row compares with is up to a buffer old,
-// which costs a few more appends, and a merge serves 16 to 32 of them: the list upkeep is a few hundred
-// instructions per merge and K ln(n / K) / 25 merges per row. 200 001 x 128, K = 64: 133 ms with a list
-// update per improvement and a list per half of the tiles, 26 ms this way.
+// A row meets about K (1 + ln(n / K)) improvements in all. To start with a bar, the block first visits
+// every few tiles just for the least value of each column of the tiles, up to 128 registers a thread: the
+// K-th smallest of these has K rows at or below it, so nothing beyond it is in the answer. A thread only
+// appends an improvement (value, row) to a short buffer of its row in shared memory; when one of a warp's
+// rows has no room for eight more, the warp sorts that buffer (bitonic, a key per lane) and merges it into
+// the row's K best, which stand in order in the output arrays (L2 cache). So the bar a row compares with is
+// up to a buffer old, which costs a few more appends, and a merge of a few hundred instructions serves 16
+// to 32 of them.
 //
-// Roles: warp 0 issues the TMA copies, warp 1 the MMAs (one lane each); the other warps are the
-// epilogue, in sets of four (one per quarter of the TMEM lanes).
+// What bounds it: the epilogue, two warps to a scheduler (168 registers a thread) at about five cycles an
+// instruction; 16 MMAs take 1 024 of the 4 600 cycles a tile takes. 200 001 x 128, K = 64: 133 ms with a
+// list update per improvement and a list per half of the tiles; 26 with buffers and resident query rows;
+// 21 with the bars, a warp per set for the MMAs, operands in uniform registers, and one mask of the
+// groups of columns that hold improvements where there was a vote and a branch for each.
+//
+// Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues); the other warps
+// are the epilogue, in sets of four (one per quarter of the TMEM lanes).
 // Every wait on an mbarrier is bounded; a wait that runs out raises a flag the other roles see, the
 // block waits for its copies in flight, frees its TMEM and returns with the error word set.
 
@@ -36,15 +43,16 @@ namespace octex_b200::kernels {
 namespace {
 
 constexpr int kTile       = 128;  // query rows per set = rows per tile = TMEM lanes
-constexpr int kKnnThreads = 320;  // copy warp, MMA warp, two sets of four epilogue warps
+constexpr int kKnnThreads = 352;  // copy warp, an MMA warp per set, two sets of four epilogue warps
 constexpr int kTmemCols   = 512;  // two accumulators of 128 fp32 columns per set
 constexpr int kMaxStages  = 6;
+constexpr int kVisitsPerK = 3;    // tiles looked at for the bars, per entry of a list
 constexpr uint32_t kPartBytes = kTile * kTileK * 2;  // 128 rows x 64 halves of an operand
 
 struct knn_ctl {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t queries;
-  uint64_t acc_full[2], acc_empty[2];
+  uint64_t acc_full[2][2], acc_empty[2][2];  // [set][accumulator]
   uint32_t tmem_base;
   int failed;
   alignas(16) float nb[8][kTile];  // norms of the rows of the tile an epilogue warp works on
@@ -93,6 +101,20 @@ __device__ __forceinline__ void tmem_ld_wait()
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+/// True in one lane of the warp, always the same.
+__device__ __forceinline__ bool elect_one()
+{
+  uint32_t p;
+  asm volatile(
+    "{\n\t"
+    ".reg .pred p;\n\t"
+    "elect.sync _|p, 0xffffffff;\n\t"
+    "selp.u32 %0, 1, 0, p;\n\t"
+    "}"
+    : "=r"(p));
+  return p != 0;
+}
+
 /// (a, b) * -2 + (x, y): two fused multiply-adds in one instruction.
 __device__ __forceinline__ void minus_twice(uint32_t a, uint32_t b, float x, float y, float& u, float& v)
 {
@@ -113,6 +135,22 @@ __device__ __forceinline__ float min3(float a, float b, float c)
   float d;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
+}
+
+/// Appends (value, row) at the shared-memory address `at` when the value is below the bar; no branch.
+__device__ __forceinline__ void note_below(float value, float bar, int row, uint32_t& at)
+{
+  asm volatile(
+    "{\n\t"
+    ".reg .pred p;\n\t"
+    "setp.lt.f32 p, %1, %2;\n\t"
+    "@p st.shared.b32 [%0], %1;\n\t"
+    "@p st.shared.b32 [%0 + 4], %3;\n\t"
+    "@p add.u32 %0, %0, 8;\n\t"
+    "}"
+    : "+r"(at)
+    : "f"(value), "f"(bar), "r"(row)
+    : "memory");
 }
 
 /// Keys in the order of (value, row); no value is NaN or -0.
@@ -195,10 +233,11 @@ __device__ __forceinline__ float merge_noted(const float2* noted, int count, int
 
 template <int kRegs>
 __global__ void __launch_bounds__(kKnnThreads, 1)
-  knn_tc_kernel(const __grid_constant__ CUtensorMap map, const float* __restrict__ norm, int64_t n, int nkb,
-                int K, const knn_shape shape, int wide_blocks, int64_t q_first, int64_t q_count,
+  knn_tc_kernel(const __grid_constant__ CUtensorMap map, const float* __restrict__ norm, int n,
+                int D, int K, const knn_shape shape, int sampled, int spread, int wide_blocks, int q_first, int q_count,
                 int32_t* best_id, float* best_d, int* __restrict__ error)
 {
+  const int nkb = (D + kTileK - 1) / kTileK;  // steps of 64 dimensions
   extern __shared__ unsigned char raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t{1023});
   // [set][64 dimensions][128 x 64] query rows that stay; [stages][tile | query rows of both sets]
@@ -209,24 +248,30 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
   float2* noted   = reinterpret_cast<float2*>(after + kCtlBytes);  // [set][row][room + 1]
   constexpr int kPart = kPartBytes / 2;                            // halves
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool wide      = static_cast<int>(blockIdx.x) < wide_blocks;
-  const int64_t q_end  = min(q_first + q_count, n);
-  const int64_t q0     = q_first + (static_cast<int64_t>(blockIdx.x) + min(static_cast<int>(blockIdx.x), wide_blocks)) * kTile;
-  const int sets       = wide && q0 + kTile < q_end ? 2 : 1;
-  const int64_t ntiles = (n + kTile - 1) / kTile;
-  const int stages     = shape.stages;
+  // the same for all lanes, and known to be: what the copies and the MMAs take is then computed and kept
+  // in uniform registers
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
+  const bool wide  = static_cast<int>(blockIdx.x) < wide_blocks;
+  const int q_end  = min(q_first + q_count, n);
+  const int q0     = q_first + (static_cast<int>(blockIdx.x) + min(static_cast<int>(blockIdx.x), wide_blocks)) * kTile;
+  const int sets   = wide && q0 + kTile < q_end ? 2 : 1;
+  const int ntiles = (n + kTile - 1) / kTile;
+  const int stages = shape.stages;
+  // the tiles in the order of their visits: every spread-th for the bars, then all
+  const int visits = sampled + ntiles;
+  auto tile_of     = [&](int visit) { return visit < sampled ? visit * spread : visit - sampled; };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; s++) {
       mbar_init(&ctl.full[s], 1);
-      mbar_init(&ctl.empty[s], 1);
+      mbar_init(&ctl.empty[s], sets);
     }
     mbar_init(&ctl.queries, 1);
-    for (int b = 0; b < 2; b++) {
-      mbar_init(&ctl.acc_full[b], 1);
-      mbar_init(&ctl.acc_empty[b], 4 * sets);  // one arrival per epilogue warp
-    }
+    for (int set = 0; set < 2; set++)
+      for (int b = 0; b < 2; b++) {
+        mbar_init(&ctl.acc_full[set][b], 1);
+        mbar_init(&ctl.acc_empty[set][b], 4);  // one arrival per epilogue warp
+      }
     ctl.failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -239,183 +284,268 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem      = ctl.tmem_base;
+  const uint32_t tmem      = __shfl_sync(0xffffffffu, ctl.tmem_base, 0);
   const volatile int* stop = &ctl.failed;
 
   if (warp == 0) {
-    // ---- copies ------------------------------------------------------------------------------
-    if (lane == 0) {
-      bool ok = true;
-      if (shape.resident) {
-        mbar_expect_tx(&ctl.queries, static_cast<uint32_t>(sets * nkb) * kPartBytes);
-        for (int set = 0; set < sets; set++)
-          for (int kb = 0; kb < nkb; kb++)
-            tma_load_2d(queries + (set * nkb + kb) * kPart, &map, kb * kTileK, static_cast<int>(q0) + set * kTile, &ctl.queries);
-      }
-      int s         = 0;
-      uint32_t turn = 0;
-      for (int64_t t = 0; t < ntiles && ok; t++) {
-        for (int kb = 0; kb < nkb; kb++) {
-          if (turn > 0) ok = mbar_wait(&ctl.empty[s], (turn & 1u) ^ 1u, stop);
-          if (!ok) break;
-          __half* b = tiles + s * (shape.stage_bytes() / 2);
+    // ---- copies: the warp goes through the loop together, one lane issues --------------------------
+    const bool issues = elect_one();
+    bool ok           = true;
+    if (shape.resident && issues) {
+      mbar_expect_tx(&ctl.queries, static_cast<uint32_t>(sets * nkb) * kPartBytes);
+      for (int set = 0; set < sets; set++)
+        for (int kb = 0; kb < nkb; kb++)
+          tma_load_2d(queries + (set * nkb + kb) * kPart, &map, kb * kTileK, q0 + set * kTile, &ctl.queries);
+    }
+    int s         = 0;
+    uint32_t turn = 0;
+    for (int t = 0; t < visits && ok; t++) {
+      for (int kb = 0; kb < nkb; kb++) {
+        if (turn > 0) ok = __all_sync(0xffffffffu, mbar_wait(&ctl.empty[s], (turn & 1u) ^ 1u, stop));
+        if (!ok) break;
+        __half* b = tiles + s * (shape.stage_bytes() / 2);
+        if (issues) {
           mbar_expect_tx(&ctl.full[s], shape.resident ? kPartBytes : kPartBytes * (1 + sets));
-          tma_load_2d(b, &map, kb * kTileK, static_cast<int>(t * kTile), &ctl.full[s]);
+          tma_load_2d(b, &map, kb * kTileK, tile_of(t) * kTile, &ctl.full[s]);
           if (!shape.resident)
             for (int set = 0; set < sets; set++)
-              tma_load_2d(b + (1 + set) * kPart, &map, kb * kTileK, static_cast<int>(q0) + set * kTile, &ctl.full[s]);
-          if (++s == stages) s = 0, turn++;
+              tma_load_2d(b + (1 + set) * kPart, &map, kb * kTileK, q0 + set * kTile, &ctl.full[s]);
         }
+        __syncwarp();
+        if (++s == stages) s = 0, turn++;
       }
-      if (!ok && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 1);
     }
-  } else if (warp == 1) {
-    // ---- MMAs --------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 1);
+  } else if (warp <= 2) {
+    // ---- MMAs: a warp per set, so that one set's waits pass under the other's MMAs ----------------
+    const int set = warp - 1;
+    if (set < sets) {
       constexpr uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(kTile >> 3) << 17) |
                                  (static_cast<uint32_t>(kTile >> 4) << 24);
-      bool ok       = !shape.resident || mbar_wait(&ctl.queries, 0, stop);
-      int s         = 0;
-      uint32_t turn = 0;
-      for (int64_t t = 0; t < ntiles && ok; t++) {
-        const int b      = static_cast<int>(t & 1);
+      constexpr uint64_t kPartUnits = kPartBytes >> 4;  // of a descriptor's address
+      const uint64_t stage_units    = shape.stage_bytes() >> 4;
+      const uint64_t tiles_desc     = umma_desc(tiles);
+      const uint64_t own_desc       = shape.resident ? umma_desc(queries + set * nkb * kPart) : tiles_desc + (1 + set) * kPartUnits;
+      const bool issues = elect_one();
+      bool ok           = !shape.resident || __all_sync(0xffffffffu, mbar_wait(&ctl.queries, 0, stop));
+      int s             = 0;
+      uint32_t turn     = 0;
+      for (int t = 0; t < visits && ok; t++) {
+        const int b      = t & 1;
         const uint32_t u = static_cast<uint32_t>(t >> 1);
-        if (t >= 2) ok = mbar_wait(&ctl.acc_empty[b], (u & 1u) ^ 1u, stop);
+        if (t >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&ctl.acc_empty[set][b], (u & 1u) ^ 1u, stop));
         if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + static_cast<uint32_t>((2 * b + set) * kTile);
         for (int kb = 0; kb < nkb; kb++) {
-          ok = mbar_wait(&ctl.full[s], turn & 1u, stop);
+          ok = __all_sync(0xffffffffu, mbar_wait(&ctl.full[s], turn & 1u, stop));
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const __half* tile = tiles + s * (shape.stage_bytes() / 2);
-          const uint64_t db  = umma_desc(tile);
-          for (int set = 0; set < sets; set++) {
-            const uint64_t da = umma_desc(shape.resident ? queries + (set * nkb + kb) * kPart : tile + (1 + set) * kPart);
+          const uint64_t db = tiles_desc + s * stage_units;
+          const uint64_t da = own_desc + (shape.resident ? kb * kPartUnits : s * stage_units);
+          if (issues) {
 #pragma unroll
             for (int k = 0; k < kTileK / 16; k++)
-              umma_f16(tmem + static_cast<uint32_t>((2 * b + set) * kTile), da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              if (kb * kTileK + 16 * k < D)  // beyond it a tile's columns are zero
+                umma_f16(acc, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit(&ctl.empty[s]);  // arrives when the MMAs reading this stage are done
+            if (kb + 1 == nkb) umma_commit(&ctl.acc_full[set][b]);
           }
-          umma_commit(&ctl.empty[s]);  // arrives when the MMAs reading this stage are done
+          __syncwarp();
           if (++s == stages) s = 0, turn++;
         }
-        if (ok) umma_commit(&ctl.acc_full[b]);
       }
-      if (!ok && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 2);
+      if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 2);
     }
-  } else if (const int set = (warp - 2) >> 2; set < sets) {
+  } else if (const int set = (warp - 3) >> 2; set < sets) {
     // ---- epilogue: one query row per thread ----------------------------------------------------
     const int quarter  = warp & 3;  // the TMEM lanes this warp may read
-    const int64_t wrow = q0 + set * kTile + quarter * 32;  // the warp's first query row
-    const int64_t row  = wrow + lane;
+    const int wrow     = q0 + set * kTile + quarter * 32;  // the warp's first query row
+    const int row      = wrow + lane;
     const bool live    = row < q_end;
     const int room     = shape.room;
     float2* rows_noted = noted + static_cast<size_t>(set * kTile + quarter * 32) * (room + 1);  // of the warp's 32 rows
     float2* mine       = rows_noted + lane * (room + 1);  // an odd number of entries apart: no bank conflicts either way
-    int32_t* ids       = best_id + (wrow - q_first) * K;
-    float* vals        = best_d + (wrow - q_first) * K;
+    int32_t* ids       = best_id + static_cast<int64_t>(wrow - q_first) * K;
+    float* vals        = best_d + static_cast<int64_t>(wrow - q_first) * K;
     float kth          = live ? INFINITY : -INFINITY;  // what a row has to beat: its K-th best at the last merge
     int have           = 0;                            // entries of the row in the output arrays
-    int count          = 0;                            // entries noted since
-    float* nb          = ctl.nb[warp - 2];
+    const uint32_t at0     = smem_u32(mine);
+    const uint32_t last_at = at0 + 8 * (room - 8);  // beyond it there is no room for eight more
+    uint32_t at            = at0;                   // where the next improvement goes
+    float* nb              = ctl.nb[warp - 3];
     auto merge_rows = [&](unsigned which) {
       while (which != 0) {
         const int L = __ffs(which) - 1;
         which &= which - 1;
-        const int c = __shfl_sync(0xffffffffu, count, L), h = __shfl_sync(0xffffffffu, have, L);
+        const int c = static_cast<int>(__shfl_sync(0xffffffffu, at - at0, L) >> 3), h = __shfl_sync(0xffffffffu, have, L);
         __syncwarp();
         const float last = merge_noted<kRegs>(rows_noted + L * (room + 1), c, h, K, vals + static_cast<int64_t>(L) * K,
                                               ids + static_cast<int64_t>(L) * K);
         __syncwarp();
         if (lane == L) {
-          kth   = last;
-          have  = min(K, h + c);
-          count = 0;
+          kth  = fminf(kth, last);
+          have = min(K, h + c);
+          at   = at0;
         }
       }
     };
-    // 32 columns of the tile: the least of every eight is looked at first; where one of the warp's rows
-    // has an improvement among them, every thread appends its own. Once a row has no room for eight
-    // more, the full rows are merged and the scan goes on with the columns after.
-    auto scan = [&](const uint32_t (&r)[32], int col, int64_t first) {
-      float d[32];
+    // t of 32 columns; a row itself is infinitely far
+    auto distances = [&](const uint32_t (&r)[32], int col, int first, float* d) {
 #pragma unroll
       for (int g = 0; g < 8; g++) {
         const float4 nn = *reinterpret_cast<const float4*>(nb + col + g * 4);
         minus_twice(r[g * 4 + 0], r[g * 4 + 1], nn.x, nn.y, d[g * 4 + 0], d[g * 4 + 1]);
         minus_twice(r[g * 4 + 2], r[g * 4 + 3], nn.z, nn.w, d[g * 4 + 2], d[g * 4 + 3]);
       }
-      if (first < wrow + 32 && first + 32 > wrow) {  // the rows themselves
+      if (first < wrow + 32 && first + 32 > wrow) {
 #pragma unroll
         for (int i = 0; i < 32; i++)
           if (first + i == row) d[i] = INFINITY;
       }
-      float least[4];
+    };
+    // 64 columns of the tile: the least of every eight is looked at first; where one of the warp's rows
+    // has an improvement among them, every thread appends its own; a row without room for eight more is
+    // merged. (A vote and a branch per eight columns: 25 ms where this takes 21.)
+    auto scan = [&](const uint32_t (&r)[2][32], int col, int first) {
+      float d[64];
+      distances(r[0], col, first, d);
+      distances(r[1], col + 32, first + 32, d + 32);
+      float least[8];
 #pragma unroll
-      for (int g = 0; g < 4; g++)
+      for (int g = 0; g < 8; g++)
         least[g] = fminf(min3(min3(d[8 * g], d[8 * g + 1], d[8 * g + 2]), d[8 * g + 3], d[8 * g + 4]),
                          min3(d[8 * g + 5], d[8 * g + 6], d[8 * g + 7]));
-      if (!__any_sync(0xffffffffu, fminf(min3(least[0], least[1], least[2]), least[3]) < kth)) return;
-      int from = 0;
-      for (;;) {
-        bool full = false;
+      const float all = fminf(min3(min3(least[0], least[1], least[2]), least[3], least[4]), min3(least[5], least[6], least[7]));
+      if (!__any_sync(0xffffffffu, all < kth)) return;
+      // groups of eight with an improvement, of the thread and of the warp
+      unsigned own = 0;
 #pragma unroll
-        for (int g = 0; g < 4; g++)
-          if (!full && g >= from && __any_sync(0xffffffffu, least[g] < kth)) {
+      for (int g = 0; g < 8; g++)
+        own |= least[g] < kth ? 1u << g : 0u;
+      unsigned todo = __reduce_or_sync(0xffffffffu, own);
+      while (todo != 0) {
+        // all of them at once when every row has the room, else one by one
+        const bool room_for_all = __all_sync(0xffffffffu, at + 64 * __popc(own & todo) <= last_at + 64);
+        const unsigned now      = room_for_all ? todo : todo & (0u - todo);
+#pragma unroll
+        for (int g = 0; g < 8; g++)
+          if (now & (1u << g)) {
 #pragma unroll
             for (int i = 0; i < 8; i++)
-              if (d[8 * g + i] < kth) {
-                mine[count] = make_float2(d[8 * g + i], __int_as_float(static_cast<int32_t>(first) + 8 * g + i));
-                count++;
-              }
-            full = __any_sync(0xffffffffu, count > room - 8);
-            from = g + 1;
+              note_below(d[8 * g + i], kth, first + 8 * g + i, at);
           }
-        if (!full) break;
-        merge_rows(__ballot_sync(0xffffffffu, count > room - 8));
+        todo ^= now;
+        const unsigned full = __ballot_sync(0xffffffffu, at > last_at);
+        if (full != 0) merge_rows(full);
       }
     };
-    // norms of the rows of a tile, four per lane; rows beyond the matrix never win
-    auto fetch_norms = [&](int64_t t, float (&v)[4]) {
+    // norms of the rows of a visit's tile, four per lane; rows beyond the matrix never win
+    auto fetch_norms = [&](int visit, float (&v)[4]) {
+      const int first = tile_of(visit) * kTile + lane;
 #pragma unroll
       for (int i = 0; i < 4; i++) {
-        const int64_t r = t * kTile + i * 32 + lane;
-        v[i]            = r < n ? __ldg(norm + r) : INFINITY;
+        const int r = first + i * 32;
+        v[i]        = r < n ? __ldg(norm + r) : INFINITY;
       }
     };
     float ahead[4];
     fetch_norms(0, ahead);
     bool ok = true;
-    for (int64_t t = 0; t < ntiles; t++) {
-      const int b      = static_cast<int>(t & 1);
-      const uint32_t u = static_cast<uint32_t>(t >> 1);
+    // the accumulator of a visit is there, and so are the norms of its tile
+    auto begin = [&](int visit) {
       __syncwarp();  // every lane is done with the norms of the tile before
 #pragma unroll
       for (int i = 0; i < 4; i++)
         nb[i * 32 + lane] = ahead[i];
-      fetch_norms(t + 1, ahead);  // in flight behind this tile
+      fetch_norms(visit + 1, ahead);  // in flight behind this tile
       __syncwarp();
-      ok = mbar_wait(&ctl.acc_full[b], u & 1u, stop);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      ok = __all_sync(0xffffffffu, mbar_wait(&ctl.acc_full[set][visit & 1], static_cast<uint32_t>(visit >> 1) & 1u, stop));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>((2 * b + set) * kTile);
+      return ok;
+    };
+    // 32 columns of the visit's accumulator; once the last are there the tensor cores may overwrite it
+    const uint32_t tmem_rows = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(set * kTile);
+    auto columns             = [&](int visit, int c, uint32_t (&r)[32]) {
+      tmem_ld32(tmem_rows + static_cast<uint32_t>(visit & 1) * 2 * kTile + static_cast<uint32_t>(c * 32), r);
+    };
+    auto arrived = [&](int visit, bool last) {
+      tmem_ld_wait();
+      if (last) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.acc_empty[set][visit & 1]);
+      }
+    };
+    int visit = 0;
+    {
+      // one least value per column of a tile, columns 32 kParts apart sharing one: neighbors that stand
+      // next to each other in the matrix still count one by one
+      constexpr int kParts = kRegs == 1 ? 2 : kRegs == 2 ? 3 : 4;
+      float least[kParts][32];
+#pragma unroll
+      for (int c = 0; c < kParts; c++)
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+          least[c][i] = INFINITY;
 #pragma unroll 1
-      for (int c = 0; c < 4; c++) {
-        uint32_t r[32];
-        tmem_ld32(taddr + static_cast<uint32_t>(c * 32), r);
-        tmem_ld_wait();
-        if (c == 3) {
-          // the accumulator is in registers: the tensor cores may overwrite it
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl.acc_empty[b]);
+      for (; visit < sampled; visit++) {
+        if (!begin(visit)) break;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          uint32_t r[32];
+          float d[32];
+          columns(visit, c, r);
+          arrived(visit, c == 3);
+          distances(r, c * 32, tile_of(visit) * kTile + c * 32, d);
+#pragma unroll
+          for (int i = 0; i < 32; i++)
+            least[c % kParts][i] = fminf(least[c % kParts][i], d[i]);
         }
-        scan(r, c * 32, t * kTile + c * 32);
+      }
+      // halving of the range between the least and the largest of them, never below K of them
+      float low = INFINITY, high = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < kParts; c++)
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+          low  = fminf(low, least[c][i]);
+          high = fmaxf(high, least[c][i]);
+        }
+      auto below = [&](float bar) {
+        int many = 0;
+#pragma unroll
+        for (int c = 0; c < kParts; c++)
+#pragma unroll
+          for (int i = 0; i < 32; i++)
+            many += least[c][i] <= bar ? 1 : 0;
+        return many;
+      };
+#pragma unroll 1
+      for (int step = 0; step < 12; step++) {
+        const float middle = 0.5f * low + 0.5f * high;
+        if (below(middle) >= K)
+          high = middle;
+        else
+          low = middle;
+      }
+      // rows as far as the bar may still be wanted: the bar that a row has to beat lies above it
+      if (live && fabsf(high) < 3e38f && below(high) >= K) kth = fmaf(fabsf(high), 2.4e-7f, high) + 1e-37f;
+    }
+#pragma unroll 1
+    for (; ok && visit < visits; visit++) {
+      if (!begin(visit)) break;
+#pragma unroll 1
+      for (int c = 0; c < 4; c += 2) {
+        uint32_t r[2][32];
+        columns(visit, c, r[0]);
+        columns(visit, c + 1, r[1]);
+        arrived(visit, c == 2);
+        scan(r, c * 32, tile_of(visit) * kTile + c * 32);
       }
     }
     if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 3);
     if (ok) {
-      merge_rows(__ballot_sync(0xffffffffu, count > 0));
+      merge_rows(__ballot_sync(0xffffffffu, at != at0));
       for (int L = 0; L < 32 && wrow + L < q_end; L++) {
         const int h    = __shfl_sync(0xffffffffu, have, L);
         const float qn = __ldg(norm + wrow + L);
@@ -483,9 +613,15 @@ void knn_tc(const __half* x, const float* norm, int64_t n, int D, int K, int64_t
   const int64_t round  = int64_t{2} * kTile * sms;
   const int64_t rest   = q_count % round;
   const int64_t narrow = rest <= round / 2 ? (rest + kTile - 1) / kTile : 0;
+  // Tiles that are looked at for the bars: a visit costs the same whatever it saves, an improvement the
+  // same work at any n, and K ln(n / visits) of them are left: the best number of visits grows with K
+  // alone. 266 665 x 96, K = 64: 34.5 ms with 16 visits, 33.5 with 2 K and 4 K, 45.5 with every tile.
+  const int64_t ntiles = (n + kTile - 1) / kTile;
+  const int64_t spread = std::max<int64_t>(1, ntiles / std::max(16, kVisitsPerK * K));
   const int64_t wide   = narrow > 0 || rest == 0 ? (q_count - rest) / (2 * kTile) : (q_count + 2 * kTile - 1) / (2 * kTile);
-  kernel<<<static_cast<unsigned>(wide + narrow), kKnnThreads, smem, s>>>(map, norm, n, nkb, K, shape, static_cast<int>(wide), q_first,
-                                                                         q_count, best_id, best_d, error);
+  kernel<<<static_cast<unsigned>(wide + narrow), kKnnThreads, smem, s>>>(
+    map, norm, static_cast<int>(n), D, K, shape, static_cast<int>((ntiles + spread - 1) / spread), static_cast<int>(spread),
+    static_cast<int>(wide), static_cast<int>(q_first), static_cast<int>(q_count), best_id, best_d, error);
 }
 
 }  // namespace octex_b200::kernels

@@ -39,7 +39,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
 {
   const uint32_t addr = smem_u32(bar);
   for (uint32_t i = 0; i < kSpinLimit; i++) {
-    if (give_up != nullptr && *give_up != 0) return false;
+    if (give_up != nullptr && (i & 7u) == 7u && *give_up != 0) return false;
     uint32_t ok;
     asm volatile(
       "{\n\t"
