@@ -340,6 +340,44 @@ __device__ __forceinline__ void rank_sort(const unsigned long long* src, int cnt
   }
 }
 
+/// The first `want` keys of the ascending list old[0, n) and the m distinct keys add[0, m), none of them in
+/// the list, into dst, ascending; order [m] is scratch. A new key's place is the number of new keys below
+/// it, counted, and of old ones, found by halving; an old key's is its own plus the new ones below it,
+/// halving in their order. One barrier where a sorting network over all of them has 36 (256 keys) to 55
+/// (1 024 keys): 1 000 queries with the default parameters 356 -> 331 us, 10 000 embeddings with 256 start
+/// points and three waves 9.59 -> 9.20 ms. All threads of the block call it.
+__device__ __forceinline__ void merge_sorted(const unsigned long long* old, int n, const unsigned long long* add, int m,
+                                             unsigned long long* order, int want, unsigned long long* dst)
+{
+  auto below = [](const unsigned long long* list, int count, unsigned long long key) {
+    int lo = 0, hi = count;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (list[mid] < key)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    return lo;
+  };
+  for (int j = threadIdx.x; j < m; j += blockDim.x) {
+    const unsigned long long mine = add[j];
+    int at                        = 0;
+#pragma unroll 4
+    for (int i = 0; i < m; i++)
+      at += add[i] < mine;
+    order[at]       = mine;
+    const int place = at + below(old, n, mine);
+    if (place < want) dst[place] = mine;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned long long mine = old[i];
+    const int place               = i + below(order, m, mine);
+    if (place < want) dst[place] = mine;
+  }
+}
+
 /// float(h) - q for an fp16 bit pattern h: the mixed-precision subtract of sm_100 (PTX ISA 8.6),
 /// the same value as converting first (the conversion is exact) without the conversion.
 __device__ __forceinline__ float half_minus(unsigned short h, float q)
@@ -781,6 +819,8 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
   if (total <= 2 * P) {
     if (total <= kRankMax) {
       rank_sort(pool, total, sorted);
+    } else if (nk > 0 && total - nk <= P) {
+      merge_sorted(pool, nk, pool + nk, total - nk, sorted + P, KO, sorted);
     } else {
       int width = P;
       while (width < total)
@@ -1114,8 +1154,31 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // cut in any order)
   const int R = a.sketch_rank ? a.KO : a.R;
   int ns      = n;
-  if (n > R) {
-    auto key_at = [&](int i) { return rank_key(dist[i], static_cast<unsigned>(cand[i])); };
+  auto key_at = [&](int i) { return rank_key(dist[i], static_cast<unsigned>(cand[i])); };
+  // A search that ranks by sketch distance keeps what it selects here, so a key beyond the last one of a
+  // full kept list is out already. Where the keys that are left fit, they need no selection: which of them
+  // stay is the merge's to say, and the kept list comes out the same (with the merge by places: 2 500
+  // embeddings, 512 start points and three waves 5.17 -> 4.98 ms).
+  bool selected = false;
+  if (a.sketch_rank && !fresh && kid[a.KO - 1] >= 0) {
+    const unsigned long long bound = rank_key(kd[a.KO - 1], static_cast<unsigned>(kid[a.KO - 1]));
+    if (threadIdx.x == 0) ctrl[0] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      if (key_at(i) < bound) {
+        const int s = atomicAdd(&ctrl[0], 1);
+        if (s < R) {
+          sid[s] = cand[i];
+          sdv[s] = dist[i];
+        }
+      }
+    __syncthreads();
+    if (ctrl[0] <= R) {
+      ns       = ctrl[0];
+      selected = true;
+    }
+  }
+  if (!selected && n > R) {
     auto hi_at          = [&](int i) { return __float_as_uint(dist[i]); };
     auto lo_at          = [&](int i) { return static_cast<unsigned>(cand[i]); };
     const radix_cut_t c = smallest_cut(hi_at, lo_at, n, R, hist, ctrl);
@@ -1131,7 +1194,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
       }
     }
     ns = R;
-  } else {
+  } else if (!selected) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       sid[i] = cand[i];
       sdv[i] = dist[i];

@@ -170,6 +170,23 @@ def test_k_larger_than_starts_and_k_one(oracle, gpu_small):
         assert np.array_equal(dist.view(np.uint32), want_dist.view(np.uint32))
 
 
+@pytest.mark.parametrize("kw", [
+    dict(starts=100, waves=2, rerank=100, wave_rerank=28), dict(starts=100, waves=2, rerank=100, wave_rerank=29),
+    dict(starts=128, waves=3, rerank=128, wave_rerank=128), dict(starts=128, waves=2, rerank=128, wave_rerank=200),
+    dict(starts=65, waves=2, rerank=400, wave_rerank=64), dict(starts=512, waves=2, rerank=40, wave_rerank=512),
+    dict(starts=65, waves=3, sketch_rank=True, final_rerank=32), dict(starts=128, waves=3, sketch_rank=True, final_rerank=0),
+    dict(starts=257, waves=2, sketch_rank=True, final_rerank=200), dict(starts=1000, waves=2, sketch_rank=True, final_rerank=64)])
+def test_merge_forms(oracle, gpu_small, gpu_wide, kw):
+    """The merge at the lengths where its form changes (128 keys in all, as many new keys as the kept list
+    takes rounded up to a power of two), full and short kept lists, and searches ranked by sketch distance
+    whose later rounds take what beats the kept list without a selection, or have too much of it."""
+    for idx, arrays, meta, _, queries in (gpu_small, gpu_wide):
+        for k in (1, 10, 32):
+            dist, ids, want_dist, want_ids, _, _ = check_against_checker(oracle, idx, arrays, meta, queries, k=k, read=8, **kw)
+            assert np.array_equal(ids, want_ids), (kw, k)
+            assert np.array_equal(dist.view(np.uint32), want_dist.view(np.uint32)), (kw, k)
+
+
 def test_batches_partial_and_empty(gpu_small):
     """batch splitting, a padded last batch and an empty query set (tests/test_api.py of the
     reference: batch=37, empty input)."""
