@@ -278,6 +278,13 @@ OCTEX_B200_EXPORT cuvsError_t octexB200SearchWait(cuvsResources_t res, cuvsOctex
                                                   cuvsOctexIndex_t index, const float* queries,
                                                   int64_t n_queries, int64_t dim, int64_t* neighbors,
                                                   float* distances, int64_t k, int32_t on_device);
+/* *in_place = 1 when a search with these device arrays works on them where they are: one process, all
+ * three in the memory of the index's GPU (and on the boundaries of their types), and that GPU current.
+ * Otherwise (another GPU's memory, managed or page-locked memory) they are copied in and out. */
+OCTEX_B200_EXPORT cuvsError_t octexB200SearchInPlace(cuvsOctexIndex_t index, const float* queries,
+                                                     const int64_t* neighbors, const float* distances,
+                                                     int32_t* in_place);
+
 /* detail::resident_search (cpp/src/neighbors/octex/search.cu:983-997): search again the queries of
  * the previous call, which are still on the GPU, and leave the results there. The timing protocol
  * of the reference's benchmark uses it (cpp/bench/octex_bench.cu:223-253). */

@@ -89,7 +89,8 @@ SYMBOLS = (
     "cuvsOctexIndexGetDim", "cuvsOctexIndexGetCopies", "cuvsOctexIndexGetNumDevices",
     "cuvsOctexIndexGetDevices", "cuvsOctexIndexGetDeviceBytes", "cuvsOctexBuild", "cuvsOctexLoad",
     "cuvsOctexSearch", "octexB200Search", "octexB200LoadRank", "octexB200Attach",
-    "octexB200SearchWait", "octexB200SearchResident", "octexB200ProfileBatch", "octexB200SetDebug", "octexB200Fetch",
+    "octexB200SearchWait", "octexB200SearchInPlace", "octexB200SearchResident", "octexB200ProfileBatch",
+    "octexB200SetDebug", "octexB200Fetch",
     "octexB200CellCodes", "octexB200QueryCodesStatic", "octexB200SetProjection",
     "octexB200CommUniqueId", "octexB200CommInit", "octexB200CommDisconnect", "octexB200CheckLast",
     "octexB200MemoryReport", "octexB200Build", "octexB200ExactNeighbors", "octexB200SetTable", "octexB200SearchedTable",

@@ -484,6 +484,15 @@ cuvsError_t octexB200SearchWait(cuvsResources_t res, cuvsOctexSearchParams_t par
   });
 }
 
+cuvsError_t octexB200SearchInPlace(cuvsOctexIndex_t index, const float* queries, const int64_t* neighbors,
+                                   const float* distances, int32_t* in_place)
+{
+  return translate([=] {
+    OCTEX_EXPECTS(index != nullptr && in_place != nullptr, "octex: a search argument is NULL");
+    *in_place = octex_b200::detail::search_in_place(as_index(*index)->impl(), queries, neighbors, distances);
+  });
+}
+
 cuvsError_t octexB200SearchResident(cuvsResources_t res, cuvsOctexSearchParams_t params,
                                     cuvsOctexIndex_t index, int64_t n_queries, int64_t k)
 {

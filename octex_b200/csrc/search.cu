@@ -4,7 +4,7 @@
 // search_impl :816-961, the two search overloads :1020-1064) for one process per GPU. Parameter
 // limits and error texts are the reference's. A batch is two kernels and one per wave: projection
 // with cell lookup and sketch-space queries, first round, waves, the last of which writes the
-// results. Queries and results in device memory are used where they are, on the caller's stream, and
+// results. Queries and results in the memory of the index's GPU are used where they are, on the caller's stream, and
 // every kernel is launched for the queries there are: no copies, no padding. A batch that stays in the
 // plan's buffers (resident searches, several processes) is replayed as one CUDA graph.
 
@@ -622,6 +622,19 @@ auto device_reaches(const void* p) -> bool
   return at.type != cudaMemoryTypeUnregistered;
 }
 
+/// True when p is memory of this GPU itself and on a boundary of `align` bytes: what the kernels of a
+/// search may load and store themselves. Another GPU's memory is not mapped here, managed and
+/// page-locked memory is better copied once than read over the bus by every block.
+auto own_memory(const void* p, int device, size_t align) -> bool
+{
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == device && reinterpret_cast<uintptr_t>(p) % align == 0;
+}
+
 /// Page-locked staging of at least `bytes`, kept with the plan.
 void* staging(dbuf& b, int device, size_t bytes)
 {
@@ -652,10 +665,11 @@ auto search_device(index_impl& ix, search_params const& sp, cudaStream_t caller,
   return pl;
 }
 
-/// A search by one process with queries and results in host memory (or in another GPU's): the copies
-/// are queued around the kernels. Several batches alternate between two lanes, each a plan on a stream
-/// of its own: the copies of one batch run under the kernels of the other. Page-locked arrays are
-/// copied from and to directly; ordinary ones pass through page-locked staging of the plan.
+/// A search by one process with queries and results that are not all memory of its GPU (host memory,
+/// another GPU's): the copies are queued around the kernels. Several batches alternate between two
+/// lanes, each a plan on a stream of its own: the copies of one batch run under the kernels of the
+/// other. Page-locked arrays are copied from and to directly; ordinary ones pass through page-locked
+/// staging of the plan.
 void search_copied(index_impl& ix, search_params const& sp, cudaStream_t caller, int cur, const float* queries,
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
 {
@@ -744,6 +758,15 @@ void search_copied(index_impl& ix, search_params const& sp, cudaStream_t caller,
 
 }  // namespace
 
+auto search_in_place(index_impl const& ix, const float* queries, const int64_t* neighbors, const float* distances) -> bool
+{
+  int cur = 0;
+  OCTEX_CUDA_TRY(cudaGetDevice(&cur));
+  const int device = ix.part.device;
+  return ix.world == 1 && cur == device && own_memory(queries, device, alignof(float)) &&
+         own_memory(neighbors, device, alignof(int64_t)) && own_memory(distances, device, alignof(float));
+}
+
 void search_impl(resources const& res,
                  search_params const& sp,
                  index const& idx,
@@ -765,7 +788,7 @@ void search_impl(resources const& res,
   OCTEX_CUDA_TRY(cudaGetDevice(&cur));
   cudaStream_t caller = res.stream;
   auto& p             = ix.part;
-  if (ix.world == 1 && !resident && !host_out && cur == p.device) {
+  if (!resident && !host_out && search_in_place(ix, queries, neighbors, distances)) {
     auto pl = search_device(ix, sp, caller, queries, nq, neighbors, distances, k);
     if (wait) {
       OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));

@@ -73,6 +73,10 @@ void search_impl(resources const& res,
                  bool resident,
                  bool wait = false);
 
+/// True when a search with these device arrays works on them where they are (one process, everything in
+/// the memory of the index's GPU, which is the current device); otherwise they are copied in and out.
+auto search_in_place(index_impl const& ix, const float* queries, const int64_t* neighbors, const float* distances) -> bool;
+
 /// One batch of the queries already on the GPU, launched kernel by kernel with an event between
 /// them: milliseconds of center+sketch, projection, cell codes, lookup, first round, each wave,
 /// best k (the per-kernel counterpart of detail::timed_batch, search.cu:965-981 of the reference).

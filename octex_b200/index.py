@@ -330,6 +330,12 @@ class Index:
                 raise ValueError("octex: queries must be a matrix [m, dim]")
             m, d = q.shape
             on_device = q.is_cuda
+            if on_device and q.device.index != torch.cuda.current_device():
+                # the call works on a stream of the queries' device
+                with torch.cuda.device(q.device):
+                    return self.search(q, k, read=read, starts=starts, waves=waves, rerank=rerank,
+                                       wave_rerank=wave_rerank, batch=batch, sketch_rank=sketch_rank,
+                                       final_rerank=final_rerank, neighbors=neighbors, distances=distances)
             def usable(g, dt):
                 return (_is_torch(g) and g.dtype == dt and g.device == q.device
                         and g.is_contiguous() and tuple(g.shape) == (m, k))

@@ -96,3 +96,81 @@ def test_batches_of_any_size_share_a_plan():
         t.join()
     assert not failures
     idx.close()
+
+
+def search_at(idx, queries, ids, dist, m, dim, k, on_device=1, wait=True, stream=0, **kw):
+    """The C call on addresses, as a program that has no torch tensors makes it."""
+    import ctypes as C
+    from octex_b200 import _lib
+    p = octex_b200.search_params(**kw)
+    fn = _lib.lib().octexB200SearchWait if wait else _lib.lib().octexB200Search
+    _lib.check(fn(idx._resources(stream).h, C.byref(p), idx._h, C.c_void_p(queries), C.c_int64(m), C.c_int64(dim),
+                  C.c_void_p(ids), C.c_void_p(dist), C.c_int64(k), C.c_int32(on_device)))
+
+
+def in_place(idx, queries, ids, dist):
+    import ctypes as C
+    from octex_b200 import _lib
+    out = C.c_int32(-1)
+    _lib.check(_lib.lib().octexB200SearchInPlace(idx._h, C.c_void_p(queries), C.c_void_p(ids), C.c_void_p(dist),
+                                                 C.byref(out)))
+    return out.value
+
+
+def test_arrays_outside_the_index_gpu_are_copied():
+    """A device search works in place only on aligned memory of the index's own GPU. Page-locked and
+    ordinary host memory given as device arrays, and results off the boundaries of their types, are
+    copied, as they were when every search copied. The route is asserted before the search: a kernel
+    never gets an address it may not use."""
+    import torch
+    from octex_b200 import synth
+    dim, n, k = 64, 97, 10
+    idx, _ = make_index(dim, copies=8, blocks=4)
+    kw = dict(read=8, starts=32, waves=1, rerank=64, wave_rerank=64)
+    queries = synth.plumbing(n, dim, seed=1)
+    want = idx.search(queries, k, **kw)
+    q = torch.as_tensor(queries, device="cuda")
+    ids, dist = torch.empty((n, k), dtype=torch.int64, device="cuda"), torch.empty((n, k), device="cuda")
+    assert in_place(idx, q.data_ptr(), ids.data_ptr(), dist.data_ptr()) == 1
+    host = (np.ascontiguousarray(queries), np.zeros((n, k), np.int64), np.zeros((n, k), np.float32))
+    addresses = [a.ctypes.data for a in host]
+    for at in range(3):  # one of the three elsewhere is enough
+        three = [q.data_ptr(), ids.data_ptr(), dist.data_ptr()]
+        three[at] = addresses[at]
+        assert in_place(idx, *three) == 0
+    assert in_place(idx, *addresses) == 0
+    search_at(idx, *addresses, n, dim, k, **kw)
+    assert same((host[2], host[1]), want)
+    pinned = [torch.as_tensor(a).pin_memory() for a in (queries, np.zeros((n, k), np.int64), np.zeros((n, k), np.float32))]
+    addresses = [t.data_ptr() for t in pinned]
+    assert in_place(idx, *addresses) == 0
+    search_at(idx, *addresses, n, dim, k, **kw)
+    assert same((pinned[2].numpy(), pinned[1].numpy()), want)
+    words = torch.zeros(2 * n * k + 1, dtype=torch.int32, device="cuda")  # ids four bytes off
+    off = words.data_ptr() + (4 if words.data_ptr() % 8 == 0 else 0)
+    assert in_place(idx, q.data_ptr(), off, dist.data_ptr()) == 0
+    search_at(idx, q.data_ptr(), off, dist.data_ptr(), n, dim, k, **kw)
+    got = words.cpu().numpy()[1:].tobytes()
+    assert same((dist.cpu().numpy(), np.frombuffer(got, np.int64).reshape(n, k)), want)
+    idx.close()
+
+
+def test_queries_on_another_gpu():
+    """Torch queries on a GPU the index is not on, with either device current: copied, ordered after
+    the stream of the queries' device, results there."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    from octex_b200 import synth
+    idx, _ = make_index(64, copies=8, blocks=4)
+    kw = dict(read=8, starts=32, waves=1, rerank=64, wave_rerank=64)
+    queries = synth.plumbing(300, 64, seed=1)
+    want = idx.search(queries, 10, **kw)
+    for current in (0, 1):
+        with torch.cuda.device(current):
+            q = torch.as_tensor(queries, device="cuda:1")
+            for batch in (10000, 70):
+                d, i = idx.search(q + 0, 10, batch=batch, **kw)
+                assert d.device == i.device == q.device
+                assert same((d.cpu().numpy(), i.cpu().numpy()), want)
+    idx.close()
