@@ -221,15 +221,20 @@ __device__ __forceinline__ long long cell_code_tame(const float (&y)[8 * B], flo
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same code again with half the instructions of block_code_tame (117 against 248), for the
-// kernel that decodes every query. Rounding v to r leaves e = v - r (exact); the other coset leaves
+// The same code again with about half the arithmetic of block_code_tame (one coset repaired instead of two),
+// for the kernel that decodes every query. Rounding v to r leaves e = v - r (exact); the other coset leaves
 // 1/2 - |e| in every coordinate. With A = sum |e|, m = max |e|, n = min |e| the squared errors of the
 // two cosets after their parity repairs differ by
 //     D = A - 2 + (odd ? 1 - 2 m : 0) - (odd' ? 2 n : 0)
 // so the nearer coset is known before either is worked out, and only the one taken is repaired. D is
-// good to 4e-6 (eight additions of terms up to 1/2, and the 2^-25 by which v - 1/2 may be rounded), and
-// the two sums that block_code_tame compares, of at most eight squares up to 1, to 1e-6 each: where
-// |D| < 2e-5 the block is `doubtful` and goes to block_code_tame. The rest is exact: both parities come
+// good to 4e-6 (eight additions of terms up to 1/2), and the two sums that block_code_tame compares, of
+// at most eight squares up to 1, to 1e-6 each. What grows with the coordinates is the rounding of
+// v - 1/2, which the half coset starts from: exact for v >= 1/2, but a v just above -2^k crosses a
+// binade, so it is off by up to d = (V + 1/2) 2^-24 where no |v| exceeds V. A coordinate within d of a
+// tie may then be rounded the other way (its squared error changes by 2 d, in all eight at worst), and
+// the coordinate repaired may be one within 2 d of the worst (4 d), or one of those at a tie (2 d): 22 d
+// in all. Where |D| is below decode_margin = 2.1e-5 + V 2^-19 >= 6e-6 + 22 d the block is `doubtful`
+// and goes to block_code_tame. The rest is exact: both parities come
 // from the low bits of the rounded values, and the coset taken is rounded and repaired by the same
 // operations on the same values as in nearest_d8_tame. Two coordinates at a time share an instruction
 // (the packed fp32 arithmetic of sm_100, each half rounded as on its own).
@@ -274,8 +279,20 @@ __device__ __forceinline__ float min3_abs(float a, float b, float c)
   return fminf(fminf(fabsf(a), fabsf(b)), fabsf(c));
 }
 
-/// Block code of the four pairs y scaled by inv; primes: the eight cell primes in shared memory.
-__device__ __forceinline__ unsigned long long block_code_fast(const f32_pair (&y)[4], float inv,
+/// The larger magnitude, NaN when either is none (fmaxf would drop it).
+__device__ __forceinline__ float max_abs_nan(float a, float b)
+{
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b)));
+  return d;
+}
+
+/// Below this |D| a block with no coordinate beyond `reach` (before the scaling by inv) is doubtful.
+__device__ __forceinline__ float decode_margin(float reach, float inv) { return fmaf(reach * inv, 1.9073486e-6f, 2.1e-5f); }
+
+/// Block code of the four pairs y scaled by inv; primes: the eight cell primes in shared memory;
+/// margin: decode_margin of the block.
+__device__ __forceinline__ unsigned long long block_code_fast(const f32_pair (&y)[4], float inv, float margin,
                                                               const unsigned long long* primes, bool& doubtful)
 {
   const f32_pair up = pack2(kRintMagic, kRintMagic), down = pack2(-kRintMagic, -kRintMagic);
@@ -305,7 +322,7 @@ __device__ __forceinline__ unsigned long long block_code_fast(const f32_pair (&y
   float D = A - 2.f;
   if (odd_i & 1u) D += fmaf(-2.f, m, 1.f);
   if (odd_h & 1u) D = fmaf(-2.f, n, D);
-  doubtful         = fabsf(D) < 2e-5f;
+  doubtful         = fabsf(D) < margin;
   const bool halves = D > 0.f;
   const bool odd    = ((halves ? odd_h : odd_i) & 1u) != 0;
   // the coset taken, from its own rounding on

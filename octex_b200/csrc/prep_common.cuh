@@ -35,12 +35,13 @@ static __device__ __noinline__ unsigned long long block_code_rare(float v0, floa
   return wild ? block_code(v) : block_code_tame(v);
 }
 
-/// Code of a block whose coordinates (scaled by inv) may be any; wild: one of them may be large.
-__device__ __forceinline__ unsigned long long block_code_any(const f32_pair (&own)[4], float inv,
+/// Code of a block whose coordinates (scaled by inv) may be any; wild: one of them may be beyond
+/// kTameLimit, margin: decode_margin of them.
+__device__ __forceinline__ unsigned long long block_code_any(const f32_pair (&own)[4], float inv, float margin,
                                                              const unsigned long long* primes, bool wild)
 {
   bool doubtful;
-  unsigned long long hb = block_code_fast(own, inv, primes, doubtful);
+  unsigned long long hb = block_code_fast(own, inv, margin, primes, doubtful);
   if (wild || doubtful) {
     float v[8];
 #pragma unroll
@@ -67,6 +68,7 @@ struct group_decoder {
   f32_pair y[4 * kOwn];
   const unsigned long long* primes;
   unsigned long long weight;
+  float reach;  // the largest magnitude of the coordinates (NaN: one of them is none)
   bool wild;
 
   __device__ __forceinline__ group_decoder(int sub, const unsigned long long* p) : primes(p)
@@ -77,28 +79,30 @@ struct group_decoder {
       for (int k = 0; k < kOwn; k++)
         weight *= kGolden;
   }
-  /// Which of the two decodes the coordinates need; call it when y is set.
+  /// Which of the decodes the coordinates need; call it when y is set.
   __device__ __forceinline__ void settle(float tame_y)
   {
-    wild = false;
+    reach = 0.f;
 #pragma unroll
     for (int i = 0; i < 4 * kOwn; i++) {
       float a, b;
       unpack2(y[i], a, b);
-      wild = wild || !(fabsf(a) < tame_y) || !(fabsf(b) < tame_y);
+      reach = max_abs_nan(reach, max_abs_nan(a, b));
     }
+    wild = !(reach < tame_y);
   }
   /// All lanes of the warp call it together.
   __device__ __forceinline__ long long code(float inv_f) const
   {
     unsigned long long h = 0;
+    const float margin   = decode_margin(reach, inv_f);
 #pragma unroll
     for (int j = 0; j < kOwn; j++) {
       f32_pair own[4];
 #pragma unroll
       for (int i = 0; i < 4; i++)
         own[i] = y[4 * j + i];
-      const unsigned long long hb = block_code_any(own, inv_f, primes, wild);
+      const unsigned long long hb = block_code_any(own, inv_f, margin, primes, wild);
       h = j == 0 ? hb : h * kGolden + hb;
     }
     if constexpr (kGroup<B> > 1) {
@@ -248,11 +252,12 @@ __device__ __forceinline__ void lookup_pairs(const tc_lookup& look, Fetch fetch,
 
 /// The segment of one (query, copy) by one thread with all of its coordinates (4 B pairs): the form for
 /// large batches, where the instructions of a step count and not how long a warp takes for it. A lane
-/// per block repeats what follows the decode (final mixing, lookup: about 90 instructions) in every
-/// lane of the group. All lanes of the warp call it together; lv [L] are the levels of the copy.
+/// per block repeats what follows the decode (final mixing, lookup) in every lane of the group. reach:
+/// the largest magnitude of the coordinates; wild: it is beyond the short decodes. All lanes of the
+/// warp call it together; lv [L] are the levels of the copy.
 template <int B>
-__device__ __forceinline__ void lookup_alone(const tc_lookup& look, const f32_pair (&y)[4 * B], bool live, bool wild,
-                                             const float* inv_f, const cell_level* lv,
+__device__ __forceinline__ void lookup_alone(const tc_lookup& look, const f32_pair (&y)[4 * B], bool live, float reach,
+                                             bool wild, const float* inv_f, const cell_level* lv,
                                              const unsigned long long* primes, int L, int64_t row, int c, int Cg)
 {
   int first = -1, asked = 0;
@@ -270,13 +275,14 @@ __device__ __forceinline__ void lookup_alone(const tc_lookup& look, const f32_pa
       continue;
     }
     unsigned long long h = 0;
+    const float margin   = decode_margin(reach, inv_f[j]);
 #pragma unroll
     for (int b = 0; b < B; b++) {
       f32_pair own[4];
 #pragma unroll
       for (int i = 0; i < 4; i++)
         own[i] = y[4 * b + i];
-      h = h * kGolden + block_code_any(own, inv_f[j], primes, wild);
+      h = h * kGolden + block_code_any(own, inv_f[j], margin, primes, wild);
     }
     const long long code = finish_code(h);
     answer();

@@ -348,18 +348,18 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
       }
     } else if constexpr (kMode == tc_mode::bulk) {
       f32_pair y[16];
-      bool wild = false;  // a coordinate too large for the short decode (or not a number)
+      float reach = 0.f;  // the largest magnitude (NaN: a coordinate is not a number)
   #pragma unroll
       for (int i = 0; i < 16; i++) {
         const float2 sh = *reinterpret_cast<const float2*>(sm.shift[set] + cc * 32 + 2 * i);
         const float a   = __half2float(__float2half_rn(__fadd_rn(__uint_as_float(r[2 * i]), sh.x)));
         const float b   = __half2float(__float2half_rn(__fadd_rn(__uint_as_float(r[2 * i + 1]), sh.y)));
-        wild            = wild || !(fabsf(a) < tame_y) || !(fabsf(b) < tame_y);
+        reach           = max_abs_nan(reach, max_abs_nan(a, b));
         y[i]            = pack2(a, b);
       }
       // a row beyond the batch holds anything: it goes through the motions of the short decode
       const bool live = ready && row < m && c < Cg;
-      lookup_alone<4>(look, y, live, wild && live, sm.inv_f, sm.lv[set] + cc * L, sm.primes, L, row, c, Cg);
+      lookup_alone<4>(look, y, live, live ? reach : 0.f, live && !(reach < tame_y), sm.inv_f, sm.lv[set] + cc * L, sm.primes, L, row, c, Cg);
     } else {
       // The coordinates change hands through shared memory: row e of the tile is a line of 128 bytes,
       // chunk 4 cc + j (16 bytes) holds block j of copy cc, at chunk ^ (e % 8) so that neither side has

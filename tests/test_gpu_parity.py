@@ -82,6 +82,26 @@ def test_cell_codes_large_coordinates(oracle):
         assert np.array_equal(got, want), (inv, int((got != want).sum()))
 
 
+@pytest.mark.parametrize("blocks", [1, 3, 4])
+def test_cell_codes_across_binades(oracle, blocks):
+    """The decode that decides between the cosets first, where v - 1/2 is rounded: coordinates just above
+    -2^k, in one, three and all coordinates of a block. The first row once got the other coset (its
+    errors are 0.81506 and 0.81541, v - 1/2 is off by 2^-10)."""
+    rng = np.random.default_rng(23)
+    known = np.array([-17.247255, 3.8654776, 21.901697, 14.626226, 8.2977238, -9.6680155, -16383.901, 3.3852804], np.float32)
+    for k in range(0, 20):
+        x = rng.uniform(-30, 30, size=(60000, blocks, 8)).astype(np.float32)
+        for rows, many in ((slice(0, 20000), 1), (slice(20000, 40000), 3), (slice(40000, 60000), 8)):
+            at = rng.permuted(np.tile(np.arange(8), (20000, blocks, 1)), axis=2)[..., :many]
+            value = -(2.0 ** k) + rng.uniform(0, 0.5, at.shape) * rng.choice([1.0, 1e-2, 1e-4], at.shape)
+            np.put_along_axis(x[rows], at, value.astype(np.float32), axis=2)
+        x[0] = known
+        x = x.reshape(len(x), 8 * blocks)
+        got = octex_b200.cell_codes(x, blocks, 1.0)
+        want = oracle.cell_code(x, blocks, 1.0)
+        assert np.array_equal(got, want), (k, int((got != want).sum()))
+
+
 def test_cell_codes_against_reference_device_code(oracle):
     """The reference's e8b_hash64 compiled as device code, run on this GPU, on the same points."""
     if oracle.ref_e8_cuda() is None:
