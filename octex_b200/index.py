@@ -122,11 +122,17 @@ def search_params(**kw) -> _lib.SearchParams:
 
 
 @functools.lru_cache(maxsize=64)
-def _search_params_ref(read, starts, waves, rerank, wave_rerank, batch, sketch_rank, final_rerank):
-    """A pointer to the struct of these parameters, made once (the library only reads it)."""
-    p = search_params(read=read, starts=starts, waves=waves, rerank=rerank, wave_rerank=wave_rerank,
-                      batch=batch, sketch_rank=sketch_rank, final_rerank=final_rerank)
-    return C.pointer(p)
+def _params_of_numbers(*values):
+    return C.pointer(search_params(**dict(zip(SEARCH_PARAMS, values))))
+
+
+def _search_params_ref(*values):
+    """A pointer to the struct of these parameters (in the order of ``SEARCH_PARAMS``), made once for
+    the same numbers (the library only reads it). Whatever else stands for a number (a numpy or torch
+    scalar, which may change) is read now."""
+    return _params_of_numbers(*[v if type(v) in (int, bool) or v is None else
+                                bool(v) if name == "sketch_rank" else int(v)
+                                for name, v in zip(SEARCH_PARAMS, values)])
 
 
 def load_params(placement="shard", sketch="replicate", **kw):
@@ -313,13 +319,7 @@ class Index:
                                wave_rerank=wave_rerank, batch=batch, sketch_rank=sketch_rank,
                                final_rerank=final_rerank, neighbors=neighbors, distances=distances)
             return back(D), back(I)
-        try:
-            p = _search_params_ref(read, starts, waves, rerank, wave_rerank, batch, sketch_rank,
-                                   final_rerank)
-        except TypeError:  # an unhashable number (a 0-d array)
-            p = C.pointer(search_params(read=read, starts=starts, waves=waves, rerank=rerank,
-                                        wave_rerank=wave_rerank, batch=batch, sketch_rank=sketch_rank,
-                                        final_rerank=final_rerank))
+        p = _search_params_ref(read, starts, waves, rerank, wave_rerank, batch, sketch_rank, final_rerank)
         torch = _torch()
         if _is_torch(queries):
             q = queries.detach() if queries.requires_grad else queries

@@ -116,3 +116,36 @@ def test_python_argument_checks(tmp_path):
         octex_b200.load(tmp_path)
     p = octex_b200.search_params(read=8, sketch_rank=True)
     assert p.read == 8 and p.sketch_rank and p.starts == 128
+
+
+def test_search_parameters_are_read_at_every_call(L):
+    """A parameter may be a scalar of numpy or torch: its value at the call counts, also when the same
+    object held another one at a call before, and nothing keeps the object."""
+    import gc
+    import weakref
+    import torch
+    from octex_b200.index import _search_params_ref
+    fields = ("read", "starts", "waves", "rerank", "wave_rerank", "batch", "sketch_rank", "final_rerank")
+
+    def values(**kw):
+        given = dict(dict(read=32, starts=128, waves=2, rerank=128, wave_rerank=128, batch=10000, sketch_rank=False,
+                          final_rerank=32), **kw)
+        p = _search_params_ref(*[given[f] for f in fields]).contents
+        return [getattr(p, f) for f in fields]
+
+    starts = torch.tensor(32)
+    assert values(starts=starts)[1] == 32
+    starts.fill_(64)
+    assert values(starts=starts)[1] == 64
+    array = np.array(7)
+    assert values(read=array)[0] == 7
+    array[...] = 9
+    assert values(read=array)[0] == 9
+    assert values(sketch_rank=np.bool_(True), waves=np.int64(1), rerank=16.0) == [32, 128, 1, 16, 128, 10000, True, 32]
+    assert values(final_rerank=None)[7] == 32  # the default
+    gone = weakref.ref(starts)
+    del starts
+    gc.collect()
+    assert gone() is None
+    with pytest.raises((TypeError, ValueError)):
+        values(read="many")
