@@ -650,12 +650,11 @@ cuvsError_t octexB200Fetch(cuvsOctexIndex_t index, const char* name, void* dst, 
     else if (n == "phase_rows") b = &pl->phase2;
     OCTEX_EXPECTS(b != nullptr, "octex: unknown array name \"" + n + "\"");
     OCTEX_EXPECTS(b->ptr != nullptr, "octex: \"" + n + "\" is not kept (see octexB200SetDebug)");
-    // the rows of the last batch; every one of these arrays has a row per query
-    const size_t size = b->size / static_cast<size_t>(std::max(pl->cap, 1)) * static_cast<size_t>(rows_used(*pl));
+    std::lock_guard<std::mutex> lock(pl->mu);
+    const size_t size = octex_b200::detail::bytes_used(pl->world, pl->cap, pl->m, b->size);
     if (bytes != nullptr) *bytes = static_cast<int64_t>(size);
     if (dst == nullptr) return;
     OCTEX_EXPECTS(capacity >= static_cast<int64_t>(size), "octex: the destination is too small");
-    std::lock_guard<std::mutex> lock(pl->mu);
     OCTEX_CUDA_TRY(cudaSetDevice(pl->device));
     if (pl->used) OCTEX_CUDA_TRY(cudaEventSynchronize(pl->done_ev));
     OCTEX_CUDA_TRY(cudaStreamSynchronize(ix.part.stream));

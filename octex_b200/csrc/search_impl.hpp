@@ -90,7 +90,12 @@ void check_tc(plan const& pl);
 /// The plan of these parameters for batches of up to m queries.
 auto get_plan(index_impl& ix, search_params const& sp, int m, int k, int lane = 0) -> std::shared_ptr<plan>;
 
-/// Rows of the plan's buffers that hold something of the last batch, of `cap` allocated.
-inline auto rows_used(plan const& pl) -> int { return pl.world > 1 ? pl.cap : pl.m; }
+/// Bytes of one of the plan's arrays (`size` allocated) that belong to the last batch of m queries: a row
+/// per query, `cap` rows allocated. With several processes the arrays hold this process's rows of a
+/// batch, which is always a whole one.
+inline auto bytes_used(int world, int cap, int m, size_t size) -> size_t
+{
+  return world > 1 ? size : size / static_cast<size_t>(cap > 0 ? cap : 1) * static_cast<size_t>(m);
+}
 
 }  // namespace octex_b200::detail

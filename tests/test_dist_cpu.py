@@ -120,3 +120,30 @@ def test_rows_dealt_over_ranks(tmp_path, world):
     spans = [np.load(tmp_path / f"rows{r}.npy") for r in range(world)]
     assert spans[0][0] == 0 and spans[-1][1] == 1003
     assert all(spans[r][1] == spans[r + 1][0] for r in range(world - 1))
+
+
+def test_bytes_of_the_last_batch(tmp_path):
+    """What Index.fetch gets of an array: with one process the rows of the last batch, with several the
+    whole array of the process's own rows (37 queries over two processes: 18 and 19 rows, neither a
+    multiple of 37), always a whole number of rows."""
+    import shutil
+    import subprocess
+    cxx, cuda = shutil.which("g++"), "/usr/local/cuda/include"
+    if cxx is None or not os.path.isdir(cuda):
+        pytest.skip("needs g++ and the CUDA headers")
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('''
+#include "search_impl.hpp"
+#include <cstdio>
+int main()
+{
+  using octex_b200::detail::bytes_used;
+  const size_t row = 32 * sizeof(long long);
+  std::printf("%zu %zu %zu %zu %zu\\n", bytes_used(2, 37, 37, 18 * row), bytes_used(2, 37, 37, 19 * row),
+              bytes_used(2, 37, 37, 37 * row), bytes_used(1, 100, 33, 100 * row), bytes_used(1, 1, 1, row));
+}
+''')
+    subprocess.run([cxx, "-std=c++17", "-I", os.path.join(ROOT, "octex_b200", "csrc"), "-I", os.path.join(ROOT, "include"),
+                    "-I", cuda, str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    assert [int(v) for v in out.split()] == [rows * 256 for rows in (18, 19, 37, 33, 1)]

@@ -36,6 +36,10 @@ def worker(rank, world, port, path, out, placement, tiers):
                      ("c", dict(read=8, starts=32, waves=1, rerank=64, wave_rerank=64, batch=37))):
         d, i = idx.search(queries, 10, **kw)
         res[name + "_i"], res[name + "_d"] = i, d
+    # what the last batch of 37 left here: this process's rows of it
+    kept = idx.fetch("kept_ids", np.int64)
+    mine = 37 * (rank + 1) // world - 37 * rank // world if placement == "replicate" else 37
+    assert kept.shape == (mine * 32,)
     # device arrays in and out as well
     q = torch.as_tensor(queries, device="cuda")
     d, i = idx.search(q, 10, read=8, starts=32, waves=2, rerank=64, wave_rerank=64)
