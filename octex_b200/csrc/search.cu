@@ -116,6 +116,7 @@ plan::~plan()
   if (used) cudaEventSynchronize(done_ev);  // its kernels may be running on a caller's stream
   if (graph != nullptr) cudaGraphExecDestroy(graph);
   if (done_ev != nullptr) cudaEventDestroy(done_ev);
+  if (join_ev != nullptr) cudaEventDestroy(join_ev);
   if (tc_error_host != nullptr) cudaFreeHost(tc_error_host);
   cudaSetDevice(cur);
 }
@@ -143,25 +144,28 @@ struct batch_io {
 /// The plan's own buffers.
 auto own_io(plan const& pl) -> batch_io { return {pl.qbuf.as<float>(), pl.bi, pl.bd}; }
 
+auto capturing(cudaStream_t s) -> bool
+{
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  OCTEX_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 /// What is queued on s from here on comes after the plan's last batch, whose buffers it uses.
 void follow_last_batch(plan& pl, cudaStream_t s)
 {
-  if (!pl.used) return;
+  // a graph the caller is capturing is ordered by whoever launches it (and a capturing stream does not
+  // say its id)
+  if (!pl.used || capturing(s)) return;
   unsigned long long id = 0;
   OCTEX_CUDA_TRY(cudaStreamGetId(s, &id));
-  if (id == pl.last_stream) return;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  OCTEX_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
-  // a graph the caller is capturing is ordered by whoever launches it
-  if (cap == cudaStreamCaptureStatusNone) OCTEX_CUDA_TRY(cudaStreamWaitEvent(s, pl.done_ev, 0));
+  if (id != pl.last_stream) OCTEX_CUDA_TRY(cudaStreamWaitEvent(s, pl.done_ev, 0));
 }
 
 /// The plan's last batch is what s holds now.
 void mark_last_batch(plan& pl, cudaStream_t s)
 {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  OCTEX_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
-  if (cap != cudaStreamCaptureStatusNone) return;
+  if (capturing(s)) return;
   OCTEX_CUDA_TRY(cudaEventRecord(pl.done_ev, s));
   OCTEX_CUDA_TRY(cudaStreamGetId(s, &pl.last_stream));
   pl.used = true;
@@ -575,6 +579,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   kernels::round_allow_smem(pl.smem_max);
 
   OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.done_ev, cudaEventDisableTiming));
+  OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.join_ev, cudaEventDisableTiming));
   OCTEX_CUDA_TRY(cudaDeviceSynchronize());  // the buffers are filled on the default stream
   if (ix.world > 1) capture_batch(ix, pl, p.stream);
   return plp;
@@ -670,16 +675,13 @@ auto search_device(index_impl& ix, search_params const& sp, cudaStream_t caller,
 /// lanes, each a plan on a stream of its own: the copies of one batch run under the kernels of the
 /// other. Page-locked arrays are copied from and to directly; ordinary ones pass through page-locked
 /// staging of the plan.
-void search_copied(index_impl& ix, search_params const& sp, cudaStream_t caller, int cur, const float* queries,
+void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStream_t caller, int cur, const float* queries,
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
 {
   auto& p            = ix.part;
   const int D        = static_cast<int>(ix.dim);
   const int64_t most = std::max(sp.batch, 1), batches = (nq + most - 1) / most;
   const int m        = static_cast<int>((nq + batches - 1) / batches);
-  const debug_options dbg = ix_debug(ix);
-  // one lane when there is one batch and when the plan keeps observations
-  const int lanes = batches > 1 && !dbg.stats && !dbg.taps ? 2 : 1;
   std::shared_ptr<plan> lane[2];
   for (int l = 0; l < lanes; l++)
     lane[l] = get_plan(ix, sp, m, static_cast<int>(k), l);
@@ -750,9 +752,11 @@ void search_copied(index_impl& ix, search_params const& sp, cudaStream_t caller,
       check_tc(*lane[l]);
     }
   } else {
+    for (int l = 0; l < lanes; l++)
+      OCTEX_CUDA_TRY(cudaEventRecord(lane[l]->join_ev, stream[l]));
     OCTEX_CUDA_TRY(cudaSetDevice(cur));
     for (int l = 0; l < lanes; l++)
-      OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->done_ev, 0));
+      OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->join_ev, 0));
   }
 }
 
@@ -802,10 +806,11 @@ void search_impl(resources const& res,
     int device;
     ~back_to() { cudaSetDevice(device); }
   } back{cur};
+  // streams: a second one for the batches of one process, unless the plan keeps observations
+  const debug_options dbg = ix_debug(ix);
+  const int lanes = ix.world == 1 && !resident && nq > std::max(sp.batch, 1) && !dbg.stats && !dbg.taps ? 2 : 1;
   std::unique_lock<std::mutex> one_start(ix.start_mu);
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  OCTEX_CUDA_TRY(cudaStreamIsCapturing(caller, &cap));
-  const bool busy = cap != cudaStreamCaptureStatusNone || cudaStreamQuery(caller) != cudaSuccess;
+  const bool busy = capturing(caller) || cudaStreamQuery(caller) != cudaSuccess;
   if (busy) {
     cudaGetLastError();  // "not ready" is no failure
     if (ix.start_ev == nullptr || ix.start_dev != cur) {
@@ -817,15 +822,15 @@ void search_impl(resources const& res,
     OCTEX_CUDA_TRY(cudaEventRecord(ix.start_ev, caller));
   }
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
-  if (p.second == nullptr && ix.world == 1 && nq > sp.batch)
+  if (p.second == nullptr && lanes > 1)
     OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&p.second, cudaStreamNonBlocking));
   if (busy) {
     OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.stream, ix.start_ev, 0));
-    if (p.second != nullptr) OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.second, ix.start_ev, 0));
+    if (lanes > 1) OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.second, ix.start_ev, 0));
   }
   one_start.unlock();
   if (ix.world == 1 && !resident) {
-    search_copied(ix, sp, caller, cur, queries, nq, neighbors, distances, k, host_out);
+    search_copied(ix, sp, lanes, caller, cur, queries, nq, neighbors, distances, k, host_out);
     if (wait && !host_out) OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
     return;
   }
@@ -877,8 +882,9 @@ void search_impl(resources const& res,
     }
   }
   mark_last_batch(w, s);
+  OCTEX_CUDA_TRY(cudaEventRecord(w.join_ev, s));
   OCTEX_CUDA_TRY(cudaSetDevice(cur));
-  OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, w.done_ev, 0));
+  OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, w.join_ev, 0));
   if (host_out || wait) {
     OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
     check_tc(w);

@@ -47,6 +47,7 @@ struct plan {
   cudaGraphExec_t graph = nullptr;  // of a batch of graph_m queries in the plan's own buffers
   int graph_m           = 0;
   cudaEvent_t done_ev   = nullptr;  // the end of the plan's last batch
+  cudaEvent_t join_ev   = nullptr;  // the same for the caller's stream to wait for, also while it is captured
   // the stream done_ev was recorded on (cudaStreamGetId): a batch on another one waits for it first
   unsigned long long last_stream = 0;
   bool used                      = false;

@@ -174,3 +174,43 @@ def test_queries_on_another_gpu():
                 assert d.device == i.device == q.device
                 assert same((d.cpu().numpy(), i.cpu().numpy()), want)
     idx.close()
+
+
+def test_captured_searches():
+    """The C call that does not wait, captured on a stream of the caller and replayed with other queries:
+    arrays used in place and arrays copied in and out (page-locked ones given as device arrays), one batch
+    (also after a call that brought a second stream in) and several. use_graph = False, as a capture
+    always needed."""
+    import torch
+    from octex_b200 import synth
+    dim, k, n = 64, 10, 300
+    idx, _ = make_index(dim, copies=8, blocks=4)
+    kw = dict(read=8, starts=32, waves=2, rerank=64, wave_rerank=64)
+    queries = synth.plumbing(2 * n, dim, seed=1)
+    want = idx.search(queries, k, **kw)
+    side = torch.cuda.Stream()
+    for batch, pinned in ((1000, False), (1000, True), (130, True), (1000, True), (130, False), (1000, False)):
+        q, ids, dist = torch.empty((n, dim)), torch.empty((n, k), dtype=torch.int64), torch.empty((n, k))
+        q, ids, dist = (t.pin_memory() if pinned else t.cuda() for t in (q, ids, dist))
+        q.copy_(torch.as_tensor(queries[:n]))
+        at = (q.data_ptr(), ids.data_ptr(), dist.data_ptr())
+        assert in_place(idx, *at) == (0 if pinned else 1)
+
+        def call():
+            search_at(idx, *at, n, dim, k, wait=False, stream=side.cuda_stream, batch=batch, use_graph=False, **kw)
+
+        with torch.cuda.stream(side):
+            call()  # a plan is made outside of a capture
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            call()
+        for a in (0, n, 0):
+            q.copy_(torch.as_tensor(queries[a:a + n]))
+            ids.fill_(-5)
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert same((dist.cpu().numpy(), ids.cpu().numpy()), (want[0][a:a + n], want[1][a:a + n])), (batch, pinned, a)
+        del graph
+    idx.close()
