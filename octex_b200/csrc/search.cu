@@ -11,6 +11,7 @@
 #include "search_impl.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 
@@ -647,27 +648,81 @@ void* staging(dbuf& b, int device, size_t bytes)
   return b.ptr;
 }
 
-/// A search by one process with queries and results in the memory of its GPU: every batch runs on
-/// the caller's stream from the caller's arrays and into them.
-auto search_device(index_impl& ix, search_params const& sp, cudaStream_t caller, const float* queries, int64_t nq,
-                   int64_t* neighbors, float* distances, int64_t k) -> std::shared_ptr<plan>
+/// The event of the index for streams of device `dev`, the current one; ix.start_mu guards it.
+auto start_event(index_impl& ix, int dev) -> cudaEvent_t
 {
-  // equal batches rather than full ones and a rest
-  const int64_t most = std::max(sp.batch, 1), batches = (nq + most - 1) / most;
-  const int m        = static_cast<int>((nq + batches - 1) / batches);
-  auto pl            = get_plan(ix, sp, m, static_cast<int>(k));
-  std::lock_guard<std::mutex> lock(pl->mu);
-  // a search with device outputs returns before its kernels ran; had one of them given up, the
-  // word is still set and this is the first host code to see it
-  check_tc(*pl);
-  follow_last_batch(*pl, caller);
-  for (int64_t b0 = 0; b0 < nq; b0 += m) {
-    set_rows(*pl, static_cast<int>(std::min<int64_t>(m, nq - b0)));
-    run_batch(ix, *pl, {queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k},
-              caller, nullptr);
+  if (ix.start_ev == nullptr || ix.start_dev != dev) {
+    if (ix.start_ev != nullptr) cudaEventDestroy(ix.start_ev);
+    ix.start_ev = nullptr;
+    OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&ix.start_ev, cudaEventDisableTiming));
+    ix.start_dev = dev;
   }
-  mark_last_batch(*pl, caller);
-  return pl;
+  return ix.start_ev;
+}
+
+/// The stream of the second lane, made when first needed (its device is current; ix.start_mu guards it).
+auto second_stream(index_impl& ix) -> cudaStream_t
+{
+  auto& p = ix.part;
+  if (p.second == nullptr) OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&p.second, cudaStreamNonBlocking));
+  return p.second;
+}
+
+/// Queries of the batches a call is cut into. Two are halves, since nothing is left to run under the end
+/// of the second: 10 100 queries, batch 10 000, 600 us against 650 as 10 000 and 100, and 12 345 from host
+/// memory 1 097 against 1 213. Three and more are whole batches and a rest (1 067 queries, batch 400, 256
+/// start points and three waves: 646 us against 706 in thirds).
+auto batch_rows(int64_t nq, int batch) -> int
+{
+  const int64_t most = std::max(batch, 1);
+  return static_cast<int>(nq <= most ? nq : nq <= 2 * most ? (nq + 1) / 2 : most);
+}
+
+/// The plans of a call: one, or one per lane.
+using lane_plans = std::array<std::shared_ptr<plan>, 2>;
+
+/// A search by one process with queries and results in the memory of its GPU: the batches run from the
+/// caller's arrays and into them. One batch stays on the caller's stream; several alternate between it
+/// and a second one, each with a plan of its own: the rounds of a batch end in blocks that leave
+/// multiprocessors idle, whatever its size. 200 000 rows x 128, one stream and two: 3 x 300 queries with
+/// 256 start points and three waves 830 and 636 us, 10 x 1 000 queries 1 016 and 727, 3 x 10 000
+/// 1 787 and 1 700.
+auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStream_t caller, const float* queries,
+                   int64_t nq, int64_t* neighbors, float* distances, int64_t k) -> lane_plans
+{
+  const int m = batch_rows(nq, sp.batch);
+  lane_plans lane;
+  for (int l = 0; l < lanes; l++)
+    lane[l] = get_plan(ix, sp, m, static_cast<int>(k), l);
+  std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
+  if (lanes > 1) lock1 = std::unique_lock<std::mutex>(lane[1]->mu);
+  cudaStream_t stream[2] = {caller, caller};
+  if (lanes > 1) {
+    std::lock_guard<std::mutex> one_start(ix.start_mu);
+    stream[1] = second_stream(ix);
+    OCTEX_CUDA_TRY(cudaEventRecord(start_event(ix, ix.part.device), caller));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(stream[1], ix.start_ev, 0));
+  }
+  for (int l = 0; l < lanes; l++) {
+    // a search with device outputs returns before its kernels ran; had one of them given up, the
+    // word is still set and this is the first host code to see it
+    check_tc(*lane[l]);
+    follow_last_batch(*lane[l], stream[l]);
+  }
+  int64_t batch = 0;
+  for (int64_t b0 = 0; b0 < nq; b0 += m, batch++) {
+    const int l = static_cast<int>(batch % lanes);
+    set_rows(*lane[l], static_cast<int>(std::min<int64_t>(m, nq - b0)));
+    run_batch(ix, *lane[l], {queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k},
+              stream[l], nullptr);
+  }
+  for (int l = 0; l < lanes; l++)
+    mark_last_batch(*lane[l], stream[l]);
+  if (lanes > 1) {
+    OCTEX_CUDA_TRY(cudaEventRecord(lane[1]->join_ev, stream[1]));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[1]->join_ev, 0));
+  }
+  return lane;
 }
 
 /// A search by one process with queries and results that are not all memory of its GPU (host memory,
@@ -680,9 +735,8 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
 {
   auto& p            = ix.part;
   const int D        = static_cast<int>(ix.dim);
-  const int64_t most = std::max(sp.batch, 1), batches = (nq + most - 1) / most;
-  const int m        = static_cast<int>((nq + batches - 1) / batches);
-  std::shared_ptr<plan> lane[2];
+  const int m        = batch_rows(nq, sp.batch);
+  lane_plans lane;
   for (int l = 0; l < lanes; l++)
     lane[l] = get_plan(ix, sp, m, static_cast<int>(k), l);
   std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
@@ -792,11 +846,15 @@ void search_impl(resources const& res,
   OCTEX_CUDA_TRY(cudaGetDevice(&cur));
   cudaStream_t caller = res.stream;
   auto& p             = ix.part;
+  // streams: a second one for the batches of one process, unless the plan keeps observations
+  const debug_options dbg = ix_debug(ix);
+  const int lanes = ix.world == 1 && !resident && nq > std::max(sp.batch, 1) && !dbg.stats && !dbg.taps ? 2 : 1;
   if (!resident && !host_out && search_in_place(ix, queries, neighbors, distances)) {
-    auto pl = search_device(ix, sp, caller, queries, nq, neighbors, distances, k);
+    const lane_plans used = search_device(ix, sp, lanes, caller, queries, nq, neighbors, distances, k);
     if (wait) {
       OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
-      check_tc(*pl);
+      for (auto const& pl : used)
+        if (pl != nullptr) check_tc(*pl);
     }
     return;
   }
@@ -806,24 +864,14 @@ void search_impl(resources const& res,
     int device;
     ~back_to() { cudaSetDevice(device); }
   } back{cur};
-  // streams: a second one for the batches of one process, unless the plan keeps observations
-  const debug_options dbg = ix_debug(ix);
-  const int lanes = ix.world == 1 && !resident && nq > std::max(sp.batch, 1) && !dbg.stats && !dbg.taps ? 2 : 1;
   std::unique_lock<std::mutex> one_start(ix.start_mu);
   const bool busy = capturing(caller) || cudaStreamQuery(caller) != cudaSuccess;
   if (busy) {
     cudaGetLastError();  // "not ready" is no failure
-    if (ix.start_ev == nullptr || ix.start_dev != cur) {
-      if (ix.start_ev != nullptr) cudaEventDestroy(ix.start_ev);
-      ix.start_ev = nullptr;
-      OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&ix.start_ev, cudaEventDisableTiming));
-      ix.start_dev = cur;
-    }
-    OCTEX_CUDA_TRY(cudaEventRecord(ix.start_ev, caller));
+    OCTEX_CUDA_TRY(cudaEventRecord(start_event(ix, cur), caller));
   }
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
-  if (p.second == nullptr && lanes > 1)
-    OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&p.second, cudaStreamNonBlocking));
+  if (lanes > 1) second_stream(ix);
   if (busy) {
     OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.stream, ix.start_ev, 0));
     if (lanes > 1) OCTEX_CUDA_TRY(cudaStreamWaitEvent(p.second, ix.start_ev, 0));

@@ -214,3 +214,48 @@ def test_captured_searches():
             assert same((dist.cpu().numpy(), ids.cpu().numpy()), (want[0][a:a + n], want[1][a:a + n])), (batch, pinned, a)
         del graph
     idx.close()
+
+
+def test_device_batches_alternate_between_two_streams():
+    """Several batches of device queries: the same answers as one batch for whole and ragged counts, after
+    work on the caller's stream that makes the queries, before work there that reads the results (the
+    C call that does not wait), from several threads."""
+    import threading
+    import torch
+    from octex_b200 import synth
+    dim, k = 64, 10
+    idx, _ = make_index(dim, copies=8, blocks=4)
+    kw = dict(read=8, starts=32, waves=2, rerank=64, wave_rerank=64)
+    queries = synth.plumbing(1200, dim, seed=1)
+    want = idx.search(queries, k, **kw)
+    q = torch.as_tensor(queries, device="cuda")
+    for batch in (1, 37, 300, 400, 599, 600, 1199):
+        m = min(len(queries), 12 * batch)
+        d, i = idx.search(q[:m], k, batch=batch, **kw)
+        assert same((d.cpu().numpy(), i.cpu().numpy()), (want[0][:m], want[1][:m])), batch
+    failures = []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            for _ in range(20):
+                m, batch = int(rng.integers(2, 1200)), int(rng.integers(100, 700))
+                mine = torch.empty((m, dim), device="cuda")
+                ids, dist = torch.empty((m, k), dtype=torch.int64, device="cuda"), torch.empty((m, k), device="cuda")
+                torch.empty(1 << 24, device="cuda").fill_(1.0)
+                mine.copy_(q[:m])
+                search_at(idx, mine.data_ptr(), ids.data_ptr(), dist.data_ptr(), m, dim, k, wait=False,
+                          stream=side.cuda_stream, batch=batch, **kw)
+                mine.zero_()
+                got = (dist + 0).cpu().numpy(), (ids + 0).cpu().numpy()
+                if not same(got, (want[0][:m], want[1][:m])):
+                    failures.append((seed, m, batch))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
+    idx.close()
