@@ -286,7 +286,8 @@ OCTEX_B200_EXPORT cuvsError_t octexB200SearchInPlace(cuvsOctexIndex_t index, con
                                                      int32_t* in_place);
 
 /* detail::resident_search (cpp/src/neighbors/octex/search.cu:983-997): search again the queries of
- * the previous call, which are still on the GPU, and leave the results there. The timing protocol
+ * the previous call, which are still on the GPU, and leave the results there: all of a call of one
+ * batch, the first `batch` of a call of two, of a longer one what its last batches left. The timing protocol
  * of the reference's benchmark uses it (cpp/bench/octex_bench.cu:223-253). */
 OCTEX_B200_EXPORT cuvsError_t octexB200SearchResident(cuvsResources_t res,
                                                       cuvsOctexSearchParams_t params,

@@ -27,6 +27,7 @@
 
 #include <octex_b200.hpp>
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -103,6 +104,7 @@ struct index_impl {
   device_part part;
   std::mutex mu;  // guards plans
   std::map<std::string, std::shared_ptr<plan>> plans;
+  std::atomic<unsigned long long> calls{0};  // searches so far
   debug_options debug;
   // recorded on the caller's stream at the start of a search that runs on the index's own streams
   std::mutex start_mu;

@@ -586,22 +586,31 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   return plp;
 }
 
+namespace {
+
+/// The name of a configuration. One process: a plan serves every batch it has room for. Several: their
+/// slices and exchanges depend on the number of queries.
+auto plan_key(index_impl const& ix, search_params const& sp, int m, int k, debug_options dbg) -> std::string
+{
+  return std::to_string(ix.world > 1 ? m : 0) + "/" + std::to_string(k) + "/" + std::to_string(sp.read) + "/" +
+         std::to_string(sp.starts) + "/" + std::to_string(sp.waves) + "/" + std::to_string(sp.rerank) + "/" +
+         std::to_string(sp.wave_rerank) + "/" + std::to_string(sp.sketch_rank) + "/" +
+         std::to_string(sp.final_rerank) + "/" + std::to_string(dbg.stats) + std::to_string(dbg.taps) +
+         std::to_string(dbg.ordered_projection);
+}
+auto lane_name(std::string const& key, int lane) -> std::string { return lane == 0 ? key : key + "#" + std::to_string(lane); }
+
+}  // namespace
+
 auto get_plan(index_impl& ix, search_params const& sp, int m, int k, int lane) -> std::shared_ptr<plan>
 {
   const debug_options dbg = ix_debug(ix);
-  // One process: a plan serves every batch it has room for. Several: their slices and exchanges
-  // depend on the number of queries.
-  std::string key = std::to_string(ix.world > 1 ? m : 0) + "/" + std::to_string(k) + "/" + std::to_string(sp.read) +
-                    "/" + std::to_string(sp.starts) + "/" + std::to_string(sp.waves) + "/" +
-                    std::to_string(sp.rerank) + "/" + std::to_string(sp.wave_rerank) + "/" +
-                    std::to_string(sp.sketch_rank) + "/" + std::to_string(sp.final_rerank) + "/" +
-                    std::to_string(dbg.stats) + std::to_string(dbg.taps) +
-                    std::to_string(dbg.ordered_projection);
+  const std::string key   = plan_key(ix, sp, m, k, dbg);
   std::lock_guard<std::mutex> lock(ix.mu);
   // one cached configuration: the previous buffers and graphs go before the new ones come
   // (search.cu:807-812); a configuration has one plan per lane (see search_impl)
   if (ix.plans.find(key) == ix.plans.end()) ix.plans.clear();
-  const std::string name = lane == 0 ? key : key + "#" + std::to_string(lane);
+  const std::string name = lane_name(key, lane);
   auto& pl               = ix.plans[name];
   if (pl == nullptr || pl->cap < m) {
     pl.reset();
@@ -681,6 +690,53 @@ auto batch_rows(int64_t nq, int batch) -> int
 /// The plans of a call: one, or one per lane.
 using lane_plans = std::array<std::shared_ptr<plan>, 2>;
 
+/// The plans of a call by one process. The first has room for a whole batch, also when the call is cut
+/// into halves: a resident search takes the whole batch from it (gather_resident).
+auto plans_of(index_impl& ix, search_params const& sp, int lanes, int64_t nq, int64_t k) -> lane_plans
+{
+  lane_plans lane;
+  for (int l = 0; l < lanes; l++)
+    lane[l] = get_plan(ix, sp, l == 0 ? static_cast<int>(std::min<int64_t>(nq, std::max(sp.batch, 1))) : batch_rows(nq, sp.batch),
+                       static_cast<int>(k), l);
+  return lane;
+}
+
+/// The next batch of a call on a plan: n queries from row b0 of it on.
+void set_batch(plan& pl, unsigned long long call, int64_t b0, int n)
+{
+  set_rows(pl, n);
+  pl.call  = call;
+  pl.first = b0;
+  pl.held  = n;
+}
+
+/// The m queries a resident search of the plan repeats, of which it may hold fewer: what the other lane
+/// of the same call holds behind them comes over, the rest is filled with copies of the first query
+/// (search.cu:870-883 of the reference). Queued on s; the plan's lock is held.
+void gather_resident(index_impl& ix, search_params const& sp, plan& pl, int m, int k, cudaStream_t s)
+{
+  if (pl.held >= m || pl.held == 0) return;
+  std::shared_ptr<plan> other;
+  {
+    std::lock_guard<std::mutex> lock(ix.mu);
+    const auto at = ix.plans.find(lane_name(plan_key(ix, sp, m, k, pl.dbg), 1));
+    if (at != ix.plans.end()) other = at->second;
+  }
+  const auto D = static_cast<size_t>(ix.dim);
+  if (other != nullptr) {
+    std::lock_guard<std::mutex> lock(other->mu);
+    if (other->call == pl.call && other->first == pl.first + pl.held) {
+      const int n = std::min(other->held, m - pl.held);
+      follow_last_batch(*other, s);
+      OCTEX_CUDA_TRY(cudaMemcpyAsync(pl.qbuf.as<float>() + pl.held * D, other->qbuf.ptr, sizeof(float) * n * D,
+                                     cudaMemcpyDeviceToDevice, s));
+      mark_last_batch(*other, s);  // its next batch comes after the copy
+      pl.held += n;
+    }
+  }
+  kernels::pad_rows(pl.qbuf.as<float>(), pl.held, m, static_cast<int>(D), s);
+}
+
 /// A search by one process with queries and results in the memory of its GPU: the batches run from the
 /// caller's arrays and into them. One batch stays on the caller's stream; several alternate between it
 /// and a second one, each with a plan of its own: the rounds of a batch end in blocks that leave
@@ -690,10 +746,9 @@ using lane_plans = std::array<std::shared_ptr<plan>, 2>;
 auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStream_t caller, const float* queries,
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k) -> lane_plans
 {
-  const int m = batch_rows(nq, sp.batch);
-  lane_plans lane;
-  for (int l = 0; l < lanes; l++)
-    lane[l] = get_plan(ix, sp, m, static_cast<int>(k), l);
+  const int m                   = batch_rows(nq, sp.batch);
+  const unsigned long long call = ++ix.calls;
+  const lane_plans lane         = plans_of(ix, sp, lanes, nq, k);
   std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
   if (lanes > 1) lock1 = std::unique_lock<std::mutex>(lane[1]->mu);
   cudaStream_t stream[2] = {caller, caller};
@@ -712,7 +767,7 @@ auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStrea
   int64_t batch = 0;
   for (int64_t b0 = 0; b0 < nq; b0 += m, batch++) {
     const int l = static_cast<int>(batch % lanes);
-    set_rows(*lane[l], static_cast<int>(std::min<int64_t>(m, nq - b0)));
+    set_batch(*lane[l], call, b0, static_cast<int>(std::min<int64_t>(m, nq - b0)));
     run_batch(ix, *lane[l], {queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k},
               stream[l], nullptr);
   }
@@ -734,11 +789,10 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
 {
   auto& p            = ix.part;
-  const int D        = static_cast<int>(ix.dim);
-  const int m        = batch_rows(nq, sp.batch);
-  lane_plans lane;
-  for (int l = 0; l < lanes; l++)
-    lane[l] = get_plan(ix, sp, m, static_cast<int>(k), l);
+  const int D                   = static_cast<int>(ix.dim);
+  const int m                   = batch_rows(nq, sp.batch);
+  const unsigned long long call = ++ix.calls;
+  const lane_plans lane         = plans_of(ix, sp, lanes, nq, k);
   std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
   if (lanes > 1) lock1 = std::unique_lock<std::mutex>(lane[1]->mu);
   cudaStream_t stream[2] = {p.stream, p.second};
@@ -779,7 +833,7 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
       src = pin;
     }
     OCTEX_CUDA_TRY(cudaMemcpyAsync(w.qbuf.ptr, src, bytes, cudaMemcpyDefault, s));
-    set_rows(w, n);
+    set_batch(w, call, b0, n);
     batch_io io = own_io(w);
     if (stage_out) {
       // the last kernel writes through to host memory
@@ -893,6 +947,7 @@ void search_impl(resources const& res,
   follow_last_batch(w, s);
   if (ix.world == 1) {
     set_rows(w, m);
+    gather_resident(ix, sp, w, m, static_cast<int>(k), s);
     if (sp.use_graph && (w.graph == nullptr || w.graph_m != m)) capture_batch(ix, w, s);
   }
   for (int64_t b0 = 0; b0 < nq; b0 += m) {

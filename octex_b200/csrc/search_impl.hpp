@@ -48,6 +48,10 @@ struct plan {
   int graph_m           = 0;
   cudaEvent_t done_ev   = nullptr;  // the end of the plan's last batch
   cudaEvent_t join_ev   = nullptr;  // the same for the caller's stream to wait for, also while it is captured
+  // the queries of the last call that qbuf still holds, [first, first + held) of it, and which call that was
+  int64_t first              = 0;
+  int held                   = 0;
+  unsigned long long call    = 0;
   // the stream done_ev was recorded on (cudaStreamGetId): a batch on another one waits for it first
   unsigned long long last_stream = 0;
   bool used                      = false;

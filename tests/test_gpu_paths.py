@@ -259,3 +259,34 @@ def test_device_batches_alternate_between_two_streams():
         t.join()
     assert not failures
     idx.close()
+
+
+@pytest.mark.parametrize("where", ["device", "host"])
+def test_resident_after_a_call_of_several_batches(where):
+    """A resident search repeats queries of the call before it, also when that call was cut into batches: of
+    one of two batches the first `batch`. More than the call had are filled with copies of the first."""
+    import torch
+    from octex_b200 import synth
+    dim, k = 64, 10
+    idx, _ = make_index(dim, copies=8, blocks=4)
+    kw = dict(read=8, starts=32, waves=2, rerank=64, wave_rerank=64)
+    queries = synth.plumbing(500, dim, seed=1)
+    want = idx.search(queries, k, **kw)[1]
+    q = torch.as_tensor(queries, device="cuda") if where == "device" else queries
+
+    def resident(n):
+        idx.search_resident(n, k, batch=300, **kw)
+        return idx.fetch("kept_ids", np.int64, (n, -1))[:, :k]
+
+    for total in (500, 301, 333):
+        idx.search(q[:total], k, batch=300, **kw)
+        assert np.array_equal(resident(300), want[:300]), total
+        assert np.array_equal(resident(300), want[:300]), total  # the graph of the batch
+        assert np.array_equal(resident(20), want[:20]), total
+        assert np.array_equal(idx.search(q[100:400], k, batch=300, **kw)[1] if where == "host" else
+                              idx.search(q[100:400], k, batch=300, **kw)[1].cpu().numpy(), want[100:400])
+        assert np.array_equal(resident(300), want[100:400]), total
+    idx.search(q[:40], k, batch=300, **kw)
+    got = resident(50)
+    assert np.array_equal(got[:40], want[:40]) and (got[40:] == want[0]).all()
+    idx.close()
