@@ -764,19 +764,18 @@ auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStrea
     check_tc(*lane[l]);
     follow_last_batch(*lane[l], stream[l]);
   }
-  int64_t batch = 0;
-  for (int64_t b0 = 0; b0 < nq; b0 += m, batch++) {
-    const int l = static_cast<int>(batch % lanes);
-    set_batch(*lane[l], call, b0, static_cast<int>(std::min<int64_t>(m, nq - b0)));
+  auto run = [&](int l, int64_t b0, int n) {
+    set_batch(*lane[l], call, b0, n);
     run_batch(ix, *lane[l], {queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k},
               stream[l], nullptr);
-  }
-  for (int l = 0; l < lanes; l++)
+  };
+  auto close = [&](int l, bool) {
     mark_last_batch(*lane[l], stream[l]);
-  if (lanes > 1) {
-    OCTEX_CUDA_TRY(cudaEventRecord(lane[1]->join_ev, stream[1]));
-    OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[1]->join_ev, 0));
-  }
+    if (l == 0) return;
+    OCTEX_CUDA_TRY(cudaEventRecord(lane[l]->join_ev, stream[l]));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->join_ev, 0));
+  };
+  each_batch(nq, m, lanes, run, close);
   return lane;
 }
 
@@ -788,7 +787,7 @@ auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStrea
 void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStream_t caller, int cur, const float* queries,
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
 {
-  auto& p            = ix.part;
+  auto& p                       = ix.part;
   const int D                   = static_cast<int>(ix.dim);
   const int m                   = batch_rows(nq, sp.batch);
   const unsigned long long call = ++ix.calls;
@@ -818,11 +817,9 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
     out[l].n = 0;
   };
   int64_t batch = 0;
-  for (int64_t b0 = 0; b0 < nq; b0 += m, batch++) {
-    const int l    = static_cast<int>(batch % lanes);
-    plan& w        = *lane[l];
-    cudaStream_t s = stream[l];
-    const int n    = static_cast<int>(std::min<int64_t>(m, nq - b0));
+  auto run      = [&](int l, int64_t b0, int n) {
+    plan& w            = *lane[l];
+    cudaStream_t s     = stream[l];
     const size_t bytes = sizeof(float) * static_cast<size_t>(n) * D;
     if (stage_out) deliver(l);  // the lane's staging is free again, its queries too
     const void* src = queries + b0 * D;
@@ -849,22 +846,27 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
       OCTEX_CUDA_TRY(cudaMemcpyAsync(neighbors + b0 * k, w.bi, sizeof(int64_t) * n * k, cudaMemcpyDefault, s));
       OCTEX_CUDA_TRY(cudaMemcpyAsync(distances + b0 * k, w.bd, sizeof(float) * n * k, cudaMemcpyDefault, s));
     }
-  }
-  for (int l = 0; l < lanes; l++)
+    batch++;
+  };
+  auto close = [&](int l, bool failed) {
     mark_last_batch(*lane[l], stream[l]);
-  if (host_out) {
-    if (stage_out && lanes > 1) deliver(static_cast<int>(batch % lanes));  // the older of the two first
-    for (int l = 0; l < lanes; l++) {
-      if (stage_out) deliver(l);
-      OCTEX_CUDA_TRY(cudaStreamSynchronize(stream[l]));
-      check_tc(*lane[l]);
+    if (host_out) {
+      // nothing may still be on its way from or to the caller's arrays or the staging
+      if (failed) OCTEX_CUDA_TRY(cudaStreamSynchronize(stream[l]));
+      return;
     }
-  } else {
-    for (int l = 0; l < lanes; l++)
-      OCTEX_CUDA_TRY(cudaEventRecord(lane[l]->join_ev, stream[l]));
+    OCTEX_CUDA_TRY(cudaEventRecord(lane[l]->join_ev, stream[l]));
     OCTEX_CUDA_TRY(cudaSetDevice(cur));
-    for (int l = 0; l < lanes; l++)
-      OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->join_ev, 0));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, lane[l]->join_ev, 0));
+    OCTEX_CUDA_TRY(cudaSetDevice(p.device));
+  };
+  each_batch(nq, m, lanes, run, close);
+  if (!host_out) return;
+  if (stage_out && lanes > 1) deliver(static_cast<int>(batch % lanes));  // the older of the two first
+  for (int l = 0; l < lanes; l++) {
+    if (stage_out) deliver(l);
+    OCTEX_CUDA_TRY(cudaStreamSynchronize(stream[l]));
+    check_tc(*lane[l]);
   }
 }
 
@@ -950,8 +952,7 @@ void search_impl(resources const& res,
     gather_resident(ix, sp, w, m, static_cast<int>(k), s);
     if (sp.use_graph && (w.graph == nullptr || w.graph_m != m)) capture_batch(ix, w, s);
   }
-  for (int64_t b0 = 0; b0 < nq; b0 += m) {
-    const int n = static_cast<int>(std::min<int64_t>(m, nq - b0));
+  auto run = [&](int, int64_t b0, int n) {
     if (!resident) {
       // rows [q1, q1 + m1) of the batch, the part beyond its end filled with copies of a row
       // (search.cu:870-883)
@@ -983,11 +984,14 @@ void search_impl(resources const& res,
                                        cudaMemcpyDefault, s));
       }
     }
-  }
-  mark_last_batch(w, s);
-  OCTEX_CUDA_TRY(cudaEventRecord(w.join_ev, s));
-  OCTEX_CUDA_TRY(cudaSetDevice(cur));
-  OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, w.join_ev, 0));
+  };
+  auto close = [&](int, bool) {
+    mark_last_batch(w, s);
+    OCTEX_CUDA_TRY(cudaEventRecord(w.join_ev, s));
+    OCTEX_CUDA_TRY(cudaSetDevice(cur));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(caller, w.join_ev, 0));
+  };
+  each_batch(nq, m, 1, run, close);
   if (host_out || wait) {
     OCTEX_CUDA_TRY(cudaStreamSynchronize(caller));
     check_tc(w);

@@ -92,6 +92,29 @@ auto profile_batch(resources const& res, search_params const& sp, index const& i
 /// report).
 void check_tc(plan const& pl);
 
+/// The batches of a call, dealt to its lanes in turn: run(lane, first row, rows) queues one, close(lane,
+/// failed) is called once for every lane after the last, also when a batch could not be queued: what the
+/// lanes hold by then runs all the same, and the next user of their plans has to come after it.
+template <typename Run, typename Close>
+void each_batch(int64_t nq, int m, int lanes, Run run, Close close)
+{
+  try {
+    int64_t batch = 0;
+    for (int64_t b0 = 0; b0 < nq; b0 += m, batch++)
+      run(static_cast<int>(batch % lanes), b0, static_cast<int>(nq - b0 < m ? nq - b0 : m));
+  } catch (...) {
+    for (int l = 0; l < lanes; l++) {
+      try {
+        close(l, true);
+      } catch (...) {  // the first error is the one to report
+      }
+    }
+    throw;
+  }
+  for (int l = 0; l < lanes; l++)
+    close(l, false);
+}
+
 /// The plan of these parameters for batches of up to m queries.
 auto get_plan(index_impl& ix, search_params const& sp, int m, int k, int lane = 0) -> std::shared_ptr<plan>;
 

@@ -122,17 +122,25 @@ def test_rows_dealt_over_ranks(tmp_path, world):
     assert all(spans[r][1] == spans[r + 1][0] for r in range(world - 1))
 
 
-def test_bytes_of_the_last_batch(tmp_path):
-    """What Index.fetch gets of an array: with one process the rows of the last batch, with several the
-    whole array of the process's own rows (37 queries over two processes: 18 and 19 rows, neither a
-    multiple of 37), always a whole number of rows."""
+def run_cpp(tmp_path, source):
+    """The standard output of a C++ program over the library's internal headers."""
     import shutil
     import subprocess
     cxx, cuda = shutil.which("g++"), "/usr/local/cuda/include"
     if cxx is None or not os.path.isdir(cuda):
         pytest.skip("needs g++ and the CUDA headers")
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
-    src.write_text('''
+    src.write_text(source)
+    subprocess.run([cxx, "-std=c++17", "-I", os.path.join(ROOT, "octex_b200", "csrc"), "-I", os.path.join(ROOT, "include"),
+                    "-I", cuda, str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+
+
+def test_bytes_of_the_last_batch(tmp_path):
+    """What Index.fetch gets of an array: with one process the rows of the last batch, with several the
+    whole array of the process's own rows (37 queries over two processes: 18 and 19 rows, neither a
+    multiple of 37), always a whole number of rows."""
+    out = run_cpp(tmp_path, '''
 #include "search_impl.hpp"
 #include <cstdio>
 int main()
@@ -143,7 +151,44 @@ int main()
               bytes_used(2, 37, 37, 37 * row), bytes_used(1, 100, 33, 100 * row), bytes_used(1, 1, 1, row));
 }
 ''')
-    subprocess.run([cxx, "-std=c++17", "-I", os.path.join(ROOT, "octex_b200", "csrc"), "-I", os.path.join(ROOT, "include"),
-                    "-I", cuda, str(src), "-o", str(exe)], check=True)
-    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
     assert [int(v) for v in out.split()] == [rows * 256 for rows in (18, 19, 37, 33, 1)]
+
+
+def test_lanes_are_closed_when_a_batch_fails(tmp_path):
+    """The end of every lane is marked after the last batch of a call, also when one could not be queued
+    (here: an exception on the host) or when marking fails itself; the first error is the one that comes out."""
+    out = run_cpp(tmp_path, '''
+#include "search_impl.hpp"
+#include <cstdio>
+#include <stdexcept>
+void call(int64_t nq, int m, int lanes, int fails_at, int close_fails)
+{
+  int batch = 0;
+  try {
+    octex_b200::detail::each_batch(
+      nq, m, lanes,
+      [&](int l, int64_t b0, int n) {
+        if (batch++ == fails_at) throw std::runtime_error("batch");
+        std::printf("%d:%d+%d ", l, static_cast<int>(b0), n);
+      },
+      [&](int l, bool failed) {
+        std::printf(failed ? "abandon%d " : "close%d ", l);
+        if (l == close_fails) throw std::runtime_error("close");
+      });
+  } catch (std::exception const& e) {
+    std::printf("error:%s ", e.what());
+  }
+  std::printf("\\n");
+}
+int main()
+{
+  call(25, 10, 2, -1, -1);
+  call(25, 10, 2, 1, -1);
+  call(25, 10, 2, 2, 0);
+  call(5, 10, 1, 0, -1);
+  call(30, 10, 1, -1, 0);
+}
+''')
+    assert out.split(" \n")[:5] == [
+        "0:0+10 1:10+10 0:20+5 close0 close1", "0:0+10 abandon0 abandon1 error:batch",
+        "0:0+10 1:10+10 abandon0 abandon1 error:batch", "abandon0 error:batch", "0:0+10 0:10+10 0:20+10 close0 error:close"]
