@@ -779,11 +779,32 @@ auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStrea
   return lane;
 }
 
+/// Queries of a batch in ordinary host memory go through staging of the plan below this many bytes: a
+/// memcpy and a copy that need not be waited for. Above it the driver's copy from ordinary memory, which
+/// stages piece by piece while the pieces before cross the bus, is the faster one, although the call
+/// waits in it. us a call, staged and not: 100 queries x 128 (51 KB) 86 and 87, three batches of them 174
+/// and 212, 500 x 128 (256 KB) 122 and 125, 3 x 800 (410 KB) 354 and 341, 1 000 x 128 (512 KB) 173 and 170,
+/// 200 x 960 (768 KB) 239 and 229, 2 000 x 960 1 268 and 1 101, 10 000 x 128 1 090 and 987.
+constexpr size_t kStagedQueries = size_t{384} << 10;
+
+/// Results in ordinary host memory: true when they are made on the GPU and copied by the driver, false when
+/// the last kernel stores them through to staging. The stores cross the bus under the kernel's other
+/// work where it has enough of it; a round that gathers few entries per result ends waiting for them.
+/// 10 000 queries x 100 results (12 MB), stored and copied: 2 048 entries a query 1 721 and 1 797 us, 256
+/// entries a query 1 286 and 1 168; with 5 000 queries 690 and 659, 3 000 (3.6 MB) 440 and 437, 2 000 317 and 321.
+auto copies_results(plan const& pl, int m) -> bool
+{
+  constexpr size_t kLarge = size_t{4} << 20;
+  const size_t bytes      = (sizeof(int64_t) + sizeof(float)) * static_cast<size_t>(m) * pl.k;
+  const int entries       = pl.sp.waves > 0 ? pl.r2.nmax : pl.r1.nmax;
+  return bytes >= kLarge && entries < 8 * pl.k;
+}
+
 /// A search by one process with queries and results that are not all memory of its GPU (host memory,
 /// another GPU's): the copies are queued around the kernels. Several batches alternate between two
 /// lanes, each a plan on a stream of its own: the copies of one batch run under the kernels of the
 /// other. Page-locked arrays are copied from and to directly; ordinary ones pass through page-locked
-/// staging of the plan.
+/// staging of the plan where that is faster (kStagedQueries, copies_results).
 void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStream_t caller, int cur, const float* queries,
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
 {
@@ -799,8 +820,9 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
     check_tc(*lane[l]);
     follow_last_batch(*lane[l], stream[l]);
   }
-  const bool stage_in  = host_out && !device_reaches(queries);
-  const bool stage_out = host_out && !(device_reaches(neighbors) && device_reaches(distances));
+  const bool stage_in  = host_out && sizeof(float) * static_cast<size_t>(m) * D < kStagedQueries && !device_reaches(queries);
+  const bool stage_out = host_out && !(lanes == 1 && copies_results(*lane[0], m)) &&
+                         !(device_reaches(neighbors) && device_reaches(distances));
   struct pending {
     int64_t b0 = 0;
     int n      = 0;

@@ -290,3 +290,27 @@ def test_resident_after_a_call_of_several_batches(where):
     got = resident(50)
     assert np.array_equal(got[:40], want[:40]) and (got[40:] == want[0]).all()
     idx.close()
+
+
+@pytest.mark.parametrize("dim", [64, 960])
+def test_host_arrays_of_any_size(dim):
+    """Ordinary host memory on both sides of the sizes at which queries stop being staged and results stop
+    being stored through: the answers of the same queries in device memory. (4 000 x 100 results are
+    above 4 MB, with 128 entries a query from the last round.)"""
+    import torch
+    from octex_b200 import synth
+    idx, _ = make_index(dim, copies=6, blocks=4, table_len=16)
+    kw = dict(read=8, starts=8, waves=1, rerank=128, wave_rerank=64)
+    queries = synth.plumbing(9000, dim, seed=1)
+    edge = (384 << 10) // (4 * dim)
+    for n, k, batch in ((1, 1, 10000), (edge - 1, 10, 10000), (edge, 10, 10000), (edge + 1, 100, 10000), (3 * edge + 5, 10, edge),
+                        (3 * edge - 7, 10, edge - 1), (3495, 100, 10000), (3496, 100, 10000), (4000, 100, 10000),
+                        (9000, 100, 4000), (8000, 100, 4000)):
+        q = queries[:n]
+        d, i = idx.search(torch.as_tensor(q, device="cuda"), k, **kw)
+        want = d.cpu().numpy(), i.cpu().numpy()
+        assert same(idx.search(q, k, batch=batch, **kw), want), (n, k, batch)
+        out = np.full((n, k), -7, np.int64), np.full((n, k), -7, np.float32)
+        idx.search(q, k, batch=batch, neighbors=out[0], distances=out[1], **kw)
+        assert same((out[1], out[0]), want), (n, k, batch)
+    idx.close()
