@@ -121,6 +121,9 @@ def search_params(**kw) -> _lib.SearchParams:
     return p
 
 
+_PLAIN_NUMBERS = {int, bool, type(None)}
+
+
 @functools.lru_cache(maxsize=64)
 def _params_of_numbers(*values):
     return C.pointer(search_params(**dict(zip(SEARCH_PARAMS, values))))
@@ -130,9 +133,10 @@ def _search_params_ref(*values):
     """A pointer to the struct of these parameters (in the order of ``SEARCH_PARAMS``), made once for
     the same numbers (the library only reads it). Whatever else stands for a number (a numpy or torch
     scalar, which may change) is read now."""
-    return _params_of_numbers(*[v if type(v) in (int, bool) or v is None else
-                                bool(v) if name == "sketch_rank" else int(v)
-                                for name, v in zip(SEARCH_PARAMS, values)])
+    if not _PLAIN_NUMBERS.issuperset(map(type, values)):
+        values = [v if v is None else bool(v) if name == "sketch_rank" else int(v)
+                  for name, v in zip(SEARCH_PARAMS, values)]
+    return _params_of_numbers(*values)
 
 
 def load_params(placement="shard", sketch="replicate", **kw):
