@@ -327,6 +327,8 @@ class Index:
         torch = _torch()
         if _is_torch(queries):
             q = queries.detach() if queries.requires_grad else queries
+            if type(q) is not torch.Tensor:
+                q = q.as_subclass(torch.Tensor)  # the results are plain tensors
             if q.dtype != torch.float32:
                 raise TypeError("octex: queries must be float32")
             q = q.contiguous()

@@ -314,3 +314,27 @@ def test_host_arrays_of_any_size(dim):
         idx.search(q, k, batch=batch, neighbors=out[0], distances=out[1], **kw)
         assert same((out[1], out[0]), want), (n, k, batch)
     idx.close()
+
+
+def test_results_are_plain_tensors():
+    """Queries that need gradients, are a parameter or of a subclass of torch.Tensor: the results are plain
+    tensors without history."""
+    import torch
+    from octex_b200 import synth
+
+    class Named(torch.Tensor):
+        pass
+
+    idx, _ = make_index(64, copies=8, blocks=4)
+    kw = dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)
+    queries = synth.plumbing(5, 64, seed=1)
+    want = idx.search(queries, 10, **kw)
+    for device in ("cuda", "cpu"):
+        plain = torch.as_tensor(queries, device=device)
+        for q in (plain.as_subclass(Named), torch.nn.Parameter(plain.clone()), torch.nn.Parameter(plain, requires_grad=False),
+                  (plain.clone().requires_grad_() * 1)):
+            for t in idx.search(q, 10, **kw):
+                assert type(t) is torch.Tensor and not t.requires_grad and t.device == q.device
+            d, i = idx.search(q, 10, **kw)
+            assert same((d.cpu().numpy(), i.cpu().numpy()), want)
+    idx.close()
