@@ -558,11 +558,7 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
     }
   }
   __syncwarp();
-  if (*stop != 0) {
-    // let the copies this block still has in flight land before its shared memory goes away
-    for (int i = 0; i < 2048; i++)
-      __nanosleep(512);
-  }
+  if (*stop != 0) let_copies_land();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {

@@ -17,7 +17,7 @@
 // TMA (cp.async.bulk.tensor, no cluster forms), 64 rows x 64 halves (128 bytes, the swizzle span) a
 // step; the queries are read as fp32 by all threads and written in the same swizzled layout; one
 // thread issues the copies and the MMAs; every wait on an mbarrier is bounded and a wait that runs out
-// sets an error word, lets the block free its TMEM and return. The sketch-space queries (sketch_block),
+// sets an error word, lets the copies in flight land, frees the block's TMEM and returns. The sketch-space queries (sketch_block),
 // which the rounds need and the projection does not, are made by blocks of the same launch.
 //
 // What bounds it: instruction issue of the decode (about 130 instructions per block of eight
@@ -60,9 +60,11 @@ struct __align__(1024) tc_smem {
   cell_level lv[2][kCopies * 16];
   unsigned long long primes[8];
 };
-static_assert(sizeof(__half) * kStages * (kTileM + 2 * kTileN) * kTileK >=
-                sizeof(float) * (sketch_tile<1>::kWords > sketch_tile<4>::kWords ? sketch_tile<1>::kWords : sketch_tile<4>::kWords),
+// only a: TMA writes b, and nothing orders it after what threads did there
+static_assert(sizeof(tc_smem::a) >= sizeof(float) * (sketch_tile<1>::kWords > sketch_tile<4>::kWords ? sketch_tile<1>::kWords
+                                                                                                      : sketch_tile<4>::kWords),
               "staging of the sketch blocks");
+
 /// Centred fp16 queries [row0, row0 + 128) x dimensions [d0, d0 + 64) into an operand tile with the
 /// 128-byte swizzle (16-byte chunk c of row r at chunk c ^ (r % 8)). Rows beyond the batch are left
 /// as they are: an accumulator row depends on its own operand row only.
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
       }
     }
   }
+  if (!ready) let_copies_land();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {

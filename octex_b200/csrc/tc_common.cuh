@@ -55,6 +55,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   return false;
 }
 
+/// About a millisecond: for a block that gave up, before its shared memory and TMEM go away, so that the
+/// copies and MMAs it still has in flight land.
+__device__ __forceinline__ void let_copies_land()
+{
+  for (int i = 0; i < 2048; i++)
+    __nanosleep(512);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
 {
   asm volatile(
@@ -74,7 +82,8 @@ __device__ __forceinline__ uint64_t umma_desc(const void* tile)
          | (uint64_t{2} << 61);          // layout: 128-byte swizzle
 }
 
-/// D (fp32, TMEM) (+)= A (fp16, K-major) x B^T (fp16, K-major), 128 x 128 x 16.
+/// D (fp32, TMEM) (+)= A (fp16, K-major) x B^T (fp16, K-major), 16 of the inner dimension; the other two
+/// are in idesc.
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
                                          uint32_t accumulate)
 {
