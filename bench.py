@@ -89,7 +89,7 @@ LADDER = [
 # DRAM bytes (read + write) of one launch, from the ncu capture of this bench at its default workload
 # and the first rung of LADDER (profiles/round_kernel_descriptor-1m.md). Reported as
 # roofline.traffic only when the run uses exactly that workload and those parameters.
-NCU_TRAFFIC = {"round_rows": 1.156e9, "round_lists": 0.651e9}
+NCU_TRAFFIC = {"round_rows": 1.154e9, "round_lists": 0.651e9}
 
 
 def torch_build(w):
@@ -255,9 +255,11 @@ def algorithmic_bytes(stats, sp, meta, k):
     S4 = S + 4  # a sketch row of the first round: its codes and its fp32 constant
     lists = (4 * stats[:, 2] + n1 * S4 + r1 * 2 * D + 4 * D + 4 * S + KO * 12).sum()
     pairs = len(stats) * meta["copies"]
-    # the cell lookup happens inside the projection kernel: 16-byte table slots examined and the
-    # segment written per (query, copy), next to the fp16 queries read
-    out = {"project": int((stats[:, 1] * 16).sum() + pairs * 8 + len(stats) * 2 * D),
+    # the cell lookup happens inside the projection kernel: 8-byte table slots examined, the whole code
+    # that confirms a cell found and the segment written per (query, copy), next to the fp32 queries
+    # read and the sketch-space queries written
+    found = stats[:, 2] / min(sp["read"], meta["list_len"])
+    out = {"project": int((stats[:, 1] * 8 + found * 8).sum() + pairs * 8 + len(stats) * (4 * D + 4 * S)),
            "round_lists": int(lists)}
     if waves:
         rerank_w = stats[:, 7] - r1  # rows the waves read (ids already kept are not read again)
@@ -433,7 +435,7 @@ def main():
     ap.add_argument("--cpu-sample", type=int, default=2000)
     ap.add_argument("--ladder-start", type=int, default=0)
     ap.add_argument("--e2e-batch", type=int, default=0,
-                    help="queries per captured batch of the host-buffer call (search_params.batch); 0: half the call")
+                    help="queries per batch of the host-buffer call (search_params.batch); 0: half the call")
     ap.add_argument("--builder", default="native", choices=["native", "torch"],
                     help="native: the library's own GPU builder writes the index directory (to "
                          "--index-dir) and the index is loaded from it; torch: the package's torch "
@@ -600,9 +602,9 @@ def main():
         torch.cuda.synchronize()
         return time.perf_counter() - t0
 
-    # One process: the call's queries go through in captured batches of --e2e-batch on two streams
+    # One process: the call's queries go through in batches of --e2e-batch on two streams
     # (search_params.batch), so the copies of one batch run under the kernels of the other; the
-    # figure with the whole call as one captured batch is kept beside it. Several processes
+    # figure with the whole call as one batch is kept beside it. Several processes
     # exchange inside a batch and take the call as one.
     e2e_one_s = host_call_seconds(0)
     ids_one_batch = on.copy()

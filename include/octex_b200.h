@@ -129,7 +129,8 @@ struct cuvsOctexSearchParams {
   int32_t final_rerank;
   bool balanced_gather; /* accepted, ignored: one implementation */
   bool fused_merge;     /* accepted, ignored */
-  bool use_graph;       /* false: direct kernel launches instead of replaying the batch graph */
+  bool use_graph;       /* false: resident searches and batches shared by several processes launch their
+                           kernels instead of replaying a graph; all other searches always launch them */
 };
 typedef struct cuvsOctexSearchParams* cuvsOctexSearchParams_t;
 /* octex.h:189-192 */
@@ -169,7 +170,7 @@ OCTEX_B200_EXPORT cuvsError_t octexB200Build(cuvsResources_t res, cuvsOctexIndex
  * reference calls cuVS brute force there, cpp/src/neighbors/octex/detail/build_table.cuh:60-142).
  * ids int32 / distances float [n, k] in device memory: nearest first, equal distances by ascending
  * id, -1 / +inf where a row has fewer than k others. method 0: tensor cores when dim is a multiple
- * of 8 and k <= 120, else the plain scan; 1: tensor cores or an error; 2: the plain scan. Returns
+ * of 8 and k <= 122, else the plain scan; 1: tensor cores or an error; 2: the plain scan. Returns
  * when the work on the resources' stream is done. */
 OCTEX_B200_EXPORT cuvsError_t octexB200ExactNeighbors(cuvsResources_t res, const void* rows_f16, int64_t n,
                                                       int32_t dim, int32_t k, int32_t method, int32_t* ids,

@@ -39,14 +39,15 @@ struct search_params {
   int waves            = 2;     ///< secondary waves over the neighbor table (0: first round only)
   int rerank           = 128;   ///< exact rerank depth of the first round
   int wave_rerank      = 128;   ///< exact rerank depth of every wave
-  int batch            = 10000; ///< queries per captured batch
+  int batch            = 10000; ///< queries per batch
   bool sketch_rank     = false; ///< rank by the sketch, rerank exactly only at the end
   int final_rerank     = 32;    ///< sketch-rank mode: kept entries reranked exactly at the end
   /// Ablation switches of the reference. This library has one implementation of the gather and of
   /// the merge; those two fields are accepted and ignored.
   bool balanced_gather = true;
   bool fused_merge     = true;
-  /// false: direct kernel launches for every batch instead of replaying its CUDA graph.
+  /// false: resident searches and batches shared by several processes launch their kernels instead of
+  /// replaying a CUDA graph. All other searches always launch them.
   bool use_graph       = true;
 };
 

@@ -790,7 +790,7 @@ void exact_neighbors(const __half* x, int64_t n, int D, int K, int method, int32
   norms<<<grid_for(n, 128), 128, 0, s>>>(x, n, D, norm.as<float>());
   const bool covered = kernels::knn_tc_supported(n, D, K);
   OCTEX_EXPECTS(method != 1 || covered,
-                "octex: the tensor-core neighbor scan needs a dimension that is a multiple of 8 and K <= 120");
+                "octex: the tensor-core neighbor scan needs a dimension that is a multiple of 8 and K <= 122");
   if (method == 1 || (method == 0 && covered)) {
     dbuf error(dev, sizeof(int));
     OCTEX_CUDA_TRY(cudaMemsetAsync(error.ptr, 0, sizeof(int), s));

@@ -44,10 +44,8 @@ void project_ordered(const __half* qh, int ldq, const __half* ut, int ldu, const
                      int m, int N, int D, __half* Y, cudaStream_t s);
 
 /// codes [pairs, L] = cell code at every level of the 8*blocks coordinates of each (query, copy)
-/// pair of Y [pairs, 8*blocks]. level_on [C, L] (may be null) marks the levels that hold cells;
-/// the others get code 0 and are never looked at.
-void decode_codes(const __half* Y, int64_t pairs, int C, int blocks, int L, const float* inv_f,
-                  const unsigned char* level_on, long long* codes, cudaStream_t s);
+/// pair of Y [pairs, 8*blocks].
+void decode_codes(const __half* Y, int64_t pairs, int blocks, int L, const float* inv_f, long long* codes, cudaStream_t s);
 
 /// The sketch-space queries of a batch, computed by extra blocks of the projection's launch:
 /// qs [m, S] = (q - mean) @ basis in fp32 (one fused multiply-add per dimension, in dimension

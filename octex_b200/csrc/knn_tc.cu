@@ -21,11 +21,13 @@
 // up to a buffer old, which costs a few more appends, and a merge of a few hundred instructions serves 16
 // to 32 of them.
 //
-// What bounds it: the epilogue, two warps to a scheduler (168 registers a thread) at about five cycles an
-// instruction; 16 MMAs take 1 024 of the 4 600 cycles a tile takes. 200 001 x 128, K = 64: 133 ms with a
-// list update per improvement and a list per half of the tiles; 26 with buffers and resident query rows;
-// 21 with the bars, a warp per set for the MMAs, operands in uniform registers, and one mask of the
-// groups of columns that hold improvements where there was a vote and a branch for each.
+// What bounds it: the epilogue, two warps to a scheduler (168 registers a thread, and ptxas still spills 72,
+// 176 and 304 bytes with one, two and four keys a lane), each at an instruction every five cycles; the
+// MMAs are 29 % of a tile's time (262 144 x 128, K = 64: 30.2 ms, tensor pipe 28.9 %, issue slots 40.7 % busy).
+// 200 001 x 128, K = 64: 133 ms with a list update per improvement and a list per half of the tiles; 26 with
+// buffers and resident query rows; 21 with the bars, a warp per set for the MMAs, operands in uniform
+// registers, and one mask of the groups of columns that hold improvements where there was a vote and a
+// branch for each.
 //
 // Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues); the other warps
 // are the epilogue, in sets of four (one per quarter of the TMEM lanes).
@@ -612,6 +614,8 @@ void knn_tc(const __half* x, const float* norm, int64_t n, int D, int K, int64_t
   // Tiles that are looked at for the bars: a visit costs the same whatever it saves, an improvement the
   // same work at any n, and K ln(n / visits) of them are left: the best number of visits grows with K
   // alone. 266 665 x 96, K = 64: 34.5 ms with 16 visits, 33.5 with 2 K and 4 K, 45.5 with every tile.
+  // With fewer tiles than that (24 576 rows at K = 64) all of them are looked at, which still pays: 3 000 x
+  // 128, K = 64, 0.95 ms a call and 1.16 without the bars, 16 000 1.29 and 1.63, K = 100 1.58 and 2.22.
   const int64_t ntiles = (n + kTile - 1) / kTile;
   const int64_t spread = std::max<int64_t>(1, ntiles / std::max(16, kVisitsPerK * K));
   const int64_t wide   = narrow > 0 || rest == 0 ? (q_count - rest) / (2 * kTile) : (q_count + 2 * kTile - 1) / (2 * kTile);

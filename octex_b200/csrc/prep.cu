@@ -176,15 +176,12 @@ __global__ void __launch_bounds__(256) project_ordered_kernel(const __half* __re
 template <int B>
 __global__ void decode_codes_kernel(const __half* __restrict__ Y,
                                     int64_t pairs,
-                                    int C,
                                     int L,
                                     const float* __restrict__ inv_f,
-                                    const unsigned char* __restrict__ level_on,
                                     long long* __restrict__ codes)
 {
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= pairs) return;
-  const int c = static_cast<int>(t % C);
   float y[8 * B];
   const uint4* yp = reinterpret_cast<const uint4*>(Y + t * 8 * B);
 #pragma unroll
@@ -198,11 +195,8 @@ __global__ void decode_codes_kernel(const __half* __restrict__ Y,
       y[8 * i + 2 * j + 1] = f.y;
     }
   }
-  for (int j = 0; j < L; j++) {
-    long long h = 0;
-    if (level_on == nullptr || level_on[c * L + j]) h = cell_code<B>(y, inv_f[j]);
-    codes[t * L + j] = h;
-  }
+  for (int j = 0; j < L; j++)
+    codes[t * L + j] = cell_code<B>(y, inv_f[j]);
 }
 
 // Cell code of rows of 8 * B float32 coordinates at one scale (the decode of the search kernels on
@@ -353,19 +347,18 @@ void project_ordered(const __half* qh, int ldq, const __half* ut, int ldu, const
   project_ordered_kernel<<<grid, 256, 0, s>>>(qh, ldq, ut, ldu, shift, m, N, D, Y);
 }
 
-void decode_codes(const __half* Y, int64_t pairs, int C, int blocks, int L, const float* inv_f,
-                  const unsigned char* level_on, long long* codes, cudaStream_t s)
+void decode_codes(const __half* Y, int64_t pairs, int blocks, int L, const float* inv_f, long long* codes, cudaStream_t s)
 {
   if (pairs <= 0) return;
   const unsigned g = blocks_for(pairs, 128);
   switch (blocks) {
-    case 1: decode_codes_kernel<1><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
-    case 2: decode_codes_kernel<2><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
-    case 3: decode_codes_kernel<3><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
-    case 4: decode_codes_kernel<4><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
-    case 5: decode_codes_kernel<5><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
-    case 6: decode_codes_kernel<6><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
-    case 8: decode_codes_kernel<8><<<g, 128, 0, s>>>(Y, pairs, C, L, inv_f, level_on, codes); break;
+    case 1: decode_codes_kernel<1><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
+    case 2: decode_codes_kernel<2><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
+    case 3: decode_codes_kernel<3><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
+    case 4: decode_codes_kernel<4><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
+    case 5: decode_codes_kernel<5><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
+    case 6: decode_codes_kernel<6><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
+    case 8: decode_codes_kernel<8><<<g, 128, 0, s>>>(Y, pairs, L, inv_f, codes); break;
     default: break;  // the loader rejects other block counts
   }
 }

@@ -17,11 +17,12 @@
 // TMA (cp.async.bulk.tensor, no cluster forms), 64 rows x 64 halves (128 bytes, the swizzle span) a
 // step; the queries are read as fp32 by all threads and written in the same swizzled layout; one
 // thread issues the copies and the MMAs; every wait on an mbarrier is bounded and a wait that runs out
-// sets an error word, lets the copies in flight land, frees the block's TMEM and returns. The sketch-space queries (sketch_block),
-// which the rounds need and the projection does not, are made by blocks of the same launch.
+// sets an error word, lets the copies in flight land, frees the block's TMEM and returns. The
+// sketch-space queries (sketch_block), which the rounds need and the projection does not, are made by
+// blocks of the same launch.
 //
-// What bounds it: instruction issue of the decode (about 130 instructions per block of eight
-// coordinates and spacing, half of what block_code_tame takes) and the random sectors of
+// What bounds it: instruction issue of the decode (51 % of the slots at 16 warps a multiprocessor, 8.0 k warp
+// instructions a query where the decode that repairs both cosets took 12.2 k) and the random sectors of
 // the lookup. Two forms (tc_mode). 10 000 queries x 64 copies x 128 dimensions: 163 us in the bulk form
 // with the sketch-space queries in it, against 188 + 27 us for a kernel that decoded two copies per
 // thread after a 128-column tile and a centring kernel before it. One query: 10 us in the spread form
@@ -441,6 +442,13 @@ void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, c
   const int tiles = ((p.copies + kCopies - 1) / kCopies) * ((job.m + kTileM - 1) / kTileM);
   // rows of the caller's array are read sixteen bytes at a time where they all start on such a boundary
   const bool vec   = job.D % 4 == 0 && reinterpret_cast<uintptr_t>(job.q) % 16 == 0;
+  // A tile for every place on the GPU: the bulk form. Where the line belongs, us of a search of one round
+  // in the form taken and in the other: 64 copies x 128 dimensions, 1 150 queries (288 tiles) 97 and 92,
+  // 1 200 (320) 111 and 109, 1 400 118 and 113, 1 800 123 and 132, 10 000 401 and 465. Up to 128
+  // dimensions it is right to 4 %. Wider rows do not stay in the operand stages from tile to tile, and the
+  // bulk form overtakes later: 200 dimensions, 1 280 queries 135 and 124, 5 000 626 and 631; 512 dimensions,
+  // 1 200 queries 201 and 169, 2 300 229 and 228; 960 dimensions x 48 copies, 1 800 queries 334 and 257,
+  // 6 000 1 115 and 1 161.
   const int places = kBulkBlocks * p.sms;
   const auto mode  = look.table == nullptr ? tc_mode::taps : tiles >= places ? tc_mode::bulk : tc_mode::spread;
   const auto pick  = [&](auto taps, auto spread, auto bulk) {

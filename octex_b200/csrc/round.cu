@@ -344,8 +344,11 @@ __device__ __forceinline__ void rank_sort(const unsigned long long* src, int cnt
 /// the list, into dst, ascending; order [m] is scratch. A new key's place is the number of new keys below
 /// it, counted, and of old ones, found by halving; an old key's is its own plus the new ones below it,
 /// halving in their order. One barrier where a sorting network over all of them has 36 (256 keys) to 55
-/// (1 024 keys): 1 000 queries with the default parameters 356 -> 331 us, 10 000 embeddings with 256 start
-/// points and three waves 9.59 -> 9.20 ms. All threads of the block call it.
+/// (1 024 keys). The counting is quadratic in the new keys, and still the faster of the two over the whole
+/// range (200 000 rows x 128, us a search, by places and by the network): up to 128 new keys into 128 267
+/// and 288 (1 000 queries), into 512 1 159 and 1 497 (4 000 queries); up to 300 into 200 833 and 942; up to
+/// 512 into 65 548 and 567, into 512 1 774 and 1 938 (2 000 queries); 1 000 ranked by sketch distance into
+/// 1 000 2 120 and 2 257. All threads of the block call it.
 __device__ __forceinline__ void merge_sorted(const unsigned long long* old, int n, const unsigned long long* add, int m,
                                              unsigned long long* order, int want, unsigned long long* dst)
 {
@@ -1387,9 +1390,10 @@ namespace {
 
 /// Launch that may begin while the kernel before it in the stream is finishing; the kernel waits for
 /// it where it first needs its results (wait_for_previous_kernel).
-/// Only where it matters, in batches that leave multiprocessors idle: the first blocks of a kernel
-/// that starts under the last of another find the L1 cache split for the other's shared memory, and no
-/// block that follows on the multiprocessor gets it back (10 000 queries: 1 131 us a batch against 990).
+/// Only where it matters, in batches that leave multiprocessors idle: us a search of one round and one
+/// wave, early and not, 1 query 64 and 72, 100 queries 82 and 86, 148 84 and 86, 800 124 and 115, 1 000 132
+/// and 126, 10 000 617 and 620. (The first blocks of a kernel that starts under the last of another find the
+/// L1 cache split for the other's shared memory.)
 template <typename... P, typename... A>
 void launch_overlapped(bool early, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
                        A&&... args)
@@ -1410,7 +1414,10 @@ void launch_overlapped(bool early, void (*kernel)(P...), unsigned grid, unsigned
 /// Threads per query block. A multiprocessor runs 1024 threads of this kernel whatever the block size
 /// (64 registers each): a.threads makes the most of the blocks its shared memory holds. A batch of
 /// fewer blocks than the multiprocessors can hold at once is a matter of latency: its blocks get as
-/// many threads as still run side by side (one query, 1 M rows: 25 us a round with 128 threads).
+/// many threads as still run side by side. us a search, with that and with a.threads: 1 query of 64 copies
+/// 64 and 81, 300 queries 91 and 105, 592 100 and 107, from 800 on the same; 100 queries with 256 start
+/// points 180 and 226. Rounds of a few hundred entries lose to the wider barriers (one query of 8 copies x
+/// 8 entries: 59 and 54).
 int round_threads(const round_args& a)
 {
   int threads = a.threads;
@@ -1485,6 +1492,7 @@ void final_rerank(const long long* si, int KO, int R, const __half* vectors, row
     P <<= 1;
   const size_t words = 2 * static_cast<size_t>((k + R + 1) & ~1) + 2 * static_cast<size_t>(std::max(2 * P, 64)) +
                        2 * static_cast<size_t>((R + 3) & ~3) + ((D + 63) & ~63) + 256 + 16 + 8;
+  // early while there is a multiprocessor for every block, as in launch_round
   launch_overlapped(m <= 128, final_rerank_kernel, static_cast<unsigned>(m), kRoundThreads, sizeof(int) * words, s, si, KO, R,
                     vectors, vector_map, D, Q, k, P, bi, bd, stats);
 }

@@ -1,12 +1,13 @@
-// Batched search: plan (limits, buffers, one CUDA graph per batch shape) and the per-batch loop.
+// Batched search: plan (limits, buffers, the graph of a batch that stays in them) and the per-batch loop.
 //
 // Answers cpp/src/neighbors/octex/search.cu of hpdic/octex (make_plan :619-794, get_plan :796-814,
 // search_impl :816-961, the two search overloads :1020-1064) for one process per GPU. Parameter
 // limits and error texts are the reference's. A batch is two kernels and one per wave: projection
 // with cell lookup and sketch-space queries, first round, waves, the last of which writes the
-// results. Queries and results in the memory of the index's GPU are used where they are, on the caller's stream, and
-// every kernel is launched for the queries there are: no copies, no padding. A batch that stays in the
-// plan's buffers (resident searches, several processes) is replayed as one CUDA graph.
+// results. Queries and results in the memory of the index's GPU are used where they are, on the caller's
+// stream (the batches of a call of several on a second one in turn), and every kernel is launched for
+// the queries there are: no copies, no padding. A batch that stays in the plan's buffers (resident
+// searches, several processes) is replayed as one CUDA graph.
 
 #include "search_impl.hpp"
 
@@ -130,9 +131,8 @@ void check_tc(plan const& pl)
   if (pl.tc_error_host == nullptr || *pl.tc_error_host == 0) return;
   const int code    = *pl.tc_error_host;
   *pl.tc_error_host = 0;
-  throw error("octex: a kernel gave up waiting for data it had asked for (code " + std::to_string(code) +
-              ": 1, 2 the projection's operands, 3 the segments of a gather, 4 the rows of a rerank); "
-              "the results of that batch are not valid");
+  throw error("octex: the projection gave up waiting for data it had asked for (code " + std::to_string(code) +
+              "); the results of that batch are not valid");
 }
 
 /// Where a batch's queries are and its results go (device-accessible memory).
@@ -240,8 +240,8 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
       kernels::project_ordered(pl.qh.as<__half>(), p.ldu, p.ut.as<__half>(), p.ldu, p.shift.as<__half>(), pl.m1, wdt, D,
                                pl.Y.as<__half>(), s);
       mark();
-      kernels::decode_codes(pl.Y.as<__half>(), int64_t{pl.m1} * p.copies, p.copies, ix.blocks, L, p.inv_f.as<float>(),
-                            nullptr, pl.codes.as<long long>(), s);
+      kernels::decode_codes(pl.Y.as<__half>(), int64_t{pl.m1} * p.copies, ix.blocks, L, p.inv_f.as<float>(),
+                            pl.codes.as<long long>(), s);
     }
     mark();
     kernels::probe(pl.codes.as<long long>(), pl.m1, p.copies, L, look, s);

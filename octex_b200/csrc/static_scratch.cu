@@ -103,8 +103,8 @@ extern "C" cuvsError_t octexB200QueryCodesStatic(cuvsOctexIndex_t index, const f
                            sw, qh, p.ldu, qs, s);
     kernels::project_ordered(qh, p.ldu, p.ut.as<__half>(), p.ldu, p.shift.as<__half>(),
                              static_cast<int>(m), N, D, Y, s);
-    kernels::decode_codes(Y, static_cast<int64_t>(m) * p.copies, p.copies, ix.blocks, L,
-                          p.inv_f.as<float>(), nullptr, reinterpret_cast<long long*>(codes), s);
+    kernels::decode_codes(Y, static_cast<int64_t>(m) * p.copies, ix.blocks, L, p.inv_f.as<float>(),
+                          reinterpret_cast<long long*>(codes), s);
     OCTEX_CUDA_TRY(cudaPeekAtLastError());
     cuvsSetLastErrorText(nullptr);
     return CUVS_SUCCESS;

@@ -562,7 +562,7 @@ def exact_neighbors(rows, k, method="auto"):
     """The ``k`` nearest other rows of every row of ``rows`` [n, dim] (a torch CUDA tensor, used as
     float16) by squared L2: ``(ids int32 [n, k], distances float32 [n, k])`` as torch tensors on the
     same GPU, nearest first (``octexB200ExactNeighbors``).  ``method``: "auto", "tensor" (the
-    tcgen05 scan; dim a multiple of 8, k <= 120) or "plain"."""
+    tcgen05 scan; dim a multiple of 8, k <= 122) or "plain"."""
     torch = _torch()
     if not (_is_torch(rows) and rows.is_cuda and rows.dim() == 2):
         raise TypeError("octex: exact_neighbors takes a torch CUDA matrix [n, dim]")

@@ -534,10 +534,20 @@ def test_fused_lookup_path_100k(oracle, gpu_100k):
 
 
 def test_direct_launches_equal_graph(gpu_wide):
-    """use_graph = false (search.cu:885-920 of the reference: the same kernels launched directly)."""
+    """use_graph = false (search.cu:885-920 of the reference: the same kernels launched directly). A resident
+    search replays the graph of its batch or launches its kernels; an ordinary one always launches."""
     idx, _, _, _, queries = gpu_wide
     kw = dict(read=8, starts=32, waves=2, rerank=64, wave_rerank=64)
+    idx.search(queries[::-1].copy(), 10, **kw)
     d0, i0 = idx.search(queries, 10, **kw)
+    kept = idx.fetch("kept_ids", np.int64), idx.fetch("kept_dist", np.uint32)
+    assert np.array_equal(kept[0].reshape(len(queries), -1)[:, :10], i0)
+    for use_graph in (True, False, True):
+        for n in (len(queries), 7, len(queries)):
+            idx.search_resident(n, 10, use_graph=use_graph, **kw)
+            for name, dtype, want in (("kept_ids", np.int64, kept[0]), ("kept_dist", np.uint32, kept[1])):
+                rows = want.reshape(len(queries), -1)[:n]
+                assert np.array_equal(idx.fetch(name, dtype, (n, -1)), rows), (use_graph, n, name)
     p = octex_b200.search_params(use_graph=False, **kw)
     I = np.zeros((len(queries), 10), np.int64)
     D = np.zeros((len(queries), 10), np.float32)
