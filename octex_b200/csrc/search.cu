@@ -914,7 +914,8 @@ void search_impl(resources const& res,
                  int64_t k,
                  bool host_out,
                  bool resident,
-                 bool wait)
+                 bool wait,
+                 int max_lanes)
 {
   auto& ix = idx.impl();
   OCTEX_EXPECTS(qdim == ix.dim, "octex: query dimension differs from the index");
@@ -926,7 +927,7 @@ void search_impl(resources const& res,
   auto& p             = ix.part;
   // streams: a second one for the batches of one process, unless the plan keeps observations
   const debug_options dbg = ix_debug(ix);
-  const int lanes = ix.world == 1 && !resident && nq > std::max(sp.batch, 1) && !dbg.stats && !dbg.taps ? 2 : 1;
+  const int lanes = ix.world == 1 && !resident && nq > std::max(sp.batch, 1) && !dbg.stats && !dbg.taps ? max_lanes : 1;
   if (!resident && !host_out && search_in_place(ix, queries, neighbors, distances)) {
     const lane_plans used = search_device(ix, sp, lanes, caller, queries, nq, neighbors, distances, k);
     if (wait) {

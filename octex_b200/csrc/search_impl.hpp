@@ -76,7 +76,8 @@ void search_impl(resources const& res,
                  int64_t k,
                  bool host_out,
                  bool resident,
-                 bool wait = false);
+                 bool wait     = false,
+                 int max_lanes = 2);
 
 /// True when a search with these device arrays works on them where they are (one process, everything in
 /// the memory of the index's GPU, which is the current device); otherwise they are copied in and out.
