@@ -165,6 +165,7 @@ struct round_args {
   int done_stride = 0;
   int done_off = 0;  // entries of earlier waves
   int pick_slots = 0;  // hash slots for the earlier start points (power of two)
+  int kept_slots = 0;  // hash slots for the ids of the kept list (power of two)
   // sketch: rows of sw codes; sketch_norm [n]: the constant of every row (sketch_row_norms),
   // whole on every GPU even when the rows are dealt
   const signed char* sketch = nullptr;
@@ -179,7 +180,6 @@ struct round_args {
   int R = 0;                 // rerank depth (exact) — ignored when sketch_rank
   int KO = 0;
   int sketch_rank = 0;
-  int fresh = 0;  // the kept list starts empty
   long long* si = nullptr;  // kept ids [m, KO]
   float* sd = nullptr;      // kept distances [m, KO]
   // sizes of the shared-memory carve-up (host decides)

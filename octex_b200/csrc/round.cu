@@ -27,9 +27,26 @@ namespace {
 constexpr unsigned kIdHash          = 2654435761u;
 constexpr unsigned long long kNoKey = ~0ULL;
 
+/// Words every thread of a block shares: counters, and what a selection finds out.
+enum ctl {
+  kEmitted,   // keys taken by a selection
+  kBin,       // bin of the R-th key, keys still needed from it, its size
+  kLeft,
+  kSize,
+  kDistinct,  // distinct ids of the gather
+  kStarts,    // start points of a wave
+  kMerged,    // new keys of a merge
+  kSide,      // members of the bin of the R-th key
+  kLow,       // range of the high words a selection bins
+  kHigh,
+  kValid,     // entries of the kept list with an id
+  kWithin,    // ranking by sketch distance: candidates below the last key of a full kept list
+  kCtlWords
+};
+
 /// Offsets (in 4-byte words) of the regions of a round block's shared memory.
 struct round_layout {
-  int table, cand, dist, pool, sorted, sid, sdv, qv, sc, fq, st, len, hist, wsum, ctrl, kid, kd, words;
+  int table, cand, dist, pool, sorted, sid, sdv, qv, sc, fq, st, len, hist, wsum, ctrl, kid, kd, kset, words;
   __host__ __device__ explicit round_layout(const round_args& a)
   {
     const int in_smem = a.cand_global == nullptr ? a.nmax : 0;
@@ -41,9 +58,8 @@ struct round_layout {
       return o;
     };
     // Two regions are used twice. The sketch distances are written where the hash set of the gather
-    // was (the set is dead once the ids are collected; the filter of kept ids, which builds a small
-    // set there again, starts after the selection has copied out the distances it needs). The keys of
-    // the merge are written where the candidates were (dead after the selection).
+    // was (the set is dead once the ids are collected). The keys of the merge are written where the
+    // candidates were (dead after the selection).
     const int pool_words = 2 * (a.KO + rm);
     const int sort_words = a.P > 32 ? 4 * a.P : 128;  // 2 P keys, 64 at least (the one-warp sort)
     table  = take(a.ht_slots > in_smem ? a.ht_slots : in_smem);
@@ -61,10 +77,11 @@ struct round_layout {
     st     = take(a.nseg);
     len    = take(a.nseg);
     hist   = take(256);
-    wsum   = take(36);  // one word per warp of at most 32, and the total
-    ctrl   = take(8);
+    wsum   = take(32);  // one word per warp
+    ctrl   = take(kCtlWords);
     kid    = take(a.KO);
     kd     = take(a.KO);
+    kset   = take(a.kept_slots);
     words  = at;
   }
 };
@@ -75,14 +92,13 @@ __device__ __forceinline__ unsigned home_slot(int id, int slots)
   return __umulhi(static_cast<unsigned>(id) * kIdHash, static_cast<unsigned>(slots));
 }
 
-/// Exclusive prefix of v over the block (kThreads threads); total = the sum. wsum: kThreads / 32 + 1
-/// words.
+/// Exclusive prefix of v over the block (kThreads threads); total = the sum. wsum: kThreads / 32 words that
+/// nothing else uses until the block's next barrier.
 template <int kThreads = kRoundThreads>
 __device__ __forceinline__ int block_scan(int v, int* wsum, int& total)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int nw = kThreads / 32;
-  int inc          = v;
+  int inc        = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int u = __shfl_up_sync(0xffffffffu, inc, o);
@@ -90,22 +106,32 @@ __device__ __forceinline__ int block_scan(int v, int* wsum, int& total)
   }
   if (lane == 31) wsum[warp] = inc;
   __syncthreads();
-  if (warp == 0) {
-    const int w = lane < nw ? wsum[lane] : 0;
-    int winc    = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, winc, o);
-      if (lane >= o) winc += u;
-    }
-    if (lane < nw) wsum[lane] = winc - w;
-    if (lane == nw - 1) wsum[nw] = winc;
+  const int w = lane < kThreads / 32 ? wsum[lane] : 0;
+  total       = __reduce_add_sync(0xffffffffu, w);
+  return __reduce_add_sync(0xffffffffu, lane < warp ? w : 0) + inc - v;
+}
+
+/// Puts an id (none when negative) into a small set of `slots` (a power of two, never full) ids.
+__device__ __forceinline__ void insert_id(int* set, int slots, int id)
+{
+  if (id < 0) return;
+  unsigned h = (static_cast<unsigned>(id) * kIdHash) & (slots - 1);
+  for (int p = 0; p < slots; p++) {
+    const int prev = atomicCAS(&set[h], -1, id);
+    if (prev == -1 || prev == id) return;
+    h = (h + 1) & (slots - 1);
   }
-  __syncthreads();
-  const int out = wsum[warp] + inc - v;
-  total         = wsum[nw];
-  __syncthreads();
-  return out;
+}
+__device__ __forceinline__ bool holds_id(const int* set, int slots, int id)
+{
+  unsigned h = (static_cast<unsigned>(id) * kIdHash) & (slots - 1);
+  for (int p = 0; p < slots; p++) {
+    const int t = set[h];
+    if (t == -1) return false;
+    if (t == id) return true;
+    h = (h + 1) & (slots - 1);
+  }
+  return false;
 }
 
 /// (distance bits << 32) | id: the total order of every kept list (search_kernels.cuh:365-368).
@@ -196,13 +222,13 @@ __device__ __forceinline__ radix_cut_t radix_cut(HiAt hi_at, LoAt lo_at, int n, 
           }
           cum += h[t];
         }
-        ctrl[1] = 8 * lane + d;                  // digit
-        ctrl[2] = need - static_cast<int>(cum);  // still needed from that bucket
-        ctrl[3] = static_cast<int>(size);        // bucket size
+        ctrl[kBin]  = 8 * lane + d;                  // digit
+        ctrl[kLeft] = need - static_cast<int>(cum);  // still needed from that bucket
+        ctrl[kSize] = static_cast<int>(size);        // bucket size
       }
     }
     __syncthreads();
-    const int digit = ctrl[1], left = ctrl[2], bucket = ctrl[3];
+    const int digit = ctrl[kBin], left = ctrl[kLeft], bucket = ctrl[kSize];
     if (word == 1) {
       prefix_hi |= static_cast<unsigned>(digit) << shift;
       mask_hi |= 255u << shift;
@@ -218,48 +244,61 @@ __device__ __forceinline__ radix_cut_t radix_cut(HiAt hi_at, LoAt lo_at, int n, 
                      (static_cast<unsigned long long>(mask_hi) << 32) | mask_lo};
 }
 
-/// The same threshold as radix_cut with, in the usual case, one counting pass instead of three or
-/// four: the high words (distances of one query: a narrow range of bit patterns) are binned over
-/// their own range [min, max] into 256 bins, the bin that holds the R-th key is found, and the
-/// R-th key itself is ranked among the few members of that bin. Falls back on radix_cut when that
-/// bin holds more than 128 keys (many equal or nearly equal distances). hist: 256 words, used as
-/// counters and then as the list of the bin's members; ctrl[1], [2], [3], [7] are used.
-template <typename HiAt, typename LoAt>
-__device__ __forceinline__ radix_cut_t smallest_cut(HiAt hi_at, LoAt lo_at, int n, int R, unsigned* hist,
-                                                    int* ctrl)
+/// What a selection expects: counters at zero, no range yet. A barrier belongs behind it.
+__device__ __forceinline__ void selection_begin(unsigned* hist, int* ctrl)
 {
-  constexpr int kSide = 128;
-  const int lane = threadIdx.x & 31;
-  unsigned* uc   = reinterpret_cast<unsigned*>(ctrl);
   for (int i = threadIdx.x; i < 256; i += blockDim.x)
     hist[i] = 0;
   if (threadIdx.x == 0) {
-    uc[1] = ~0u;
-    uc[2] = 0u;
-    uc[7] = 0u;
+    ctrl[kEmitted] = 0;
+    ctrl[kSide]    = 0;
+    ctrl[kLow]     = -1;
+    ctrl[kHigh]    = 0;
   }
-  __syncthreads();
-  unsigned lo = ~0u, hi = 0u;
+}
+
+/// The range of the high words of n keys, in ctrl[kLow] and ctrl[kHigh]. After selection_begin and a barrier;
+/// ends in one.
+template <typename HiAt>
+__device__ __forceinline__ void find_range(HiAt hi_at, int n, int* ctrl)
+{
+  unsigned low = ~0u, high = 0u;
+#pragma unroll 4
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const unsigned h = hi_at(i);
-    lo               = min(lo, h);
-    hi               = max(hi, h);
+    low              = min(low, h);
+    high             = max(high, h);
   }
-  lo = __reduce_min_sync(0xffffffffu, lo);
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  if (lane == 0) {
-    atomicMin(&uc[1], lo);
-    atomicMax(&uc[2], hi);
+  low  = __reduce_min_sync(0xffffffffu, low);
+  high = __reduce_max_sync(0xffffffffu, high);
+  if ((threadIdx.x & 31) == 0 && low <= high) {
+    atomicMin(reinterpret_cast<unsigned*>(&ctrl[kLow]), low);
+    atomicMax(reinterpret_cast<unsigned*>(&ctrl[kHigh]), high);
   }
   __syncthreads();
-  lo           = uc[1];
-  hi           = uc[2];
+}
+
+/// emit(high word, low word) for the R smallest of n distinct keys (n > R), in any order; hi_at(i) /
+/// lo_at(i) give the two words of key i. The high words (distances of one query: a narrow range of bit
+/// patterns, known to be [ctrl[kLow], ctrl[kHigh]]) are counted in 256 bins over their range, the bin
+/// that holds the R-th key is found, and a second pass takes what lies below it and puts the bin's own
+/// members aside, which are ranked among themselves. With more than 128 of those (many equal or nearly
+/// equal distances) radix_cut finds the threshold. With the range three passes over the keys and five
+/// barriers; passes of their own for the members and the taking made it four and nine. hist: 256 words,
+/// counters and then the members. After selection_begin and find_range; all threads of the block call it,
+/// and a barrier belongs behind it.
+template <typename HiAt, typename LoAt, typename Emit>
+__device__ __forceinline__ void take_smallest(HiAt hi_at, LoAt lo_at, int n, int R, unsigned* hist, int* ctrl, Emit emit)
+{
+  constexpr unsigned kSideRoom = 128;
+  const unsigned lo = static_cast<unsigned>(ctrl[kLow]), hi = static_cast<unsigned>(ctrl[kHigh]);
   const int sh = max(0, 24 - __clz(static_cast<int>(hi - lo)));  // (hi - lo) >> sh < 256
   for (int i = threadIdx.x; i < n; i += blockDim.x)
     atomicAdd(&hist[(hi_at(i) - lo) >> sh], 1u);
   __syncthreads();
   if (threadIdx.x < 32) {
     // lane l owns bins 8l .. 8l+7: the bin at which the running count reaches R
+    const int lane = threadIdx.x;
     unsigned h[8], mine = 0;
 #pragma unroll
     for (int t = 0; t < 8; t++) {
@@ -285,59 +324,60 @@ __device__ __forceinline__ radix_cut_t smallest_cut(HiAt hi_at, LoAt lo_at, int 
         }
         cum += h[t];
       }
-      ctrl[1] = 8 * lane + d;               // bin
-      ctrl[2] = R - static_cast<int>(cum);  // still needed from that bin
-      ctrl[3] = static_cast<int>(size);     // its size
+      ctrl[kBin]  = 8 * lane + d;
+      ctrl[kLeft] = R - static_cast<int>(cum);
+      ctrl[kSize] = static_cast<int>(size);
     }
   }
   __syncthreads();
-  const unsigned bin = static_cast<unsigned>(ctrl[1]);
-  const int left = ctrl[2], bucket = ctrl[3];
-  if (bucket == left) {
-    // the bin is taken whole: every key whose high word is below the next bin's first value
-    unsigned long long top = static_cast<unsigned long long>(lo) + ((static_cast<unsigned long long>(bin) + 1) << sh) - 1;
-    if (top > 0xffffffffULL) top = 0xffffffffULL;
-    __syncthreads();
-    return radix_cut_t{(top << 32) | 0xffffffffULL, ~0ULL};
-  }
-  if (bucket > kSide) {
-    __syncthreads();
-    return radix_cut(hi_at, lo_at, n, R, hist, ctrl);
+  const unsigned bin  = static_cast<unsigned>(ctrl[kBin]);
+  const unsigned left = static_cast<unsigned>(ctrl[kLeft]), size = static_cast<unsigned>(ctrl[kSize]);
+  if (left < size && size > kSideRoom) {
+    const radix_cut_t c = radix_cut(hi_at, lo_at, n, R, hist, ctrl);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const unsigned h = hi_at(i), l = lo_at(i);
+      if ((((static_cast<unsigned long long>(h) << 32) | l) & c.mask) <= c.prefix) emit(h, l);
+    }
+    return;
   }
   unsigned long long* side = reinterpret_cast<unsigned long long*>(hist);  // the counters are dead
+  const unsigned taken     = left == size ? bin + 1 : bin;                // the bins below are taken whole
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const unsigned h = hi_at(i);
-    if (((h - lo) >> sh) == bin) side[atomicAdd(&uc[7], 1u)] = (static_cast<unsigned long long>(h) << 32) | lo_at(i);
+    const unsigned h = hi_at(i), b = (h - lo) >> sh;
+    if (b < taken)
+      emit(h, lo_at(i));
+    else if (b == bin)
+      side[atomicAdd(&ctrl[kSide], 1)] = (static_cast<unsigned long long>(h) << 32) | lo_at(i);
   }
+  if (left == size) return;
   __syncthreads();
-  if (threadIdx.x < bucket) {
+  if (threadIdx.x < size) {
     const unsigned long long mine = side[threadIdx.x];
-    int below                     = 0;
-    for (int j = 0; j < bucket; j++)
+    unsigned below                = 0;
+    for (unsigned j = 0; j < size; j++)
       below += side[j] < mine;
-    if (below == left - 1) {  // the left-th smallest of the bin is the R-th smallest of all
-      uc[2] = static_cast<unsigned>(mine >> 32);
-      uc[3] = static_cast<unsigned>(mine);
-    }
+    if (below < left) emit(static_cast<unsigned>(mine >> 32), static_cast<unsigned>(mine));
   }
-  __syncthreads();
-  const unsigned long long cut = (static_cast<unsigned long long>(uc[2]) << 32) | uc[3];
-  __syncthreads();
-  return radix_cut_t{cut, ~0ULL};
 }
 
-/// Ascending order of cnt <= blockDim.x distinct keys src[0, cnt) into dst (another array): a
-/// thread counts the keys below its own and puts it there. No step depends on another, which
-/// suits the short lists a merge usually sorts better than a sorting network run by one warp.
-__device__ __forceinline__ void rank_sort(const unsigned long long* src, int cnt, unsigned long long* dst)
+/// The `want` smallest of cnt distinct keys src[0, cnt) into dst (another array), ascending: a group of
+/// lanes counts the keys below its own and puts it there. No step depends on another, which suits the
+/// short lists a merge usually sorts better than a sorting network run by one warp. cnt <= blockDim.x.
+__device__ __forceinline__ void rank_sort(const unsigned long long* src, int cnt, unsigned long long* dst, int want)
 {
-  if (threadIdx.x < cnt) {
-    const unsigned long long mine = src[threadIdx.x];
-    int below                     = 0;
-    for (int j = 0; j < cnt; j++)
-      below += src[j] < mine;
-    dst[below] = mine;
-  }
+  int lanes = 1;  // per key
+  while (lanes < 32 && 2 * lanes * cnt <= static_cast<int>(blockDim.x))
+    lanes *= 2;
+  const int at = threadIdx.x / lanes, sub = threadIdx.x & (lanes - 1);
+  if ((threadIdx.x & ~31u) / lanes >= static_cast<unsigned>(cnt)) return;  // a warp without a key
+  const unsigned long long mine = src[min(at, cnt - 1)];
+  int below                     = 0;
+#pragma unroll 4
+  for (int j = sub; j < cnt; j += lanes)
+    below += src[j] < mine;
+  for (int o = 1; o < lanes; o <<= 1)
+    below += __shfl_xor_sync(0xffffffffu, below, o);
+  if (sub == 0 && at < cnt && below < want) dst[below] = mine;
 }
 
 /// The first `want` keys of the ascending list old[0, n) and the m distinct keys add[0, m), none of them in
@@ -770,9 +810,10 @@ __device__ __forceinline__ void exact_distances(const int* sid, int ns, const __
 /// with (-1, +inf), written to pb / pd. Same result as sorting kept + new and taking the first KO
 /// distinct keys (search_kernels.cuh:372-415). A new key beyond the last entry of a full kept list
 /// cannot make it and is dropped at once; what remains is sorted directly when it is short, or the
-/// KO smallest are cut out by radix passes first. kid / kd: the kept list as it was (shared
-/// memory), null when it starts empty. pool holds KO + ns keys, sorted holds 2 * P (P a power of
-/// two >= KO). oi / od (k > 0): the first k entries go there too, the results of a last round.
+/// KO smallest are selected first. kid / kd: the kept list as it was (shared memory), nk its entries with
+/// an id (it is packed: those come first); ctrl[kMerged] is zero. pool holds KO + ns keys, sorted holds
+/// 2 * P (P a power of two >= KO). oi / od (k > 0): the first k entries go there too, the results of a
+/// last round.
 __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
                                                 unsigned long long* sorted,
                                                 int P,
@@ -781,6 +822,7 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
                                                 int KO,
                                                 const int* kid,
                                                 const float* kd,
+                                                int nk,
                                                 const int* sid,
                                                 const float* sdv,
                                                 int ns,
@@ -790,39 +832,27 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
                                                 float* od = nullptr,
                                                 int k = 0)
 {
-  const bool fresh = kid == nullptr;
-  if (threadIdx.x == 0) ctrl[6] = 0;
-  // the kept list is packed (valid entries first): nk = first index without an id
-  int nk = 0;
-  if (!fresh) {
-    int lo = 0, hi = KO;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (kid[mid] >= 0)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    nk = lo;
-  }
   const unsigned long long bound =
     nk == KO && KO > 0 ? rank_key(kd[KO - 1], static_cast<unsigned>(kid[KO - 1])) : kNoKey;
-  __syncthreads();
   for (int i = threadIdx.x; i < nk; i += blockDim.x)
     pool[i] = rank_key(kd[i], static_cast<unsigned>(kid[i]));
   for (int i = threadIdx.x; i < ns; i += blockDim.x) {
     if (sid[i] < 0) continue;
     const unsigned long long k = rank_key(sdv[i], static_cast<unsigned>(sid[i]));
-    if (k < bound) pool[nk + atomicAdd(&ctrl[6], 1)] = k;
+    if (k < bound) pool[nk + atomicAdd(&ctrl[kMerged], 1)] = k;
   }
   __syncthreads();
-  const int total = nk + ctrl[6];
-  int cnt         = min(total, KO);
-  constexpr int kRankMax = 128;  // keys sorted by ranking, one thread per key (blocks have >= 128 threads)
-  if (total <= 2 * P) {
-    if (total <= kRankMax) {
-      rank_sort(pool, total, sorted);
-    } else if (nk > 0 && total - nk <= P) {
+  const int total = nk + ctrl[kMerged];
+  const int cnt   = min(total, KO);
+  // Short lists are sorted by ranking, at most kRankSteps comparisons a thread. A block of 128 threads, of
+  // which many share a multiprocessor, rather selects first where KO keys are few of the total.
+  constexpr int kRankSteps = 128;
+  const int threads        = blockDim.x;
+  const auto few           = [&](int keys) { return keys <= threads && keys * keys <= kRankSteps * threads; };
+  if (few(total) && (total <= 2 * P || threads > kRoundThreads)) {
+    rank_sort(pool, total, sorted, KO);
+  } else if (total <= 2 * P) {
+    if (nk > 0 && total - nk <= P) {
       merge_sorted(pool, nk, pool + nk, total - nk, sorted + P, KO, sorted);
     } else {
       int width = P;
@@ -834,23 +864,20 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
       bitonic_sort(sorted, width);
     }
   } else {
-    // the KO smallest are cut out first (into the upper half of the sort region), then sorted
+    // the KO smallest are selected first (into the upper half of the sort region), then sorted
     unsigned long long* picked = sorted + max(P, 32);
-    auto hi_at          = [&](int i) { return static_cast<unsigned>(pool[i] >> 32); };
-    auto lo_at          = [&](int i) { return static_cast<unsigned>(pool[i]); };
-    const radix_cut_t c = smallest_cut(hi_at, lo_at, total, KO, hist, ctrl);
-    if (threadIdx.x == 0) ctrl[0] = 0;
+    auto hi_at                 = [&](int i) { return static_cast<unsigned>(pool[i] >> 32); };
+    auto lo_at                 = [&](int i) { return static_cast<unsigned>(pool[i]); };
+    selection_begin(hist, ctrl);
     __syncthreads();
-    for (int i = threadIdx.x; i < total; i += blockDim.x) {
-      const unsigned long long k = pool[i];
-      if ((k & c.mask) <= c.prefix) {
-        const int s = atomicAdd(&ctrl[0], 1);
-        if (s < P) picked[s] = k;
-      }
-    }
+    find_range(hi_at, total, ctrl);
+    take_smallest(hi_at, lo_at, total, KO, hist, ctrl, [&](unsigned high, unsigned low) {
+      const int s = atomicAdd(&ctrl[kEmitted], 1);
+      if (s < P) picked[s] = (static_cast<unsigned long long>(high) << 32) | low;
+    });
     __syncthreads();
-    if (KO <= kRankMax) {
-      rank_sort(picked, KO, sorted);
+    if (few(KO)) {
+      rank_sort(picked, KO, sorted, KO);
     } else {
       for (int i = threadIdx.x; i < P; i += blockDim.x)
         sorted[i] = i < KO ? picked[i] : kNoKey;
@@ -903,7 +930,6 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   const int S    = a.sw;
   long long* pb  = a.si + static_cast<int64_t>(q) * a.KO;
   float* pd      = a.sd + static_cast<int64_t>(q) * a.KO;
-  const bool fresh = a.fresh != 0;
 
   // The integer form of the sketch distance serves the first round of a search that reranks
   // exactly. Waves take the fp32 sum (see sketch_rows_f32), and so does every round of a search
@@ -922,16 +948,26 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   if (!a.sketch_rank)
     for (int i = threadIdx.x; i < a.D; i += blockDim.x)
       fq[(a.D & 7) ? i : query_slot(i)] = a.Q[static_cast<int64_t>(q) * a.D + i];
-  if (threadIdx.x == 0) ctrl[4] = 0;  // distinct ids
-  // the kept list as the round finds it: read once, used by the start points, by the filter of
-  // already kept ids and by the merge
+  selection_begin(hist, ctrl);
+  if (threadIdx.x == 0) {
+    ctrl[kDistinct] = 0;
+    ctrl[kMerged]   = 0;
+    ctrl[kValid]    = 0;
+    ctrl[kWithin]   = 0;
+  }
+  // the kept list as the round finds it (empty in a first round): read once, used by the start points, by
+  // the filter of already kept ids and by the merge
   int* kid  = smem + lay.kid;
   float* kd = reinterpret_cast<float*>(smem + lay.kd);
-  if (!fresh)
+  int* kset = smem + lay.kset;
+  if constexpr (kRows) {
     for (int i = threadIdx.x; i < a.KO; i += blockDim.x) {
       kid[i] = static_cast<int>(pb[i]);
       kd[i]  = pd[i];
     }
+    for (int i = threadIdx.x; i < a.kept_slots; i += blockDim.x)
+      kset[i] = -1;
+  }
 
   // cycles per phase of this block (observation only): start points / segments, gather, sketch
   // scoring, selection, filter + prefetch, exact distances, merge
@@ -947,41 +983,30 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   int total = 0, nseg = a.nseg;
   if constexpr (kRows) {
     // start points: the first nseg kept entries that no earlier wave expanded
-    // (search_kernels.cuh:571-631); earlier start points go through a hash set in the table region
-    int* pdone = a.done + static_cast<int64_t>(q) * a.done_stride;
-    for (int i = threadIdx.x; i < a.pick_slots; i += blockDim.x)
-      table[i] = -1;
+    // (search_kernels.cuh:571-631); earlier start points, if there are any, go through a hash set in the
+    // table region
+    int* pdone       = a.done + static_cast<int64_t>(q) * a.done_stride;
+    const bool again = a.done_off > 0;
+    if (again)
+      for (int i = threadIdx.x; i < a.pick_slots; i += blockDim.x)
+        table[i] = -1;
     __syncthreads();
-    for (int i = threadIdx.x; i < a.done_off; i += blockDim.x) {
-      const int v = pdone[i];
-      if (v < 0) continue;
-      unsigned h = (static_cast<unsigned>(v) * kIdHash) & (a.pick_slots - 1);
-      for (int p = 0; p < a.pick_slots; p++) {
-        const int prev = atomicCAS(&table[h], -1, v);
-        if (prev == -1 || prev == v) break;
-        h = (h + 1) & (a.pick_slots - 1);
-      }
+    if (again)
+      for (int i = threadIdx.x; i < a.done_off; i += blockDim.x)
+        insert_id(table, a.pick_slots, pdone[i]);
+    for (int i = threadIdx.x; i < a.KO; i += blockDim.x) {
+      const int v = kid[i];
+      insert_id(kset, a.kept_slots, v);
+      if (v >= 0 && (i + 1 == a.KO || kid[i + 1] < 0)) ctrl[kValid] = i + 1;
     }
-    __syncthreads();
+    if (again) __syncthreads();
     const int per       = (a.KO + kThreads - 1) / kThreads;
     const int i0        = threadIdx.x * per;
     unsigned fresh_bits = 0;
     int mine            = 0;
     for (int i = i0; i < min(a.KO, i0 + per); i++) {
       const int v = kid[i];
-      bool f      = v >= 0;
-      if (f) {
-        unsigned h = (static_cast<unsigned>(v) * kIdHash) & (a.pick_slots - 1);
-        for (int p = 0; p < a.pick_slots; p++) {
-          const int t = table[h];
-          if (t == -1) break;
-          if (t == v) {
-            f = false;
-            break;
-          }
-          h = (h + 1) & (a.pick_slots - 1);
-        }
-      }
+      const bool f = v >= 0 && !(again && holds_id(table, a.pick_slots, v));
       if (f) {
         fresh_bits |= 1u << (i - i0);
         mine++;
@@ -1008,8 +1033,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
     for (int o = nseg + threadIdx.x; o < a.nseg; o += blockDim.x)
       pdone[a.done_off + o] = -1;
     total = nseg * a.table_len;
-    if (threadIdx.x == 0) ctrl[5] = nseg;
-    __syncthreads();
+    if (threadIdx.x == 0) ctrl[kStarts] = nseg;
   } else {
     // segment starts and lengths; every segment is either empty or `read` entries long
     int mine = 0;
@@ -1094,7 +1118,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
           if (lane >= o) inc += up;
         }
         int base = 0;
-        if (lane == 31 && inc > 0) base = atomicAdd(&ctrl[4], inc);
+        if (lane == 31 && inc > 0) base = atomicAdd(&ctrl[kDistinct], inc);
         base   = __shfl_sync(0xffffffffu, base, 31);
         int at = base + inc - mine;
 #pragma unroll
@@ -1107,7 +1131,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
     }
   }
   __syncthreads();
-  const int n = min(ctrl[4], a.nmax);
+  const int n = min(ctrl[kDistinct], a.nmax);
   tick(1);
 
   // int8 sketch distances (search_kernels.cuh:228-251), sixteen codes per lane, S / 16 lanes
@@ -1155,47 +1179,40 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
 
   // the nearest by (sketch distance, id) (search_kernels.cuh:259-322 takes equal distances at the
   // cut in any order)
-  const int R = a.sketch_rank ? a.KO : a.R;
-  int ns      = n;
-  auto key_at = [&](int i) { return rank_key(dist[i], static_cast<unsigned>(cand[i])); };
+  const int R   = a.sketch_rank ? a.KO : a.R;
+  int ns        = n;
+  bool selected = false;
   // A search that ranks by sketch distance keeps what it selects here, so a key beyond the last one of a
   // full kept list is out already. Where the keys that are left fit, they need no selection: which of them
   // stay is the merge's to say, and the kept list comes out the same (with the merge by places: 2 500
   // embeddings, 512 start points and three waves 5.17 -> 4.98 ms).
-  bool selected = false;
-  if (a.sketch_rank && !fresh && kid[a.KO - 1] >= 0) {
+  if (kRows && a.sketch_rank && ctrl[kValid] == a.KO) {
     const unsigned long long bound = rank_key(kd[a.KO - 1], static_cast<unsigned>(kid[a.KO - 1]));
-    if (threadIdx.x == 0) ctrl[0] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-      if (key_at(i) < bound) {
-        const int s = atomicAdd(&ctrl[0], 1);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += kThreads)
+      if (__float_as_uint(dist[i]) <= static_cast<unsigned>(bound >> 32) &&
+          rank_key(dist[i], static_cast<unsigned>(cand[i])) < bound) {
+        const int s = atomicAdd(&ctrl[kWithin], 1);
         if (s < R) {
           sid[s] = cand[i];
           sdv[s] = dist[i];
         }
       }
     __syncthreads();
-    if (ctrl[0] <= R) {
-      ns       = ctrl[0];
-      selected = true;
-    }
+    selected = ctrl[kWithin] <= R;
+    if (selected) ns = ctrl[kWithin];
   }
   if (!selected && n > R) {
-    auto hi_at          = [&](int i) { return __float_as_uint(dist[i]); };
-    auto lo_at          = [&](int i) { return static_cast<unsigned>(cand[i]); };
-    const radix_cut_t c = smallest_cut(hi_at, lo_at, n, R, hist, ctrl);
-    if (threadIdx.x == 0) ctrl[0] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      if ((key_at(i) & c.mask) <= c.prefix) {
-        const int s = atomicAdd(&ctrl[0], 1);
-        if (s < R) {
-          sid[s] = cand[i];
-          sdv[s] = dist[i];
-        }
+    auto hi_at = [&](int i) { return __float_as_uint(dist[i]); };
+    auto lo_at = [&](int i) { return static_cast<unsigned>(cand[i]); };
+    find_range(hi_at, n, ctrl);
+    take_smallest(hi_at, lo_at, n, R, hist, ctrl, [&](unsigned high, unsigned low) {
+      const int s = atomicAdd(&ctrl[kEmitted], 1);
+      if (s < R) {
+        sid[s] = static_cast<int>(low);
+        sdv[s] = __uint_as_float(high);
       }
-    }
+    });
     ns = R;
   } else if (!selected) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1206,52 +1223,25 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   __syncthreads();
 
   tick(3);
-  // a selected id that is already in the kept list brings the key it already has there: drop it
-  // before the vectors are read (the reference reranks it again and collapses the equal keys)
-  if (!fresh) {
-    int HK = 64;
-    while (HK < 2 * a.KO)
-      HK <<= 1;
-    for (int i = threadIdx.x; i < HK; i += blockDim.x)
-      table[i] = -1;
-    __syncthreads();
-    for (int i = threadIdx.x; i < a.KO; i += blockDim.x) {
-      const int v = kid[i];
-      if (v < 0) continue;
-      unsigned h = (static_cast<unsigned>(v) * kIdHash) & (HK - 1);
-      for (int p = 0; p < HK; p++) {
-        const int prev = atomicCAS(&table[h], -1, v);
-        if (prev == -1 || prev == v) break;
-        h = (h + 1) & (HK - 1);
-      }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < ns; i += blockDim.x) {
-      const int v = sid[i];
-      unsigned h  = (static_cast<unsigned>(v) * kIdHash) & (HK - 1);
-      for (int p = 0; p < HK; p++) {
-        const int t = table[h];
-        if (t == -1) break;
-        if (t == v) {
-          sid[i] = -1;
-          break;
-        }
-        h = (h + 1) & (HK - 1);
-      }
-    }
-    __syncthreads();
-  }
-  int reranked = 0;
-  if (!a.sketch_rank) {
-    // every row about to be read is asked for at once (128-byte lines into L2), so the distance
-    // loop below finds most of them on the way
-    const int row_bytes = a.D * 2;
-    for (int r = threadIdx.x; r < (may_prefetch<kDealt>(a.vector_map) ? ns : 0); r += blockDim.x) {
-      if (sid[r] < 0) continue;
-      const char* row = reinterpret_cast<const char*>(a.vectors + static_cast<int64_t>(sid[r]) * a.D);
+  // A selected id that is already in the kept list brings the key it already has there: drop it
+  // before the vectors are read (the reference reranks it again and collapses the equal keys). Every row
+  // about to be read is asked for at once (128-byte lines into L2), so the distance loop below finds
+  // most of them on the way.
+  const bool ahead    = !a.sketch_rank && may_prefetch<kDealt>(a.vector_map);
+  const int row_bytes = a.D * 2;
+  for (int r = threadIdx.x; r < ns; r += blockDim.x) {
+    const int v = sid[r];
+    if (kRows && holds_id(kset, a.kept_slots, v)) {
+      sid[r] = -1;
+    } else if (ahead) {
+      const char* row = reinterpret_cast<const char*>(a.vectors + static_cast<int64_t>(v) * a.D);
       for (int b = 0; b < row_bytes; b += 128)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
     }
+  }
+  if (kRows) __syncthreads();
+  int reranked = 0;
+  if (!a.sketch_rank) {
     if (a.stats != nullptr) {
       int mine = 0;
       for (int i = threadIdx.x; i < ns; i += blockDim.x)
@@ -1262,16 +1252,15 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
     exact_distances<kDealt>(sid, ns, a.vectors, a.vector_map, a.D, fq, sdv);
     tick(5);
   }
-  merge_into_kept(pool, sorted, a.P, pb, pd, a.KO, fresh ? nullptr : kid, kd, sid, sdv, ns, hist, ctrl,
+  merge_into_kept(pool, sorted, a.P, pb, pd, a.KO, kid, kd, kRows ? ctrl[kValid] : 0, sid, sdv, ns, hist, ctrl,
                   a.out_i == nullptr ? nullptr : a.out_i + static_cast<int64_t>(q) * a.k,
                   a.out_i == nullptr ? nullptr : a.out_d + static_cast<int64_t>(q) * a.k,
                   a.out_i == nullptr ? 0 : a.k);
-  __syncthreads();
   tick(6);
   if (a.stats != nullptr && threadIdx.x == 0) {
     long long* s = a.stats + static_cast<int64_t>(q) * 8;
     if constexpr (kRows) {
-      s[4] += ctrl[5];
+      s[4] += ctrl[kStarts];
       s[5] += n;
     } else {
       s[2] += total;
@@ -1304,9 +1293,10 @@ __global__ void __launch_bounds__(kRoundThreads) final_rerank_kernel(const long 
   float* fq                  = sdv + ((R + 3) & ~3);                         // [D]
   unsigned* hist             = reinterpret_cast<unsigned*>(fq + ((D + 63) & ~63));
   int* wsum                  = reinterpret_cast<int*>(hist + 256);
-  int* ctrl                  = wsum + 16;
+  int* ctrl                  = wsum + 32;
   const int q                = blockIdx.x;
   const long long* ps        = si + static_cast<int64_t>(q) * KO;
+  if (threadIdx.x == 0) ctrl[kMerged] = 0;
   wait_for_previous_kernel();
   for (int i = threadIdx.x; i < D; i += blockDim.x)
     fq[(D & 7) ? i : query_slot(i)] = Q[static_cast<int64_t>(q) * D + i];
@@ -1321,7 +1311,7 @@ __global__ void __launch_bounds__(kRoundThreads) final_rerank_kernel(const long 
   block_scan(mine, wsum, ns);
   exact_distances<true>(sid, ns, vectors, vector_map, D, fq, sdv);
   merge_into_kept(pool, sorted, P, bi + static_cast<int64_t>(q) * k, bd + static_cast<int64_t>(q) * k,
-                  k, nullptr, nullptr, sid, sdv, ns, hist, ctrl);
+                  k, nullptr, nullptr, 0, sid, sdv, ns, hist, ctrl);
   if (stats != nullptr && threadIdx.x == 0) {
     stats[static_cast<int64_t>(q) * 8 + 6] += ns;
     stats[static_cast<int64_t>(q) * 8 + 7] += ns;
@@ -1491,7 +1481,7 @@ void final_rerank(const long long* si, int KO, int R, const __half* vectors, row
   while (P < k)
     P <<= 1;
   const size_t words = 2 * static_cast<size_t>((k + R + 1) & ~1) + 2 * static_cast<size_t>(std::max(2 * P, 64)) +
-                       2 * static_cast<size_t>((R + 3) & ~3) + ((D + 63) & ~63) + 256 + 16 + 8;
+                       2 * static_cast<size_t>((R + 3) & ~3) + ((D + 63) & ~63) + 256 + 32 + kCtlWords;
   // early while there is a multiprocessor for every block, as in launch_round
   launch_overlapped(m <= 128, final_rerank_kernel, static_cast<unsigned>(m), kRoundThreads, sizeof(int) * words, s, si, KO, R,
                     vectors, vector_map, D, Q, k, P, bi, bd, stats);

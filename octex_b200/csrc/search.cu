@@ -50,7 +50,7 @@ constexpr size_t kSmemSoftLimit = size_t{96} << 10;   // above this the candidat
 constexpr size_t kSmemHardLimit = size_t{227} << 10;  // shared memory a block can opt in to
 
 /// Fill the size fields of a round and decide where its candidate arrays live.
-void size_round(plan& pl, kernels::round_args& r, int entries_max, int pick_entries, int device,
+void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, int pick_entries, int device,
                 int64_t sketch_bytes)
 {
   r.pick_slots = 0;
@@ -59,9 +59,12 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, int pick_entr
     while (r.pick_slots * 3 < pick_entries * 4)  // at most 75 % full
       r.pick_slots <<= 1;
   }
-  int kept_slots = 64;  // the set of kept ids a round filters its selection with
-  while (kept_slots < 2 * r.KO)
-    kept_slots <<= 1;
+  r.kept_slots = 0;  // the set of kept ids a wave filters its selection with
+  if (waves) {
+    r.kept_slots = 64;
+    while (r.kept_slots < 2 * r.KO)
+      r.kept_slots <<= 1;
+  }
   r.nmax = std::max(entries_max, 1);
   r.P    = 2;
   while (r.P < r.KO)
@@ -74,7 +77,7 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, int pick_entr
   for (int twelfths : {24, 18, 16}) {
     r.hash_twelfths = twelfths;
     r.cap_slots = kernels::hash_slots_of(std::min(entries_max, kernels::kMaxHash), kernels::kMaxHash, twelfths);
-    r.ht_slots  = std::max({r.cap_slots, r.pick_slots, kept_slots});
+    r.ht_slots  = std::max(r.cap_slots, r.pick_slots);
     if (kernels::round_smem_bytes(r) <= kEightBlocks) break;
   }
   if (kernels::round_smem_bytes(r) > kSmemSoftLimit) {
@@ -532,7 +535,6 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   r1.sketch_rank = sp.sketch_rank ? 1 : 0;
   r1.sketch_map  = map_of(ix, p.sketch_rows);
   r1.vector_map  = map_of(ix, p.vector_rows);
-  r1.fresh       = 1;
   r1.si          = pl.si.as<long long>();
   r1.sd          = pl.sd.as<float>();
   r1.stats       = pl.stats.as<long long>();
@@ -545,7 +547,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   }
   // sketch rows of this GPU's own memory (not the host tier, not dealt over GPUs) plus their constants
   const int64_t sketch_bytes = (p.sketch.host || p.sketch_rows.on) ? 0 : static_cast<int64_t>(p.sketch.size + p.sketch_norm.size);
-  size_round(pl, r1, p.copies * pl.lr, 0, p.device, sketch_bytes);
+  size_round(pl, r1, p.copies * pl.lr, false, 0, p.device, sketch_bytes);
   // waves: table rows of the start points
   if (sp.waves > 0) {
     auto& r2       = pl.r2;
@@ -570,12 +572,11 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
     r2.R           = pl.R2;
     r2.KO          = pl.KO;
     r2.sketch_rank = r1.sketch_rank;
-    r2.fresh       = 0;
     r2.si          = pl.wsi;
     r2.sd          = pl.wsd;
     r2.stats       = r1.stats;
     r2.phase       = pl.phase2.as<long long>();
-    size_round(pl, r2, S * ix.table_len, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes);
+    size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes);
   }
   kernels::round_allow_smem(pl.smem_max);
 
