@@ -26,6 +26,7 @@ namespace {
 
 constexpr unsigned kIdHash          = 2654435761u;
 constexpr unsigned long long kNoKey = ~0ULL;
+constexpr int kAheadBytes           = 512;  // fp16 rows up to this are asked for ahead of the exact distances
 
 /// Words every thread of a block shares: counters, and what a selection finds out.
 enum ctl {
@@ -109,6 +110,28 @@ __device__ __forceinline__ int block_scan(int v, int* wsum, int& total)
   const int w = lane < kThreads / 32 ? wsum[lane] : 0;
   total       = __reduce_add_sync(0xffffffffu, w);
   return __reduce_add_sync(0xffffffffu, lane < warp ? w : 0) + inc - v;
+}
+
+/// True when an id was not in the set of the gather yet and is now. The steps grow by one slot each (the
+/// longest way among the 32 ids of a warp is what a step of the gather takes, and ways grow together into
+/// runs where every step is one slot); from kGrowing steps on, one slot each, so that a free slot is met.
+/// There is one: as many slots as entries. Against steps of one slot, thousand cycles of a block's gathers:
+/// 16 384 entries and 21 848 slots, three waves, 115 and 105; 32 768 in as many slots 171 and 121 (the search
+/// 4 888 and 4 340 us). Reading a slot before the exchange, or four entries' exchanges side by side, take
+/// longer (179 and 178 for the first): what counts is how many steps a warp makes, and the reads come on top.
+__device__ __forceinline__ bool claim(int* set, int slots, int id)
+{
+  constexpr int kGrowing = 32;
+  unsigned s             = home_slot(id, slots);
+#pragma unroll 1
+  for (int p = 1; p < kGrowing + slots; p++) {
+    const int was = atomicCAS(&set[s], -1, id);
+    if (was == -1) return true;
+    if (was == id) return false;
+    s += p < kGrowing ? p : 1;
+    if (s >= static_cast<unsigned>(slots)) s -= slots;
+  }
+  return false;
 }
 
 /// Puts an id (none when negative) into a small set of `slots` (a power of two, never full) ids.
@@ -1095,16 +1118,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
           const int id = v[u];
           bool is_new  = false;
           if (id >= 0) {  // else nothing read, or the padding of a table row
-            unsigned s = home_slot(id, HT);
-            for (int p = 0; p < HT; p++) {
-              const int prev = atomicCAS(&table[s], -1, id);
-              if (prev == -1) {
-                is_new = true;
-                break;
-              }
-              if (prev == id) break;
-              s = s + 1 == static_cast<unsigned>(HT) ? 0u : s + 1;
-            }
+            is_new = claim(table, HT, id);
           }
           if (!is_new) v[u] = -1;
           mine += is_new;
@@ -1226,9 +1240,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // A selected id that is already in the kept list brings the key it already has there: drop it
   // before the vectors are read (the reference reranks it again and collapses the equal keys). Every row
   // about to be read is asked for at once (128-byte lines into L2), so the distance loop below finds
-  // most of them on the way.
-  const bool ahead    = !a.sketch_rank && may_prefetch<kDealt>(a.vector_map);
+  // most of them on the way; not wide rows, of which the loop has enough on the way itself (999 queries, 382 rows of 1 920 bytes
+  // each, a first round: 144 us asked for and 129 not; 10 000 queries, 370 rows of 256 bytes, a wave: 411 and 418).
   const int row_bytes = a.D * 2;
+  const bool ahead    = !a.sketch_rank && row_bytes <= kAheadBytes && may_prefetch<kDealt>(a.vector_map);
   for (int r = threadIdx.x; r < ns; r += blockDim.x) {
     const int v = sid[r];
     if (kRows && holds_id(kset, a.kept_slots, v)) {

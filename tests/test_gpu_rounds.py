@@ -20,6 +20,35 @@ def against_checker(oracle, idx, arrays, meta, queries, k, **kw):
         assert np.array_equal(dist.view(np.uint32), want_dist.view(np.uint32)), (len(queries), kw)
 
 
+@pytest.fixture(scope="module")
+def many_rows(tmp_path_factory):
+    """700 000 rows: a bit for each takes 21 876 words, more than most hash sets and fewer than the largest."""
+    import torch
+    from octex_b200 import index_dir
+    g = torch.Generator("cuda").manual_seed(5)
+    centers = torch.randn(500, 32, generator=g, device="cuda") * 2
+    rows = centers[torch.randint(500, (700_000,), generator=g, device="cuda")] + torch.randn(700_000, 32, generator=g, device="cuda")
+    path = str(tmp_path_factory.mktemp("many_rows"))
+    octex_b200.build_native(rows, path, copies=8, blocks=2, pca_dims=32, list_len=16, min_cell=4, log_buckets=12,
+                            sketch_width=32, table_len=64, seed=3)
+    idx = octex_b200.load(path, placement="replicate", devices=0)
+    arrays, meta = index_dir.read_index(path)
+    yield idx, arrays, meta, (rows[::9973][:60] + 0.1).cpu().numpy()
+    idx.close()
+
+
+@pytest.mark.parametrize("kw", [
+    dict(read=16, starts=16, waves=2, rerank=64, wave_rerank=64),            # eight blocks a multiprocessor
+    dict(read=16, starts=96, waves=2, rerank=64, wave_rerank=128),           # four
+    dict(read=16, starts=256, waves=2, rerank=128, wave_rerank=512),         # two, the hash set three quarters full at most
+    dict(read=16, starts=300, waves=2, rerank=128, wave_rerank=512),         # one, bits
+    dict(read=16, starts=512, waves=2, sketch_rank=True, final_rerank=32),   # one, bits, distances over them
+])
+def test_gathered_ids(oracle, many_rows, kw):
+    idx, arrays, meta, queries = many_rows
+    against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+
+
 @pytest.mark.parametrize("distinct", [1, 3, 40, 4000])
 def test_selection_among_equal_distances(oracle, distinct):
     """Rows that repeat: the bin of the last selected key holds any number of keys, more than are ranked
