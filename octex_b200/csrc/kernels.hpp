@@ -185,6 +185,7 @@ struct round_args {
   // sizes of the shared-memory carve-up (host decides)
   int ht_slots = 0;   // ints of the hash set region (>= largest set used, >= pick_slots)
   int cap_slots = 0;  // largest gather hash set (slots)
+  int map_words = 0;  // words (a multiple of four) of a bit for every row, which then takes the set's place
   int hash_twelfths = 16;  // slots per 12 gathered entries (host: as sparse as shared memory allows)
   int keep_sketch = 0;  // the sketch and its row constants fit the L2 cache with room to spare: load them
                         // with an evict-last policy, the large arrays with evict-first (host decides)

@@ -1078,9 +1078,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // threads walks one segment, so consecutive threads read consecutive entries, and every thread
   // has four segments' loads in flight before it touches the set
   tick(0);
-  const int HT = hash_slots_of(total, a.cap_slots, a.hash_twelfths);
+  const int HT = a.map_words > 0 ? a.map_words : hash_slots_of(total, a.cap_slots, a.hash_twelfths);
+  const int empty = a.map_words > 0 ? 0 : -1;
   for (int i = threadIdx.x; i < HT / 4; i += blockDim.x)
-    reinterpret_cast<int4*>(table)[i] = make_int4(-1, -1, -1, -1);
+    reinterpret_cast<int4*>(table)[i] = make_int4(empty, empty, empty, empty);
   __syncthreads();
   {
     const int maxlen = kRows ? a.table_len : a.lr;
@@ -1118,7 +1119,12 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
           const int id = v[u];
           bool is_new  = false;
           if (id >= 0) {  // else nothing read, or the padding of a table row
-            is_new = claim(table, HT, id);
+            if (a.map_words > 0) {
+              const unsigned bit = 1u << (id & 31);
+              is_new             = (atomicOr(reinterpret_cast<unsigned*>(&table[id >> 5]), bit) & bit) == 0;
+            } else {
+              is_new = claim(table, HT, id);
+            }
           }
           if (!is_new) v[u] = -1;
           mine += is_new;

@@ -51,7 +51,7 @@ constexpr size_t kSmemHardLimit = size_t{227} << 10;  // shared memory a block c
 
 /// Fill the size fields of a round and decide where its candidate arrays live.
 void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, int pick_entries, int device,
-                int64_t sketch_bytes)
+                int64_t sketch_bytes, int64_t rows)
 {
   r.pick_slots = 0;
   if (pick_entries > 0) {
@@ -80,12 +80,36 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
     r.ht_slots  = std::max(r.cap_slots, r.pick_slots);
     if (kernels::round_smem_bytes(r) <= kEightBlocks) break;
   }
-  if (kernels::round_smem_bytes(r) > kSmemSoftLimit) {
-    // placeholders: non-null makes the layout drop the two arrays; the real buffers follow
-    r.cand_global = reinterpret_cast<int*>(1);
-    r.dist_global = reinterpret_cast<float*>(1);
-    OCTEX_EXPECTS(kernels::round_smem_bytes(r) <= kSmemHardLimit,
-                  "octex: the round does not fit shared memory");
+  // placeholders: non-null makes the layout drop the two arrays; the real buffers follow
+  auto settle = [&] {
+    r.cand_global = nullptr;
+    r.dist_global = nullptr;
+    if (kernels::round_smem_bytes(r) > kSmemSoftLimit) {
+      r.cand_global = reinterpret_cast<int*>(1);
+      r.dist_global = reinterpret_cast<float*>(1);
+    }
+    return (size_t{228} << 10) / (kernels::round_smem_bytes(r) + 1024);  // blocks of a multiprocessor
+  };
+  // A bit for every row of the index instead of the set, where that takes no more room, or where the set
+  // leaves a multiprocessor one block anyway: one exchange an entry, and no way to a free slot.
+  // A million rows, 32 768 entries a query: 121 and 62 thousand cycles of gathers, the search 4 340 and 3 798 us;
+  // 100 003 rows, 8 192 entries, 502 and 487. Where two blocks fit with the set the bits at one block lose what
+  // the blocks do side by side: a million rows, 16 384 entries, 8 670 and 9 605.
+  const size_t blocks = settle();
+  const int slots     = r.ht_slots;
+  const int words     = static_cast<int>(std::min<int64_t>((rows + 127) / 128 * 4, 1 << 20));
+  if (words <= slots || blocks < 2) {
+    r.map_words = words;
+    r.ht_slots  = std::max({words, r.pick_slots, slots >= r.nmax ? r.nmax : 0});
+    settle();
+    if (r.ht_slots > slots && kernels::round_smem_bytes(r) > kSmemHardLimit) {
+      r.map_words = 0;
+      r.ht_slots  = slots;
+      settle();
+    }
+  }
+  OCTEX_EXPECTS(kernels::round_smem_bytes(r) <= kSmemHardLimit, "octex: the round does not fit shared memory");
+  if (r.cand_global != nullptr) {
     pl.scratch_cand.push_back(alloc<int>(pl, device, int64_t{r.m} * r.nmax));
     r.cand_global = pl.scratch_cand.back().as<int>();
     // the sketch distances still go where the hash set was when that region holds them all (the
@@ -100,8 +124,8 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
   // threads per block: a multiprocessor runs 1024 threads of this kernel (64 registers each); when
   // fewer than eight blocks fit its shared memory, the blocks get more threads to make up for it
   const size_t per_block = kernels::round_smem_bytes(r) + 1024;
-  const int fit          = static_cast<int>(std::max<size_t>((size_t{228} << 10) / per_block, 1));
-  r.threads              = fit >= 8 ? 128 : fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
+  const int held         = static_cast<int>(std::max<size_t>((size_t{228} << 10) / per_block, 1));
+  r.threads              = held >= 8 ? 128 : held >= 4 ? 256 : held >= 2 ? 512 : 1024;
   OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, device));
   {
     // the sketch stays in the L2 cache when it and its constants take at most 60 % of it
@@ -547,7 +571,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   }
   // sketch rows of this GPU's own memory (not the host tier, not dealt over GPUs) plus their constants
   const int64_t sketch_bytes = (p.sketch.host || p.sketch_rows.on) ? 0 : static_cast<int64_t>(p.sketch.size + p.sketch_norm.size);
-  size_round(pl, r1, p.copies * pl.lr, false, 0, p.device, sketch_bytes);
+  size_round(pl, r1, p.copies * pl.lr, false, 0, p.device, sketch_bytes, ix.n);
   // waves: table rows of the start points
   if (sp.waves > 0) {
     auto& r2       = pl.r2;
@@ -576,7 +600,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
     r2.sd          = pl.wsd;
     r2.stats       = r1.stats;
     r2.phase       = pl.phase2.as<long long>();
-    size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes);
+    size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes, ix.n);
   }
   kernels::round_allow_smem(pl.smem_max);
 

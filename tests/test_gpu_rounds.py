@@ -49,6 +49,18 @@ def test_gathered_ids(oracle, many_rows, kw):
     against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
 
 
+@pytest.mark.parametrize("rows", [511, 512, 513, 8191, 8193])
+def test_rows_around_a_word_of_bits(oracle, rows):
+    """Ids up to the last bit of the last word; a bit for every row or a set of as many slots as entries."""
+    from octex_b200 import build_index, synth
+    arrays, meta = build_index.build_arrays(synth.plumbing(rows, 32, seed=0), small_params(copies=4, table_len=24), device="cpu")
+    idx = octex_b200.attach(arrays, meta, borrow=False)
+    queries = synth.plumbing(50, 32, seed=1)
+    for kw in (dict(read=16, starts=12, waves=2, rerank=48, wave_rerank=32), dict(read=4, starts=100, waves=1, rerank=16, wave_rerank=256)):
+        against_checker(oracle, idx, arrays, meta, queries, 7, **kw)
+    idx.close()
+
+
 @pytest.mark.parametrize("distinct", [1, 3, 40, 4000])
 def test_selection_among_equal_distances(oracle, distinct):
     """Rows that repeat: the bin of the last selected key holds any number of keys, more than are ranked
