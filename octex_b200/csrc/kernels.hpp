@@ -189,6 +189,7 @@ struct round_args {
   int hash_twelfths = 16;  // slots per 12 gathered entries (host: as sparse as shared memory allows)
   int keep_sketch = 0;  // the sketch and its row constants fit the L2 cache with room to spare: load them
                         // with an evict-last policy, the large arrays with evict-first (host decides)
+  int pass_vectors = 0;  // the fp16 rows leave the L2 cache first (evict-first; host decides)
   int threads = kRoundThreads;  // threads per query block in a large batch: 128 to 1024 (host: the smallest
                                 // that still fills a multiprocessor with the blocks that fit it)
   int sms = 1;                  // multiprocessors of the GPU

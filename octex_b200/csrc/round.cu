@@ -711,8 +711,8 @@ __device__ __forceinline__ int query_slot(int i)
 /// (shared memory, read 16 bytes at a time).
 /// Both row pointers are valid (a row that is not wanted is replaced by any row by the caller, who
 /// drops the result). kMode 0: any D that is a multiple of 8; 1: D a multiple of 128, so no step
-/// needs a bounds check; 2: D = 128, one step with constant offsets.
-template <int kMode>
+/// needs a bounds check; 2: D = 128, one step with constant offsets. kPass: the rows leave the L2 cache first.
+template <int kMode, bool kPass>
 __device__ __forceinline__ void exact_pair(const uint4* const (&row)[2], int Drt, int sub, const float* fq,
                                            float (&out)[2])
 {
@@ -731,7 +731,10 @@ __device__ __forceinline__ void exact_pair(const uint4* const (&row)[2], int Drt
     for (int s = 0; s < 2; s++)
 #pragma unroll
       for (int u = 0; u < 2; u++)
-        if (kWhole || h0 + 64 * s < D) v[s][u] = __ldg(row[u] + ((h0 + 64 * s) >> 3));
+        if (kWhole || h0 + 64 * s < D) {
+          const uint4* at = row[u] + ((h0 + 64 * s) >> 3);
+          v[s][u]         = kPass ? ldg16_hint(at, l2_policy_stream()) : __ldg(at);
+        }
 #pragma unroll
     for (int s = 0; s < 2; s++) {
       const int hs = h0 + 64 * s;
@@ -769,7 +772,7 @@ __device__ __forceinline__ void exact_pair(const uint4* const (&row)[2], int Drt
 /// 1, 2, 4, 8, 16 (search_kernels.cuh:325-342 is the reference's warp-per-row form of the same
 /// sum). Eight lanes own a row, each reading 16 bytes per step (partial sums 4 lane .. 4 lane + 3);
 /// a warp works on eight rows at a time.
-template <bool kDealt, int kMode>
+template <bool kDealt, int kMode, bool kPass>
 __device__ __forceinline__ void exact_rows(const int* sid, int ns, const __half* __restrict__ vectors,
                                            const row_map& map, int Drt, const float* fq, float* sdv)
 {
@@ -790,24 +793,24 @@ __device__ __forceinline__ void exact_rows(const int* sid, int ns, const __half*
       row[u] = reinterpret_cast<const uint4*>(row_of<kDealt>(vectors, map, wanted[u] ? id : map.local, D));
     }
     float out[2];
-    exact_pair<kMode>(row, D, sub, fq, out);
+    exact_pair<kMode, kPass>(row, D, sub, fq, out);
 #pragma unroll
     for (int u = 0; u < 2; u++)
       if (wanted[u] && sub == 0) sdv[j[u]] = out[u];
   }
 }
 
-template <bool kDealt>
+template <bool kDealt, bool kPass>
 __device__ __forceinline__ void exact_distances(const int* sid, int ns, const __half* __restrict__ vectors,
                                                 const row_map& map, int D, const float* fq, float* sdv)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (D == 128) {
-    exact_rows<kDealt, 2>(sid, ns, vectors, map, D, fq, sdv);
+    exact_rows<kDealt, 2, kPass>(sid, ns, vectors, map, D, fq, sdv);
   } else if ((D & 127) == 0) {
-    exact_rows<kDealt, 1>(sid, ns, vectors, map, D, fq, sdv);
+    exact_rows<kDealt, 1, kPass>(sid, ns, vectors, map, D, fq, sdv);
   } else if ((D & 7) == 0) {
-    exact_rows<kDealt, 0>(sid, ns, vectors, map, D, fq, sdv);
+    exact_rows<kDealt, 0, kPass>(sid, ns, vectors, map, D, fq, sdv);
   } else {
     for (int j = warp; j < ns; j += nw) {
       if (sid[j] < 0) continue;
@@ -1270,7 +1273,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
       block_scan<kThreads>(mine, wsum, reranked);
     }
     tick(4);
-    exact_distances<kDealt>(sid, ns, a.vectors, a.vector_map, a.D, fq, sdv);
+    // (rows of other GPUs do not pass through this cache)
+    if (!kDealt && a.pass_vectors != 0)
+      exact_distances<kDealt, true>(sid, ns, a.vectors, a.vector_map, a.D, fq, sdv);
+    else
+      exact_distances<kDealt, false>(sid, ns, a.vectors, a.vector_map, a.D, fq, sdv);
     tick(5);
   }
   merge_into_kept(pool, sorted, a.P, pb, pd, a.KO, kid, kd, kRows ? ctrl[kValid] : 0, sid, sdv, ns, hist, ctrl,
@@ -1330,7 +1337,7 @@ __global__ void __launch_bounds__(kRoundThreads) final_rerank_kernel(const long 
   }
   int ns = 0;
   block_scan(mine, wsum, ns);
-  exact_distances<true>(sid, ns, vectors, vector_map, D, fq, sdv);
+  exact_distances<true, false>(sid, ns, vectors, vector_map, D, fq, sdv);
   merge_into_kept(pool, sorted, P, bi + static_cast<int64_t>(q) * k, bd + static_cast<int64_t>(q) * k,
                   k, nullptr, nullptr, 0, sid, sdv, ns, hist, ctrl);
   if (stats != nullptr && threadIdx.x == 0) {

@@ -132,6 +132,12 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
     int l2 = 0;
     OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device));
     r.keep_sketch = sketch_bytes > 0 && static_cast<double>(sketch_bytes) <= 0.6 * l2 ? 1 : 0;
+    // One that takes a fifth of it or more is pushed out in part by the fp16 rows, read once or twice a batch,
+    // unless those go first: 64 MB of sketch, 10 000 queries at 384 rows a wave 883 and 874 us a search, 512
+    // rows and three waves 8 666 and 8 528 (waves' scoring 188 and 172 thousand cycles). A smaller sketch
+    // stays anyway, and rows that many queries share are better kept: 13 MB of sketch, rows of 1 920 bytes,
+    // 487 and 532 us.
+    r.pass_vectors = r.keep_sketch != 0 && static_cast<double>(sketch_bytes) >= 0.2 * l2 ? 1 : 0;
   }
 }
 
