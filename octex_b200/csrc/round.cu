@@ -674,15 +674,25 @@ __device__ __forceinline__ void sketch_rows_f32(const int* cand, int n, const si
     cq[4 * b] = q4.x, cq[4 * b + 1] = q4.y, cq[4 * b + 2] = q4.z, cq[4 * b + 3] = q4.w;
   }
   const int rpp = nw * kG;  // rows per step of the block
+  if (n <= 0) return;
+  // The ids of a step come in behind the step before: where they are in global memory they took a third of a
+  // step's time (three waves of 16 384 entries: 178 and 149 thousand cycles of scoring, 8 582 and 8 287 us a
+  // search). The rows a step ahead as well: no faster (8 316).
+  int id[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++)
+    id[u] = cand[min(u * rpp + warp * kG + grp, n - 1)];
   for (int jb = 0; jb < n; jb += 2 * rpp) {
     uint4 w[2];
     int j[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      j[u]         = jb + u * rpp + warp * kG + grp;
-      const int id = cand[min(j[u], n - 1)];
-      w[u] = __ldg(reinterpret_cast<const uint4*>(row_of<kDealt>(sketch, map, id, S)) + subc);
+      j[u] = jb + u * rpp + warp * kG + grp;
+      w[u] = __ldg(reinterpret_cast<const uint4*>(row_of<kDealt>(sketch, map, id[u], S)) + subc);
     }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      id[u] = cand[min(j[u] + 2 * rpp, n - 1)];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       const float d0 = sketch_chunk8(w[u].x, w[u].y, cs, cq);
