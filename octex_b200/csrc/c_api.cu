@@ -633,6 +633,16 @@ cuvsError_t octexB200Fetch(cuvsOctexIndex_t index, const char* name, void* dst, 
       pl = ix.plans.begin()->second;
     }
     const std::string n(name != nullptr ? name : "");
+    if (n == "shapes") {
+      std::lock_guard<std::mutex> lock(pl->mu);
+      const auto shapes = octex_b200::detail::round_shapes(*pl);
+      const auto size   = static_cast<int64_t>(shapes.size() * sizeof(int32_t));
+      if (bytes != nullptr) *bytes = size;
+      if (dst == nullptr) return;
+      OCTEX_EXPECTS(capacity >= size, "octex: the destination is too small");
+      std::memcpy(dst, shapes.data(), size);
+      return;
+    }
     octex_b200::dbuf const* b = nullptr;
     if (n == "y") b = &pl->Y;
     else if (n == "qs") b = &pl->qs;

@@ -183,7 +183,7 @@ struct round_args {
   long long* si = nullptr;  // kept ids [m, KO]
   float* sd = nullptr;      // kept distances [m, KO]
   // sizes of the shared-memory carve-up (host decides)
-  int ht_slots = 0;   // ints of the hash set region (>= largest set used, >= pick_slots)
+  int ht_slots = 0;   // ints of the hash set region (>= largest set used, >= pick_slots, >= kept_slots)
   int cap_slots = 0;  // largest gather hash set (slots)
   int map_words = 0;  // words (a multiple of four) of a bit for every row, which then takes the set's place
   int hash_twelfths = 16;  // slots per 12 gathered entries (host: as sparse as shared memory allows)
@@ -215,6 +215,8 @@ struct round_args {
                                // (a selected id already in the kept list is not read again)
 };
 size_t round_smem_bytes(const round_args& a);
+/// Threads of a query block in a batch of a.m queries.
+int round_threads(const round_args& a);
 void round_lists(const round_args& a, cudaStream_t s);
 void round_rows(const round_args& a, cudaStream_t s);
 /// Opt every round kernel in to `bytes` of dynamic shared memory on the current device.

@@ -47,7 +47,7 @@ enum ctl {
 
 /// Offsets (in 4-byte words) of the regions of a round block's shared memory.
 struct round_layout {
-  int table, cand, dist, pool, sorted, sid, sdv, qv, sc, fq, st, len, hist, wsum, ctrl, kid, kd, kset, words;
+  int table, cand, dist, pool, sorted, sid, sdv, qv, sc, fq, st, len, hist, wsum, ctrl, kid, kd, words;
   __host__ __device__ explicit round_layout(const round_args& a)
   {
     const int in_smem = a.cand_global == nullptr ? a.nmax : 0;
@@ -59,8 +59,9 @@ struct round_layout {
       return o;
     };
     // Two regions are used twice. The sketch distances are written where the hash set of the gather
-    // was (the set is dead once the ids are collected). The keys of the merge are written where the
-    // candidates were (dead after the selection).
+    // was (the set is dead once the ids are collected), and the small set of kept ids is built there after
+    // them (once the selection has copied out the distances it took). The keys of the merge are written where
+    // the candidates were (dead after the selection).
     const int pool_words = 2 * (a.KO + rm);
     const int sort_words = a.P > 32 ? 4 * a.P : 128;  // 2 P keys, 64 at least (the one-warp sort)
     table  = take(a.ht_slots > in_smem ? a.ht_slots : in_smem);
@@ -82,7 +83,6 @@ struct round_layout {
     ctrl   = take(kCtlWords);
     kid    = take(a.KO);
     kd     = take(a.KO);
-    kset   = take(a.kept_slots);
     words  = at;
   }
 };
@@ -995,14 +995,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // the filter of already kept ids and by the merge
   int* kid  = smem + lay.kid;
   float* kd = reinterpret_cast<float*>(smem + lay.kd);
-  int* kset = smem + lay.kset;
   if constexpr (kRows) {
     for (int i = threadIdx.x; i < a.KO; i += blockDim.x) {
       kid[i] = static_cast<int>(pb[i]);
       kd[i]  = pd[i];
     }
-    for (int i = threadIdx.x; i < a.kept_slots; i += blockDim.x)
-      kset[i] = -1;
   }
 
   // cycles per phase of this block (observation only): start points / segments, gather, sketch
@@ -1030,11 +1027,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
     if (again)
       for (int i = threadIdx.x; i < a.done_off; i += blockDim.x)
         insert_id(table, a.pick_slots, pdone[i]);
-    for (int i = threadIdx.x; i < a.KO; i += blockDim.x) {
-      const int v = kid[i];
-      insert_id(kset, a.kept_slots, v);
-      if (v >= 0 && (i + 1 == a.KO || kid[i + 1] < 0)) ctrl[kValid] = i + 1;
-    }
+    for (int i = threadIdx.x; i < a.KO; i += blockDim.x)
+      if (kid[i] >= 0 && (i + 1 == a.KO || kid[i + 1] < 0)) ctrl[kValid] = i + 1;
     if (again) __syncthreads();
     const int per       = (a.KO + kThreads - 1) / kThreads;
     const int i0        = threadIdx.x * per;
@@ -1256,6 +1250,18 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   __syncthreads();
 
   tick(3);
+  // The set of kept ids, where the set of the gather was. In a region of its own it is made with the start
+  // points and saves these two barriers, which brings nothing (300 queries of 20 000 rows 82.4 and 81.6 us a
+  // search, 10 000 of a million 869 and 866, apart and here), but can cost blocks: 512 start points x 32 entries 1 174
+  // and 1 032, 128 x 16 with 512 reranked rows of 512 bytes 2 177 and 2 022.
+  if constexpr (kRows) {
+    for (int i = threadIdx.x; i < a.kept_slots; i += kThreads)
+      table[i] = -1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.KO; i += kThreads)
+      insert_id(table, a.kept_slots, kid[i]);
+    __syncthreads();
+  }
   // A selected id that is already in the kept list brings the key it already has there: drop it
   // before the vectors are read (the reference reranks it again and collapses the equal keys). Every row
   // about to be read is asked for at once (128-byte lines into L2), so the distance loop below finds
@@ -1265,7 +1271,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   const bool ahead    = !a.sketch_rank && row_bytes <= kAheadBytes && may_prefetch<kDealt>(a.vector_map);
   for (int r = threadIdx.x; r < ns; r += blockDim.x) {
     const int v = sid[r];
-    if (kRows && holds_id(kset, a.kept_slots, v)) {
+    if (kRows && holds_id(table, a.kept_slots, v)) {
       sid[r] = -1;
     } else if (ahead) {
       const char* row = reinterpret_cast<const char*>(a.vectors + static_cast<int64_t>(v) * a.D);
@@ -1414,6 +1420,21 @@ __global__ void merge_kept_kernel(const long long* __restrict__ src_i,
 
 size_t round_smem_bytes(const round_args& a) { return sizeof(int) * round_layout(a).words; }
 
+/// Threads per query block. A multiprocessor runs 1024 threads of this kernel whatever the block size
+/// (64 registers each): a.threads makes the most of the blocks its shared memory holds. A batch of
+/// fewer blocks than the multiprocessors can hold at once is a matter of latency: its blocks get as
+/// many threads as still run side by side. us a search, with that and with a.threads: 1 query of 64 copies
+/// 64 and 81, 300 queries 91 and 105, 592 100 and 107, from 800 on the same; 100 queries with 256 start
+/// points 180 and 226. Rounds of a few hundred entries lose to the wider barriers (one query of 8 copies x
+/// 8 entries: 59 and 54).
+int round_threads(const round_args& a)
+{
+  int threads = a.threads;
+  while (threads < 1024 && static_cast<int64_t>(a.m) * threads * 2 <= int64_t{1024} * a.sms)
+    threads *= 2;
+  return threads;
+}
+
 namespace {
 
 /// Launch that may begin while the kernel before it in the stream is finishing; the kernel waits for
@@ -1437,21 +1458,6 @@ void launch_overlapped(bool early, void (*kernel)(P...), unsigned grid, unsigned
   cfg.attrs                                     = &at;
   cfg.numAttrs                                  = 1;
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
-
-/// Threads per query block. A multiprocessor runs 1024 threads of this kernel whatever the block size
-/// (64 registers each): a.threads makes the most of the blocks its shared memory holds. A batch of
-/// fewer blocks than the multiprocessors can hold at once is a matter of latency: its blocks get as
-/// many threads as still run side by side. us a search, with that and with a.threads: 1 query of 64 copies
-/// 64 and 81, 300 queries 91 and 105, 592 100 and 107, from 800 on the same; 100 queries with 256 start
-/// points 180 and 226. Rounds of a few hundred entries lose to the wider barriers (one query of 8 copies x
-/// 8 entries: 59 and 54).
-int round_threads(const round_args& a)
-{
-  int threads = a.threads;
-  while (threads < 1024 && static_cast<int64_t>(a.m) * threads * 2 <= int64_t{1024} * a.sms)
-    threads *= 2;
-  return threads;
 }
 
 template <bool kRows, bool kDealt, int kThreads>

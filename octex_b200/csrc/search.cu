@@ -49,6 +49,9 @@ auto map_of(index_impl const& ix, dealt_rows const& d) -> kernels::row_map
 constexpr size_t kSmemSoftLimit = size_t{96} << 10;   // above this the candidates go to global memory
 constexpr size_t kSmemHardLimit = size_t{227} << 10;  // shared memory a block can opt in to
 
+/// Blocks of a multiprocessor, by shared memory (1 KB per block is the system's).
+auto blocks_of(kernels::round_args const& r) -> size_t { return (size_t{228} << 10) / (kernels::round_smem_bytes(r) + 1024); }
+
 /// Fill the size fields of a round and decide where its candidate arrays live.
 void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, int pick_entries, int device,
                 int64_t sketch_bytes, int64_t rows)
@@ -77,7 +80,7 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
   for (int twelfths : {24, 18, 16}) {
     r.hash_twelfths = twelfths;
     r.cap_slots = kernels::hash_slots_of(std::min(entries_max, kernels::kMaxHash), kernels::kMaxHash, twelfths);
-    r.ht_slots  = std::max(r.cap_slots, r.pick_slots);
+    r.ht_slots  = std::max({r.cap_slots, r.pick_slots, r.kept_slots});
     if (kernels::round_smem_bytes(r) <= kEightBlocks) break;
   }
   // placeholders: non-null makes the layout drop the two arrays; the real buffers follow
@@ -88,7 +91,7 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
       r.cand_global = reinterpret_cast<int*>(1);
       r.dist_global = reinterpret_cast<float*>(1);
     }
-    return (size_t{228} << 10) / (kernels::round_smem_bytes(r) + 1024);  // blocks of a multiprocessor
+    return blocks_of(r);
   };
   // A bit for every row of the index instead of the set, where that takes no more room, or where the set
   // leaves a multiprocessor one block anyway: one exchange an entry, and no way to a free slot.
@@ -100,7 +103,7 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
   const int words     = static_cast<int>(std::min<int64_t>((rows + 127) / 128 * 4, 1 << 20));
   if (words <= slots || blocks < 2) {
     r.map_words = words;
-    r.ht_slots  = std::max({words, r.pick_slots, slots >= r.nmax ? r.nmax : 0});
+    r.ht_slots  = std::max({words, r.pick_slots, r.kept_slots, slots >= r.nmax ? r.nmax : 0});
     settle();
     if (r.ht_slots > slots && kernels::round_smem_bytes(r) > kSmemHardLimit) {
       r.map_words = 0;
@@ -123,9 +126,8 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
   pl.smem_max = std::max(pl.smem_max, kernels::round_smem_bytes(r));
   // threads per block: a multiprocessor runs 1024 threads of this kernel (64 registers each); when
   // fewer than eight blocks fit its shared memory, the blocks get more threads to make up for it
-  const size_t per_block = kernels::round_smem_bytes(r) + 1024;
-  const int held         = static_cast<int>(std::max<size_t>((size_t{228} << 10) / per_block, 1));
-  r.threads              = held >= 8 ? 128 : held >= 4 ? 256 : held >= 2 ? 512 : 1024;
+  const size_t held = blocks_of(r);
+  r.threads         = held >= 8 ? 128 : held >= 4 ? 256 : held >= 2 ? 512 : 1024;
   OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, device));
   {
     // the sketch stays in the L2 cache when it and its constants take at most 60 % of it
@@ -166,6 +168,21 @@ void check_tc(plan const& pl)
   *pl.tc_error_host = 0;
   throw error("octex: the projection gave up waiting for data it had asked for (code " + std::to_string(code) +
               "); the results of that batch are not valid");
+}
+
+auto round_shapes(plan const& pl) -> std::vector<int32_t>
+{
+  std::vector<int32_t> out;
+  for (auto const* r : {&pl.r1, &pl.r2}) {
+    const bool any = r == &pl.r1 || pl.sp.waves > 0;
+    const auto put = [&](int64_t v) { out.push_back(any ? static_cast<int32_t>(v) : 0); };
+    put(any ? kernels::round_threads(*r) : 0);
+    put(any ? blocks_of(*r) : 0);
+    put(r->map_words > 0 ? 0 : r->cap_slots);
+    put(r->map_words);
+    put(r->cand_global != nullptr);
+  }
+  return out;
 }
 
 /// Where a batch's queries are and its results go (device-accessible memory).

@@ -20,6 +20,18 @@ def against_checker(oracle, idx, arrays, meta, queries, k, **kw):
         assert np.array_equal(dist.view(np.uint32), want_dist.view(np.uint32)), (len(queries), kw)
 
 
+def shapes(idx):
+    """Of the last batch's first round and waves: threads of a block, blocks of a multiprocessor, slots of the
+    gather's set, words of its bits, candidates in global memory."""
+    return idx.fetch("shapes", np.int32, (2, 5)).tolist()
+
+
+def whole_batch(threads):
+    """The fewest queries whose rounds run blocks of `threads` (128 to 512) where their shared memory asks for those."""
+    import torch
+    return 512 * torch.cuda.get_device_properties(0).multi_processor_count // threads + 1
+
+
 @pytest.fixture(scope="module")
 def many_rows(tmp_path_factory):
     """700 000 rows: a bit for each takes 21 876 words, more than most hash sets and fewer than the largest."""
@@ -47,6 +59,21 @@ def many_rows(tmp_path_factory):
 def test_gathered_ids(oracle, many_rows, kw):
     idx, arrays, meta, queries = many_rows
     against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+
+
+@pytest.mark.parametrize("starts,wave_rerank,threads,in_global", [
+    (16, 256, 128, 0), (75, 512, 256, 0), (143, 512, 512, 0), (254, 512, 512, 1)])
+def test_set_of_kept_ids_takes_no_room(oracle, many_rows, starts, wave_rerank, threads, in_global):
+    """300 kept entries and block sizes at which 2 or 4 KB more a block would make fewer and larger blocks, or send
+    the candidates to global memory."""
+    idx, arrays, meta, queries = many_rows
+    kw = dict(read=16, starts=starts, waves=1, rerank=128, wave_rerank=wave_rerank)
+    n = whole_batch(threads)
+    d, i = idx.search(np.resize(queries, (n, queries.shape[1])), 300, **kw)
+    assert shapes(idx)[1][0] == threads and shapes(idx)[1][4] == in_global
+    against_checker(oracle, idx, arrays, meta, queries, 300, **kw)
+    want_d, want_i = idx.search(queries, 300, **kw)
+    assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
 @pytest.mark.parametrize("rows", [511, 512, 513, 8191, 8193])
