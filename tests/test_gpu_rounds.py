@@ -76,6 +76,24 @@ def test_set_of_kept_ids_takes_no_room(oracle, many_rows, starts, wave_rerank, t
     assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
+@pytest.mark.parametrize("threads", [128, 256, 512, 1024])
+@pytest.mark.parametrize("k,kw", [
+    (10, dict(starts=16, waves=3, rerank=16, wave_rerank=16)),    # 16 kept, no more new ones than that: by places
+    (10, dict(starts=16, waves=3, rerank=64, wave_rerank=128)),   # more new ones: ranked, or selected first
+    (100, dict(starts=16, waves=2, rerank=128, wave_rerank=128)), # the first round's 128 sorted, then by places again
+    (100, dict(starts=16, waves=2, rerank=100, wave_rerank=300)),
+])
+def test_merges_at_every_block_size(oracle, many_rows, k, kw, threads):
+    idx, arrays, meta, queries = many_rows
+    kw = dict(read=16, **kw)
+    n = len(queries) if threads == 1024 else whole_batch(threads)
+    against_checker(oracle, idx, arrays, meta, queries, k, **kw)
+    want_d, want_i = idx.search(queries, k, **kw)
+    d, i = idx.search(np.resize(queries, (n, queries.shape[1])), k, **kw)
+    assert [shape[0] for shape in shapes(idx)] == [threads, threads]
+    assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
+
+
 @pytest.mark.parametrize("rows", [511, 512, 513, 8191, 8193])
 def test_rows_around_a_word_of_bits(oracle, rows):
     """Ids up to the last bit of the last word; a bit for every row or a set of as many slots as entries."""
