@@ -48,6 +48,9 @@ auto map_of(index_impl const& ix, dealt_rows const& d) -> kernels::row_map
 
 constexpr size_t kSmemSoftLimit = size_t{96} << 10;   // above this the candidates go to global memory
 constexpr size_t kSmemHardLimit = size_t{227} << 10;  // shared memory a block can opt in to
+// a block above this (1 KB is the system's) gets the whole 228 KB step of a multiprocessor's 256 KB, which
+// leaves the L1 cache 28 KB instead of 60
+constexpr size_t kSmemBelowLastStep = (size_t{196} << 10) - 1024;
 
 /// Blocks of a multiprocessor, by shared memory (1 KB per block is the system's).
 auto blocks_of(kernels::round_args const& r) -> size_t { return (size_t{228} << 10) / (kernels::round_smem_bytes(r) + 1024); }
@@ -95,9 +98,12 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
   };
   // A bit for every row of the index instead of the set, where that takes no more room, or where the set
   // leaves a multiprocessor one block anyway: one exchange an entry, and no way to a free slot.
-  // A million rows, 32 768 entries a query: 121 and 62 thousand cycles of gathers, the search 4 340 and 3 798 us;
-  // 100 003 rows, 8 192 entries, 502 and 487. Where two blocks fit with the set the bits at one block lose what
-  // the blocks do side by side: a million rows, 16 384 entries, 8 670 and 9 605.
+  // us a search, two waves by the set and by bits where these take no more room: 100 003 rows, 8 192 entries 502 and
+  // 487; a million, 32 768 entries ranked by sketch distance, three waves 4 340 and 3 798. One block either way and more
+  // room (19 200 entries; 22 400): a million rows 1 708 and 1 587; 1 695 and 1 575; 1.4 million 1 757 and 1 640. With the
+  // last step of shared memory the bits lose: 32 768 entries, 1.4 million rows 1 771 and 1 869, 1.5 million 1 791 and
+  // 1 903 (ranked by sketch distance 4 019 and 3 927, 4 065 and 4 035). Where two blocks fit with the set the bits at one
+  // lose what the blocks do side by side: a million rows, 16 384 entries, three waves 8 670 and 9 605.
   const size_t blocks = settle();
   const int slots     = r.ht_slots;
   const int words     = static_cast<int>(std::min<int64_t>((rows + 127) / 128 * 4, 1 << 20));
@@ -105,7 +111,7 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
     r.map_words = words;
     r.ht_slots  = std::max({words, r.pick_slots, r.kept_slots, slots >= r.nmax ? r.nmax : 0});
     settle();
-    if (r.ht_slots > slots && kernels::round_smem_bytes(r) > kSmemHardLimit) {
+    if (r.ht_slots > slots && kernels::round_smem_bytes(r) > kSmemBelowLastStep) {
       r.map_words = 0;
       r.ht_slots  = slots;
       settle();

@@ -32,20 +32,33 @@ def whole_batch(threads):
     return 512 * torch.cuda.get_device_properties(0).multi_processor_count // threads + 1
 
 
-@pytest.fixture(scope="module")
-def many_rows(tmp_path_factory):
-    """700 000 rows: a bit for each takes 21 876 words, more than most hash sets and fewer than the largest."""
+def built(path, count, **params):
+    """An index of `count` clustered rows of 32 dimensions made on the GPU, with its arrays for the checker and 60 queries."""
     import torch
     from octex_b200 import index_dir
     g = torch.Generator("cuda").manual_seed(5)
     centers = torch.randn(500, 32, generator=g, device="cuda") * 2
-    rows = centers[torch.randint(500, (700_000,), generator=g, device="cuda")] + torch.randn(700_000, 32, generator=g, device="cuda")
-    path = str(tmp_path_factory.mktemp("many_rows"))
-    octex_b200.build_native(rows, path, copies=8, blocks=2, pca_dims=32, list_len=16, min_cell=4, log_buckets=12,
-                            sketch_width=32, table_len=64, seed=3)
-    idx = octex_b200.load(path, placement="replicate", devices=0)
-    arrays, meta = index_dir.read_index(path)
-    yield idx, arrays, meta, (rows[::9973][:60] + 0.1).cpu().numpy()
+    rows = centers[torch.randint(500, (count,), generator=g, device="cuda")] + torch.randn(count, 32, generator=g, device="cuda")
+    octex_b200.build_native(rows, str(path), blocks=2, pca_dims=32, min_cell=4, log_buckets=12, sketch_width=32,
+                            table_len=64, seed=3, **params)
+    idx = octex_b200.load(str(path), placement="replicate", devices=0)
+    arrays, meta = index_dir.read_index(str(path))
+    return idx, arrays, meta, (rows[::count // 60][:60] + 0.1).cpu().numpy()
+
+
+@pytest.fixture(scope="module")
+def many_rows(tmp_path_factory):
+    """700 000 rows: a bit for each takes 21 876 words, more than most hash sets and fewer than the largest."""
+    idx, *rest = built(tmp_path_factory.mktemp("many_rows"), 700_000, copies=8, list_len=16)
+    yield idx, *rest
+    idx.close()
+
+
+@pytest.fixture(scope="module")
+def more_rows(tmp_path_factory):
+    """1 400 000 rows: a bit for each takes 43 752 words, more than any hash set, and 171 KB."""
+    idx, *rest = built(tmp_path_factory.mktemp("more_rows"), 1_400_000, copies=16, list_len=64)
+    yield idx, *rest
     idx.close()
 
 
@@ -59,6 +72,41 @@ def many_rows(tmp_path_factory):
 def test_gathered_ids(oracle, many_rows, kw):
     idx, arrays, meta, queries = many_rows
     against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+
+
+@pytest.mark.parametrize("starts,wave_rerank,words", [
+    (256, 128, 0),      # the set leaves two blocks
+    (300, 128, 43752),  # it leaves one: bits, below the last step of shared memory
+    (512, 512, 0),      # they would need that
+])
+def test_bits_that_take_more_room(oracle, more_rows, starts, wave_rerank, words):
+    idx, arrays, meta, queries = more_rows
+    kw = dict(read=64, starts=starts, waves=2, rerank=512, wave_rerank=wave_rerank)
+    idx.search(queries, 10, **kw)
+    assert shapes(idx)[1][3] == words
+    against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+
+
+@pytest.mark.parametrize("spare", [0, 1, 64])
+def test_full_set(oracle, more_rows, spare):
+    """A wave that gathers as many ids as its set has slots (32 768 of 512 table rows), none twice but for `spare`."""
+    idx, arrays, meta, queries = more_rows
+    kw = dict(read=64, starts=512, rerank=512, wave_rerank=512)
+    starts = idx.search(queries[7:8], 512, waves=0, **kw)[1][0]
+    assert starts.min() >= 0 and len(set(starts)) == 512
+    ids = np.random.default_rng(3).permutation(len(arrays["vectors"]))[:512 * 64].astype(np.int32)
+    ids[len(ids) - spare:] = ids[:spare]
+    table = np.array(arrays["table"])
+    table[starts] = ids.reshape(512, 64)
+    idx.set_table(table)
+    try:
+        idx.set_debug(stats=True)
+        idx.search(queries[7:8], 10, waves=1, **kw)
+        assert idx.fetch("stats", np.int64, (1, 8))[0, 5] == 512 * 64 - spare and shapes(idx)[1][2:4] == [32768, 0]
+        idx.set_debug()
+        against_checker(oracle, idx, dict(arrays, table=table), meta, queries[:20], 10, waves=1, **kw)
+    finally:
+        idx.set_table(arrays["table"])
 
 
 @pytest.mark.parametrize("starts,wave_rerank,threads,in_global", [
@@ -96,7 +144,7 @@ def test_merges_at_every_block_size(oracle, many_rows, k, kw, threads):
 
 @pytest.mark.parametrize("rows", [511, 512, 513, 8191, 8193])
 def test_rows_around_a_word_of_bits(oracle, rows):
-    """Ids up to the last bit of the last word; a bit for every row or a set of as many slots as entries."""
+    """Ids up to the last bit of the last word, where the set would have 256 to 4 096 slots."""
     from octex_b200 import build_index, synth
     arrays, meta = build_index.build_arrays(synth.plumbing(rows, 32, seed=0), small_params(copies=4, table_len=24), device="cpu")
     idx = octex_b200.attach(arrays, meta, borrow=False)
