@@ -330,9 +330,9 @@ OCTEX_B200_EXPORT cuvsError_t octexB200SetDebug(cuvsOctexIndex_t index, int32_t 
 OCTEX_B200_EXPORT cuvsError_t octexB200SetProjection(cuvsOctexIndex_t index, int32_t ordered);
 /* Copy a named array of the last batch to host memory: "y", "qs", "codes", "seg", "cand1",
  * "cand1_dist", "n1", "kept1_ids", "kept1_dist", "stats", "kept_ids", "kept_dist"; and
- * "shapes", int32 [2, 5], what the first round and a wave of it looked like: threads of a block, blocks of a
+ * "shapes", int32 [2, 6], what the first round and a wave of it looked like: threads of a block, blocks of a
  * multiprocessor by shared memory, slots of the gather's hash set, words of its bits, 1 when the candidates
- * are in global memory. *bytes returns its size; dst may be NULL to ask for the size only. */
+ * are in global memory, 1 when the fp16 rows leave the L2 cache first. *bytes returns its size; dst may be NULL to ask for the size only. */
 OCTEX_B200_EXPORT cuvsError_t octexB200Fetch(cuvsOctexIndex_t index, const char* name, void* dst,
                                              int64_t capacity, int64_t* bytes);
 

@@ -57,7 +57,7 @@ auto blocks_of(kernels::round_args const& r) -> size_t { return (size_t{228} << 
 
 /// Fill the size fields of a round and decide where its candidate arrays live.
 void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, int pick_entries, int device,
-                int64_t sketch_bytes, int64_t rows)
+                int64_t sketch_bytes, int64_t rows, bool vectors_here)
 {
   r.pick_slots = 0;
   if (pick_entries > 0) {
@@ -140,12 +140,15 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
     int l2 = 0;
     OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device));
     r.keep_sketch = sketch_bytes > 0 && static_cast<double>(sketch_bytes) <= 0.6 * l2 ? 1 : 0;
-    // One that takes a fifth of it or more is pushed out in part by the fp16 rows, read once or twice a batch,
-    // unless those go first: 64 MB of sketch, 10 000 queries at 384 rows a wave 883 and 874 us a search, 512
-    // rows and three waves 8 666 and 8 528 (waves' scoring 188 and 172 thousand cycles). A smaller sketch
-    // stays anyway, and rows that many queries share are better kept: 13 MB of sketch, rows of 1 920 bytes,
-    // 487 and 532 us.
-    r.pass_vectors = r.keep_sketch != 0 && static_cast<double>(sketch_bytes) >= 0.2 * l2 ? 1 : 0;
+    // One that takes a quarter of it or more is pushed out in part by the fp16 rows, read once or twice a batch,
+    // unless those go first. us a search with the rows as others and first, 10 000 queries at 384 rows a wave and
+    // 2 000 at 512 and three waves: 68 MB of sketch 1 093 and 1 075, 1 896 and 1 839; 36 MB 924 and 920, 1 328 and 1 289; 34 MB
+    // 1 016 and 1 020, 1 446 and 1 434. A smaller sketch stays anyway, and rows that many queries share are better
+    // kept: 31 MB 1 036 and 1 045, 1 445 and 1 436; 27 MB 1 001 and 1 008, 1 405 and 1 397; 13 MB, rows of 1 920 bytes
+    // 2 184 and 2 308, 1 156 and 1 180. (Rows that wide lose above the line too where the data has few clusters, and with
+    // default parameters win: 53 MB 2 612 and 2 648, 2 001 and 2 025, 513 and 497.) Rows in host memory come over the
+    // bus and are kept at any size: 2 000 queries of 400 000 x 96 4 682 and 4 957.
+    r.pass_vectors = vectors_here && r.keep_sketch != 0 && static_cast<double>(sketch_bytes) >= 0.25 * l2 ? 1 : 0;
   }
 }
 
@@ -187,6 +190,7 @@ auto round_shapes(plan const& pl) -> std::vector<int32_t>
     put(r->map_words > 0 ? 0 : r->cap_slots);
     put(r->map_words);
     put(r->cand_global != nullptr);
+    put(r->pass_vectors);
   }
   return out;
 }
@@ -600,7 +604,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   }
   // sketch rows of this GPU's own memory (not the host tier, not dealt over GPUs) plus their constants
   const int64_t sketch_bytes = (p.sketch.host || p.sketch_rows.on) ? 0 : static_cast<int64_t>(p.sketch.size + p.sketch_norm.size);
-  size_round(pl, r1, p.copies * pl.lr, false, 0, p.device, sketch_bytes, ix.n);
+  size_round(pl, r1, p.copies * pl.lr, false, 0, p.device, sketch_bytes, ix.n, !p.vectors.host);
   // waves: table rows of the start points
   if (sp.waves > 0) {
     auto& r2       = pl.r2;
@@ -629,7 +633,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
     r2.sd          = pl.wsd;
     r2.stats       = r1.stats;
     r2.phase       = pl.phase2.as<long long>();
-    size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes, ix.n);
+    size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes, ix.n, !p.vectors.host);
   }
   kernels::round_allow_smem(pl.smem_max);
 

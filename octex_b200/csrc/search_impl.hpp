@@ -89,9 +89,10 @@ auto search_in_place(index_impl const& ix, const float* queries, const int64_t* 
 auto profile_batch(resources const& res, search_params const& sp, index const& idx, int64_t nq,
                    int64_t k) -> std::vector<float>;
 
-/// What the rounds of the plan's last batch looked like, five numbers for the first round and five for a wave
+/// What the rounds of the plan's last batch looked like, six numbers for the first round and six for a wave
 /// (zeros without one): threads of a block, blocks of a multiprocessor by shared memory, slots of the
-/// gather's hash set, words of its bits (0: the set), 1 when the candidates are in global memory.
+/// gather's hash set, words of its bits (0: the set), 1 when the candidates are in global memory, 1 when the
+/// fp16 rows leave the L2 cache first.
 auto round_shapes(plan const& pl) -> std::vector<int32_t>;
 
 /// Throws when a kernel of an earlier batch of this plan reported that it gave up (and clears the

@@ -22,8 +22,8 @@ def against_checker(oracle, idx, arrays, meta, queries, k, **kw):
 
 def shapes(idx):
     """Of the last batch's first round and waves: threads of a block, blocks of a multiprocessor, slots of the
-    gather's set, words of its bits, candidates in global memory."""
-    return idx.fetch("shapes", np.int32, (2, 5)).tolist()
+    gather's set, words of its bits, candidates in global memory, fp16 rows leave the L2 cache first."""
+    return idx.fetch("shapes", np.int32, (2, 6)).tolist()
 
 
 def whole_batch(threads):
@@ -85,6 +85,21 @@ def test_bits_that_take_more_room(oracle, more_rows, starts, wave_rerank, words)
     idx.search(queries, 10, **kw)
     assert shapes(idx)[1][3] == words
     against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+
+
+def test_rows_that_leave_the_cache_first(oracle, many_rows, more_rows):
+    """With a sketch of 50 MB, a quarter of the L2 cache, but not of 25 MB, nor when the rows are in host memory."""
+    kw = dict(read=16, starts=32, waves=2, rerank=100, wave_rerank=65)
+    for (idx, arrays, meta, queries), first in ((many_rows, 0), (more_rows, 1)):
+        idx.search(queries, 10, **kw)
+        assert [shape[5] for shape in shapes(idx)] == [first, first]
+        against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+    idx, arrays, meta, queries = more_rows
+    far = octex_b200.load(idx.path, placement="replicate", devices=0, vectors_on_host=True)
+    got, want = far.search(queries, 10, **kw), idx.search(queries, 10, **kw)
+    assert [shape[5] for shape in shapes(far)] == [0, 0]
+    assert np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])
+    far.close()
 
 
 @pytest.mark.parametrize("spare", [0, 1, 64])
