@@ -62,16 +62,25 @@ def more_rows(tmp_path_factory):
     idx.close()
 
 
-@pytest.mark.parametrize("kw", [
-    dict(read=16, starts=16, waves=2, rerank=64, wave_rerank=64),            # eight blocks a multiprocessor
-    dict(read=16, starts=96, waves=2, rerank=64, wave_rerank=128),           # four
-    dict(read=16, starts=256, waves=2, rerank=128, wave_rerank=512),         # two, the hash set three quarters full at most
-    dict(read=16, starts=300, waves=2, rerank=128, wave_rerank=512),         # one, bits
-    dict(read=16, starts=512, waves=2, sketch_rank=True, final_rerank=32),   # one, bits, distances over them
+@pytest.mark.parametrize("kw,threads,slots,words", [
+    (dict(starts=16, rerank=64, wave_rerank=64), 128, 2048, 0),                   # half full at most
+    (dict(starts=64, rerank=64, wave_rerank=64), 256, 5464, 0),                   # three quarters
+    (dict(starts=96, rerank=64, wave_rerank=128), 512, 8192, 0),
+    (dict(starts=256, rerank=128, wave_rerank=512), 512, 21848, 0),               # candidates in global memory
+    (dict(starts=300, rerank=128, wave_rerank=512), 512, 0, 21876),               # bits, two blocks
+    (dict(starts=400, rerank=128, wave_rerank=512), 1024, 0, 21876),              # bits, one
+    (dict(starts=512, sketch_rank=True, final_rerank=32), 1024, 0, 21876),        # distances over the bits
 ])
-def test_gathered_ids(oracle, many_rows, kw):
+def test_gathered_ids(oracle, many_rows, kw, threads, slots, words):
+    """Every form of the set of gathered ids in blocks of the size a whole batch has, and of 1 024 threads."""
     idx, arrays, meta, queries = many_rows
+    kw = dict(read=16, waves=2, **kw)
     against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+    want_d, want_i = idx.search(queries, 10, **kw)
+    n = len(queries) if threads == 1024 else whole_batch(threads)
+    d, i = idx.search(np.resize(queries, (n, queries.shape[1])), 10, **kw)
+    assert [shapes(idx)[1][f] for f in (0, 2, 3)] == [threads, slots, words]
+    assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
 @pytest.mark.parametrize("starts,wave_rerank,words", [
@@ -171,8 +180,7 @@ def test_rows_around_a_word_of_bits(oracle, rows):
 
 @pytest.mark.parametrize("distinct", [1, 3, 40, 4000])
 def test_selection_among_equal_distances(oracle, distinct):
-    """Rows that repeat: the bin of the last selected key holds any number of keys, more than are ranked
-    aside (128) and all of them among these."""
+    """Rows that repeat: fewer candidates than are selected, or a few equal ones at the cut."""
     from octex_b200 import build_index, synth
     rng = np.random.default_rng(2)
     base = synth.plumbing(distinct, 48, seed=0)[rng.integers(0, distinct, 4000)]
@@ -181,4 +189,44 @@ def test_selection_among_equal_distances(oracle, distinct):
     queries = synth.plumbing(40, 48, seed=1)
     for kw in (dict(read=16, starts=64, waves=2, rerank=40, wave_rerank=200), dict(read=16, starts=64, waves=1, sketch_rank=True)):
         against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+    idx.close()
+
+
+@pytest.mark.parametrize("threads", [128, 1024])
+@pytest.mark.parametrize("near", [40, 200])
+@pytest.mark.parametrize("members", [1, 127, 128, 129, 300])
+def test_members_of_the_bin_at_the_cut(oracle, members, near, threads):
+    """A wave over table rows made by hand: `near` ids of equal rows, `members` of others, the rest of a third kind, and
+    the cut of the selection inside the second kind: up to 128 are ranked aside, for more the threshold is found
+    digit by digit. Blocks of 128 threads select in the merge too where more than 256 keys meet (200 near
+    ones and 127 members or more), 65 of them, all at the same distance."""
+    from octex_b200 import build_index, synth
+    rng = np.random.default_rng(2)
+    base = synth.plumbing(3000, 48, seed=0)
+    kinds = [np.arange(i, 2700, 3) for i in range(3)]
+    for i in range(3):
+        base[kinds[i]] = base[2700 + i]
+    query = (base[:1] + 0.05).astype(np.float32)
+    arrays, meta = build_index.build_arrays(base, small_params(table_len=32), device="cpu")
+    sketched = (query - arrays["mean"]).astype(np.float64) @ np.asarray(arrays["sketch_basis"], np.float64).reshape(48, -1)
+    apart = ((arrays["sketch"] * np.asarray(arrays["sketch_scale"], np.float64) - sketched) ** 2).sum(1)
+    kinds.sort(key=lambda of: apart[of[0]])
+    bits = np.float32([apart[of[0]] for of in kinds]).view(np.uint32).astype(np.int64)
+    shift = max(int(bits[2] - bits[0]).bit_length() - 8, 0)
+    assert 1 < (bits[1] - bits[0]) >> shift < ((bits[2] - bits[0]) >> shift) - 1  # bins of their own
+
+    kw = dict(read=16, starts=16, rerank=64, wave_rerank=near + (members + 1) // 2)
+    idx = octex_b200.attach(arrays, meta, borrow=False)
+    starts = idx.search(query, 65, waves=0, **kw)[1][0, :16]  # 65: more than the first round finds or reranks
+    assert starts.min() >= 0
+    ids = np.concatenate([rng.permutation(of)[:count] for of, count in zip(kinds, (near, members, 512 - near - members))])
+    table = np.array(arrays["table"])
+    table[starts] = rng.permutation(ids).astype(np.int32).reshape(16, 32)
+    idx.set_table(table)
+    n = 3 if threads == 1024 else whole_batch(threads)
+    idx.set_debug(stats=True)
+    idx.search(np.repeat(query, n, axis=0), 65, waves=1, **kw)
+    assert shapes(idx)[1][0] == threads and (idx.fetch("stats", np.int64, (n, 8))[:, 5] == 512).all()
+    idx.set_debug()
+    against_checker(oracle, idx, dict(arrays, table=table), meta, np.repeat(query, n, axis=0), 65, waves=1, **kw)
     idx.close()
