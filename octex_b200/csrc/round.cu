@@ -881,17 +881,19 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
   const int total = nk + ctrl[kMerged];
   const int cnt   = min(total, KO);
   // New keys that fit behind the kept ones go to their places among them. Other short lists are sorted by ranking,
-  // at most kRankSteps comparisons a thread; a block of 128 threads, of which many share a multiprocessor, rather
-  // selects first where KO keys are few of the total. us a search where the places were left to the ranking
-  // whenever that was short enough, and now: 1 000 queries with 128 kept and 128 reranked rows 340 and 330, 10 000 2 404
-  // and 2 322, 4 000 wide rows with 256 1 631 and 1 590. Limits of 32, 128 and 512 comparisons: one query with
-  // 256 reranked rows 91.5, 89.3 and 89.8, 148 with 512 172, 169 and 186, elsewhere alike.
+  // at most kRankSteps comparisons a thread, and a quarter of that where KO keys are few of the total, which are
+  // rather selected first (always in a block of 128 threads, of which many share a multiprocessor). us a search:
+  // where the places were left to the ranking whenever that was short enough, and now, 1 000 queries with 128 kept
+  // and 128 reranked rows 340 and 330, 10 000 2 404 and 2 322, 4 000 wide rows with 256 1 631 and 1 590. Limits of 32,
+  // 128 and 512 comparisons: one query with 256 kept and 256 reranked rows 91.5, 89.3 and 89.8, 148 with 512 172, 169
+  // and 186. The quarter, at 32 kept of 300 to 512 reranked rows: 55 queries 126.9 and 123.5, 296 135.6 and
+  // 131.5; at 32 of 128 one query takes 66 when it selects first and 63.
   constexpr int kRankSteps = 128;
   const int threads        = blockDim.x;
-  const auto few           = [&](int keys) { return keys <= threads && keys * keys <= kRankSteps * threads; };
+  const auto few           = [&](int keys, int steps) { return keys <= threads && keys * keys <= steps * threads; };
   if (nk > 0 && total - nk <= P) {
     merge_sorted(pool, nk, pool + nk, total - nk, sorted + P, KO, sorted);
-  } else if (few(total) && (total <= 2 * P || threads > kRoundThreads)) {
+  } else if (total <= 2 * P ? few(total, kRankSteps) : threads > kRoundThreads && few(total, kRankSteps / 4)) {
     rank_sort(pool, total, sorted, KO);
   } else if (total <= 2 * P) {
     int width = P;
@@ -914,7 +916,7 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
       if (s < P) picked[s] = (static_cast<unsigned long long>(high) << 32) | low;
     });
     __syncthreads();
-    if (few(KO)) {
+    if (few(KO, kRankSteps)) {
       rank_sort(picked, KO, sorted, KO);
     } else {
       for (int i = threadIdx.x; i < P; i += blockDim.x)

@@ -166,6 +166,20 @@ def test_merges_at_every_block_size(oracle, many_rows, k, kw, threads):
     assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
+@pytest.mark.parametrize("threads,rerank", [(128, 32), (128, 33), (256, 90), (256, 91), (512, 128), (512, 129), (1024, 181), (1024, 182)])
+def test_first_merges_around_the_ranking(oracle, more_rows, threads, rerank):
+    """Sixteen kept of a first round's reranked rows: ranked up to rerank^2 = 32 threads (128 threads: sorted up to 32),
+    selected first beyond."""
+    idx, arrays, meta, queries = more_rows
+    kw = dict(read=64, starts=16, waves=1, rerank=rerank, wave_rerank=64)
+    n = len(queries) if threads == 1024 else whole_batch(threads)
+    against_checker(oracle, idx, arrays, meta, queries, 10, **kw)
+    want_d, want_i = idx.search(queries, 10, **kw)
+    d, i = idx.search(np.resize(queries, (n, queries.shape[1])), 10, **kw)
+    assert shapes(idx)[0][0] == threads
+    assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
+
+
 @pytest.mark.parametrize("rows", [511, 512, 513, 8191, 8193])
 def test_rows_around_a_word_of_bits(oracle, rows):
     """Ids up to the last bit of the last word, where the set would have 256 to 4 096 slots."""
