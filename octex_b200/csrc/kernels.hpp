@@ -16,6 +16,11 @@ constexpr int kMaxSketchKO = 1024;   // kept entries when ranking by sketch
 constexpr int kMaxExpanded = 6144;   // start points expanded by earlier waves
 constexpr int kRoundThreads = 128;  // threads of a query block unless its shared memory asks for more
 
+/// Shared memory a block can opt in to. Kernels whose need varies are opted in to all of it: the opt-in belongs to
+/// the kernel and the device, not to a launch, and one for less would take it from another plan, call or
+/// thread that needs more.
+constexpr int kMaxBlockSmem = 227 << 10;
+
 /// Slots of the hash set that collects `total` entries: twelfths / 12 slots per entry (24 = half
 /// full at most, 16 = three quarters), a multiple of four, between kMinHash and cap. (The reference,
 /// search_kernels.cuh:33-38, takes a power of two at most two thirds full; only the memory taken and
@@ -31,7 +36,7 @@ __host__ __device__ inline int hash_slots_of(int total, int cap, int twelfths)
 void pad_rows(float* q, int from, int m, int D, cudaStream_t s);
 
 /// Largest dimension center_sketch takes: its block keeps 16 centred rows in shared memory.
-constexpr int kMaxDim = (227 << 10) / (16 * 4);
+constexpr int kMaxDim = kMaxBlockSmem / (16 * 4);
 
 /// qh [m, ldq] = half(q - mean) zero-padded to ldq columns; qs [m, S] = (q - mean) @ basis in fp32
 /// (one fused multiply-add per dimension, in dimension order).
@@ -219,8 +224,8 @@ size_t round_smem_bytes(const round_args& a);
 int round_threads(const round_args& a);
 void round_lists(const round_args& a, cudaStream_t s);
 void round_rows(const round_args& a, cudaStream_t s);
-/// Opt every round kernel in to `bytes` of dynamic shared memory on the current device.
-void round_allow_smem(size_t bytes);
+/// Opt every round kernel in to kMaxBlockSmem bytes of dynamic shared memory on the current device.
+void round_allow_smem();
 
 /// bi, bd [m, k] = the first k columns of si, sd [m, KO].
 void take_k(const long long* si, const float* sd, int KO, int k, int m, long long* bi, float* bd,

@@ -601,7 +601,7 @@ void knn_tc(const __half* x, const float* norm, int64_t n, int D, int K, int64_t
   const knn_shape shape = choose_shape(nkb);
   const size_t smem     = shape.smem_bytes(nkb);
   const auto kernel     = K <= 32 ? knn_tc_kernel<1> : K <= 64 ? knn_tc_kernel<2> : knn_tc_kernel<4>;
-  cudaError_t status    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t status    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
   int dev = 0, sms = 1;
   if (status == cudaSuccess) status = cudaGetDevice(&dev);
   if (status == cudaSuccess) status = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -1480,12 +1480,12 @@ void launch_round(const round_args& a, cudaStream_t s)
   }
 }
 template <bool kRows, bool kDealt>
-void allow_smem(int b)
+void allow_smem()
 {
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
 }
 bool dealt(const round_args& a)
 {
@@ -1493,13 +1493,12 @@ bool dealt(const round_args& a)
 }
 }  // namespace
 
-void round_allow_smem(size_t bytes)
+void round_allow_smem()
 {
-  const int b = static_cast<int>(bytes);
-  allow_smem<false, false>(b);
-  allow_smem<true, false>(b);
-  allow_smem<false, true>(b);
-  allow_smem<true, true>(b);
+  allow_smem<false, false>();
+  allow_smem<true, false>();
+  allow_smem<false, true>();
+  allow_smem<true, true>();
 }
 
 void round_lists(const round_args& a, cudaStream_t s)

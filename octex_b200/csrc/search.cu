@@ -47,7 +47,7 @@ auto map_of(index_impl const& ix, dealt_rows const& d) -> kernels::row_map
 }
 
 constexpr size_t kSmemSoftLimit = size_t{96} << 10;   // above this the candidates go to global memory
-constexpr size_t kSmemHardLimit = size_t{227} << 10;  // shared memory a block can opt in to
+constexpr size_t kSmemHardLimit = kernels::kMaxBlockSmem;
 // a block above this (1 KB is the system's) gets the whole 228 KB step of a multiprocessor's 256 KB, which
 // leaves the L1 cache 28 KB instead of 60
 constexpr size_t kSmemBelowLastStep = (size_t{196} << 10) - 1024;
@@ -129,7 +129,6 @@ void size_round(plan& pl, kernels::round_args& r, int entries_max, bool waves, i
       r.dist_global = pl.scratch_dist.back().as<float>();
     }
   }
-  pl.smem_max = std::max(pl.smem_max, kernels::round_smem_bytes(r));
   // threads per block: a multiprocessor runs 1024 threads of this kernel (64 registers each); when
   // fewer than eight blocks fit its shared memory, the blocks get more threads to make up for it
   const size_t held = blocks_of(r);
@@ -635,7 +634,7 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
     r2.phase       = pl.phase2.as<long long>();
     size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes, ix.n, !p.vectors.host);
   }
-  kernels::round_allow_smem(pl.smem_max);
+  kernels::round_allow_smem();
 
   OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.done_ev, cudaEventDisableTiming));
   OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.join_ev, cudaEventDisableTiming));

@@ -43,7 +43,6 @@ struct plan {
   int tap_cap = 0;
   std::vector<dbuf> scratch_cand, scratch_dist;
   kernels::round_args r1, r2;
-  size_t smem_max       = 0;
   cudaGraphExec_t graph = nullptr;  // of a batch of graph_m queries in the plan's own buffers
   int graph_m           = 0;
   cudaEvent_t done_ev   = nullptr;  // the end of the plan's last batch

@@ -180,6 +180,16 @@ def test_first_merges_around_the_ranking(oracle, more_rows, threads, rerank):
     assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
+def test_plans_of_several_indexes(many_rows, more_rows):
+    """Two indexes searched in turn, each with a plan of its own size."""
+    (one, _, _, queries), (other, _, _, others) = many_rows, more_rows
+    large, small = dict(read=16, starts=256, waves=1, wave_rerank=512), dict(read=16, starts=16, waves=1, wave_rerank=16)
+    want = one.search(queries, 10, **large), other.search(others, 10, **small)
+    for _ in range(2):
+        for got, ref in ((one.search(queries, 10, **large), want[0]), (other.search(others, 10, **small), want[1])):
+            assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
+
+
 @pytest.mark.parametrize("rows", [511, 512, 513, 8191, 8193])
 def test_rows_around_a_word_of_bits(oracle, rows):
     """Ids up to the last bit of the last word, where the set would have 256 to 4 096 slots."""
