@@ -385,21 +385,30 @@ __device__ __forceinline__ void take_smallest(HiAt hi_at, LoAt lo_at, int n, int
 
 /// The `want` smallest of cnt distinct keys src[0, cnt) into dst (another array), ascending: a group of
 /// lanes counts the keys below its own and puts it there. No step depends on another, which suits the
-/// short lists a merge usually sorts better than a sorting network run by one warp. cnt <= blockDim.x.
+/// short lists a merge usually sorts better than a sorting network run by one warp. A lane counts eight keys at
+/// least: with 32 lanes for each of 32 keys a merge of 1 024 threads took 3.3 thousand cycles, with four 2.8. One
+/// lane a key has a loop of its own, which reads two keys a load: 7 499 queries whose first round keeps 128 of
+/// 128 keys 303 us without it, 293 with it; 10 000 with default parameters 2 322 and 2 277. cnt <= blockDim.x.
 __device__ __forceinline__ void rank_sort(const unsigned long long* src, int cnt, unsigned long long* dst, int want)
 {
   int lanes = 1;  // per key
-  while (lanes < 32 && 2 * lanes * cnt <= static_cast<int>(blockDim.x))
+  while (cnt > 8 * lanes && 2 * lanes * cnt <= static_cast<int>(blockDim.x))
     lanes *= 2;
   const int at = threadIdx.x / lanes, sub = threadIdx.x & (lanes - 1);
   if ((threadIdx.x & ~31u) / lanes >= static_cast<unsigned>(cnt)) return;  // a warp without a key
   const unsigned long long mine = src[min(at, cnt - 1)];
   int below                     = 0;
+  if (lanes == 1) {
+#pragma unroll 8
+    for (int j = 0; j < cnt; j++)
+      below += src[j] < mine;
+  } else {
 #pragma unroll 4
-  for (int j = sub; j < cnt; j += lanes)
-    below += src[j] < mine;
-  for (int o = 1; o < lanes; o <<= 1)
-    below += __shfl_xor_sync(0xffffffffu, below, o);
+    for (int j = sub; j < cnt; j += lanes)
+      below += src[j] < mine;
+    for (int o = 1; o < lanes; o <<= 1)
+      below += __shfl_xor_sync(0xffffffffu, below, o);
+  }
   if (sub == 0 && at < cnt && below < want) dst[below] = mine;
 }
 
