@@ -531,9 +531,10 @@ __device__ __forceinline__ void sketch_query_setup(const float* __restrict__ qs,
 // The int8 sketch and its row constants are the arrays every query reads most often (hundreds of
 // rows per round) and, for an index of a million rows, small enough to stay in the 126 MB L2 cache
 // next to everything else; the fp16 vectors, the lists and the neighbor table are read once or a
-// few times per batch and are many times larger. When the host finds that the sketch fits, the
-// kernels load sketch rows and constants with an evict-last policy and the large arrays with an
-// evict-first policy, so that the streaming reads do not push the sketch out.
+// few times per batch and are many times larger. When the host finds that the sketch fits
+// (keep_sketch), the first round loads sketch rows and constants with an evict-last policy, and every
+// round the lists and the table with an evict-first policy, so that the streaming reads do not push
+// the sketch out; the fp16 rows go first too where a large sketch needs the room (pass_vectors).
 
 __device__ __forceinline__ unsigned long long l2_policy_keep()
 {
@@ -737,6 +738,8 @@ __device__ __forceinline__ void exact_pair(const uint4* const (&row)[2], int Drt
 {
   constexpr bool kWhole = kMode != 0;
   const int D           = kMode == 2 ? 128 : Drt;
+  // (The policy is made at each load: held in two registers over the loop it is no faster at 128 dimensions, 1 074 and
+  // 1 076 us a search, and slower at others: 32 dimensions 920 and 935, 64 1 007 and 1 026, 256 1 472 and 1 487.)
   float acc[2][4];
 #pragma unroll
   for (int u = 0; u < 2; u++)
@@ -1278,8 +1281,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // A selected id that is already in the kept list brings the key it already has there: drop it
   // before the vectors are read (the reference reranks it again and collapses the equal keys). Every row
   // about to be read is asked for at once (128-byte lines into L2), so the distance loop below finds
-  // most of them on the way; not wide rows, of which the loop has enough on the way itself (999 queries, 382 rows of 1 920 bytes
-  // each, a first round: 144 us asked for and 129 not; 10 000 queries, 370 rows of 256 bytes, a wave: 411 and 418).
+  // most of them on the way; not wide rows, of which the loop has enough on the way itself. us a search, asked for and
+  // not, 1 000 queries at 128 rows a round, at 512, and 5 000 at 128 and 384: 512 bytes a row 421 and 425, 723 and 722, 681 and
+  // 682; 768 bytes 421 and 425, 737 and 728, 766 and 753; 1 024 bytes 426 and 432, 759 and 743, 876 and 853; 1 920 bytes 500 and
+  // 502, 992 and 944, 1 360 and 1 265. (64 wide rows a round are the exception, 1 024 bytes 333 and 339, 1 920 393 and 402.)
   const int row_bytes = a.D * 2;
   const bool ahead    = !a.sketch_rank && row_bytes <= kAheadBytes && may_prefetch<kDealt>(a.vector_map);
   for (int r = threadIdx.x; r < ns; r += blockDim.x) {
