@@ -254,6 +254,56 @@ def test_tensor_core_scan_is_exact(n, dim, k, order):
     assert (ids[:, kept:] == -1).all() and torch.isinf(d[:, kept:]).all()
 
 
+@pytest.mark.parametrize("scale", [1e-4, 1.0, 600.0])
+@pytest.mark.parametrize("n,dim,k", [(1500, 64, 20), (2000, 256, 64), (700, 320, 100)])
+def test_tensor_core_scan_of_any_magnitude(n, dim, k, scale):
+    """The scan adds the norms on the tensor cores, in three parts of eight bits. Distances against float64 over rows
+    of small, ordinary and large values (squares up to 1e6 and sums of them beyond fp16, parts down to 2^-30)."""
+    import torch
+    g = torch.Generator("cuda").manual_seed(dim)
+    x = (torch.randn(n, dim, generator=g, device="cuda") * scale).half()
+    ids, d = octex_b200.exact_neighbors(x, k, method="tensor")
+    xd = x.double()
+    sq = (xd * xd).sum(1)
+    full = sq[:, None] + sq[None, :] - 2 * (xd @ xd.T)
+    full.fill_diagonal_(float("inf"))
+    want = full.topk(k, dim=1, largest=False, sorted=True).values
+    # A chain of dim multiply-adds per norm, and dim / 16 + 2 sums of at most |a|^2 + |b|^2: at most half a unit in the
+    # last place each for the former, one for the sums, which the tensor cores may truncate.
+    bound = (2 * sq.max()) * 2.0 ** -24 * (dim + 2 * (dim / 16 + 2))
+    assert (full.gather(1, ids.long()) - d.double()).abs().max() < bound
+    assert (want - d.double()).abs().max() < bound
+
+
+def test_scans_on_two_streams():
+    """Scans of two threads at a time, each on a stream of its own, give what each gives alone: blocks of both take
+    their places for notes from the same memory."""
+    import threading
+
+    import torch
+    g = torch.Generator("cuda").manual_seed(3)
+    rows = [torch.randn(n, 64, generator=g, device="cuda").half() for n in (9001, 20000)]
+    alone = [octex_b200.exact_neighbors(x, 40) for x in rows]
+    got = [[], []]
+
+    def scan(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(4):
+                got[i].append(octex_b200.exact_neighbors(rows[i], 40))
+            torch.cuda.current_stream().synchronize()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=scan, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        assert len(got[i]) == 4
+        for ids, d in got[i]:
+            assert torch.equal(ids, alone[i][0]) and torch.equal(d, alone[i][1])
+
+
 def test_searched_table(built, oracle, tmp_path):
     """The table by the index's own search (octexB200SearchedTable; cuvsOctexBuild above
     exact_table_max), the way the reference checks its own (cpp/tests/test_build.cu, table quality):
