@@ -785,18 +785,19 @@ void exact_neighbors(const __half* x, int64_t n, int D, int K, int method, int32
   OCTEX_EXPECTS(method >= 0 && method <= 2, "octex: exact_neighbors method is 0 (choose), 1 (tensor cores) or 2 (plain)");
   int dev = 0;
   OCTEX_CUDA_TRY(cudaGetDevice(&dev));
-  dbuf norm(dev, sizeof(float) * n);
+  dbuf norm(dev, sizeof(float) * (n + 1));  // and the error word of the scan on the tensor cores
   const auto norms = D % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 ? row_norms_kernel<true> : row_norms_kernel<false>;
   norms<<<grid_for(n, 128), 128, 0, s>>>(x, n, D, norm.as<float>());
   const bool covered = kernels::knn_tc_supported(n, D, K);
   OCTEX_EXPECTS(method != 1 || covered,
                 "octex: the tensor-core neighbor scan needs a dimension that is a multiple of 8 and K <= 122");
   if (method == 1 || (method == 0 && covered)) {
-    dbuf error(dev, sizeof(int));
-    OCTEX_CUDA_TRY(cudaMemsetAsync(error.ptr, 0, sizeof(int), s));
-    kernels::knn_tc(x, norm.as<float>(), n, D, K, 0, n, ids, dist, error.as<int>(), s);
+    int* error = norm.as<int>() + n;
+    OCTEX_CUDA_TRY(cudaMemsetAsync(error, 0, sizeof(int), s));
+    kernels::knn_tc(x, norm.as<float>(), n, D, K, 0, n, ids, dist, error, s);
     OCTEX_CUDA_TRY(cudaPeekAtLastError());
-    const int gave_up = to_host<int>(error.ptr, 1)[0];
+    OCTEX_CUDA_TRY(cudaStreamSynchronize(s));
+    const int gave_up = to_host<int>(error, 1)[0];
     OCTEX_EXPECTS(gave_up == 0, "octex: the neighbor scan gave up waiting inside the kernel (code " +
                                   std::to_string(gave_up) + "); its lists are incomplete");
   } else {
@@ -810,31 +811,60 @@ void exact_neighbors(const __half* x, int64_t n, int D, int K, int method, int32
 
 namespace {
 
+/// Pieces of one block of memory, on 256-byte boundaries.
+struct pieces {
+  char* at;
+  template <typename T>
+  auto take(int64_t count) -> T*
+  {
+    T* p = reinterpret_cast<T*>(at);
+    at += size_of<T>(count);
+    return p;
+  }
+  template <typename T>
+  static auto size_of(int64_t count) -> size_t { return (sizeof(T) * static_cast<size_t>(count) + 255) / 256 * 256; }
+};
+
+/// Bytes the sort of a reverse-edge merge works with.
+auto edge_sort_bytes(int64_t edges) -> size_t
+{
+  size_t tb = 0;
+  unsigned long long* none = nullptr;
+  int32_t* no_rows         = nullptr;
+  cub::DeviceRadixSort::SortPairs(nullptr, tb, none, none, no_rows, no_rows, edges);
+  return tb;
+}
+
+/// Scratch memory of reverse_merge.
+auto reverse_scratch(int64_t n, int ks) -> size_t
+{
+  const int64_t edges = n * ks;
+  return 2 * pieces::size_of<unsigned long long>(edges) + 2 * pieces::size_of<int32_t>(edges) + pieces::size_of<int64_t>(n + 1) +
+         pieces::size_of<char>(static_cast<int64_t>(edge_sort_bytes(edges)));
+}
+
 // Reverse-edge merge of forward rows fwd / fd [n, K] (nearest first, -1 padded) into table rows
 // out [n, k]: every row v proposes itself to the rows among its first ks neighbors, a row takes its
 // first kf forward neighbors, up to kr nearest proposers, then its other forward neighbors
-// (half_rule_kernel). All pointers are device memory of `dev`.
-void reverse_merge(int dev, const int32_t* fwd, const float* fd, int64_t n, int K, int ks, int kf, int kr, int k,
-                   int32_t* out, cudaStream_t s)
+// (half_rule_kernel). All pointers are device memory of one GPU; scratch: reverse_scratch(n, ks) bytes.
+void reverse_merge(const int32_t* fwd, const float* fd, int64_t n, int K, int ks, int kf, int kr, int k,
+                   int32_t* out, void* scratch, cudaStream_t s)
 {
   OCTEX_EXPECTS(K + kr <= kMergeMax && ks <= K && kf <= K && k <= K + kr, "octex: reverse merge: rows too long");
   const int64_t edges = n * ks;
-  dbuf ekey(dev, 8 * edges), ekey_s(dev, 8 * edges), esrc(dev, 4 * edges), esrc_s(dev, 4 * edges),
-    efirst(dev, 8 * (n + 1));
-  reverse_edges_kernel<<<grid_for(edges, 256), 256, 0, s>>>(fwd, fd, n, K, ks, ekey.as<unsigned long long>(),
-                                                            esrc.as<int32_t>());
-  size_t tb = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tb, ekey.as<unsigned long long>(), ekey_s.as<unsigned long long>(),
-                                  esrc.as<int32_t>(), esrc_s.as<int32_t>(), edges);
-  dbuf tmp(dev, tb);
-  cub::DeviceRadixSort::SortPairs(tmp.ptr, tb, ekey.as<unsigned long long>(), ekey_s.as<unsigned long long>(),
-                                  esrc.as<int32_t>(), esrc_s.as<int32_t>(), edges, 0, 64, s);
-  edge_bounds_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(ekey_s.as<unsigned long long>(), edges, n,
-                                                          efirst.as<int64_t>());
-  half_rule_kernel<<<grid_for(n, 4), 128, 0, s>>>(fwd, fd, K, ekey_s.as<unsigned long long>(), esrc_s.as<int32_t>(),
-                                                  efirst.as<int64_t>(), n, k, kf, kr, out);
+  pieces from{static_cast<char*>(scratch)};
+  auto* ekey   = from.take<unsigned long long>(edges);
+  auto* ekey_s = from.take<unsigned long long>(edges);
+  auto* esrc   = from.take<int32_t>(edges);
+  auto* esrc_s = from.take<int32_t>(edges);
+  auto* efirst = from.take<int64_t>(n + 1);
+  reverse_edges_kernel<<<grid_for(edges, 256), 256, 0, s>>>(fwd, fd, n, K, ks, ekey, esrc);
+  size_t tb = edge_sort_bytes(edges);
+  cub::DeviceRadixSort::SortPairs(from.at, tb, ekey, ekey_s, esrc, esrc_s, edges, 0, 64, s);
+  edge_bounds_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(ekey_s, edges, n, efirst);
+  half_rule_kernel<<<grid_for(n, 4), 128, 0, s>>>(fwd, fd, K, ekey_s, esrc_s, efirst, n, k, kf, kr, out);
   OCTEX_CUDA_TRY(cudaPeekAtLastError());
-  OCTEX_CUDA_TRY(cudaStreamSynchronize(s));  // the scratch arrays go with this scope
+  OCTEX_CUDA_TRY(cudaStreamSynchronize(s));  // the caller may free the scratch memory
 }
 
 // ---- the directory ---------------------------------------------------------------------------------
@@ -960,9 +990,19 @@ void searched_table(resources const& res, index& idx, int k, int passes, bool re
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
   cudaStream_t s = res.stream;
   const int64_t chunk = std::min<int64_t>(n, 100000);
-  dbuf q(p.device, sizeof(float) * chunk * D), ids(p.device, sizeof(long long) * chunk * kq),
-    dist(p.device, sizeof(float) * chunk * kq), fwd(p.device, sizeof(int32_t) * n * kin),
-    fd(p.device, sizeof(float) * n * kin), merged(p.device, sizeof(int32_t) * n * k);
+  // one block for all: with an allocation for each array, and for each array of a merge, 100 001 rows spent 30 of
+  // 75 ms in allocations and their releases
+  dbuf block(p.device, pieces::size_of<float>(chunk * D) + pieces::size_of<long long>(chunk * kq) + pieces::size_of<float>(chunk * kq) +
+                         pieces::size_of<int32_t>(n * kin) + pieces::size_of<float>(n * kin) + pieces::size_of<int32_t>(n * k) +
+                         (reverse_edges ? reverse_scratch(n, kin) : 0));
+  pieces from{block.as<char>()};
+  auto* q      = from.take<float>(chunk * D);
+  auto* ids    = from.take<long long>(chunk * kq);
+  auto* dist   = from.take<float>(chunk * kq);
+  auto* fwd    = from.take<int32_t>(n * kin);
+  auto* fd     = from.take<float>(n * kin);
+  auto* merged = from.take<int32_t>(n * k);
+  const size_t table_bytes = sizeof(int32_t) * static_cast<size_t>(n) * k;
   for (int v = 0; v < passes; v++) {
     const auto t0 = std::chrono::steady_clock::now();
     search_params sp;
@@ -975,30 +1015,35 @@ void searched_table(resources const& res, index& idx, int k, int passes, bool re
     for (int64_t r0 = 0; r0 < n; r0 += chunk) {
       const int64_t m = std::min(chunk, n - r0);
       OCTEX_CUDA_TRY(cudaStreamSynchronize(p.stream));  // the rows' owner stream, before this one reads them
-      rows_to_float_kernel<<<grid_for(m * D, 256), 256, 0, s>>>(p.vectors.as<__half>() + r0 * D, m * D, q.as<float>());
+      rows_to_float_kernel<<<grid_for(m * D, 256), 256, 0, s>>>(p.vectors.as<__half>() + r0 * D, m * D, q);
       // one lane: batches this large gain 3 % from a second stream, and a second plan for every pass costs
       // more (100 001 rows: 77 ms with one, 93 with two)
-      detail::search_impl(res, sp, idx, q.as<float>(), m, D, reinterpret_cast<int64_t*>(ids.ptr), dist.as<float>(), kq, false,
-                          false, false, 1);
-      forward_rows_kernel<<<grid_for(m, 128), 128, 0, s>>>(ids.as<long long>(), dist.as<float>(), r0, m, kq, kin,
-                                                          fwd.as<int32_t>(), fd.as<float>());
+      detail::search_impl(res, sp, idx, q, m, D, reinterpret_cast<int64_t*>(ids), dist, kq, false, false, false, 1);
+      forward_rows_kernel<<<grid_for(m, 128), 128, 0, s>>>(ids, dist, r0, m, kq, kin, fwd, fd);
       OCTEX_CUDA_TRY(cudaPeekAtLastError());
+    }
+    if (v + 1 == passes && table_host != nullptr) {
+      // The pages of the result come into being while the GPU works: a copy to 13 MB of new ones takes 6.6 ms, to
+      // others 0.9.
+      auto* bytes = reinterpret_cast<volatile char*>(table_host);
+      for (size_t at = 0; at < table_bytes; at += 4096)
+        bytes[at] = bytes[at];
     }
     OCTEX_CUDA_TRY(cudaStreamSynchronize(s));
     if (reverse_edges) {
-      reverse_merge(p.device, fwd.as<int32_t>(), fd.as<float>(), n, kin, kin, kf, kr, k, merged.as<int32_t>(), s);
+      reverse_merge(fwd, fd, n, kin, kin, kf, kr, k, merged, from.at, s);
     } else {
-      OCTEX_CUDA_TRY(cudaMemcpy2DAsync(merged.ptr, sizeof(int32_t) * k, fwd.ptr, sizeof(int32_t) * kin, sizeof(int32_t) * k,
+      OCTEX_CUDA_TRY(cudaMemcpy2DAsync(merged, sizeof(int32_t) * k, fwd, sizeof(int32_t) * kin, sizeof(int32_t) * k,
                                        n, cudaMemcpyDeviceToDevice, s));
       OCTEX_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    detail::set_table(ix, merged.as<int32_t>(), k);
+    detail::set_table(ix, merged, k);
     if (verbose)
       std::fprintf(stderr, "octex: searched table, pass %d of %d (%d waves, %d starts): %.2f s\n", v + 1, passes,
                    sp.waves, sp.starts, seconds_since(t0));
   }
   if (table_host != nullptr)
-    OCTEX_CUDA_TRY(cudaMemcpy(table_host, merged.ptr, merged.size, cudaMemcpyDeviceToHost));
+    OCTEX_CUDA_TRY(cudaMemcpy(table_host, merged, table_bytes, cudaMemcpyDeviceToHost));
   OCTEX_CUDA_TRY(cudaSetDevice(cur));
 }
 
@@ -1133,7 +1178,8 @@ void build(resources const& res, index_params const& given, build_dataset const&
     dbuf out(dev, sizeof(int32_t) * n * k);
     const int h = std::max(1, k / 2);
     if (params.reverse_edges) {
-      reverse_merge(dev, fwd.as<int32_t>(), fd.as<float>(), n, K, h, h, h, k, out.as<int32_t>(), s);
+      dbuf scratch(dev, reverse_scratch(n, h));
+      reverse_merge(fwd.as<int32_t>(), fd.as<float>(), n, K, h, h, h, k, out.as<int32_t>(), scratch.ptr, s);
       OCTEX_CUDA_TRY(cudaPeekAtLastError());
       table = to_host<int32_t>(out.ptr, static_cast<size_t>(n) * k);
     } else {

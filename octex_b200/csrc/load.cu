@@ -410,12 +410,14 @@ void set_table(index_impl& ix, const int32_t* table, int table_len)
   OCTEX_CUDA_TRY(cudaGetDevice(&cur));
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
   OCTEX_CUDA_TRY(cudaStreamSynchronize(p.stream));
+  const size_t bytes = static_cast<size_t>(ix.n) * table_len * sizeof(int32_t);
   if (!p.table.host) p.bytes -= static_cast<int64_t>(p.table.size);
-  p.table      = dbuf();
+  // one of the same size that is the index's own is written over
+  if (bytes == 0 || p.table.size != bytes || p.table.host || !p.table.owned) p.table = dbuf();
   p.table_rows = dealt_rows{};
   ix.table_len = table_len;
   if (table_len > 0) {
-    p.table = dbuf(p.device, static_cast<size_t>(ix.n) * table_len * sizeof(int32_t));
+    if (p.table.ptr == nullptr) p.table = dbuf(p.device, bytes);
     p.bytes += static_cast<int64_t>(p.table.size);
     OCTEX_CUDA_TRY(cudaMemcpyAsync(p.table.ptr, table, p.table.size, cudaMemcpyDefault, p.stream));
     OCTEX_CUDA_TRY(cudaStreamSynchronize(p.stream));

@@ -22,13 +22,29 @@ namespace detail {
 
 namespace {
 
+constexpr size_t kPiece = 256;  // arrays of a plan begin on such boundaries
+
+/// The rest of the plan's memory is to hold arrays of these sizes.
+void reserve(plan& pl, int device, std::initializer_list<size_t> bytes)
+{
+  size_t total = 0;
+  for (size_t b : bytes)
+    total += (b + kPiece - 1) / kPiece * kPiece;
+  pl.memory.emplace_back(device, total);
+  pl.memory_used = 0;
+}
+
+/// An array of the plan: a piece of the memory reserved for it, where there is room, else of a new block.
 template <typename T>
 auto alloc(plan& pl, int device, int64_t count, int fill = -2) -> dbuf
 {
-  dbuf b(device, static_cast<size_t>(std::max<int64_t>(count, 1)) * sizeof(T));
+  const size_t bytes = static_cast<size_t>(std::max<int64_t>(count, 1)) * sizeof(T);
+  if (pl.memory.empty() || pl.memory.back().size - pl.memory_used < bytes) reserve(pl, device, {bytes});
+  const dbuf b = dbuf::borrow(device, pl.memory.back().as<char>() + pl.memory_used, bytes);
+  pl.memory_used += std::min((bytes + kPiece - 1) / kPiece * kPiece, pl.memory.back().size - pl.memory_used);
   if (fill != -2) OCTEX_CUDA_TRY(cudaMemset(b.ptr, fill, b.size));
-  pl.buffer_bytes += static_cast<int64_t>(b.size);
-  return b;
+  pl.buffer_bytes += static_cast<int64_t>(bytes);
+  return dbuf::borrow(device, b.ptr, bytes);
 }
 
 /// The kernels' view of an array dealt by rows (empty when the array is whole).
@@ -162,7 +178,7 @@ plan::~plan()
   if (graph != nullptr) cudaGraphExecDestroy(graph);
   if (done_ev != nullptr) cudaEventDestroy(done_ev);
   if (join_ev != nullptr) cudaEventDestroy(join_ev);
-  if (tc_error_host != nullptr) cudaFreeHost(tc_error_host);
+  if (words != nullptr) words->give_back(word);
   cudaSetDevice(cur);
 }
 
@@ -511,6 +527,11 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
   OCTEX_CUDA_TRY(cudaSetDevice(p.device));
   const int m1  = std::max(pl.m1, 1);
   const int wdt = 8 * ix.blocks * p.copies;
+  const auto mb = static_cast<size_t>(std::max(pl.mwmax, 1));
+  // (the arrays of several processes and of an observed search, and candidates in global memory, come in blocks of their own)
+  reserve(pl, p.device,
+          {sizeof(float) * m1 * D, sizeof(float) * m1 * sw, sizeof(int2) * m1 * p.copies, sizeof(long long) * m1 * pl.KO,
+           sizeof(float) * m1 * pl.KO, (sizeof(long long) + sizeof(float)) * mb * k, sizeof(int) * m1 * S * sp.waves});
   pl.qbuf  = alloc<float>(pl, p.device, int64_t{m1} * D, 0);
   pl.qs    = alloc<float>(pl, p.device, int64_t{m1} * sw);
   pl.use_tc = !dbg.ordered_projection && kernels::project_tc_supported(ix.blocks, p.ldu);
@@ -520,9 +541,14 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
     pl.codes = alloc<long long>(pl, p.device, int64_t{m1} * p.copies * L);
   }
   // the word a kernel sets when one of its bounded waits (on an mbarrier) ran out
-  OCTEX_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&pl.tc_error_host), sizeof(int), cudaHostAllocMapped));
-  *pl.tc_error_host = 0;
-  OCTEX_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&pl.tc_error_dev), pl.tc_error_host, 0));
+  if (ix.words != nullptr) pl.word = ix.words->take();
+  if (pl.word < 0) {
+    ix.words = std::make_shared<pinned_words>(p.device);
+    pl.word  = ix.words->take();
+  }
+  pl.words         = ix.words;
+  pl.tc_error_host = pl.words->host(pl.word);
+  pl.tc_error_dev  = pl.words->device(pl.word);
   if (pl.use_tc) {
     int sms = 0;
     OCTEX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device));

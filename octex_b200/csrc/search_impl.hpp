@@ -38,7 +38,9 @@ struct plan {
   dbuf tap_cand, tap_dist, tap_n, kept1_i, kept1_d;
   bool use_tc = false;          // tensor-core projection with the decode in its epilogue
   kernels::project_tc_plan tc;  // its tensor maps
-  int* tc_error_host = nullptr; // pinned, device-visible: non-zero when a bounded wait in a kernel ran out
+  std::shared_ptr<pinned_words> words;  // a word of the index, non-zero when a bounded wait in a kernel ran out
+  int word           = -1;
+  int* tc_error_host = nullptr;
   int* tc_error_dev  = nullptr;
   int tap_cap = 0;
   std::vector<dbuf> scratch_cand, scratch_dist;
@@ -55,6 +57,9 @@ struct plan {
   unsigned long long last_stream = 0;
   bool used                      = false;
   int64_t buffer_bytes  = 0;
+  // what the arrays above are pieces of (see alloc): an allocation and its release take 0.6 ms of any size
+  std::vector<dbuf> memory;
+  size_t memory_used = 0;  // of the last of them
   // page-locked staging of calls with ordinary host memory, made when first needed: queries in,
   // results out (the last kernel of the batch writes them there)
   dbuf stage_q, stage_out;

@@ -338,3 +338,46 @@ def test_results_are_plain_tensors():
             d, i = idx.search(q, 10, **kw)
             assert same((d.cpu().numpy(), i.cpu().numpy()), want)
     idx.close()
+
+
+def test_more_plans_than_words():
+    """A plan's arrays are pieces of one block and its give-up word one of 64 of the index: many configurations one
+    after the other, each the answer of a handle that knows only this one."""
+    from octex_b200 import synth
+    idx, _ = make_index(64)
+    queries = synth.plumbing(70, 64, seed=3)
+    kw = dict(read=8, waves=1, rerank=32, wave_rerank=32)
+    got = [idx.search(queries[:1 + s], 5, starts=1 + s, **kw) for s in range(70)]
+    for s in (0, 1, 33, 63, 64, 69):
+        other, _ = make_index(64)
+        assert same(other.search(queries[:1 + s], 5, starts=1 + s, **kw), got[s]), s
+        other.close()
+    idx.close()
+
+
+@pytest.mark.parametrize("borrow", [False, True])
+def test_table_of_the_same_size_is_written_over(borrow):
+    """set_table writes over the index's own table where the size is the same, and never over an array that belongs to
+    the caller."""
+    import torch
+    from octex_b200 import build_index, synth
+    base = synth.plumbing(4000, 64, seed=0)
+    arrays, meta = build_index.build_arrays(base, small_params(pca_dims=64, list_len=16, min_cell=2, sketch_width=32, table_len=24),
+                                            device="cpu")
+    queries = synth.plumbing(50, 64, seed=4)
+    kw = dict(read=4, starts=16, waves=2, rerank=16, wave_rerank=16)
+    table = np.ascontiguousarray(arrays["table"])
+    turned = np.ascontiguousarray(np.roll(table, 1, axis=0))  # every row the neighbors of the row before
+    mine = torch.as_tensor(table, device="cuda")
+    idx = octex_b200.attach(dict(arrays, table=mine) if borrow else arrays, meta, borrow=borrow)
+    first = idx.search(queries, 10, **kw)
+    idx.set_table(turned)
+    second = idx.search(queries, 10, **kw)
+    idx.set_table(table)
+    assert same(idx.search(queries, 10, **kw), first)
+    idx.close()
+    assert np.array_equal(mine.cpu().numpy(), table)
+    fresh = octex_b200.attach(dict(arrays, table=turned), meta, borrow=False)
+    assert same(fresh.search(queries, 10, **kw), second)
+    assert not same(first, second)
+    fresh.close()
