@@ -5,15 +5,16 @@
 //   t[q, r] = |x_r|^2 - 2 x_q . x_r          squared distance up to the row's own constant |x_q|^2
 //
 // A block takes items of one or two sets of 128 query rows and walks over all rows in tiles of 128. Per tile and
-// set the 128 x 128 accumulators are one chain of tcgen05.mma (fp32 in TMEM): first a short one whose operands
-// are the tile's norms, each as three bf16 of eight bits, and minus a half for each of the three, then the fp16
-// rows (by TMA, 128-byte swizzle). So an accumulator is -t / 2 and the epilogue neither loads a norm nor does
-// arithmetic: norms from shared memory, an FMA for each, took half of the shared memory's time (a load whose 32
-// lanes want the same 16 bytes fills the data pipe for four cycles) beside the MMAs, which read their operands
-// from it as well. The sums start with the norm, so they end small instead of growing to |x|^2 before the
-// subtraction: against 64 bits the distances of near rows are off by 2.2e-7 (20 000 x 96 on the unit sphere, root
-// mean square), 3.3e-7 (256 dimensions) and 2.8e-4 (960, non-negative), 2.3e-7, 6.7e-7 and 6.1e-4 with the norm
-// added behind. The accumulators are double buffered, so the tensor cores work on tile i + 1 while four epilogue
+// set the 128 x 128 accumulators are one chain of tcgen05.mma (fp32 in TMEM): the fp16 rows (by TMA, 128-byte
+// swizzle), then a short one whose operands are the tile's norms, each as three bf16 of eight bits, and minus a half
+// for each of the three. So an accumulator is -t / 2 and the epilogue neither loads a norm nor does arithmetic: norms
+// from shared memory, an FMA for each, took half of the shared memory's time (a load whose 32 lanes want the same
+// 16 bytes fills the data pipe for four cycles) beside the MMAs, which read their operands from it as well. The norms
+// come last: the sums before are those of the products alone and the distances against 64 bits as far off as with
+// an FMA behind the MMAs (root mean square, relative, of near rows: 2.25e-7 at 96 dimensions on the unit sphere,
+// 6.6e-7 at 256, 6.1e-4 at 960 non-negative ones, both ways), the neighbors found the same ones. Norms first give
+// 2.2e-7, 3.3e-7 and 2.8e-4 there but 2.1e-7 instead of 1.8e-7 at 64 dimensions, and other neighbors among near ties.
+// The accumulators are double buffered, so the tensor cores work on tile i + 1 while four epilogue
 // warps per set read tile i (tcgen05.ld, one query row per thread) and compare with what the row has to beat. The
 // query rows stay in shared memory for the whole scan when they fit (256 dimensions at most), so a tile of 128
 // rows is read from the L2 cache once for 256 query rows.
@@ -31,12 +32,13 @@
 //
 // What bounds it: the MMAs. One of 128 x 128 x 16 with both operands in shared memory takes 101 cycles instead
 // of 64 (128 bytes a cycle would be needed), the norms one more of them, and a tile with nothing looked at 2 200
-// of the 2 800 cycles that it takes (200 001 x 128, K = 64: 11.2 of 14.2 ms; 64 dimensions 8.0 of 12.0); the rest is
+// of the 2 800 cycles that it takes (200 001 x 128, K = 64: 11.4 of 14.5 ms; 64 dimensions 8.2 of 12.3); the rest is
 // what the four warps of a set wait for one another when one of them looks through its improvements.
 // 200 001 x 128, K = 64, ms: 133 with a list update per improvement; 20.5 with buffers in shared memory that the
 // epilogue merges itself and norms it adds; 18.3 with list warps and norms in the MMAs; 15.0 with the groups read
 // again from TMEM (instead of 64 columns kept in registers until it is known which are wanted); 14.2 with the next 32
-// columns on their way while 32 are looked at. Two warps per row, a half of the columns each: 18.7.
+// columns on their way while 32 are looked at, 14.5 with the norms last. Two warps per row, a half of the columns each:
+// 18.7.
 //
 // Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues), warp 3 makes the norm
 // operands; eight epilogue warps, four per set, one per quarter of the TMEM lanes; four list warps of 64 rows.
@@ -438,16 +440,6 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
         if (works) ok = __all_sync(0xffffffffu, mbar_wait(&ctl.acc_empty[set][b], ((v >> 1) & 1u) ^ 1u, stop));
         if (!ok) break;
         const uint32_t acc = tmem + (2 * b + set) * kTile;
-        ok = __all_sync(0xffffffffu, mbar_wait(&ctl.norms_full[b], (v >> 1) & 1u, stop));
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!works) {
-          if (lane == 0) mbar_arrive(&ctl.norms_empty[b]);
-        } else if (issues) {
-          umma_f16(acc, norm_desc(halves), norm_desc(norms + b * kNormBytes), idesc | kBothBf16, 0u);
-          umma_commit(&ctl.norms_empty[b]);
-        }
-        __syncwarp();
         for (int kb = 0; kb < nkb; kb++) {
           ok = __all_sync(0xffffffffu, mbar_wait(&ctl.full[s], turn & 1u, stop));
           if (!ok) break;
@@ -460,13 +452,24 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
 #pragma unroll
             for (int k = 0; k < kTileK / 16; k++)
               if (kb * kTileK + 16 * k < D)  // beyond it a tile's columns are zero
-                umma_f16(acc, da + 2 * k, db + 2 * k, idesc, 1u);
+                umma_f16(acc, da + 2 * k, db + 2 * k, idesc, kb > 0 || k > 0 ? 1u : 0u);
             umma_commit(&ctl.empty[s]);  // arrives when the MMAs reading this stage are done
-            if (kb + 1 == nkb) umma_commit(&ctl.acc_full[set][b]);
           }
           __syncwarp();
           if (++s == stages) s = 0, turn++;
         }
+        // the norms come last
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(&ctl.norms_full[b], (v >> 1) & 1u, stop));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!works) {
+          if (lane == 0) mbar_arrive(&ctl.norms_empty[b]);
+        } else if (issues) {
+          umma_f16(acc, norm_desc(halves), norm_desc(norms + b * kNormBytes), idesc | kBothBf16, 1u);
+          umma_commit(&ctl.norms_empty[b]);
+          umma_commit(&ctl.acc_full[set][b]);
+        }
+        __syncwarp();
       }
       if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 2);
     } else if (warp == 3) {
