@@ -1016,8 +1016,8 @@ void searched_table(resources const& res, index& idx, int k, int passes, bool re
       const int64_t m = std::min(chunk, n - r0);
       OCTEX_CUDA_TRY(cudaStreamSynchronize(p.stream));  // the rows' owner stream, before this one reads them
       rows_to_float_kernel<<<grid_for(m * D, 256), 256, 0, s>>>(p.vectors.as<__half>() + r0 * D, m * D, q);
-      // one lane: batches this large gain 3 % from a second stream, and a second plan for every pass costs
-      // more (100 001 rows: 77 ms with one, 93 with two)
+      // one lane: the batches go in halves on two streams as it is, and a second plan for every pass costs more than it
+      // gives (100 001 rows: 77 ms with one, 93 with two)
       detail::search_impl(res, sp, idx, q, m, D, reinterpret_cast<int64_t*>(ids), dist, kq, false, false, false, 1);
       forward_rows_kernel<<<grid_for(m, 128), 128, 0, s>>>(ids, dist, r0, m, kq, kin, fwd, fd);
       OCTEX_CUDA_TRY(cudaPeekAtLastError());

@@ -72,6 +72,7 @@ struct device_part {
   dealt_rows table_rows, sketch_rows, vector_rows;
   cudaStream_t stream = nullptr;
   cudaStream_t second = nullptr;  // created when a search first alternates its batches between two streams
+  cudaStream_t half   = nullptr;  // created when a batch first goes in two halves; never part of a capture
   int64_t bytes       = 0;
 
   device_part() = default;
@@ -88,6 +89,7 @@ struct device_part {
         cudaIpcCloseMemHandle(p);
     if (stream != nullptr) cudaStreamDestroy(stream);
     if (second != nullptr) cudaStreamDestroy(second);
+    if (half != nullptr) cudaStreamDestroy(half);
     cudaSetDevice(cur);
   }
 };

@@ -247,9 +247,18 @@ void mark_last_batch(plan& pl, cudaStream_t s)
   pl.used = true;
 }
 
-/// Launch every kernel of a batch of pl.m queries on s (captured into the graph, or run directly).
-void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t s, std::vector<cudaEvent_t>* marks)
+/// Rows of a batch by one process.
+struct row_range {
+  int first, count;
+};
+
+/// Launch every kernel of a batch of pl.m queries on s (captured into the graph, or run directly), or (part given:
+/// by one process and without observation) of some of its rows. io is the whole batch's.
+void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t s, std::vector<cudaEvent_t>* marks,
+               row_range const* part = nullptr)
 {
+  const int64_t first = part != nullptr ? part->first : 0;
+  const int m1 = part != nullptr ? part->count : pl.m1, mw = part != nullptr ? part->count : pl.mw;
   // marks (profiling only): one event before the first kernel and one after every step
   auto mark = [&] {
     if (marks == nullptr) return;
@@ -273,17 +282,17 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
   for (float f : ix.spacings)
     finest = std::min(finest, f);
   kernels::sketch_job job;
-  job.q = io.q, job.mean = p.mean.as<float>(), job.basis = p.basis.as<float>();
-  job.m = pl.m1, job.D = D, job.S = sw;
-  job.qs   = pl.qs.as<float>();
-  job.keep = io.q == pl.qbuf.as<float>() ? nullptr : pl.qbuf.as<float>();
+  job.q = io.q + first * D, job.mean = p.mean.as<float>(), job.basis = p.basis.as<float>();
+  job.m = m1, job.D = D, job.S = sw;
+  job.qs   = pl.qs.as<float>() + first * sw;
+  job.keep = io.q == pl.qbuf.as<float>() ? nullptr : pl.qbuf.as<float>() + first * D;
   kernels::tc_lookup look;
   look.table    = p.cell_table.as<kernels::cell_slot>();
   look.keys     = p.cell_keys.as<long long>();
   look.levels   = p.cell_levels.as<kernels::cell_level>();
   look.list_len = ix.list_len;
   look.lr       = pl.lr;
-  look.seg      = pl.seg.as<int2>();
+  look.seg      = pl.seg.as<int2>() + first * p.copies;
   look.stats    = pl.stats.as<long long>();
   // without inspection the cells are looked up where their codes are computed: no codes array, no
   // lookup kernel
@@ -327,9 +336,20 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
   const bool last_is_lists  = pl.sp.waves == 0 && !pl.shard;
   auto with_results         = [&](kernels::round_args r, bool last) {
     if (last && !reranks_at_end) {
-      r.out_i = io.ids;
-      r.out_d = io.dist;
+      r.out_i = io.ids + first * pl.k;
+      r.out_d = io.dist + first * pl.k;
       r.k     = pl.k;
+    }
+    if (part != nullptr) {
+      r.m = part->count;
+      if (r.seg != nullptr) r.seg += first * p.copies;
+      r.qs += first * sw;
+      r.Q += first * D;
+      r.si += first * pl.KO;
+      r.sd += first * pl.KO;
+      if (r.done != nullptr) r.done += first * r.done_stride;
+      if (r.cand_global != nullptr) r.cand_global += first * r.nmax;
+      if (r.dist_global != nullptr) r.dist_global += first * r.nmax;
     }
     return r;
   };
@@ -381,8 +401,8 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
     mark();
   }
   if (reranks_at_end)
-    kernels::final_rerank(pl.wsi, pl.KO, pl.FR, p.vectors.as<__half>(), pl.r1.vector_map, D, Qw, pl.k, pl.mw, io.ids,
-                          io.dist, pl.stats.as<long long>(), s);
+    kernels::final_rerank(pl.wsi + first * pl.KO, pl.KO, pl.FR, p.vectors.as<__half>(), pl.r1.vector_map, D, Qw + first * D,
+                          pl.k, mw, io.ids + first * pl.k, io.dist + first * pl.k, pl.stats.as<long long>(), s);
   else if (pl.sp.waves == 0 && pl.shard)
     kernels::take_k(pl.wsi, pl.wsd, pl.KO, pl.k, pl.mw, io.ids, io.dist, s);
   mark();
@@ -661,6 +681,24 @@ auto make_plan(index_impl& ix, search_params const& sp, int m, int k, debug_opti
     size_round(pl, r2, S * ix.table_len, true, S * std::max(sp.waves - 1, 0), p.device, sketch_bytes, ix.n, !p.vectors.host);
   }
   kernels::round_allow_smem();
+  {
+    // Kernels of the two halves of a batch run side by side, one's under the end of the other's, where there are
+    // more query blocks than the multiprocessors hold of its heaviest round (twice as many where they hold one
+    // each) and a million entries to gather. us a search, whole and in halves: a million rows, eight blocks each, 1 000
+    // queries 161 and 176, 1 200 216 and 208, 2 500 307 and 277, 10 000 861 and 831; four blocks each, 500 195 and
+    // 194, 700 264 and 232, 4 000 982 and 930; two, 300 473 and 448, 1 200 1 212 and 1 094, 10 000 8 143 and 8 021; one,
+    // 200 527 and 587, 400 747 and 681, 2 500 3 556 and 3 432. A small index with 32 entries a query, 1 200 55 and
+    // 58, 3 000 65 and 66; 256 entries, 1 300 110 and 109; 1 088, 1 200 117 and 116, 1 500 124 and 116.
+    int64_t held = 0, entries = 0;
+    for (auto const* r : {&r1, &pl.r2}) {
+      if (r == &pl.r2 && sp.waves == 0) continue;
+      const auto per_sm = std::min<int64_t>(static_cast<int64_t>(blocks_of(*r)), 1024 / r->threads);
+      held              = held == 0 ? per_sm : std::min(held, per_sm);
+      entries += int64_t{r->nmax} * (r == &r1 ? 1 : sp.waves);
+    }
+    pl.entries     = entries;
+    pl.halves_from = std::max(held >= 2 ? held * r1.sms + 1 : int64_t{2} * r1.sms, (1 << 20) / entries);
+  }
 
   OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.done_ev, cudaEventDisableTiming));
   OCTEX_CUDA_TRY(cudaEventCreateWithFlags(&pl.join_ev, cudaEventDisableTiming));
@@ -784,6 +822,43 @@ auto plans_of(index_impl& ix, search_params const& sp, int lanes, int64_t nq, in
   return lane;
 }
 
+/// The stream of the second half of a batch of n queries, if it goes in halves: not while s is captured (so this stream
+/// never is, whatever other threads capture), nor under observation. Its device is current, ix.start_mu is held.
+auto half_stream(index_impl& ix, plan const& pl, int n, cudaStream_t s) -> cudaStream_t
+{
+  if (n < pl.halves_from || pl.dbg.stats || pl.dbg.taps || capturing(s)) return nullptr;
+  auto& p = ix.part;
+  if (p.half == nullptr) OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&p.half, cudaStreamNonBlocking));
+  return p.half;
+}
+
+/// A batch of n queries in device memory on s; in two halves where that pays: the second runs on the other stream,
+/// from where s is now, and s goes on when it is done.
+void run_in_place(index_impl& ix, plan& pl, batch_io const& io, int n, cudaStream_t s)
+{
+  std::unique_lock<std::mutex> one_start(ix.start_mu);
+  cudaStream_t other = half_stream(ix, pl, n, s);
+  if (other == nullptr) {
+    one_start.unlock();
+    run_batch(ix, pl, io, s, nullptr);
+    return;
+  }
+  OCTEX_CUDA_TRY(cudaEventRecord(start_event(ix, ix.part.device), s));
+  OCTEX_CUDA_TRY(cudaStreamWaitEvent(other, ix.start_ev, 0));
+  one_start.unlock();
+  struct joined {  // also when a half could not be queued
+    plan& pl;
+    cudaStream_t s, other;
+    ~joined()
+    {
+      if (cudaEventRecord(pl.join_ev, other) == cudaSuccess) cudaStreamWaitEvent(s, pl.join_ev, 0);
+    }
+  } join{pl, s, other};
+  const row_range halves[2] = {{0, (n + 1) / 2}, {(n + 1) / 2, n / 2}};
+  run_batch(ix, pl, io, s, nullptr, &halves[0]);
+  run_batch(ix, pl, io, other, nullptr, &halves[1]);
+}
+
 /// The next batch of a call on a plan: n queries from row b0 of it on.
 void set_batch(plan& pl, unsigned long long call, int64_t b0, int n)
 {
@@ -849,8 +924,11 @@ auto search_device(index_impl& ix, search_params const& sp, int lanes, cudaStrea
   }
   auto run = [&](int l, int64_t b0, int n) {
     set_batch(*lane[l], call, b0, n);
-    run_batch(ix, *lane[l], {queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k},
-              stream[l], nullptr);
+    const batch_io io{queries + b0 * ix.dim, reinterpret_cast<long long*>(neighbors + b0 * k), distances + b0 * k};
+    if (lanes == 1)
+      run_in_place(ix, *lane[l], io, n, stream[l]);
+    else
+      run_batch(ix, *lane[l], io, stream[l], nullptr);
   };
   auto close = [&](int l, bool) {
     mark_last_batch(*lane[l], stream[l]);
@@ -883,25 +961,48 @@ auto copies_results(plan const& pl, int m) -> bool
   return bytes >= kLarge && entries < 8 * pl.k;
 }
 
+/// Entries a batch in ordinary host memory gathers from which on it goes in two halves: the call waits twice in the
+/// copies of its queries then, under kernels that have to be long enough. us a call, whole and in halves: 3.3
+/// million (3 000 queries of a small index) 269 and 297, 3.7 (1 200 x 128) 292 and 293, 6.1 375 and 365, 6.5 482 and
+/// 451, 7.7 457 and 406, 15 743 and 745, 18 859 and 824, 31 1 414 and 1 295.
+constexpr int64_t kCopiedEntries = int64_t{1} << 22;
+
 /// A search by one process with queries and results that are not all memory of its GPU (host memory,
 /// another GPU's): the copies are queued around the kernels. Several batches alternate between two
 /// lanes, each a plan on a stream of its own: the copies of one batch run under the kernels of the
-/// other. Page-locked arrays are copied from and to directly; ordinary ones pass through page-locked
+/// other. So do the halves of a batch that goes in two, on the two streams with one plan. Page-locked arrays are copied from and to directly; ordinary ones pass through page-locked
 /// staging of the plan where that is faster (kStagedQueries, copies_results).
 void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStream_t caller, int cur, const float* queries,
                    int64_t nq, int64_t* neighbors, float* distances, int64_t k, bool host_out)
 {
   auto& p                       = ix.part;
   const int D                   = static_cast<int>(ix.dim);
-  const int m                   = batch_rows(nq, sp.batch);
+  int m                         = batch_rows(nq, sp.batch);
   const unsigned long long call = ++ix.calls;
-  const lane_plans lane         = plans_of(ix, sp, lanes, nq, k);
+  lane_plans lane               = plans_of(ix, sp, lanes, nq, k);
   std::unique_lock<std::mutex> lock0(lane[0]->mu), lock1;
   if (lanes > 1) lock1 = std::unique_lock<std::mutex>(lane[1]->mu);
   cudaStream_t stream[2] = {p.stream, p.second};
   for (int l = 0; l < lanes; l++) {
     check_tc(*lane[l]);
     follow_last_batch(*lane[l], stream[l]);
+  }
+  bool halves = false;  // of the one batch there is, lane l's from row l * m of the plan's arrays on
+  if (lanes == 1 && nq == m) {
+    stream[1] = nullptr;
+    std::lock_guard<std::mutex> one_start(ix.start_mu);
+    // (a copy of results to ordinary memory would hold up the second half)
+    if (!(host_out && (copies_results(*lane[0], m) || m * lane[0]->entries < kCopiedEntries)))
+      stream[1] = half_stream(ix, *lane[0], m, stream[0]);
+    halves = stream[1] != nullptr;
+  }
+  if (halves) {
+    lanes     = 2;
+    m         = (m + 1) / 2;
+    lane[1]   = lane[0];
+    set_batch(*lane[0], call, 0, static_cast<int>(nq));
+    OCTEX_CUDA_TRY(cudaEventRecord(lane[0]->join_ev, stream[0]));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(stream[1], lane[0]->join_ev, 0));
   }
   const bool stage_in  = host_out && sizeof(float) * static_cast<size_t>(m) * D < kStagedQueries && !device_reaches(queries);
   const bool stage_out = host_out && !(lanes == 1 && copies_results(*lane[0], m)) &&
@@ -914,11 +1015,12 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
   auto deliver = [&](int l) {
     if (out[l].n == 0) return;
     OCTEX_CUDA_TRY(cudaStreamSynchronize(stream[l]));
-    plan& w          = *lane[l];
-    const size_t cnt = static_cast<size_t>(out[l].n) * k;
-    std::memcpy(neighbors + out[l].b0 * k, w.stage_out.ptr, cnt * sizeof(int64_t));
-    std::memcpy(distances + out[l].b0 * k, w.stage_out.as<char>() + sizeof(int64_t) * static_cast<size_t>(w.cap) * k,
-                cnt * sizeof(float));
+    plan& w            = *lane[l];
+    const size_t cnt   = static_cast<size_t>(out[l].n) * k;
+    const size_t from  = halves ? static_cast<size_t>(l) * m * k : 0;
+    const auto* dist   = reinterpret_cast<const float*>(w.stage_out.as<int64_t>() + static_cast<size_t>(w.cap) * k);
+    std::memcpy(neighbors + out[l].b0 * k, w.stage_out.as<int64_t>() + from, cnt * sizeof(int64_t));
+    std::memcpy(distances + out[l].b0 * k, dist + from, cnt * sizeof(float));
     out[l].n = 0;
   };
   int64_t batch = 0;
@@ -926,16 +1028,19 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
     plan& w            = *lane[l];
     cudaStream_t s     = stream[l];
     const size_t bytes = sizeof(float) * static_cast<size_t>(n) * D;
+    const row_range part{halves ? l * m : 0, n};
+    float* own_q = w.qbuf.as<float>() + static_cast<size_t>(part.first) * D;
     if (stage_out) deliver(l);  // the lane's staging is free again, its queries too
     const void* src = queries + b0 * D;
     if (stage_in) {
       if (!stage_out && batch >= lanes) OCTEX_CUDA_TRY(cudaStreamSynchronize(s));
-      void* pin = staging(w.stage_q, p.device, sizeof(float) * static_cast<size_t>(w.cap) * D);
+      float* pin = static_cast<float*>(staging(w.stage_q, p.device, sizeof(float) * static_cast<size_t>(w.cap) * D)) +
+                   static_cast<size_t>(part.first) * D;
       std::memcpy(pin, src, bytes);
       src = pin;
     }
-    OCTEX_CUDA_TRY(cudaMemcpyAsync(w.qbuf.ptr, src, bytes, cudaMemcpyDefault, s));
-    set_batch(w, call, b0, n);
+    OCTEX_CUDA_TRY(cudaMemcpyAsync(own_q, src, bytes, cudaMemcpyDefault, s));
+    if (!halves) set_batch(w, call, b0, n);
     batch_io io = own_io(w);
     if (stage_out) {
       // the last kernel writes through to host memory
@@ -943,17 +1048,24 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
       io.ids    = reinterpret_cast<long long*>(pin);
       io.dist   = reinterpret_cast<float*>(pin + sizeof(int64_t) * static_cast<size_t>(w.cap) * k);
     }
-    run_batch(ix, w, io, s, nullptr);
+    run_batch(ix, w, io, s, nullptr, halves ? &part : nullptr);
     if (stage_out) {
       out[l].b0 = b0;
       out[l].n  = n;
     } else {
-      OCTEX_CUDA_TRY(cudaMemcpyAsync(neighbors + b0 * k, w.bi, sizeof(int64_t) * n * k, cudaMemcpyDefault, s));
-      OCTEX_CUDA_TRY(cudaMemcpyAsync(distances + b0 * k, w.bd, sizeof(float) * n * k, cudaMemcpyDefault, s));
+      const int64_t from = int64_t{part.first} * k;
+      OCTEX_CUDA_TRY(cudaMemcpyAsync(neighbors + b0 * k, w.bi + from, sizeof(int64_t) * n * k, cudaMemcpyDefault, s));
+      OCTEX_CUDA_TRY(cudaMemcpyAsync(distances + b0 * k, w.bd + from, sizeof(float) * n * k, cudaMemcpyDefault, s));
     }
     batch++;
   };
   auto close = [&](int l, bool failed) {
+    if (halves && l == 0) return;
+    if (halves) {  // what the plan's last batch is ends on the first stream
+      OCTEX_CUDA_TRY(cudaEventRecord(lane[1]->join_ev, stream[1]));
+      OCTEX_CUDA_TRY(cudaStreamWaitEvent(stream[0], lane[1]->join_ev, 0));
+      l = 0;
+    }
     mark_last_batch(*lane[l], stream[l]);
     if (host_out) {
       // nothing may still be on its way from or to the caller's arrays or the staging

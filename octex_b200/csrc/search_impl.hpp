@@ -56,6 +56,8 @@ struct plan {
   // the stream done_ev was recorded on (cudaStreamGetId): a batch on another one waits for it first
   unsigned long long last_stream = 0;
   bool used                      = false;
+  int64_t entries       = 0;  // list and table entries that a query gathers at most
+  int64_t halves_from   = 0;  // queries from which on a batch goes in two halves on two streams
   int64_t buffer_bytes  = 0;
   // what the arrays above are pieces of (see alloc): an allocation and its release take 0.6 ms of any size
   std::vector<dbuf> memory;

@@ -381,3 +381,80 @@ def test_table_of_the_same_size_is_written_over(borrow):
     assert same(fresh.search(queries, 10, **kw), second)
     assert not same(first, second)
     fresh.close()
+
+
+@pytest.mark.parametrize("dim,kw", [
+    (64, dict(read=8, starts=16, waves=2, rerank=32, wave_rerank=32)),
+    (98, dict(read=8, starts=16, waves=0, rerank=32)),                                # rows on 8-byte boundaries
+    (48, dict(read=16, starts=512, waves=1, sketch_rank=True, final_rerank=40)),      # a block a multiprocessor
+    (64, dict(read=16, starts=32, waves=1, sketch_rank=True, final_rerank=0)),
+])
+def test_batches_in_halves(dim, kw):
+    """A batch of more query blocks than the multiprocessors hold goes in two halves on two streams: the answer and
+    the segments of the inspected run, which does not, for arrays on the GPU, in ordinary and in page-locked memory;
+    one query less than the line and whole batches of odd numbers; searches before and after on another stream; what
+    a resident search repeats."""
+    import torch
+    from octex_b200 import synth
+    idx, _ = make_index(dim, copies=6, rows=6000, table_len=32)
+    queries = synth.plumbing(2601, dim, seed=5)
+    for n in (1183, 1184, 1185, 2601):
+        want, seg = inspected(idx, queries[:n], 10, **kw)
+        on_gpu = torch.as_tensor(queries[:n], device="cuda")
+        d, i = idx.search(on_gpu, 10, **kw)
+        assert same((d.cpu().numpy(), i.cpu().numpy()), want), n
+        assert np.array_equal(idx.fetch("seg", np.int32), seg), n
+        assert same(idx.search(queries[:n], 10, **kw), want), n
+        assert np.array_equal(idx.fetch("seg", np.int32), seg), n
+        with torch.cuda.stream(torch.cuda.Stream()):
+            d, i = idx.search(on_gpu, 10, **kw)
+            torch.cuda.current_stream().synchronize()
+        assert same((d.cpu().numpy(), i.cpu().numpy()), want), n
+        pinned = torch.as_tensor(queries[:n]).pin_memory()
+        got = idx.search(pinned, 10, **kw)
+        got = [t.cpu().numpy() if torch.is_tensor(t) else t for t in got]
+        assert same(got, want), n
+    idx.close()
+
+
+def test_halves_and_graphs():
+    """A search whose stream is captured keeps to it, and the graph gives the answer of the search in halves, also
+    while other searches go in halves between its launches; arrays used in place and arrays copied."""
+    import torch
+    from octex_b200 import synth
+    dim, k, n = 64, 10, 2500
+    idx, _ = make_index(dim, copies=6)
+    kw = dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)
+    queries = torch.as_tensor(synth.plumbing(n, dim, seed=6))
+    want = [t.cpu().numpy() for t in idx.search(queries.cuda(), k, **kw)]
+    side = torch.cuda.Stream()
+    for pinned in (False, True):
+        q, ids, dist = queries, torch.empty((n, k), dtype=torch.int64), torch.empty((n, k))
+        q, ids, dist = (t.pin_memory() if pinned else t.cuda() for t in (q, ids, dist))
+        at = (q.data_ptr(), ids.data_ptr(), dist.data_ptr())
+
+        def call():
+            search_at(idx, *at, n, dim, k, wait=False, stream=side.cuda_stream, use_graph=False, **kw)
+
+        torch.cuda.synchronize()
+        call()
+        side.synchronize()
+        assert same((dist.cpu().numpy(), ids.cpu().numpy()), want)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            call()
+        for _ in range(2):
+            ids.fill_(-5)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                graph.replay()
+            call()  # in halves, behind the graph
+            side.synchronize()
+            assert same((dist.cpu().numpy(), ids.cpu().numpy()), want)
+            ids.fill_(-5)
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert same((dist.cpu().numpy(), ids.cpu().numpy()), want)
+        del graph
+    idx.close()
