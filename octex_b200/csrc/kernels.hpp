@@ -60,6 +60,7 @@ struct sketch_job {
   const float* mean  = nullptr;
   const float* basis = nullptr;
   int m = 0, D = 0, S = 0;
+  int beside  = 1;  // such launches that share the GPU
   float* qs   = nullptr;
   float* keep = nullptr;
 };
@@ -102,7 +103,7 @@ void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, c
 /// The same step for indexes of another number of blocks per copy (project_ord.cu): projection in
 /// dimension order (the order of project_ordered), decode and lookup in one kernel.
 void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
-                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, cudaStream_t s);
+                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, int sms, cudaStream_t s);
 
 /// codes [n] = cell code of each row of y [n, 8*blocks] float32 scaled by inv_f.
 void cell_codes_f32(const float* y, int64_t n, int blocks, float inv_f, long long* codes,

@@ -16,6 +16,8 @@
 
 #include "prep_common.cuh"
 
+#include <algorithm>
+
 namespace octex_b200::kernels {
 
 namespace {
@@ -29,7 +31,7 @@ struct ord_shape {
 };
 
 template <int B>
-__global__ void __launch_bounds__(256) project_lookup_kernel(const sketch_job job, int sk_blocks,
+__global__ void __launch_bounds__(256) project_lookup_kernel(const sketch_job job, int sk_blocks, int per_block,
                                                              const __half* __restrict__ ut, int ldu, int Cg, int L,
                                                              const __half* __restrict__ shift,
                                                              const float* __restrict__ inv_f, float tame_y,
@@ -52,9 +54,9 @@ __global__ void __launch_bounds__(256) project_lookup_kernel(const sketch_job jo
   float* sb = smem + kStep * kLd;  // [32 dims][68 columns]
   const int tiles = (Cg + kC - 1) / kC;
   const int c0    = ((blockIdx.x - sk_blocks) % tiles) * kC;
-  const int row0  = ((blockIdx.x - sk_blocks) / tiles) * kRows;
+  const int row0  = ((blockIdx.x - sk_blocks) / tiles) * per_block;
   const int m = job.m, D = job.D, N = Cg * 8 * B, col0 = c0 * 8 * B;
-  const int rows = min(kRows, m - row0);
+  const int rows = min(per_block, m - row0);
   fill_primes(primes);
   if (threadIdx.x < kC * L) lv[threadIdx.x] = c0 + threadIdx.x / L < Cg ? look.levels[c0 * L + threadIdx.x] : cell_level{0, 0, -1, 0};
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -144,23 +146,34 @@ __global__ void __launch_bounds__(256) project_lookup_kernel(const sketch_job jo
 }  // namespace
 
 void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
-                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, cudaStream_t s)
+                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, int sms,
+                            cudaStream_t s)
 {
   if (job.m <= 0 || copies <= 0) return;
   const float tame_y = finest > 0.f ? kTameLimit * finest * 0.99f : 0.f;
   const int sk       = sketch_blocks<1>(job);
-  auto launch        = [&](auto kernel, int per_block) {
-    const unsigned grid = static_cast<unsigned>(sk + ((copies + per_block - 1) / per_block) * ((job.m + kRows - 1) / kRows));
-    kernel<<<grid, 256, 0, s>>>(job, sk, ut, ldu, copies, L, shift, inv_f, tame_y, look);
+  // A block goes through its pairs in turns of 256 lanes, so one of 64 rows takes several times the latency of a turn
+  // where there are multiprocessors left for more blocks of fewer: as few rows as give each of them a block, but not
+  // fewer than a turn takes with all levels at once. us a search, 64 rows and these: 8 copies x 48 dimensions in two
+  // blocks, 64 queries 78 and 71, 300 79.5 and 73.7, 1 000 92 and 87; 64 copies, one round, 100 49 and 43; 20 x 96 in
+  // three blocks, 300 51 and 47. The sums of a block take as long for fewer rows: with three blocks for a
+  // multiprocessor 64 copies and 1 000 queries take 73 us instead of 62, 40 x 768 dimensions and 300 111 instead of 97.
+  auto launch        = [&](auto kernel, int copies_a_block, int group) {
+    const int tiles = (copies + copies_a_block - 1) / copies_a_block;
+    const int fit   = std::max(1, (sms / job.beside - sk) / tiles);
+    const int least = 256 / (group * copies_a_block * std::max(L, 1));
+    const int rows  = std::min(kRows, (std::max({(job.m + fit - 1) / fit, least, 1}) + 3) & ~3);
+    const unsigned grid = static_cast<unsigned>(sk + tiles * ((job.m + rows - 1) / rows));
+    kernel<<<grid, 256, 0, s>>>(job, sk, rows, ut, ldu, copies, L, shift, inv_f, tame_y, look);
   };
   switch (blocks) {
-    case 1: launch(project_lookup_kernel<1>, ord_shape<1>::kC); break;
-    case 2: launch(project_lookup_kernel<2>, ord_shape<2>::kC); break;
-    case 3: launch(project_lookup_kernel<3>, ord_shape<3>::kC); break;
-    case 4: launch(project_lookup_kernel<4>, ord_shape<4>::kC); break;
-    case 5: launch(project_lookup_kernel<5>, ord_shape<5>::kC); break;
-    case 6: launch(project_lookup_kernel<6>, ord_shape<6>::kC); break;
-    case 8: launch(project_lookup_kernel<8>, ord_shape<8>::kC); break;
+    case 1: launch(project_lookup_kernel<1>, ord_shape<1>::kC, kGroup<1>); break;
+    case 2: launch(project_lookup_kernel<2>, ord_shape<2>::kC, kGroup<2>); break;
+    case 3: launch(project_lookup_kernel<3>, ord_shape<3>::kC, kGroup<3>); break;
+    case 4: launch(project_lookup_kernel<4>, ord_shape<4>::kC, kGroup<4>); break;
+    case 5: launch(project_lookup_kernel<5>, ord_shape<5>::kC, kGroup<5>); break;
+    case 6: launch(project_lookup_kernel<6>, ord_shape<6>::kC, kGroup<6>); break;
+    case 8: launch(project_lookup_kernel<8>, ord_shape<8>::kC, kGroup<8>); break;
     default: break;  // the loader rejects other block counts
   }
 }

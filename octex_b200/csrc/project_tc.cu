@@ -13,7 +13,7 @@
 // rounds them to fp16 and hands them through shared memory to groups of four lanes, one block of
 // eight coordinates each, which decode the populated spacings and look their cells up.
 //
-// A tile is 128 queries x 64 coordinates (two copies), a block 256 threads. The projections come in by
+// A tile is 128 queries (fewer in the spread form) x 64 coordinates (two copies), a block 256 threads. The projections come in by
 // TMA (cp.async.bulk.tensor, no cluster forms), 64 rows x 64 halves (128 bytes, the swizzle span) a
 // step; the queries are read as fp32 by all threads and written in the same swizzled layout; one
 // thread issues the copies and the MMAs; every wait on an mbarrier is bounded and a wait that runs out
@@ -33,6 +33,7 @@
 #include "prep_common.cuh"
 #include "tc_common.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 namespace octex_b200::kernels {
@@ -45,7 +46,8 @@ constexpr int kTileN    = 32 * kCopies;
 constexpr int kStages   = 2;
 constexpr int kThreads  = 256;  // two warps per TMEM lane quarter, one copy each
 constexpr int kTmemCols = 2 * kTileN;  // two fp32 accumulators
-constexpr int kBulkBlocks = 2;  // blocks per SM of the form for large batches: 128 registers per thread
+constexpr int kBulkBlocks   = 2;  // blocks per SM of the form for large batches: 128 registers per thread
+constexpr int kSpreadBlocks = 3;  // and of the form for others: 80
 constexpr uint32_t kBBytes = kTileN * kTileK * 2;
 
 struct __align__(1024) tc_smem {
@@ -66,12 +68,12 @@ static_assert(sizeof(tc_smem::a) >= sizeof(float) * (sketch_tile<1>::kWords > sk
                                                                                                       : sketch_tile<4>::kWords),
               "staging of the sketch blocks");
 
-/// Centred fp16 queries [row0, row0 + 128) x dimensions [d0, d0 + 64) into an operand tile with the
-/// 128-byte swizzle (16-byte chunk c of row r at chunk c ^ (r % 8)). Rows beyond the batch are left
+/// Centred fp16 queries [row0, end) (128 at most) x dimensions [d0, d0 + 64) into an operand tile with the
+/// 128-byte swizzle (16-byte chunk c of row r at chunk c ^ (r % 8)). Rows beyond are left
 /// as they are: an accumulator row depends on its own operand row only.
 template <bool kVec>
 __device__ __forceinline__ void fill_queries(__half* tile, const float* __restrict__ q, const float* __restrict__ mean,
-                                             int row0, int m, int D, int d0)
+                                             int row0, int end, int D, int d0)
 {
   const int part = threadIdx.x & 15, d = d0 + 4 * part;
   float mu[4];
@@ -85,7 +87,7 @@ __device__ __forceinline__ void fill_queries(__half* tile, const float* __restri
 #pragma unroll
     for (int i = 0; i < 4; i++)
       v[u][i] = mu[i];
-    if (row0 + r < m) {
+    if (row0 + r < end) {
       const float* src = q + static_cast<int64_t>(row0 + r) * D + d;
       if constexpr (kVec) {
         if (d < D) {
@@ -102,7 +104,7 @@ __device__ __forceinline__ void fill_queries(__half* tile, const float* __restri
 #pragma unroll
   for (int u = 0; u < 8; u++) {
     const int r = (threadIdx.x >> 4) + 16 * u;
-    if (row0 + r >= m) continue;
+    if (row0 + r >= end) continue;
     __half h[4];
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -122,11 +124,12 @@ __device__ __forceinline__ void fill_queries(__half* tile, const float* __restri
 // fit its two stages. Which: project_decode_tc.
 enum class tc_mode { taps, spread, bulk };
 template <bool kVec, tc_mode kMode>
-__global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode == tc_mode::spread ? 3 : kBulkBlocks)
+__global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode == tc_mode::spread ? kSpreadBlocks : kBulkBlocks)
   project_decode_tc_kernel(
   const __grid_constant__ CUtensorMap map_b,
   const sketch_job job,
   int sk_blocks,
+  int rows,
   int Cg,
   int L,
   int nkb,
@@ -153,7 +156,7 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
   const int m = job.m, D = job.D;
   const int N       = Cg * 32;
   const int tiles_n = (Cg + kCopies - 1) / kCopies;
-  const int tiles   = tiles_n * ((m + kTileM - 1) / kTileM);
+  const int tiles   = tiles_n * ((m + rows - 1) / rows);
   // the block's tiles, the copies of a tile of queries side by side
   int tile = blockIdx.x - sk_blocks, last = tile + 1;
   if constexpr (kMode == tc_mode::bulk) {
@@ -226,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
   // all threads: the queries of a tile into the operand stages, when they fit whole
   auto fill_all = [&](int tile_m) {
     for (int kb = 0; kb < nkb; kb++)
-      fill_queries<kVec>(sm.a[kb], job.q, job.mean, tile_m * kTileM, m, D, kb * kTileK);
+      fill_queries<kVec>(sm.a[kb], job.q, job.mean, tile_m * rows, min(m, (tile_m + 1) * rows), D, kb * kTileK);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read what was just written
     __syncthreads();
   };
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
           if (!ready) sm.failed = 1;
           if (ready && threadIdx.x == 0) load_projections(tile, kb, 0);
         }
-        if (ready) fill_queries<kVec>(sm.a[s], job.q, job.mean, tile_m * kTileM, m, D, kb * kTileK);
+        if (ready) fill_queries<kVec>(sm.a[s], job.q, job.mean, tile_m * rows, min(m, (tile_m + 1) * rows), D, kb * kTileK);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0 && ready) {
@@ -314,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
 
     // warp w reads TMEM lanes 32 (w % 4) .. + 31; warps 0-3 take the first copy of the tile, 4-7 the second
     const int quarter = warp & 3, cc = warp >> 2;
-    const int row = tile_m * kTileM + quarter * 32 + lane;
+    const int row = tile_m * rows + quarter * 32 + lane;  // (a tile has all 128 in the forms that use it)
     const int c   = tile_n * kCopies + cc;
     uint32_t r[32];
     const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(set * kTileN + cc * 32);
@@ -393,8 +396,8 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
           y[i]           = pack2(f.x, f.y);
         }
       };
-      const int pairs    = min(kTileM, m - tile_m * kTileM) * kCopies;
-      const int64_t row0 = static_cast<int64_t>(tile_m) * kTileM;
+      const int pairs    = min(rows, m - tile_m * rows) * kCopies;
+      const int64_t row0 = static_cast<int64_t>(tile_m) * rows;
       if (!all_ready) {
         // no accumulators: nothing to look up
       } else if (look.stats == nullptr && spread_pays<4>(pairs, L)) {
@@ -442,15 +445,16 @@ void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, c
   const int tiles = ((p.copies + kCopies - 1) / kCopies) * ((job.m + kTileM - 1) / kTileM);
   // rows of the caller's array are read sixteen bytes at a time where they all start on such a boundary
   const bool vec   = job.D % 4 == 0 && reinterpret_cast<uintptr_t>(job.q) % 16 == 0;
-  // A tile for every place on the GPU: the bulk form. Where the line belongs, us of a search of one round
-  // in the form taken and in the other: 64 copies x 128 dimensions, 1 150 queries (288 tiles) 97 and 92,
-  // 1 200 (320) 111 and 109, 1 400 118 and 113, 1 800 123 and 132, 10 000 401 and 465. Up to 128
-  // dimensions it is right to 4 %. Wider rows do not stay in the operand stages from tile to tile, and the
-  // bulk form overtakes later: 200 dimensions, 1 280 queries 135 and 124, 5 000 626 and 631; 512 dimensions,
-  // 1 200 queries 201 and 169, 2 300 229 and 228; 960 dimensions x 48 copies, 1 800 queries 334 and 257,
-  // 6 000 1 115 and 1 161.
-  const int places = kBulkBlocks * p.sms;
-  const auto mode  = look.table == nullptr ? tc_mode::taps : tiles >= places ? tc_mode::bulk : tc_mode::spread;
+  // More tiles than the GPU has places for blocks of the spread form (half of them where two launches share it, for the
+  // halves of a batch): the bulk form, a block for each of its own places. us of a search of one round, 64 copies x 128
+  // dimensions, in this form and, with the line at a tile for each place of the bulk form, in the other: 1 184
+  // queries (320 tiles) 104 spread and 112 bulk; halves of 800 127 bulk and 148 spread, of 1 000 134 and 173; of 1 250 164
+  // bulk, 205 spread. Wider rows do not stay in the operand stages from tile to tile, and the line stays where it was:
+  // 200 dimensions x 200 copies, 300 queries 101 bulk and 84 spread, but 256 x 64, 1 200 107 and 116; 512 x 64, 1 200
+  // 121 and 116, 2 300 168 and 161; 960 x 48, 6 000 1 115 and 1 161.
+  const int places = kBulkBlocks * p.sms, spread_places = kSpreadBlocks * p.sms / job.beside;
+  const bool many  = p.ldu <= kStages * kTileK ? tiles > spread_places - sketch_blocks<1>(job) : tiles >= places;
+  const auto mode  = look.table == nullptr ? tc_mode::taps : many ? tc_mode::bulk : tc_mode::spread;
   const auto pick  = [&](auto taps, auto spread, auto bulk) {
     return mode == tc_mode::taps ? taps : mode == tc_mode::spread ? spread : bulk;
   };
@@ -460,8 +464,23 @@ void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, c
         : pick(project_decode_tc_kernel<false, tc_mode::taps>, project_decode_tc_kernel<false, tc_mode::spread>,
                project_decode_tc_kernel<false, tc_mode::bulk>);
   const int sk        = mode == tc_mode::bulk ? sketch_blocks<4>(job) : sketch_blocks<1>(job);
-  const unsigned grid = static_cast<unsigned>(mode == tc_mode::bulk ? places : sk + tiles);
-  kernel<<<grid, kThreads, sizeof(tc_smem) + 1024, s>>>(b, job, sk, p.copies, L, p.ldu / kTileK, shift, inv_f, tame_y,
+  // Queries of a tile in the spread form: a block goes through its pairs in turns of 64, so a tile of 128 queries takes
+  // four times a block's latency where three blocks of fewer would fit a multiprocessor. As few as give every place
+  // a block, but not fewer than keep its threads busy in one turn. us of a search of one round, 128 a tile and these: 64
+  // copies x 128 dimensions, 17 queries 48.5 and 46.0, 100 64.3 and 52.6, 300 74.8 and 62.2, 600 85.6 and 78.8, 1 000 100 and
+  // 95; 8 x 64, 300 62 and 47, 1 000 66 and 53. The operands of wide rows are most of a tile's time: 256 dimensions 148
+  // 68 and 58, 300 71 and 67, but 600 (48 a tile) 78.1 and 79.7, 1 000 94 and 99; 960, 999 132 and 146.
+  int rows = kTileM;
+  if (mode == tc_mode::spread) {
+    const int tiles_n = (p.copies + kCopies - 1) / kCopies;
+    const int fit     = std::max(1, (spread_places - sk) / tiles_n);
+    const int least   = std::max(1, kThreads / (4 * kCopies * L));
+    const int split   = std::min(kTileM, (std::max((job.m + fit - 1) / fit, least) + 3) & ~3);
+    if (p.ldu <= kStages * kTileK || (p.ldu <= 2 * kStages * kTileK && split <= kTileM / 3)) rows = split;
+  }
+  const unsigned grid = static_cast<unsigned>(
+    mode == tc_mode::bulk ? places : sk + ((p.copies + kCopies - 1) / kCopies) * ((job.m + rows - 1) / rows));
+  kernel<<<grid, kThreads, sizeof(tc_smem) + 1024, s>>>(b, job, sk, rows, p.copies, L, p.ldu / kTileK, shift, inv_f, tame_y,
                                                         codes, Yout, look, error);
 }
 

@@ -284,6 +284,7 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
   kernels::sketch_job job;
   job.q = io.q + first * D, job.mean = p.mean.as<float>(), job.basis = p.basis.as<float>();
   job.m = m1, job.D = D, job.S = sw;
+  job.beside = part != nullptr ? 2 : 1;
   job.qs   = pl.qs.as<float>() + first * sw;
   job.keep = io.q == pl.qbuf.as<float>() ? nullptr : pl.qbuf.as<float>() + first * D;
   kernels::tc_lookup look;
@@ -305,7 +306,7 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
   } else if (!pl.dbg.taps) {
     mark();
     kernels::project_lookup_ordered(job, ix.blocks, p.ut.as<__half>(), p.ldu, p.copies, L, p.shift.as<__half>(),
-                                    p.inv_f.as<float>(), finest, look, s);
+                                    p.inv_f.as<float>(), finest, look, pl.r1.sms, s);
     mark();
     mark();
   } else {

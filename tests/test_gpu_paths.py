@@ -340,6 +340,21 @@ def test_results_are_plain_tensors():
     idx.close()
 
 
+@pytest.mark.parametrize("copies,dim,n", [(64, 128, 149), (64, 128, 300), (64, 64, 1001), (63, 128, 1184), (64, 128, 1700),
+                                          (40, 200, 150), (40, 200, 500), (64, 256, 301)])
+def test_projection_tiles_of_fewer_queries(copies, dim, n):
+    """The spread form of the projection with the tiles that give every place on the GPU a block: rows that are no
+    multiple of them, wide rows where they are split and where not, the line to the bulk form, halves of a batch."""
+    from octex_b200 import synth
+    idx, _ = make_index(dim, rows=3000, copies=copies, blocks=4, pca_dims=64)
+    kw = dict(read=8, starts=16, waves=0, rerank=32)
+    queries = synth.plumbing(n, dim, seed=8)
+    want, seg = inspected(idx, queries, 10, **kw)
+    assert same(idx.search(queries, 10, **kw), want)
+    assert np.array_equal(idx.fetch("seg", np.int32), seg)
+    idx.close()
+
+
 def test_more_plans_than_words():
     """A plan's arrays are pieces of one block and its give-up word one of 64 of the index: many configurations one
     after the other, each the answer of a handle that knows only this one."""
