@@ -37,7 +37,7 @@
 // 200 001 x 128, K = 64, ms: 133 with a list update per improvement; 20.5 with buffers in shared memory that the
 // epilogue merges itself and norms it adds; 18.3 with list warps and norms in the MMAs; 15.0 with the groups read
 // again from TMEM (instead of 64 columns kept in registers until it is known which are wanted); 14.2 with the next 32
-// columns on their way while 32 are looked at, 14.5 with the norms last. Two warps per row, a half of the columns each:
+// columns on their way while 32 are looked at, 14.5 with the norms last, 14.3 looking through without votes. Two warps per row, a half of the columns each:
 // 18.7.
 //
 // Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues), warp 3 makes the norm
@@ -60,7 +60,6 @@ constexpr int kKnnThreads = 512;  // a copy warp, an MMA warp per set, a warp fo
 constexpr int kTmemCols   = 512;  // two accumulators of 128 fp32 columns per set
 constexpr int kMaxStages  = 6;
 constexpr int kNoted      = 32;   // improvements a row notes for a merge, in global memory, twice
-constexpr int kHitRoom    = 6;    // groups of four columns a thread may have set aside
 constexpr int kHitBytes   = 640;  // of a warp's groups at one place: four values and a row per lane
 constexpr uint32_t kIdleLimit = 1u << 28;  // looks of a list warp for something to merge before it gives up
 constexpr int kVisitsPerK = 3;    // tiles looked at for the bars, per entry of a list
@@ -87,11 +86,12 @@ static_assert(sizeof(knn_ctl) <= kCtlBytes && kCtlBytes % 16 == 0, "control bloc
 struct knn_shape {
   int stages;    // of 64 dimensions of a tile (and of the query rows, when those do not stay)
   int resident;  // the query rows stay in shared memory
+  int room;      // groups of four columns a thread may have set aside, at most kNoted / 4
   __host__ __device__ size_t stage_bytes() const { return (resident ? 1 : 3) * static_cast<size_t>(kPartBytes); }
   __host__ __device__ size_t query_bytes(int nkb) const { return resident ? 2 * static_cast<size_t>(nkb) * kPartBytes : 0; }
   size_t smem_bytes(int nkb) const
   {
-    return 1024 + query_bytes(nkb) + stages * stage_bytes() + 3 * kNormBytes + kCtlBytes + 8 * kHitRoom * kHitBytes;
+    return 1024 + query_bytes(nkb) + stages * stage_bytes() + 3 * kNormBytes + kCtlBytes + 8 * room * kHitBytes;
   }
 };
 
@@ -192,12 +192,23 @@ __device__ __forceinline__ unsigned above_bar(const float (&v)[4], float bar)
   return __funnelshift_l(d[0], __funnelshift_l(d[1], __funnelshift_l(d[2], d[3] >> 31, 1), 1), 1);
 }
 
-/// Sets four accumulators and the row of the first aside at the shared-memory address `at`, which moves on.
-__device__ __forceinline__ void set_aside(uint32_t& at, uint32_t to_first, const uint32_t (&v)[4], int first)
+/// Sets four accumulators and the row of the first aside at the shared-memory address `at`, which moves on, where
+/// `wanted` is not zero; no branch.
+__device__ __forceinline__ void set_aside(unsigned wanted, uint32_t& at, uint32_t to_first, const uint32_t (&v)[4], int first)
 {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-  asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + to_first), "r"(first) : "memory");
-  at += kHitBytes;
+  asm volatile(
+    "{\n\t"
+    ".reg .pred p;\n\t"
+    ".reg .b32 a;\n\t"
+    "setp.ne.u32 p, %1, 0;\n\t"
+    "add.u32 a, %0, %2;\n\t"
+    "@p st.shared.v4.b32 [%0], {%3, %4, %5, %6};\n\t"
+    "@p st.shared.b32 [a], %7;\n\t"
+    "@p add.u32 %0, %0, %8;\n\t"
+    "}"
+    : "+r"(at)
+    : "r"(wanted), "r"(to_first), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(first), "n"(kHitBytes)
+    : "memory");
 }
 
 /// Keys in the order of (value, row); no value is NaN or -0.
@@ -513,9 +524,9 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
       volatile float* list_bar  = ctl.bar + set * kTile + quarter * 32 + lane;
       *list_bar                 = -INFINITY;
       // groups of four columns with an improvement: the four values, and the first one's row `to_first` bytes behind
-      const uint32_t hit0     = smem_u32(hits) + (warp - 4) * kHitRoom * kHitBytes + lane * 16;
+      const uint32_t hit0     = smem_u32(hits) + (warp - 4) * shape.room * kHitBytes + lane * 16;
       const uint32_t to_first = 512 - 12 * lane;
-      const uint32_t hit_end  = hit0 + (kHitRoom - 2) * kHitBytes;  // beyond it there is no room for two more
+      const uint32_t hit_end  = hit0 + (shape.room - 4) * kHitBytes;  // beyond it there is no room for four more
       uint32_t hit            = hit0;                               // where the next one goes
       // the notes of the rows whose lanes ask for it go to the list warps; the lanes go on in the other buffer
       auto hand_over = [&](bool asks) {
@@ -534,25 +545,25 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
         }
         __syncwarp();
       };
-      // the improvements among the groups of columns set aside; a row without room for four more hands its notes over
+      // the improvements among the groups of columns set aside; a row whose notes may not hold them hands these over first
       auto look_through = [&]() {
+        const bool asks = count != 0 && count + 4 * static_cast<int>((hit - hit0) / kHitBytes) > kNoted;
+        if (__any_sync(0xffffffffu, asks)) hand_over(asks);
 #pragma unroll 1
-        for (uint32_t e = hit0; ok && __any_sync(0xffffffffu, e < hit); e += kHitBytes) {
-          if (__any_sync(0xffffffffu, count > kNoted - 4)) hand_over(count > kNoted - 4);
-          if (ok && e < hit) {
-            float v[4];
-            int first;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                         : "r"(e)
-                         : "memory");
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(first) : "r"(e + to_first) : "memory");
+        for (uint32_t e = hit0; ok && e < hit; e += kHitBytes) {
+          float v[4];
+          int first;
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                       : "r"(e)
+                       : "memory");
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(first) : "r"(e + to_first) : "memory");
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-              if (v[i] > bar && first + i != row)
-                mine[buffer * kNoted + count++] = make_float2(fmaf(-2.0f, v[i], 0.0f), __int_as_float(first + i));
-          }
+          for (int i = 0; i < 4; i++)
+            if (v[i] > bar && first + i != row)
+              mine[buffer * kNoted + count++] = make_float2(fmaf(-2.0f, v[i], 0.0f), __int_as_float(first + i));
         }
+        __syncwarp();
         hit = hit0;
       };
       // a row itself is no neighbor
@@ -566,8 +577,8 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
       // The 128 columns of an accumulator, the next 32 on their way while the ones before are looked at. The largest of
       // every four is compared with the bar, which leaves a bit for each. Of the few groups in which one of the warp's
       // rows has an improvement the columns are read once more, two groups at a time, and set aside by the rows that
-      // want them: to keep them in registers for that, or to set the groups aside at once, every one under a predicate,
-      // takes longer than the second reading.
+      // want them: to keep them in registers for that, to choose a row's group among them by its bits or to set the
+      // groups aside at once, every one under a predicate, takes longer than the second reading.
       auto scan = [&](uint32_t columns, int first) {
         auto improvements = [&](const uint32_t (&r)[32]) {
           unsigned bits = 0;
@@ -602,8 +613,8 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
           tmem_ld4(columns + 4 * g, v[0]);
           tmem_ld4(columns + 4 * g2, v[1]);
           tmem_ld_wait();
-          if (own >> g & 1u) set_aside(hit, to_first, v[0], first + 4 * g);
-          if (g2 != g && (own >> g2 & 1u)) set_aside(hit, to_first, v[1], first + 4 * g2);
+          set_aside(own >> g & 1u, hit, to_first, v[0], first + 4 * g);
+          set_aside(g2 != g ? own >> g2 & 1u : 0u, hit, to_first, v[1], first + 4 * g2);
           if (__any_sync(0xffffffffu, hit > hit_end)) look_through();
         }
       };
@@ -773,10 +784,13 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
 knn_shape choose_shape(int nkb)
 {
   constexpr size_t kLimit = 227 * 1024;
-  knn_shape fit{kMaxStages, 1};
-  while (fit.stages > 3 && fit.smem_bytes(nkb) > kLimit)
-    fit.stages--;
-  return fit.smem_bytes(nkb) <= kLimit ? fit : knn_shape{3, 0};
+  for (const int room : {8, 6}) {
+    knn_shape fit{kMaxStages, 1, room};
+    while (fit.stages > 3 && fit.smem_bytes(nkb) > kLimit)
+      fit.stages--;
+    if (fit.smem_bytes(nkb) <= kLimit) return fit;
+  }
+  return knn_shape{3, 0, 8};
 }
 
 }  // namespace
