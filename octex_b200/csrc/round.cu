@@ -653,6 +653,41 @@ __device__ __forceinline__ float sketch_chunk8(unsigned w0, unsigned w1, const f
   return d;
 }
 
+/// Two fp32 values side by side.
+using f32_two = unsigned long long;
+__device__ __forceinline__ f32_two two_of(float a, float b)
+{
+  f32_two r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+/// Sixteen int8 codes: sketch_chunk8 of either eight, side by side in packed multiply-adds, then the sum of the two.
+/// s [8] and minus_q [8]: scale and negated query value of codes i and 8 + i.
+__device__ __forceinline__ float sketch_chunk16(const uint4& w, const f32_two* s, const f32_two* minus_q)
+{
+  const unsigned x[4] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u, w.z ^ 0x80808080u, w.w ^ 0x80808080u};  // code + 128
+  f32_two d           = 0;
+#pragma unroll
+  for (int p = 0; p < 4; p++) {
+    const unsigned two = (p & 1) ? 0x4342 : 0x4140;
+    const unsigned a   = __byte_perm(x[p < 2 ? 0 : 1], 0x64646464u, two);
+    const unsigned b   = __byte_perm(x[p < 2 ? 2 : 3], 0x64646464u, two);
+    const f32_two c0   = two_of(half_minus(static_cast<unsigned short>(a & 0xffffu), 1152.0f),
+                                half_minus(static_cast<unsigned short>(b & 0xffffu), 1152.0f));
+    const f32_two c1   = two_of(half_minus(static_cast<unsigned short>(a >> 16), 1152.0f),
+                                half_minus(static_cast<unsigned short>(b >> 16), 1152.0f));
+    f32_two t;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t) : "l"(c0), "l"(s[2 * p]), "l"(minus_q[2 * p]));
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(t), "l"(d));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t) : "l"(c1), "l"(s[2 * p + 1]), "l"(minus_q[2 * p + 1]));
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(t), "l"(d));
+  }
+  float d0, d1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d0), "=f"(d1) : "l"(d));
+  return __fadd_rn(d0, d1);
+}
+
 /// The sketch distance in the reference's own fp32 terms, sum_k (c_k s_k - q_k)^2
 /// (search_kernels.cuh:228-251), for the waves: there a candidate's row arrives from memory later
 /// than the arithmetic on it takes, so the form that needs nothing but the row (no row constant)
@@ -663,7 +698,11 @@ __device__ __forceinline__ float sketch_chunk8(unsigned w0, unsigned w1, const f
 /// holds two neighbouring chunks (one 16-byte load) and adds them itself (stride 1); kLw (a power
 /// of two >= S / 16) lanes own a row; two rows per lane group are in flight. A lane past the last
 /// chunk works on chunk 0 with scales and query 0 and adds exactly 0.
-template <int kLw, bool kDealt>
+/// kPaired: the two chunks of a lane in packed operations, half as many to issue, for the waves (us a search, one by one
+/// and packed: three waves of 16 384 entries 7 992 and 7 869, of 32 768 ranked by sketch distance 3 429 and 3 334, of 4 096
+/// 1 807 and 1 734, 10 000 tuned 835 and 829, 1 000 with default parameters 291 and 287). First rounds that rank by
+/// sketch distance spill with it: 355 and 366.
+template <int kLw, bool kDealt, bool kPaired>
 __device__ __forceinline__ void sketch_rows_f32(const int* cand, int n, const signed char* __restrict__ sketch,
                                                 const row_map& map, int S, const float* sc, const float* qv,
                                                 float* dist)
@@ -682,6 +721,12 @@ __device__ __forceinline__ void sketch_rows_f32(const int* cand, int n, const si
     const float4 q4 = live ? reinterpret_cast<const float4*>(qv + sub * 16)[b] : make_float4(0.f, 0.f, 0.f, 0.f);
     cs[4 * b] = s4.x, cs[4 * b + 1] = s4.y, cs[4 * b + 2] = s4.z, cs[4 * b + 3] = s4.w;
     cq[4 * b] = q4.x, cq[4 * b + 1] = q4.y, cq[4 * b + 2] = q4.z, cq[4 * b + 3] = q4.w;
+  }
+  f32_two s2[8], q2[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    s2[i] = two_of(cs[i], cs[8 + i]);
+    q2[i] = two_of(-cq[i], -cq[8 + i]);
   }
   const int rpp = nw * kG;  // rows per step of the block
   if (n <= 0) return;
@@ -705,9 +750,11 @@ __device__ __forceinline__ void sketch_rows_f32(const int* cand, int n, const si
       id[u] = cand[min(j[u] + 2 * rpp, n - 1)];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const float d0 = sketch_chunk8(w[u].x, w[u].y, cs, cq);
-      const float d1 = sketch_chunk8(w[u].z, w[u].w, cs + 8, cq + 8);
-      float d        = __fadd_rn(d0, d1);
+      float d;
+      if constexpr (kPaired)
+        d = sketch_chunk16(w[u], s2, q2);
+      else
+        d = __fadd_rn(sketch_chunk8(w[u].x, w[u].y, cs, cq), sketch_chunk8(w[u].z, w[u].w, cs + 8, cq + 8));
 #pragma unroll
       for (int o = 1; o < kLw; o <<= 1)
         d = __fadd_rn(d, __shfl_xor_sync(0xffffffffu, d, o));
@@ -1195,17 +1242,17 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   if (!int_form) {
     const float* qv = reinterpret_cast<const float*>(w16);
     if (S <= 16) {
-      sketch_rows_f32<1, kDealt>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<1, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 32) {
-      sketch_rows_f32<2, kDealt>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<2, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 64) {
-      sketch_rows_f32<4, kDealt>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<4, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 128) {
-      sketch_rows_f32<8, kDealt>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<8, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 256) {
-      sketch_rows_f32<16, kDealt>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<16, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else {
-      sketch_rows_f32<32, kDealt>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<32, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     }
   } else {
     const bool keep = a.keep_sketch != 0 && may_prefetch<kDealt>(a.sketch_map);
