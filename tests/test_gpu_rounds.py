@@ -254,3 +254,36 @@ def test_members_of_the_bin_at_the_cut(oracle, members, near, threads):
     idx.set_debug()
     against_checker(oracle, idx, dict(arrays, table=table), meta, np.repeat(query, n, axis=0), 65, waves=1, **kw)
     idx.close()
+
+
+@pytest.mark.parametrize("width", [16, 32, 48, 64, 80, 128, 144, 256, 320])
+def test_sketch_distances_of_waves(width):
+    """The fp32 sketch distances a wave and a first round give, at every number of lanes a row takes and with lanes past
+    the last chunk: chunks of eight codes, two fused multiply-adds a code, then a butterfly. float64 has every
+    product and sum before a rounding exactly, but for an addition that is rounded twice about once in 2^29."""
+    from octex_b200 import build_index, synth
+    base = synth.plumbing(3000, 320, seed=0)
+    arrays, meta = build_index.build_arrays(base, small_params(pca_dims=64, list_len=16, min_cell=2, sketch_width=width, table_len=24),
+                                            device="cpu")
+    idx = octex_b200.attach(arrays, meta, borrow=False)
+    queries = synth.plumbing(40, 320, seed=9)
+    kw = dict(read=4, starts=64, sketch_rank=True, final_rerank=0)
+    scale, codes = arrays["sketch_scale"].astype(np.float32), arrays["sketch"].reshape(3000, width).astype(np.float64)
+    for waves in (0, 2):
+        d, ids = idx.search(queries, 64, waves=waves, **kw)
+        qs = idx.fetch("qs", np.float32).reshape(-1, width)[:40].astype(np.float64)
+        live = ids >= 0
+        t = (codes[ids] * scale.astype(np.float64) - qs[:, None]).astype(np.float32).astype(np.float64)
+        part = np.zeros((40, 64, width // 8), np.float32)
+        for i in range(8):
+            part = (t[:, :, i::8] ** 2 + part).astype(np.float32)
+        lanes = 1
+        while lanes < width // 8:
+            lanes *= 2
+        part = np.concatenate([part, np.zeros((40, 64, lanes - width // 8), np.float32)], 2)
+        while lanes > 1:
+            part = part[:, :, 0::2] + part[:, :, 1::2]
+            lanes //= 2
+        assert live.sum() > 400  # (the lists of a first round hold about twenty rows a query)
+        assert np.array_equal(part[:, :, 0][live], d[live]), (waves, width)
+    idx.close()
