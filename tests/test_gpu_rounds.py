@@ -256,11 +256,28 @@ def test_members_of_the_bin_at_the_cut(oracle, members, near, threads):
     idx.close()
 
 
+def sketch_distances(codes, scale, qs):
+    """fp32 sketch distances [..., rows] of int8 codes [..., rows, width] to queries [..., width], bit for bit: chunks of
+    eight codes, two fused multiply-adds a code, then a butterfly over the next power of two of them. float64 has every
+    product and sum before a rounding exactly, but for an addition that is rounded twice about once in 2^29."""
+    t = (codes.astype(np.float64) * scale.astype(np.float64) - qs.astype(np.float64)[..., None, :]).astype(np.float32).astype(np.float64)
+    part = np.zeros(t.shape[:-1] + (t.shape[-1] // 8,), np.float32)
+    for i in range(8):
+        part = (t[..., i::8] ** 2 + part).astype(np.float32)
+    lanes = 1
+    while lanes < part.shape[-1]:
+        lanes *= 2
+    part = np.concatenate([part, np.zeros(part.shape[:-1] + (lanes - part.shape[-1],), np.float32)], -1)
+    while lanes > 1:
+        part = part[..., 0::2] + part[..., 1::2]
+        lanes //= 2
+    return part[..., 0]
+
+
 @pytest.mark.parametrize("width", [16, 32, 48, 64, 80, 128, 144, 256, 320])
 def test_sketch_distances_of_waves(width):
     """The fp32 sketch distances a wave and a first round give, at every number of lanes a row takes and with lanes past
-    the last chunk: chunks of eight codes, two fused multiply-adds a code, then a butterfly. float64 has every
-    product and sum before a rounding exactly, but for an addition that is rounded twice about once in 2^29."""
+    the last chunk."""
     from octex_b200 import build_index, synth
     base = synth.plumbing(3000, 320, seed=0)
     arrays, meta = build_index.build_arrays(base, small_params(pca_dims=64, list_len=16, min_cell=2, sketch_width=width, table_len=24),
@@ -268,22 +285,48 @@ def test_sketch_distances_of_waves(width):
     idx = octex_b200.attach(arrays, meta, borrow=False)
     queries = synth.plumbing(40, 320, seed=9)
     kw = dict(read=4, starts=64, sketch_rank=True, final_rerank=0)
-    scale, codes = arrays["sketch_scale"].astype(np.float32), arrays["sketch"].reshape(3000, width).astype(np.float64)
+    codes = arrays["sketch"].reshape(3000, width)
     for waves in (0, 2):
         d, ids = idx.search(queries, 64, waves=waves, **kw)
-        qs = idx.fetch("qs", np.float32).reshape(-1, width)[:40].astype(np.float64)
+        qs = idx.fetch("qs", np.float32).reshape(-1, width)[:40]
         live = ids >= 0
-        t = (codes[ids] * scale.astype(np.float64) - qs[:, None]).astype(np.float32).astype(np.float64)
-        part = np.zeros((40, 64, width // 8), np.float32)
-        for i in range(8):
-            part = (t[:, :, i::8] ** 2 + part).astype(np.float32)
-        lanes = 1
-        while lanes < width // 8:
-            lanes *= 2
-        part = np.concatenate([part, np.zeros((40, 64, lanes - width // 8), np.float32)], 2)
-        while lanes > 1:
-            part = part[:, :, 0::2] + part[:, :, 1::2]
-            lanes //= 2
         assert live.sum() > 400  # (the lists of a first round hold about twenty rows a query)
-        assert np.array_equal(part[:, :, 0][live], d[live]), (waves, width)
+        assert np.array_equal(sketch_distances(codes[ids], arrays["sketch_scale"], qs)[live], d[live]), (waves, width)
+    idx.close()
+
+
+@pytest.mark.parametrize("starts,table_len,queries", [(16, 24, 3), (64, 24, 40), (200, 32, 700), (512, 32, 2), (512, 32, 160),
+                                                      (700, 32, 20)])
+def test_kept_lists_by_sketch(starts, table_len, queries):
+    """Waves that rank by sketch distance: a full kept list lets only nearer candidates through, which a selection
+    goes through where they are more than the list takes. Against the rule itself from the first round's candidates
+    on: a wave expands the first kept rows that none did before, and the nearest of all stay; blocks of every size,
+    fewer candidates than a step of the block's threads and several steps of them."""
+    from octex_b200 import build_index, synth
+    rows, width = 6000, 32
+    base = synth.plumbing(rows, 64, seed=0)
+    arrays, meta = build_index.build_arrays(base, small_params(pca_dims=64, list_len=64, min_cell=2, sketch_width=width,
+                                                               table_len=table_len), device="cpu")
+    idx = octex_b200.attach(arrays, meta, borrow=False)
+    q = synth.plumbing(queries, 64, seed=7)
+    kw = dict(read=64, starts=starts, waves=3, sketch_rank=True, final_rerank=0)
+    d, ids = idx.search(q, starts, **kw)
+    idx.set_debug(taps=True)
+    idx.search(q, starts, **kw)
+    qs = idx.fetch("qs", np.float32).reshape(-1, width)
+    n1, cand = idx.fetch("n1", np.int32), idx.fetch("cand1", np.int32)
+    cand = cand.reshape(len(n1), -1)
+    idx.set_debug()
+    codes, scale, table = arrays["sketch"].reshape(rows, width), arrays["sketch_scale"], arrays["table"].reshape(rows, -1)
+    for i in range(0, queries, max(1, queries // 20)):
+        dist = sketch_distances(codes, scale, qs[i])
+        seen, done = set(cand[i, :n1[i]].tolist()), set()
+        for _ in range(3):
+            kept = sorted(seen, key=lambda r: (dist[r], r))[:starts]
+            new = [r for r in kept if r not in done][:starts]
+            done |= set(new)
+            seen = set(kept) | (set(table[new].ravel().tolist()) - {-1})
+        kept = sorted(seen, key=lambda r: (dist[r], r))[:starts]
+        assert ids[i, :len(kept)].tolist() == kept, i
+        assert np.array_equal(d[i, :len(kept)], dist[kept])
     idx.close()
