@@ -440,10 +440,30 @@ void capture_batch(index_impl const& ix, plan& pl, cudaStream_t s)
     cudaGraphExecDestroy(pl.graph);
     pl.graph = nullptr;
   }
+  // a large batch of one process in two halves, side by side in the graph (see run_in_place)
+  struct side {
+    cudaStream_t s = nullptr;
+    ~side()
+    {
+      if (s != nullptr) cudaStreamDestroy(s);
+    }
+  } other;
+  if (ix.world == 1 && pl.m >= pl.halves_from && !pl.dbg.stats && !pl.dbg.taps)
+    OCTEX_CUDA_TRY(cudaStreamCreateWithFlags(&other.s, cudaStreamNonBlocking));
   cudaGraph_t graph = nullptr;
   OCTEX_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   try {
-    run_batch(ix, pl, own_io(pl), s, nullptr);
+    if (other.s == nullptr) {
+      run_batch(ix, pl, own_io(pl), s, nullptr);
+    } else {
+      const row_range halves[2] = {{0, (pl.m + 1) / 2}, {(pl.m + 1) / 2, pl.m / 2}};
+      OCTEX_CUDA_TRY(cudaEventRecord(pl.join_ev, s));
+      OCTEX_CUDA_TRY(cudaStreamWaitEvent(other.s, pl.join_ev, 0));
+      run_batch(ix, pl, own_io(pl), s, nullptr, &halves[0]);
+      run_batch(ix, pl, own_io(pl), other.s, nullptr, &halves[1]);
+      OCTEX_CUDA_TRY(cudaEventRecord(pl.join_ev, other.s));
+      OCTEX_CUDA_TRY(cudaStreamWaitEvent(s, pl.join_ev, 0));
+    }
   } catch (...) {
     cudaStreamEndCapture(s, &graph);
     if (graph != nullptr) cudaGraphDestroy(graph);

@@ -473,3 +473,18 @@ def test_halves_and_graphs():
             assert same((dist.cpu().numpy(), ids.cpu().numpy()), want)
         del graph
     idx.close()
+
+
+def test_resident_batches_in_halves():
+    """The graph of a large batch holds its halves side by side, as the search before it ran them: replayed, with
+    fewer queries than the search had, and again after a search of others."""
+    from octex_b200 import synth
+    idx, _ = make_index(64, copies=6)
+    kw = dict(read=8, starts=16, waves=2, rerank=32, wave_rerank=32)
+    queries = synth.plumbing(2600, 64, seed=6)
+    for first in (0, 100):
+        want = idx.search(queries[first:first + 2500], 10, **kw)[1]
+        for n in (2500, 2500, 1301, 40, 2500):
+            idx.search_resident(n, **kw)
+            assert np.array_equal(idx.fetch("kept_ids", np.int64, (n, -1))[:, :10], want[:n]), n
+    idx.close()
