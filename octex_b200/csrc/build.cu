@@ -825,6 +825,17 @@ struct pieces {
   static auto size_of(int64_t count) -> size_t { return (sizeof(T) * static_cast<size_t>(count) + 255) / 256 * 256; }
 };
 
+/// Device, managed or page-locked memory.
+auto known_to_cuda(const void* p) -> bool
+{
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type != cudaMemoryTypeUnregistered;
+}
+
 /// Bytes the sort of a reverse-edge merge works with.
 auto edge_sort_bytes(int64_t edges) -> size_t
 {
@@ -1022,9 +1033,9 @@ void searched_table(resources const& res, index& idx, int k, int passes, bool re
       forward_rows_kernel<<<grid_for(m, 128), 128, 0, s>>>(ids, dist, r0, m, kq, kin, fwd, fd);
       OCTEX_CUDA_TRY(cudaPeekAtLastError());
     }
-    if (v + 1 == passes && table_host != nullptr) {
+    if (v + 1 == passes && table_host != nullptr && !known_to_cuda(table_host)) {
       // The pages of the result come into being while the GPU works: a copy to 13 MB of new ones takes 6.6 ms, to
-      // others 0.9.
+      // others 0.9. (Page-locked memory has its pages, and in a GPU's the host can't write.)
       auto* bytes = reinterpret_cast<volatile char*>(table_host);
       for (size_t at = 0; at < table_bytes; at += 4096)
         bytes[at] = bytes[at];

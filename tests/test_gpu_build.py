@@ -3,14 +3,17 @@ writes, in the manner of the reference's own build tests (cpp/tests/test_build.c
 hpdic/octex): shapes and dtypes of the directory, consistency of the cell arrays, lists made of a
 cell's own rows nearest first, the sketch against its definition, the neighbor table against brute
 force with the reverse-edge rule, and the recall of a search over the result."""
+import ctypes as C
 import json
 import os
 
 import numpy as np
 import pytest
+import torch
 
 import octex_b200
 from conftest import recall
+from octex_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -302,6 +305,24 @@ def test_scans_on_two_streams():
         assert len(got[i]) == 4
         for ids, d in got[i]:
             assert torch.equal(ids, alone[i][0]) and torch.equal(d, alone[i][1])
+
+@pytest.mark.parametrize("kind", ["page-locked", "ordinary", "device"])
+def test_searched_table_destination(built, kind):
+    """The table is returned into memory of any kind, also where the host itself can't write."""
+    path, a, meta, base, queries = built
+    n, k = len(base), 16
+    idx = octex_b200.load(path, devices=[0], placement="replicate")
+    want = idx.searched_table(table_len=k, passes=1)
+    out = {"page-locked": lambda: torch.full((n, k), -7, dtype=torch.int32).pin_memory(),
+           "ordinary": lambda: torch.from_numpy(np.full((n, k), -7, np.int32)),
+           "device": lambda: torch.full((n, k), -7, dtype=torch.int32, device="cuda")}[kind]()
+    lib, res = _lib.lib(), idx._resources(0)
+    status = lib.octexB200SearchedTable(res.h, idx._h, C.c_int32(k), C.c_int32(1), C.c_int32(1), C.c_int32(0),
+                                        C.c_void_p(out.data_ptr()))
+    _lib.check(status)
+    assert np.array_equal(out.cpu().numpy(), want)
+    idx.close()
+
 
 
 def test_searched_table(built, oracle, tmp_path):
