@@ -32,13 +32,13 @@
 //
 // What bounds it: the MMAs. One of 128 x 128 x 16 with both operands in shared memory takes 101 cycles instead
 // of 64 (128 bytes a cycle would be needed), the norms one more of them, and a tile with nothing looked at 2 200
-// of the 2 800 cycles that it takes (200 001 x 128, K = 64: 11.4 of 14.5 ms; 64 dimensions 8.2 of 12.3); the rest is
+// of the 2 800 cycles that it takes (200 001 x 128, K = 64: 11.4 of 14.3 ms; 64 dimensions 8.2 of 11.9); the rest is
 // what the four warps of a set wait for one another when one of them looks through its improvements.
 // 200 001 x 128, K = 64, ms: 133 with a list update per improvement; 20.5 with buffers in shared memory that the
 // epilogue merges itself and norms it adds; 18.3 with list warps and norms in the MMAs; 15.0 with the groups read
 // again from TMEM (instead of 64 columns kept in registers until it is known which are wanted); 14.2 with the next 32
-// columns on their way while 32 are looked at, 14.5 with the norms last, 14.3 looking through without votes. Two warps per row, a half of the columns each:
-// 18.7.
+// columns on their way while 32 are looked at, 14.5 with the norms last, 14.3 looking through without votes. Two
+// warps per row, a half of the columns each: 18.7.
 //
 // Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues), warp 3 makes the norm
 // operands; eight epilogue warps, four per set, one per quarter of the TMEM lanes; four list warps of 64 rows.
