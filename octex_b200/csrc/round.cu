@@ -184,6 +184,68 @@ __device__ __forceinline__ void bitonic_sort(unsigned long long* key, int P)
   }
 }
 
+/// The key of a lane after it met the one `stride` lanes off: the smaller or the larger of the two.
+__device__ __forceinline__ unsigned long long met(unsigned long long mine, int stride, bool smaller)
+{
+  const unsigned long long other = __shfl_xor_sync(0xffffffffu, mine, stride);
+  return (mine < other) == smaller ? mine : other;
+}
+
+/// src[0, count) and kNoKey up to `width` (a power of two, 64 at least) in ascending order into key [width], another
+/// array: the network of bitonic_sort with 64 keys to a warp, two a lane, so that only steps of 64 places and more go
+/// through shared memory and have barriers (6 of the 45 of 512 keys). All threads of the block call it.
+__device__ __forceinline__ void sort_keys(const unsigned long long* src, int count, unsigned long long* key, int width)
+{
+  const int lane = threadIdx.x & 31, warp0 = (threadIdx.x >> 5) * 64, all = blockDim.x * 2;
+  auto finish    = [&](unsigned long long& lo, unsigned long long& hi, bool up) {  // steps of 32 to 1
+    const bool keep               = (lo < hi) == up;
+    const unsigned long long less = keep ? lo : hi;
+    hi                            = keep ? hi : lo;
+    lo                            = less;
+#pragma unroll 1
+    for (int stride = 16; stride > 0; stride >>= 1) {
+      const bool smaller = ((lane & stride) == 0) == up;
+      lo                 = met(lo, stride, smaller);
+      hi                 = met(hi, stride, smaller);
+    }
+  };
+  for (int at = warp0 + lane; at < width; at += all) {
+    unsigned long long lo = at < count ? src[at] : kNoKey, hi = at + 32 < count ? src[at + 32] : kNoKey;
+#pragma unroll 1
+    for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll 1
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        const bool first = (lane & stride) == 0;
+        lo               = met(lo, stride, first == ((at & size) == 0));
+        hi               = met(hi, stride, first == (((at + 32) & size) == 0));
+      }
+    finish(lo, hi, (at & 64) == 0);
+    key[at]      = lo;
+    key[at + 32] = hi;
+  }
+  __syncthreads();
+  for (int size = 128; size <= width; size <<= 1) {
+    for (int stride = size >> 1; stride >= 64; stride >>= 1) {
+      for (int p = threadIdx.x; p < width / 2; p += blockDim.x) {
+        const int i                = 2 * p - (p & (stride - 1));
+        const unsigned long long a = key[i], b = key[i + stride];
+        if ((a > b) == ((i & size) == 0)) {
+          key[i]          = b;
+          key[i + stride] = a;
+        }
+      }
+      __syncthreads();
+    }
+    for (int at = warp0 + lane; at < width; at += all) {
+      unsigned long long lo = key[at], hi = key[at + 32];
+      finish(lo, hi, (at & size) == 0);
+      key[at]      = lo;
+      key[at + 32] = hi;
+    }
+    __syncthreads();
+  }
+}
+
 struct radix_cut_t {
   unsigned long long prefix, mask;
 };
@@ -412,15 +474,16 @@ __device__ __forceinline__ void rank_sort(const unsigned long long* src, int cnt
   if (sub == 0 && at < cnt && below < want) dst[below] = mine;
 }
 
+constexpr int kCounted = 128;  // new keys whose places are counted at most (see merge_sorted)
+
 /// The first `want` keys of the ascending list old[0, n) and the m distinct keys add[0, m), none of them in
 /// the list, into dst, ascending; order [m] is scratch. A new key's place is the number of new keys below
 /// it, counted, and of old ones, found by halving; an old key's is its own plus the new ones below it,
 /// halving in their order. One barrier where a sorting network over all of them has 36 (256 keys) to 55
-/// (1 024 keys). The counting is quadratic in the new keys, and still the faster of the two over the whole
-/// range (200 000 rows x 128, us a search, by places and by the network): up to 128 new keys into 128 267
-/// and 288 (1 000 queries), into 512 1 159 and 1 497 (4 000 queries); up to 300 into 200 833 and 942; up to
-/// 512 into 65 548 and 567, into 512 1 774 and 1 938 (2 000 queries); 1 000 ranked by sketch distance into
-/// 1 000 2 120 and 2 257. All threads of the block call it.
+/// (1 024 keys). Counting is quadratic in the new keys: of more than kCounted the caller has put them into order
+/// already, ascending (sort_keys). us a search with all places counted, and with kCounted of 64, 128 and 256: 1 000
+/// queries, 512 kept and 512 reranked rows 1 470, 1 427, 1 429 and 1 424; 2 000, 256 and 256 1 550, 1 541, 1 544 and
+/// 1 553; 2 500 ranked by sketch distance into 512 3 265, 3 154, 3 154 and 3 158. All threads of the block call it.
 __device__ __forceinline__ void merge_sorted(const unsigned long long* old, int n, const unsigned long long* add, int m,
                                              unsigned long long* order, int want, unsigned long long* dst)
 {
@@ -435,17 +498,24 @@ __device__ __forceinline__ void merge_sorted(const unsigned long long* old, int 
     }
     return lo;
   };
-  for (int j = threadIdx.x; j < m; j += blockDim.x) {
-    const unsigned long long mine = add[j];
-    int at                        = 0;
+  if (m > kCounted) {
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+      const int place = j + below(old, n, order[j]);
+      if (place < want) dst[place] = order[j];
+    }
+  } else {
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+      const unsigned long long mine = add[j];
+      int at                        = 0;
 #pragma unroll 4
-    for (int i = 0; i < m; i++)
-      at += add[i] < mine;
-    order[at]       = mine;
-    const int place = at + below(old, n, mine);
-    if (place < want) dst[place] = mine;
+      for (int i = 0; i < m; i++)
+        at += add[i] < mine;
+      order[at]       = mine;
+      const int place = at + below(old, n, mine);
+      if (place < want) dst[place] = mine;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const unsigned long long mine = old[i];
     const int place               = i + below(order, m, mine);
@@ -940,28 +1010,29 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
   const int total = nk + ctrl[kMerged];
   const int cnt   = min(total, KO);
   // New keys that fit behind the kept ones go to their places among them. Other short lists are sorted by ranking,
-  // at most kRankSteps comparisons a thread, and a quarter of that where KO keys are few of the total, which are
-  // rather selected first (always in a block of 128 threads, of which many share a multiprocessor). us a search:
-  // where the places were left to the ranking whenever that was short enough, and now, 1 000 queries with 128 kept
-  // and 128 reranked rows 340 and 330, 10 000 2 404 and 2 322, 4 000 wide rows with 256 1 631 and 1 590. Limits of 32,
-  // 128 and 512 comparisons: one query with 256 kept and 256 reranked rows 91.5, 89.3 and 89.8, 148 with 512 172, 169
-  // and 186. The quarter, at 32 kept of 300 to 512 reranked rows: 55 queries 126.9 and 123.5, 296 135.6 and
-  // 131.5; at 32 of 128 one query takes 66 when it selects first and 63.
-  constexpr int kRankSteps = 128;
+  // at most kRankSteps comparisons a thread, and half of that where KO keys are few of the total, which are
+  // rather selected first (always in a block of 128 threads, of which many share a multiprocessor); longer ones by the
+  // network. us a search: where the places were left to the ranking whenever that was short enough, and now, 1 000
+  // queries with 128 kept and 128 reranked rows 340 and 330, 10 000 2 404 and 2 322, 4 000 wide rows with 256 1 631 and
+  // 1 590. Limits of 32, 64 and 128 comparisons: 10 000 queries with 256 kept and 512 reranked rows in three waves 7 606,
+  // 7 597 and 7 705 (7 867 with a barrier for every step of the network), 2 000 with 192 and 384 1 396, 1 394 and 1 400
+  // (1 428), 148 with 512 and 512 165, 165 and 165 (172). The half, at 32 kept of 300 to 512 reranked rows: 55 queries
+  // 126.9 and 123.5, 296 135.6 and 131.5; at 32 of 128 one query takes 66 when it selects first and 63.
+  constexpr int kRankSteps = 64;
   const int threads        = blockDim.x;
   const auto few           = [&](int keys, int steps) { return keys <= threads && keys * keys <= steps * threads; };
-  if (nk > 0 && total - nk <= P) {
-    merge_sorted(pool, nk, pool + nk, total - nk, sorted + P, KO, sorted);
-  } else if (total <= 2 * P ? few(total, kRankSteps) : threads > kRoundThreads && few(total, kRankSteps / 4)) {
+  const bool places        = nk > 0 && total - nk <= P;
+  // what is sorted by the network, if anything (one place in the code for all: every copy of it costs the round's
+  // other phases registers)
+  const unsigned long long* from = pool;
+  unsigned long long* to         = sorted;
+  int count = 0, width = P;
+  if (places) {
+    if (total - nk > kCounted) from = pool + nk, to = sorted + P, count = total - nk, width = 2 * kCounted;
+  } else if (total <= 2 * P ? few(total, kRankSteps) : threads > kRoundThreads && few(total, kRankSteps / 2)) {
     rank_sort(pool, total, sorted, KO);
   } else if (total <= 2 * P) {
-    int width = P;
-    while (width < total)
-      width <<= 1;
-    for (int i = threadIdx.x; i < width; i += blockDim.x)
-      sorted[i] = i < total ? pool[i] : kNoKey;
-    __syncthreads();
-    bitonic_sort(sorted, width);
+    count = total;
   } else {
     // the KO smallest are selected first (into the upper half of the sort region), then sorted
     unsigned long long* picked = sorted + max(P, 32);
@@ -978,12 +1049,15 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
     if (few(KO, kRankSteps)) {
       rank_sort(picked, KO, sorted, KO);
     } else {
-      for (int i = threadIdx.x; i < P; i += blockDim.x)
-        sorted[i] = i < KO ? picked[i] : kNoKey;
-      __syncthreads();
-      bitonic_sort(sorted, P);
+      from = picked, count = KO;
     }
   }
+  if (count > 0) {
+    while (width < count)
+      width <<= 1;
+    sort_keys(from, count, to, width);
+  }
+  if (places) merge_sorted(pool, nk, pool + nk, total - nk, sorted + P, KO, sorted);
   __syncthreads();
   for (int i = threadIdx.x; i < KO; i += blockDim.x) {
     const unsigned long long key = i < cnt ? sorted[i] : kNoKey;

@@ -180,6 +180,25 @@ def test_first_merges_around_the_ranking(oracle, more_rows, threads, rerank):
     assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
+@pytest.mark.parametrize("queries_at_once", [5, 64, 700])
+@pytest.mark.parametrize("starts,rerank,wave_rerank", [
+    (65, 128, 65),     # a first merge of 128 keys into 65 (128 threads: two chunks of a warp), new ones counted
+    (128, 129, 128),   # 129 of 256 places; the most keys whose places are counted
+    (130, 257, 129),   # 257 of 512; one more
+    (200, 512, 256),   # more than twice the kept ones: selected, then sorted
+    (512, 511, 300),
+    (512, 512, 512),   # as many as there is room for
+])
+def test_merges_of_many_keys(oracle, more_rows, starts, rerank, wave_rerank, queries_at_once):
+    """Merges whose keys the network sorts: sizes around its powers of two, blocks of few and of many threads."""
+    idx, arrays, meta, queries = more_rows
+    kw = dict(read=64, starts=starts, waves=2, rerank=rerank, wave_rerank=wave_rerank)
+    against_checker(oracle, idx, arrays, meta, queries, 32, **kw)
+    want_d, want_i = idx.search(queries, starts, **kw)
+    d, i = idx.search(np.resize(queries, (queries_at_once, queries.shape[1])), starts, **kw)
+    assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
+
+
 def test_plans_of_several_indexes(many_rows, more_rows):
     """Two indexes searched in turn, each with a plan of its own size."""
     (one, _, _, queries), (other, _, _, others) = many_rows, more_rows
