@@ -855,6 +855,29 @@ auto half_stream(index_impl& ix, plan const& pl, int n, cudaStream_t s) -> cudaS
   return p.half;
 }
 
+/// What s holds from now on comes after the half of a batch queued on `other`. A half is joined as well when the
+/// batch could not be queued whole; where not even that can be queued the host waits, so that no call returns with the
+/// caller's arrays in use on a stream that the caller does not know.
+struct half_join {
+  cudaEvent_t ev;
+  cudaStream_t s, other;
+  bool open = true;
+  half_join(plan const& pl, cudaStream_t on, cudaStream_t half) : ev(pl.join_ev), s(on), other(half) {}
+  half_join(half_join const&) = delete;
+  void close()
+  {
+    OCTEX_CUDA_TRY(cudaEventRecord(ev, other));
+    OCTEX_CUDA_TRY(cudaStreamWaitEvent(s, ev, 0));
+    open = false;
+  }
+  ~half_join()
+  {
+    if (!open || (cudaEventRecord(ev, other) == cudaSuccess && cudaStreamWaitEvent(s, ev, 0) == cudaSuccess)) return;
+    cudaStreamSynchronize(other);
+    cudaGetLastError();  // the error to report is on its way
+  }
+};
+
 /// A batch of n queries in device memory on s; in two halves where that pays: the second runs on the other stream,
 /// from where s is now, and s goes on when it is done.
 void run_in_place(index_impl& ix, plan& pl, batch_io const& io, int n, cudaStream_t s)
@@ -869,17 +892,11 @@ void run_in_place(index_impl& ix, plan& pl, batch_io const& io, int n, cudaStrea
   OCTEX_CUDA_TRY(cudaEventRecord(start_event(ix, ix.part.device), s));
   OCTEX_CUDA_TRY(cudaStreamWaitEvent(other, ix.start_ev, 0));
   one_start.unlock();
-  struct joined {  // also when a half could not be queued
-    plan& pl;
-    cudaStream_t s, other;
-    ~joined()
-    {
-      if (cudaEventRecord(pl.join_ev, other) == cudaSuccess) cudaStreamWaitEvent(s, pl.join_ev, 0);
-    }
-  } join{pl, s, other};
+  half_join join(pl, s, other);
   const row_range halves[2] = {{0, (n + 1) / 2}, {(n + 1) / 2, n / 2}};
   run_batch(ix, pl, io, s, nullptr, &halves[0]);
   run_batch(ix, pl, io, other, nullptr, &halves[1]);
+  join.close();
 }
 
 /// The next batch of a call on a plan: n queries from row b0 of it on.
@@ -1086,8 +1103,7 @@ void search_copied(index_impl& ix, search_params const& sp, int lanes, cudaStrea
   auto close = [&](int l, bool failed) {
     if (halves && l == 0) return;
     if (halves) {  // what the plan's last batch is ends on the first stream
-      OCTEX_CUDA_TRY(cudaEventRecord(lane[1]->join_ev, stream[1]));
-      OCTEX_CUDA_TRY(cudaStreamWaitEvent(stream[0], lane[1]->join_ev, 0));
+      half_join(*lane[0], stream[0], stream[1]).close();
       l = 0;
     }
     mark_last_batch(*lane[l], stream[l]);
