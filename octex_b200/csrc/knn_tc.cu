@@ -61,6 +61,12 @@ constexpr int kTmemCols   = 512;  // two accumulators of 128 fp32 columns per se
 constexpr int kMaxStages  = 6;
 constexpr int kNoted      = 32;   // improvements a row notes for a merge, in global memory, twice
 constexpr int kHitBytes   = 640;  // of a warp's groups at one place: four values and a row per lane
+// Groups of four columns a lane may have set aside; a warp looks through them when there is no room for two more in one of
+// its lanes. All are noted at once, so 4 kRoom <= kNoted. With eight rows wait longer for their notes to reach the
+// lists: ms with six and eight, 200 001 x 128, K = 64 15.7 and 16.3, 64 dimensions 13.2 and 13.7, 100 000 x 128, K = 120
+// 5.9 and 6.5, 10 007 x 64, K = 64 0.52 and 0.58 (256 dimensions: the same).
+constexpr int kRoom = 6;
+static_assert(4 * kRoom <= kNoted, "notes of a look through");
 constexpr uint32_t kIdleLimit = 1u << 28;  // looks of a list warp for something to merge before it gives up
 constexpr int kVisitsPerK = 3;    // tiles looked at for the bars, per entry of a list
 constexpr uint32_t kPartBytes = kTile * kTileK * 2;  // 128 rows x 64 halves of an operand
@@ -86,7 +92,7 @@ static_assert(sizeof(knn_ctl) <= kCtlBytes && kCtlBytes % 16 == 0, "control bloc
 struct knn_shape {
   int stages;    // of 64 dimensions of a tile (and of the query rows, when those do not stay)
   int resident;  // the query rows stay in shared memory
-  int room;      // groups of four columns a thread may have set aside, at most kNoted / 4
+  int room;      // kRoom (a constant instead: 24 bytes of the epilogue's registers spill)
   __host__ __device__ size_t stage_bytes() const { return (resident ? 1 : 3) * static_cast<size_t>(kPartBytes); }
   __host__ __device__ size_t query_bytes(int nkb) const { return resident ? 2 * static_cast<size_t>(nkb) * kPartBytes : 0; }
   size_t smem_bytes(int nkb) const
@@ -526,7 +532,7 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
       // groups of four columns with an improvement: the four values, and the first one's row `to_first` bytes behind
       const uint32_t hit0     = smem_u32(hits) + (warp - 4) * shape.room * kHitBytes + lane * 16;
       const uint32_t to_first = 512 - 12 * lane;
-      const uint32_t hit_end  = hit0 + (shape.room - 4) * kHitBytes;  // beyond it there is no room for four more
+      const uint32_t hit_end  = hit0 + (shape.room - 2) * kHitBytes;  // beyond it there is no room for two more
       uint32_t hit            = hit0;                               // where the next one goes
       // the notes of the rows whose lanes ask for it go to the list warps; the lanes go on in the other buffer
       auto hand_over = [&](bool asks) {
@@ -784,13 +790,10 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
 knn_shape choose_shape(int nkb)
 {
   constexpr size_t kLimit = 227 * 1024;
-  for (const int room : {8, 6}) {
-    knn_shape fit{kMaxStages, 1, room};
-    while (fit.stages > 3 && fit.smem_bytes(nkb) > kLimit)
-      fit.stages--;
-    if (fit.smem_bytes(nkb) <= kLimit) return fit;
-  }
-  return knn_shape{3, 0, 8};
+  knn_shape fit{kMaxStages, 1, kRoom};
+  while (fit.stages > 3 && fit.smem_bytes(nkb) > kLimit)
+    fit.stages--;
+  return fit.smem_bytes(nkb) <= kLimit ? fit : knn_shape{3, 0, kRoom};
 }
 
 }  // namespace
