@@ -26,7 +26,11 @@
 // bit), reads those again and sets them aside in shared memory, a lane its own. When one of a warp's rows has no
 // room left, all are looked through and what is still wanted is noted (value, row) in one of two buffers of the
 // row. A full buffer goes to a list warp, which sorts it (bitonic, a key per lane) and merges it into the row's K
-// best, which stand in order in the output arrays (L2 cache), and publishes the K-th. So the bar a row compares
+// best, which stand in order in the output arrays (L2 cache), and publishes the K-th. At the end of an item all rows hand
+// over at once, with nothing else left to do: then the epilogue warps merge as well, whichever row no other warp has
+// taken. (Left to four list warps the end of an item took 70 us, 64 merges one after the other; us a call, so and
+// now: 1 000 x 128, K = 64 438 and 272, K = 10 165 and 117, 10 007 x 64, K = 64 513 and 360, 200 001 x 128 15 100 and
+// 14 700, 50 000 x 768, K = 10 4 760 and 4 650.) So the bar a row compares
 // with is a buffer or two old, which costs a few more notes, and no tile waits for a merge (2 000 cycles, mostly
 // the latencies of shuffles and of the L2 cache, where a tile takes 2 200).
 //
@@ -41,7 +45,7 @@
 // warps per row, a half of the columns each: 18.7.
 //
 // Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues), warp 3 makes the norm
-// operands; eight epilogue warps, four per set, one per quarter of the TMEM lanes; four list warps of 64 rows.
+// operands; eight epilogue warps, four per set, one per quarter of the TMEM lanes; four list warps, a quarter of the rows each.
 // Every wait, on an mbarrier or a word in shared memory, is bounded; one that runs out raises a flag the other roles see, the
 // block waits for its copies in flight, frees its TMEM and returns with the error word set.
 
@@ -68,6 +72,7 @@ constexpr int kHitBytes   = 640;  // of a warp's groups at one place: four value
 constexpr int kRoom = 6;
 static_assert(4 * kRoom <= kNoted, "notes of a look through");
 constexpr uint32_t kIdleLimit = 1u << 28;  // looks of a list warp for something to merge before it gives up
+constexpr int kTaken      = 1 << 9;  // of notes handed over: a warp is merging them
 constexpr int kVisitsPerK = 3;    // tiles looked at for the bars, per entry of a list
 constexpr uint32_t kPartBytes = kTile * kTileK * 2;  // 128 rows x 64 halves of an operand
 constexpr uint32_t kNormBytes = kTile * 32;          // 128 rows x 16 bf16 of a norm operand
@@ -81,7 +86,7 @@ struct knn_ctl {
   int failed;
   int place;                // of the block's notes
   int finished[8];          // items an epilogue warp is through with
-  int handed[2 * kTile];    // notes of a row that are to be merged: 0, or their number and which of the two buffers
+  int handed[2 * kTile];    // notes of a row that are to be merged: 0, or their number, which of the two buffers, kTaken
   int have[2 * kTile];      // entries in a row's list
   float bar[2 * kTile];     // what the row's list asks for, as an accumulator
 };
@@ -401,6 +406,31 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
   const volatile int* stop = &ctl.failed;
   const bool placed        = ctl.place >= 0;
 
+  // What row r of the item has handed over goes into its list, unless another warp is at it; r is the same for all
+  // lanes. Which warp merges a row changes, which lane has which entry of its list does not.
+  auto merge_handed = [&](int r, int q0) {
+    int note = 0;
+    if (lane == 0) {
+      note = *static_cast<volatile int*>(&ctl.handed[r]);
+      if (note != 0 && ((note & kTaken) != 0 || atomicCAS(&ctl.handed[r], note, note | kTaken) != note)) note = 0;
+    }
+    note = __shfl_sync(0xffffffffu, note, 0);
+    if (note == 0) return;
+    __threadfence_block();
+    const int c = note & 255, h = *static_cast<volatile int*>(&ctl.have[r]);
+    const int64_t list = static_cast<int64_t>(q0 + r - q_first) * K;
+    const float last   = merge_noted<kRegs>(notes + ((static_cast<size_t>(ctl.place) * 2 * kTile + r) * 2 + (note >> 8 & 1)) * kNoted, c,
+                                            h, K, best_d + list, best_id + list);
+    __syncwarp();
+    if (lane == 0) {
+      *static_cast<volatile int*>(&ctl.have[r])  = min(K, h + c);
+      *static_cast<volatile float*>(&ctl.bar[r]) = -0.5f * last;
+      __threadfence_block();
+      *static_cast<volatile int*>(&ctl.handed[r]) = 0;
+    }
+    __syncwarp();
+  };
+
   // The block's items, 256 query rows each, the narrow ones of 128 last. Visits are counted on over them
   // (modulo 2^32, which the phases of the barriers divide).
   uint32_t v0   = 0;          // the item's first visit
@@ -529,6 +559,7 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
       volatile int* handed      = ctl.handed + set * kTile + quarter * 32 + lane;
       volatile float* list_bar  = ctl.bar + set * kTile + quarter * 32 + lane;
       *list_bar                 = -INFINITY;
+      *static_cast<volatile int*>(&ctl.have[set * kTile + quarter * 32 + lane]) = 0;
       // groups of four columns with an improvement: the four values, and the first one's row `to_first` bytes behind
       const uint32_t hit0     = smem_u32(hits) + (warp - 4) * shape.room * kHitBytes + lane * 16;
       const uint32_t to_first = 512 - 12 * lane;
@@ -714,63 +745,72 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
         look_through();
         hand_over(count != 0);
       }
-      if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 3);
       __threadfence_block();
       __syncwarp();
       if (lane == 0) *static_cast<volatile int*>(&ctl.finished[set * 4 + quarter]) = done_items + 1;
-    } else if (const int list = warp - 12; list >= 0 && list >> 1 < sets) {
-      // ---- lists: what the rows hand over is merged while the epilogue goes on; 64 rows a warp -----
-      const int row0 = list * 64;  // of the block's 256
-      const int wrow = q0 + row0;
-      float2* rows_noted = notes + (static_cast<size_t>(ctl.place) * 2 * kTile + row0) * 2 * kNoted;
-      int32_t* ids       = best_id + static_cast<int64_t>(wrow - q_first) * K;
-      float* vals        = best_d + static_cast<int64_t>(wrow - q_first) * K;
-      volatile int* handed   = ctl.handed + row0;
-      volatile int* finished = ctl.finished + list * 2;
-      ctl.have[row0 + lane]      = 0;
-      ctl.have[row0 + 32 + lane] = 0;
-      __syncwarp();
+      // The last notes of all rows came at once: the list warps start from the first row, the others help from the last.
+#pragma unroll 1
+      for (int L = 31; L >= 0 && ok; L--)
+        merge_handed(set * kTile + quarter * 32 + L, q0);
+      for (uint32_t i = 0; ok && __any_sync(0xffffffffu, *handed != 0); i++) {
+        ok = __all_sync(0xffffffffu, i < kSpinLimit && *stop == 0);
+        __nanosleep(64);
+      }
+      if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 3);
+      // the rows' own norms, four rows at a time
+      __threadfence_block();
+#pragma unroll 1
+      for (int L0 = 0; ok && L0 < 32 && wrow + L0 < q_end; L0 += 4) {
+        const int many = min(4, q_end - wrow - L0);
+        int h[4];
+        float qn[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          h[u]  = u < many ? *static_cast<volatile int*>(&ctl.have[set * kTile + quarter * 32 + L0 + u]) : 0;
+          qn[u] = u < many ? __ldg(norm + wrow + L0 + u) : 0.f;
+        }
+        float* od   = best_d + static_cast<int64_t>(wrow + L0 - q_first) * K;
+        int32_t* oi = best_id + static_cast<int64_t>(wrow + L0 - q_first) * K;
+        for (int t = lane; t < K; t += 32) {
+          float d[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            d[u] = t < h[u] ? od[u * K + t] : INFINITY;
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (u < many) {
+              od[u * K + t] = t < h[u] ? fmaxf(__fadd_rn(qn[u], d[u]), 0.f) : INFINITY;
+              if (t >= h[u]) oi[u * K + t] = -1;
+            }
+        }
+      }
+    } else if (warp >= 12) {
+      // ---- lists: what the rows hand over is merged while the epilogue goes on; 64 rows a warp, or 32 of one set -----
+      const int list = warp - 12, row0 = list * 32 * sets;  // of the block's 256
+      const volatile int* handed   = ctl.handed + row0;
+      const volatile int* finished = ctl.finished + list * sets;
       bool ok = true;
       for (uint32_t idle = 0; ok;) {
-        const bool over = __all_sync(0xffffffffu, finished[lane & 1] == done_items + 1);
+        const bool over = __all_sync(0xffffffffu, finished[lane & (sets - 1)] == done_items + 1);
         __threadfence_block();
-        unsigned todo[2] = {__ballot_sync(0xffffffffu, handed[lane] != 0), __ballot_sync(0xffffffffu, handed[32 + lane] != 0)};
-        if ((todo[0] | todo[1]) == 0) {
+        auto waits = [&](int r) {
+          const int note = handed[r];
+          return note != 0 && (note & kTaken) == 0;
+        };
+        unsigned long long todo = __ballot_sync(0xffffffffu, waits(lane));
+        if (sets == 2) todo |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, waits(32 + lane))) << 32;
+        if (todo == 0) {
           if (over) break;
           ok = __all_sync(0xffffffffu, *stop == 0 && ++idle < kIdleLimit);
           __nanosleep(1000);
           continue;
         }
-        __threadfence_block();
         idle = 0;
 #pragma unroll 1
-        for (int half = 0; half < 2; half++)
-          while (todo[half] != 0) {
-            const int L = half * 32 + __ffs(todo[half]) - 1;
-            todo[half] &= todo[half] - 1;
-            const int note = handed[L], c = note & 255, h = ctl.have[row0 + L];
-            const float last = merge_noted<kRegs>(rows_noted + (L * 2 + (note >> 8)) * kNoted, c, h, K,
-                                                  vals + static_cast<int64_t>(L) * K, ids + static_cast<int64_t>(L) * K);
-            __syncwarp();
-            if (lane == 0) {
-              ctl.have[row0 + L] = min(K, h + c);
-              *static_cast<volatile float*>(&ctl.bar[row0 + L]) = -0.5f * last;
-              __threadfence_block();
-              handed[L] = 0;
-            }
-            __syncwarp();
-          }
+        for (; todo != 0; todo &= todo - 1)
+          merge_handed(row0 + __ffsll(todo) - 1, q0);
       }
       if (!ok && lane == 0 && atomicExch(&ctl.failed, 1) == 0) atomicExch(error, 6);
-      for (int L = 0; ok && L < 64 && wrow + L < q_end; L++) {
-        const int h    = ctl.have[row0 + L];
-        const float qn = __ldg(norm + wrow + L);
-        float* od      = vals + static_cast<int64_t>(L) * K;
-        for (int t = lane; t < K; t += 32) {
-          od[t] = t < h ? fmaxf(__fadd_rn(qn, od[t]), 0.f) : INFINITY;
-          if (t >= h) ids[static_cast<int64_t>(L) * K + t] = -1;
-        }
-      }
     }
     __syncwarp();
     // every accumulator has been read, so no MMA is left that reads the query rows
