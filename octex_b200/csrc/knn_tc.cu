@@ -65,12 +65,6 @@ constexpr int kTmemCols   = 512;  // two accumulators of 128 fp32 columns per se
 constexpr int kMaxStages  = 6;
 constexpr int kNoted      = 32;   // improvements a row notes for a merge, in global memory, twice
 constexpr int kHitBytes   = 640;  // of a warp's groups at one place: four values and a row per lane
-// Groups of four columns a lane may have set aside; a warp looks through them when there is no room for two more in one of
-// its lanes. All are noted at once, so 4 kRoom <= kNoted. With eight rows wait longer for their notes to reach the
-// lists: ms with six and eight, 200 001 x 128, K = 64 15.7 and 16.3, 64 dimensions 13.2 and 13.7, 100 000 x 128, K = 120
-// 5.9 and 6.5, 10 007 x 64, K = 64 0.52 and 0.58 (256 dimensions: the same).
-constexpr int kRoom = 6;
-static_assert(4 * kRoom <= kNoted, "notes of a look through");
 constexpr uint32_t kIdleLimit = 1u << 28;  // looks of a list warp for something to merge before it gives up
 constexpr int kTaken      = 1 << 9;  // of notes handed over: a warp is merging them
 constexpr int kVisitsPerK = 3;    // tiles looked at for the bars, per entry of a list
@@ -97,7 +91,7 @@ static_assert(sizeof(knn_ctl) <= kCtlBytes && kCtlBytes % 16 == 0, "control bloc
 struct knn_shape {
   int stages;    // of 64 dimensions of a tile (and of the query rows, when those do not stay)
   int resident;  // the query rows stay in shared memory
-  int room;      // kRoom (a constant instead: 24 bytes of the epilogue's registers spill)
+  int room;      // groups of four columns a lane may have set aside
   __host__ __device__ size_t stage_bytes() const { return (resident ? 1 : 3) * static_cast<size_t>(kPartBytes); }
   __host__ __device__ size_t query_bytes(int nkb) const { return resident ? 2 * static_cast<size_t>(nkb) * kPartBytes : 0; }
   size_t smem_bytes(int nkb) const
@@ -826,14 +820,24 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
 }
 
 /// Query rows that stay in shared memory with as many stages as fit behind them, three at least (256 dimensions).
-/// Beyond that they come in again with every tile.
+/// Beyond that they come in again with every tile, in four stages.
+/// Four places for groups: a warp looks through them when there is no room for two more in one of its lanes, and all are noted
+/// at once, so at most kNoted / 4. More hold up what the lists publish, fewer are looked through too often; us a call with
+/// six, four, three and two: 200 001 x 128, K = 64 14 820, 14 560, 14 860 and 16 470, 100 000 x 128, K = 120 5 822, 5 580,
+/// 5 795 and 6 725, 1 000 x 128, K = 64 272, 245, 236 and 232 (248 with lists that the epilogue merged alone). Where query rows
+/// do not stay three leave the room for the fourth stage; us with four places and three stages, three and four, 50 000 rows, K = 10 and 64:
+/// 768 dimensions 4 658 and 4 516, 6 567 and 6 353, 960 5 763 and 5 508, 8 124 and 7 739, 512 3 204 and 3 190, 4 488 and 4 482.
+/// What these take beyond a scan whose epilogue merges alone and adds the norms itself (3 070 at 512 dimensions and K = 10,
+/// 4 420 at 768; 4 610 and 6 350 at K = 64) are the MMAs of the norms; norms in the epilogue of this one 3 560 and 4 910, since
+/// they come out of the shared memory the MMAs wait for. One set that stays instead of two that do not, 264 to 576
+/// dimensions: 3 080 and 4 160 at 512.
 knn_shape choose_shape(int nkb)
 {
   constexpr size_t kLimit = 227 * 1024;
-  knn_shape fit{kMaxStages, 1, kRoom};
+  knn_shape fit{kMaxStages, 1, 4};
   while (fit.stages > 3 && fit.smem_bytes(nkb) > kLimit)
     fit.stages--;
-  return fit.smem_bytes(nkb) <= kLimit ? fit : knn_shape{3, 0, kRoom};
+  return fit.smem_bytes(nkb) <= kLimit ? fit : knn_shape{4, 0, 3};
 }
 
 }  // namespace
