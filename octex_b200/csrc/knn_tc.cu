@@ -295,9 +295,10 @@ __device__ __forceinline__ float merge_noted(const float2* noted, int count, int
 }
 
 // What the rows of the blocks that are running note, a place per block. It is the module's own memory, so a call
-// allocates nothing for it (9 MB more in an allocation of the call: 0.7 ms). A block takes a place when it starts
-// and leaves it when it ends; the shared memory it needs leaves no room for a second one on its multiprocessor,
-// and there are more places than multiprocessors, whatever calls run at the same time.
+// allocates nothing for it (in an allocation of the call: 0.7 ms): 21 MB, which the driver gives the process when it
+// first launches a scan (a process that only searches has none of it) and which stay with it. A block takes a place when
+// it starts and leaves it when it ends; the shared memory it needs leaves no room for a second one on its multiprocessor,
+// and there are more places than multiprocessors (knn_tc looks), whatever calls run at the same time.
 constexpr int kPlaces = 160;
 __device__ float2 notes[static_cast<size_t>(kPlaces) * 2 * kTile * 2 * kNoted];
 __device__ unsigned place_taken[kPlaces];
@@ -864,6 +865,7 @@ void knn_tc(const __half* x, const float* norm, int64_t n, int D, int K, int64_t
   if (status == cudaSuccess) status = cudaGetDevice(&dev);
   if (status == cudaSuccess) status = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (status != cudaSuccess) throw std::runtime_error(std::string("octex: ") + cudaGetErrorString(status));
+  if (sms > kPlaces) throw std::runtime_error("octex: more multiprocessors than the neighbor scan has places for notes");
   // A block per multiprocessor, which takes items of 256 query rows; what is left after the whole rounds goes out
   // in items of 128 rows when those fit one more round, which then takes half the time.
   const int64_t round  = int64_t{2} * kTile * sms;
