@@ -249,6 +249,8 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
   }
   for (; tile < last; tile++, set ^= ahead ? 1 : 0) {
     const int tile_n = tile % tiles_n, tile_m = tile / tiles_n;
+    // (worked out for every 64 dimensions anew, one query of 960 takes 86.3 us instead of 85.4)
+    const int first_row = tile_m * rows, end_row = min(m, first_row + rows);
     if (ahead) {
       ready = ready && mbar_wait(&sm.done, done_phase, &sm.failed);
       if (!ready) sm.failed = 1;
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, kMode == tc_mode::taps ? 1 : kMode =
           if (!ready) sm.failed = 1;
           if (ready && threadIdx.x == 0) load_projections(tile, kb, 0);
         }
-        if (ready) fill_queries<kVec>(sm.a[s], job.q, job.mean, tile_m * rows, min(m, (tile_m + 1) * rows), D, kb * kTileK);
+        if (ready) fill_queries<kVec>(sm.a[s], job.q, job.mean, first_row, end_row, D, kb * kTileK);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0 && ready) {
