@@ -1077,9 +1077,17 @@ __device__ __forceinline__ void merge_into_kept(unsigned long long* pool,
 // round whose hash set is too large for eight blocks runs 256, 512 or 1024 threads per block instead,
 // so that the blocks that do fit still bring 32 warps to a multiprocessor, and so does a batch with
 // too few queries to fill the multiprocessors with small blocks (round_threads).
-template <bool kRows, bool kDealt, int kThreads>
+//
+// kShort: a wave of few entries for few queries (short_wave). A block that is alone on its multiprocessor goes through
+// every phase once, and waits for its code more than for anything that code could do side by side: no loads ahead, no
+// packed sketch distances, no selection among the candidates that beat a full kept list. us a search of a million rows,
+// with the longer code and so: one query, 32 start points of 64 neighbors, one wave 63.8 and 63.1, four 96.4 and 94.8,
+// 16 start points and three waves 94.1 and 92.6, eight queries 95.2 and 94.4, two by sketch distance with 16 and two 71.9 and
+// 70.6.
+template <bool kRows, bool kDealt, int kThreads, bool kShort>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const round_args a)
 {
+  constexpr bool kAhead = kRows && !kShort;
   extern __shared__ __align__(16) int smem[];
   let_next_kernel_start();
   const round_layout lay(a);
@@ -1264,14 +1272,14 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
           }
         }
       };
-      if (kRows) fetch(0);
+      if (kAhead) fetch(0);
       for (int sb = 0; sb < nseg; sb += 4 * spp) {
-        if (!kRows) fetch(sb);
+        if (!kAhead) fetch(sb);
         int v[4];
 #pragma unroll
         for (int u = 0; u < 4; u++)
           v[u] = ahead[u];
-        if (kRows && sb + 4 * spp < nseg) fetch(sb + 4 * spp);
+        if (kAhead && sb + 4 * spp < nseg) fetch(sb + 4 * spp);
         int mine = 0;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
@@ -1317,17 +1325,17 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   if (!int_form) {
     const float* qv = reinterpret_cast<const float*>(w16);
     if (S <= 16) {
-      sketch_rows_f32<1, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<1, kDealt, kAhead>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 32) {
-      sketch_rows_f32<2, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<2, kDealt, kAhead>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 64) {
-      sketch_rows_f32<4, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<4, kDealt, kAhead>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 128) {
-      sketch_rows_f32<8, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<8, kDealt, kAhead>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else if (S <= 256) {
-      sketch_rows_f32<16, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<16, kDealt, kAhead>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     } else {
-      sketch_rows_f32<32, kDealt, kRows>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
+      sketch_rows_f32<32, kDealt, kAhead>(cand, n, a.sketch, a.sketch_map, S, kq, qv, dist);
     }
   } else {
     const bool keep = a.keep_sketch != 0 && may_prefetch<kDealt>(a.sketch_map);
@@ -1377,38 +1385,53 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) round_kernel(const 
   // 3 251, 10 000 with 128 and three 1 735 and 1 691.
   if (kRows && a.sketch_rank && ctrl[kValid] == a.KO) {
     const unsigned long long bound = rank_key(kd[a.KO - 1], static_cast<unsigned>(kid[a.KO - 1]));
-    for (int i0 = 0; i0 < n; i0 += 4 * kThreads) {
-      float d[4];
-      int id[4];
-      bool within[4];
+    if constexpr (kShort) {
+      for (int i = threadIdx.x; i < n; i += kThreads)
+        if (__float_as_uint(dist[i]) <= static_cast<unsigned>(bound >> 32) &&
+            rank_key(dist[i], static_cast<unsigned>(cand[i])) < bound) {
+          const int s = atomicAdd(&ctrl[kWithin], 1);
+          if (s < R) {
+            sid[s] = cand[i];
+            sdv[s] = dist[i];
+          }
+        }
+      __syncthreads();
+      selected = ctrl[kWithin] <= R;
+      if (selected) ns = ctrl[kWithin];
+    } else {
+      for (int i0 = 0; i0 < n; i0 += 4 * kThreads) {
+        float d[4];
+        int id[4];
+        bool within[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int i = i0 + u * kThreads + threadIdx.x;
-        d[u]        = i < n ? dist[i] : INFINITY;
-        within[u]   = i < n && __float_as_uint(d[u]) <= static_cast<unsigned>(bound >> 32);
-        id[u]       = within[u] ? cand[i] : 0;
-        within[u]   = within[u] && rank_key(d[u], static_cast<unsigned>(id[u])) < bound;
+        for (int u = 0; u < 4; u++) {
+          const int i = i0 + u * kThreads + threadIdx.x;
+          d[u]        = i < n ? dist[i] : INFINITY;
+          within[u]   = i < n && __float_as_uint(d[u]) <= static_cast<unsigned>(bound >> 32);
+          id[u]       = within[u] ? cand[i] : 0;
+          within[u]   = within[u] && rank_key(d[u], static_cast<unsigned>(id[u])) < bound;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (within[u]) {
+            const int s = atomicAdd(&ctrl[kWithin], 1);
+            cand[s]     = id[u];
+            dist[s]     = d[u];
+          }
       }
       __syncthreads();
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (within[u]) {
-          const int s = atomicAdd(&ctrl[kWithin], 1);
-          cand[s]     = id[u];
-          dist[s]     = d[u];
+      ns       = ctrl[kWithin];
+      selected = true;
+      if (ns > R) {
+        find_range(hi_at, ns, ctrl);
+        take_smallest(hi_at, lo_at, ns, R, hist, ctrl, emit);
+        ns = R;
+      } else {
+        for (int i = threadIdx.x; i < ns; i += blockDim.x) {
+          sid[i] = cand[i];
+          sdv[i] = dist[i];
         }
-    }
-    __syncthreads();
-    ns       = ctrl[kWithin];
-    selected = true;
-    if (ns > R) {
-      find_range(hi_at, ns, ctrl);
-      take_smallest(hi_at, lo_at, ns, R, hist, ctrl, emit);
-      ns = R;
-    } else {
-      for (int i = threadIdx.x; i < ns; i += blockDim.x) {
-        sid[i] = cand[i];
-        sdv[i] = dist[i];
       }
     }
   }
@@ -1614,6 +1637,17 @@ int round_threads(const round_args& a)
 
 namespace {
 
+/// Whether this is a short wave (round_kernel), of those that take blocks of 1 024 threads only because there are few
+/// queries. us a search with the longer code and with the shorter, 64 neighbors a start point, 1, 8 and 60 queries: 16 start
+/// points and three waves 94.1 and 92.6, 95.2 and 94.4, 103.5 and 103.1; 64 114.4 and 113.6, 122.3 and 122.6, 134.0 and
+/// 134.4; 128 and two 114.0 and 113.9 (descriptors 87.2 and 86.6), 123.2 and 124.3, 137.9 and 137.1; 256 123.9 and 124.4, 139.0 and
+/// 140.4, 157.0 and 156.4. Ranked by sketch distance 32 and two, 1 and 30 queries 80.8 and 80.3, 86.9 and 87.6; 128 111.4
+/// and 113.6.
+bool short_wave(const round_args& a)
+{
+  return a.threads < 1024 && a.nmax <= (a.sketch_rank ? 2048 : 8192) && static_cast<int64_t>(a.m) * a.nmax <= 16384;
+}
+
 /// Launch that may begin while the kernel before it in the stream is finishing; the kernel waits for
 /// it where it first needs its results (wait_for_previous_kernel).
 /// Only where it matters, in batches that leave multiprocessors idle: us a search of one round and one
@@ -1637,16 +1671,21 @@ void launch_overlapped(bool early, void (*kernel)(P...), unsigned grid, unsigned
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-template <bool kRows, bool kDealt, int kThreads>
+template <bool kRows, bool kDealt, int kThreads, bool kShort = false>
 void launch_round(const round_args& a, cudaStream_t s)
 {
-  launch_overlapped(a.m <= a.sms, round_kernel<kRows, kDealt, kThreads>, static_cast<unsigned>(a.m), kThreads, round_smem_bytes(a), s, a);
+  launch_overlapped(a.m <= a.sms, round_kernel<kRows, kDealt, kThreads, kShort>, static_cast<unsigned>(a.m), kThreads, round_smem_bytes(a), s, a);
 }
 template <bool kRows, bool kDealt>
 void launch_round(const round_args& a, cudaStream_t s)
 {
   switch (round_threads(a)) {
-    case 1024: launch_round<kRows, kDealt, 1024>(a, s); break;
+    case 1024:
+      if (kRows && short_wave(a))
+        launch_round<kRows, kDealt, 1024, kRows>(a, s);
+      else
+        launch_round<kRows, kDealt, 1024>(a, s);
+      break;
     case 512: launch_round<kRows, kDealt, 512>(a, s); break;
     case 256: launch_round<kRows, kDealt, 256>(a, s); break;
     default: launch_round<kRows, kDealt, 128>(a, s); break;
@@ -1655,10 +1694,11 @@ void launch_round(const round_args& a, cudaStream_t s)
 template <bool kRows, bool kDealt>
 void allow_smem()
 {
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
-  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+  cudaFuncSetAttribute(round_kernel<kRows, kDealt, 1024, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
 }
 bool dealt(const round_args& a)
 {

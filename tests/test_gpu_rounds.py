@@ -199,6 +199,24 @@ def test_merges_of_many_keys(oracle, more_rows, starts, rerank, wave_rerank, que
     assert np.array_equal(i, np.resize(want_i, i.shape)) and np.array_equal(d, np.resize(want_d, d.shape))
 
 
+@pytest.mark.parametrize("starts,sketch_rank", [(16, False), (128, False), (129, False), (16, True), (32, True), (33, True)])
+def test_short_waves(oracle, more_rows, starts, sketch_rank):
+    """Waves of few queries and few entries have a form of their own: one query, the most it takes (16 384 entries in all) and
+    one more, on both sides of the most entries a query (128 start points of 64 neighbors, 32 by sketch distance), give
+    what the same queries give in a large batch, which is the checker's answer."""
+    idx, arrays, meta, queries = more_rows
+    kw = dict(read=64, starts=starts, waves=3, rerank=64, wave_rerank=64, sketch_rank=sketch_rank, final_rerank=32)
+    most = 16384 // (64 * starts)
+    if not sketch_rank:
+        against_checker(oracle, idx, arrays, meta, queries[:most], 16, **kw)
+    many = np.resize(queries, (200, queries.shape[1]))
+    want_d, want_i = idx.search(many, 16, **kw)
+    assert shapes(idx)[1][0] < 1024
+    for n in (1, most, most + 1):
+        d, i = idx.search(many[:n], 16, **kw)
+        assert np.array_equal(i, want_i[:n]) and np.array_equal(d.view(np.uint32), want_d[:n].view(np.uint32)), n
+
+
 def test_plans_of_several_indexes(many_rows, more_rows):
     """Two indexes searched in turn, each with a plan of its own size."""
     (one, _, _, queries), (other, _, _, others) = many_rows, more_rows
