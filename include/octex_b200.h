@@ -332,7 +332,10 @@ OCTEX_B200_EXPORT cuvsError_t octexB200SetProjection(cuvsOctexIndex_t index, int
  * "cand1_dist", "n1", "kept1_ids", "kept1_dist", "stats", "kept_ids", "kept_dist"; and
  * "shapes", int32 [2, 6], what the first round and a wave of it looked like: threads of a block, blocks of a
  * multiprocessor by shared memory, slots of the gather's hash set, words of its bits, 1 when the candidates
- * are in global memory, 1 when the fp16 rows leave the L2 cache first. *bytes returns its size; dst may be NULL to ask for the size only. */
+ * are in global memory, 1 when the fp16 rows leave the L2 cache first; and "forms", int32 [4]: the queries from
+ * which on a batch goes in two halves on two streams, 1 when the last one did, how its queries were projected
+ * (0 written out for inspection, 1 small tiles spread over the GPU, 2 many tiles a block, 3 in dimension order)
+ * and how many queries a tile of that had. *bytes returns its size; dst may be NULL to ask for the size only. */
 OCTEX_B200_EXPORT cuvsError_t octexB200Fetch(cuvsOctexIndex_t index, const char* name, void* dst,
                                              int64_t capacity, int64_t* bytes);
 

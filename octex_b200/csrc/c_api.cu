@@ -633,9 +633,9 @@ cuvsError_t octexB200Fetch(cuvsOctexIndex_t index, const char* name, void* dst, 
       pl = ix.plans.begin()->second;
     }
     const std::string n(name != nullptr ? name : "");
-    if (n == "shapes") {
+    if (n == "shapes" || n == "forms") {
       std::lock_guard<std::mutex> lock(pl->mu);
-      const auto shapes = octex_b200::detail::round_shapes(*pl);
+      const auto shapes = n == "shapes" ? octex_b200::detail::round_shapes(*pl) : octex_b200::detail::batch_forms(*pl);
       const auto size   = static_cast<int64_t>(shapes.size() * sizeof(int32_t));
       if (bytes != nullptr) *bytes = size;
       if (dst == nullptr) return;

@@ -93,17 +93,24 @@ struct tc_lookup {
 /// True when the tensor-core kernel covers this index shape (4 blocks per copy).
 bool project_tc_supported(int blocks, int ldu);
 void project_tc_setup(project_tc_plan& p, const __half* ut, int copies, int ldu, int sms);
+/// Which form a projection took (project_tc.cu says when) and how many queries its tiles have.
+enum class project_form : int { written_out, spread, bulk, ordered };
+struct project_shape {
+  project_form form = project_form::written_out;
+  int rows          = 0;
+};
 /// The job's sketch-space queries, and seg of every (query, copy), or with look.table null the codes
 /// [m, copies, L] (and Yout [m, copies * 32] fp16 when not null). *error (device-visible int)
 /// becomes non-zero when a wait inside the kernel ran out. finest = the smallest spacing (host
 /// copy): coordinates small against it take the short decode.
-void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, const __half* shift, const float* inv_f,
+auto project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, const __half* shift, const float* inv_f,
                        float finest, long long* codes, __half* Yout,
-                       const tc_lookup& look, int* error, cudaStream_t s);
+                       const tc_lookup& look, int* error, cudaStream_t s) -> project_shape;
 /// The same step for indexes of another number of blocks per copy (project_ord.cu): projection in
 /// dimension order (the order of project_ordered), decode and lookup in one kernel.
-void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
-                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, int sms, cudaStream_t s);
+auto project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
+                            const __half* shift, const float* inv_f, float finest, const tc_lookup& look, int sms, cudaStream_t s)
+  -> project_shape;
 
 /// codes [n] = cell code of each row of y [n, 8*blocks] float32 scaled by inv_f.
 void cell_codes_f32(const float* y, int64_t n, int blocks, float inv_f, long long* codes,

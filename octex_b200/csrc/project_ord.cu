@@ -145,11 +145,12 @@ __global__ void __launch_bounds__(256) project_lookup_kernel(const sketch_job jo
 
 }  // namespace
 
-void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
+auto project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut, int ldu, int copies, int L,
                             const __half* shift, const float* inv_f, float finest, const tc_lookup& look, int sms,
-                            cudaStream_t s)
+                            cudaStream_t s) -> project_shape
 {
-  if (job.m <= 0 || copies <= 0) return;
+  project_shape took{project_form::ordered, 0};
+  if (job.m <= 0 || copies <= 0) return took;
   const float tame_y = finest > 0.f ? kTameLimit * finest * 0.99f : 0.f;
   const int sk       = sketch_blocks<1>(job);
   // A block goes through its pairs in turns of 256 lanes, so one of 64 rows takes several times the latency of a turn
@@ -164,6 +165,7 @@ void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut,
     const int least = 256 / (group * copies_a_block * std::max(L, 1));
     const int rows  = std::min(kRows, (std::max({(job.m + fit - 1) / fit, least, 1}) + 3) & ~3);
     const unsigned grid = static_cast<unsigned>(sk + tiles * ((job.m + rows - 1) / rows));
+    took.rows = rows;
     kernel<<<grid, 256, 0, s>>>(job, sk, rows, ut, ldu, copies, L, shift, inv_f, tame_y, look);
   };
   switch (blocks) {
@@ -176,6 +178,7 @@ void project_lookup_ordered(const sketch_job& job, int blocks, const __half* ut,
     case 8: launch(project_lookup_kernel<8>, ord_shape<8>::kC, kGroup<8>); break;
     default: break;  // the loader rejects other block counts
   }
+  return took;
 }
 
 }  // namespace octex_b200::kernels

@@ -435,13 +435,13 @@ void project_tc_setup(project_tc_plan& p, const __half* ut, int copies, int ldu,
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(tc_smem) + 1024));
 }
 
-void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, const __half* shift, const float* inv_f,
+auto project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, const __half* shift, const float* inv_f,
                        float finest, long long* codes, __half* Yout,
-                       const tc_lookup& look, int* error, cudaStream_t s)
+                       const tc_lookup& look, int* error, cudaStream_t s) -> project_shape
 {
   // |y| below this keeps |y / spacing| under the bound of the short decode at every level
   const float tame_y = finest > 0.f ? kTameLimit * finest * 0.99f : 0.f;
-  if (job.m <= 0 || p.copies <= 0) return;
+  if (job.m <= 0 || p.copies <= 0) return {};
   CUtensorMap b;
   std::memcpy(&b, p.map_b, sizeof(b));
   const int tiles = ((p.copies + kCopies - 1) / kCopies) * ((job.m + kTileM - 1) / kTileM);
@@ -484,6 +484,8 @@ void project_decode_tc(const project_tc_plan& p, const sketch_job& job, int L, c
     mode == tc_mode::bulk ? places : sk + ((p.copies + kCopies - 1) / kCopies) * ((job.m + rows - 1) / rows));
   kernel<<<grid, kThreads, sizeof(tc_smem) + 1024, s>>>(b, job, sk, rows, p.copies, L, p.ldu / kTileK, shift, inv_f, tame_y,
                                                         codes, Yout, look, error);
+  const auto form = mode == tc_mode::taps ? project_form::written_out : mode == tc_mode::bulk ? project_form::bulk : project_form::spread;
+  return {form, rows};
 }
 
 }  // namespace octex_b200::kernels

@@ -211,6 +211,11 @@ auto round_shapes(plan const& pl) -> std::vector<int32_t>
   return out;
 }
 
+auto batch_forms(plan const& pl) -> std::vector<int32_t>
+{
+  return {static_cast<int32_t>(pl.halves_from), pl.halved ? 1 : 0, static_cast<int32_t>(pl.projected.form), pl.projected.rows};
+}
+
 /// Where a batch's queries are and its results go (device-accessible memory).
 struct batch_io {
   const float* q;
@@ -260,6 +265,8 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
 {
   const int64_t first = part != nullptr ? part->first : 0;
   const int m1 = part != nullptr ? part->count : pl.m1, mw = part != nullptr ? part->count : pl.mw;
+  pl.halved    = part != nullptr;
+  pl.projected = {};
   // marks (profiling only): one event before the first kernel and one after every step
   auto mark = [&] {
     if (marks == nullptr) return;
@@ -300,14 +307,14 @@ void run_batch(index_impl const& ix, plan& pl, batch_io const& io, cudaStream_t 
   // lookup kernel
   if (!pl.dbg.taps && pl.use_tc) {
     mark();
-    kernels::project_decode_tc(pl.tc, job, L, p.shift.as<__half>(), p.inv_f.as<float>(), finest, nullptr, nullptr,
-                               look, pl.tc_error_dev, s);
+    pl.projected = kernels::project_decode_tc(pl.tc, job, L, p.shift.as<__half>(), p.inv_f.as<float>(), finest, nullptr,
+                                              nullptr, look, pl.tc_error_dev, s);
     mark();
     mark();
   } else if (!pl.dbg.taps) {
     mark();
-    kernels::project_lookup_ordered(job, ix.blocks, p.ut.as<__half>(), p.ldu, p.copies, L, p.shift.as<__half>(),
-                                    p.inv_f.as<float>(), finest, look, pl.r1.sms, s);
+    pl.projected = kernels::project_lookup_ordered(job, ix.blocks, p.ut.as<__half>(), p.ldu, p.copies, L,
+                                                   p.shift.as<__half>(), p.inv_f.as<float>(), finest, look, pl.r1.sms, s);
     mark();
     mark();
   } else {

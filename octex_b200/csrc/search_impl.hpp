@@ -58,6 +58,10 @@ struct plan {
   bool used                      = false;
   int64_t entries       = 0;  // list and table entries that a query gathers at most
   int64_t halves_from   = 0;  // queries from which on a batch goes in two halves on two streams
+  // of the batch whose kernels were launched last (a replayed graph launches none): did it go in halves, how was its last
+  // part projected
+  bool halved = false;
+  kernels::project_shape projected;
   int64_t buffer_bytes  = 0;
   // what the arrays above are pieces of (see alloc): an allocation and its release take 0.6 ms of any size
   std::vector<dbuf> memory;
@@ -100,6 +104,10 @@ auto profile_batch(resources const& res, search_params const& sp, index const& i
 /// gather's hash set, words of its bits (0: the set), 1 when the candidates are in global memory, 1 when the
 /// fp16 rows leave the L2 cache first.
 auto round_shapes(plan const& pl) -> std::vector<int32_t>;
+
+/// The queries from which on a batch of the plan goes in two halves, 1 when the last one did, the form its projection took
+/// (kernels::project_form) and the queries of a tile of it.
+auto batch_forms(plan const& pl) -> std::vector<int32_t>;
 
 /// Throws when a kernel of an earlier batch of this plan reported that it gave up (and clears the
 /// report).

@@ -274,8 +274,20 @@ def test_tensor_core_scan_of_any_magnitude(n, dim, k, scale):
     # A chain of dim multiply-adds per norm, and dim / 16 + 2 sums of at most |a|^2 + |b|^2: at most half a unit in the
     # last place each for the former, one for the sums, which the tensor cores may truncate.
     bound = (2 * sq.max()) * 2.0 ** -24 * (dim + 2 * (dim / 16 + 2))
-    assert (full.gather(1, ids.long()) - d.double()).abs().max() < bound
+    error = full.gather(1, ids.long()) - d.double()
+    assert error.abs().max() < bound
     assert (want - d.double()).abs().max() < bound
+    # Over all of them the roundings of a chain fall either way: the root mean square of dim of at most half a unit (2^-24
+    # of the norm) is below their number's root times that, for two norms; the last three sums may all be truncated, by a
+    # unit each. A norm short of its third part is further off than that.
+    typical = sq.mean() * (2.0 ** -24 * (2 * dim) ** 0.5 + 3 * 2.0 ** -23)
+    assert error.square().mean().sqrt() < typical
+    bits = sq.float().view(torch.int32)
+    first = (bits & -65536).view(torch.float32)
+    rest = sq.float() - first
+    second = (rest.view(torch.int32) & -65536).view(torch.float32)
+    third = (rest - second).double()[ids.long()]
+    assert third.square().mean().sqrt() > 2 * typical
 
 
 def test_scans_on_two_streams():

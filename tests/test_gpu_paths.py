@@ -32,12 +32,26 @@ def inspected(idx, queries, k, **kw):
     return out, seg
 
 
+WRITTEN, SPREAD, BULK, ORDERED = range(4)  # how a batch was projected
+
+
+def forms(idx):
+    """Queries from which on a batch goes in two halves, whether the last one did, how it was projected, in tiles of how many
+    queries."""
+    return idx.fetch("forms", np.int32).tolist()
+
+
+def halves_from(idx, queries, **kw):
+    idx.search(queries[:1], 10, **kw)
+    assert forms(idx)[1] == 0
+    return forms(idx)[0]
+
+
 @pytest.mark.parametrize("blocks,dim", [(1, 48), (2, 100), (3, 96), (4, 98), (4, 64), (4, 200), (5, 64), (6, 130), (8, 64)])
 def test_projection_forms(blocks, dim):
     """Lookup in the projection: a lane per block of coordinates with the levels side by side (few
-    queries), a lane group per (query, copy), a thread per (query, copy) in blocks that go through many
-    tiles (large batches, four blocks per copy; 64 dimensions fit the operand stages, 200 do not, and
-    rows of 98 floats do not start on 16-byte boundaries). An odd number of copies leaves the last tile
+    queries), a lane group per (query, copy). (64 dimensions fit the operand stages, 200 do not, and
+    rows of 98 floats do not start on 16-byte boundaries.) An odd number of copies leaves the last tile
     half empty."""
     import torch
     from octex_b200 import synth
@@ -55,6 +69,29 @@ def test_projection_forms(blocks, dim):
         q = torch.as_tensor(np.concatenate([queries[-1:], queries[:n]]), device="cuda")[1:]
         d, i = idx.search(q, 10, **kw)
         assert same((d.cpu().numpy(), i.cpu().numpy()), want), n
+    idx.close()
+
+
+@pytest.mark.parametrize("halved", [False, True])
+@pytest.mark.parametrize("copies,dim,form", [(63, 64, BULK), (63, 98, BULK), (63, 200, BULK), (63, 320, BULK),
+                                             (8, 64, SPREAD), (7, 98, SPREAD), (8, 200, SPREAD), (8, 320, SPREAD)])
+def test_projection_of_many_queries(copies, dim, form, halved):
+    """A thread per (query, copy) in blocks that go through many tiles, whose operands fit the stages (up to 128
+    dimensions) or come in again for every tile, and tiles of few copies spread over the GPU, for whole batches and
+    for halves, which share it: as the inspected run, which is neither."""
+    import torch
+    from octex_b200 import synth
+    idx, _ = make_index(dim, rows=3000, copies=copies, blocks=4, pca_dims=64)
+    kw = dict(read=8, starts=16, waves=0 if copies > 8 else 1, rerank=32, wave_rerank=32)
+    queries = synth.plumbing(6000, dim, seed=1)
+    queries[3, 5] = queries[2500, 7] = 3.0e6  # a coordinate for the general decode
+    line = halves_from(idx, queries, **kw)
+    n = line + 515 if halved else line - 1
+    want, seg = inspected(idx, queries[:n], 10, **kw)
+    d, i = idx.search(torch.as_tensor(queries[:n], device="cuda"), 10, **kw)
+    assert forms(idx)[1:3] == [halved, form]
+    assert same((d.cpu().numpy(), i.cpu().numpy()), want)
+    assert np.array_equal(idx.fetch("seg", np.int32), seg)
     idx.close()
 
 
@@ -344,13 +381,15 @@ def test_results_are_plain_tensors():
                                           (40, 200, 150), (40, 200, 500), (64, 256, 301)])
 def test_projection_tiles_of_fewer_queries(copies, dim, n):
     """The spread form of the projection with the tiles that give every place on the GPU a block: rows that are no
-    multiple of them, wide rows where they are split and where not, the line to the bulk form, halves of a batch."""
+    multiple of them, wide rows where they are split and where not, the line to the bulk form."""
     from octex_b200 import synth
     idx, _ = make_index(dim, rows=3000, copies=copies, blocks=4, pca_dims=64)
     kw = dict(read=8, starts=16, waves=0, rerank=32)
     queries = synth.plumbing(n, dim, seed=8)
     want, seg = inspected(idx, queries, 10, **kw)
     assert same(idx.search(queries, 10, **kw), want)
+    halved, form, rows = forms(idx)[1:]
+    assert not halved and form in (SPREAD, BULK) and (form == SPREAD or rows == 128), (form, rows)
     assert np.array_equal(idx.fetch("seg", np.int32), seg)
     idx.close()
 
@@ -398,28 +437,37 @@ def test_table_of_the_same_size_is_written_over(borrow):
     fresh.close()
 
 
-@pytest.mark.parametrize("dim,kw", [
-    (64, dict(read=8, starts=16, waves=2, rerank=32, wave_rerank=32)),
-    (98, dict(read=8, starts=16, waves=0, rerank=32)),                                # rows on 8-byte boundaries
-    (48, dict(read=16, starts=512, waves=1, sketch_rank=True, final_rerank=40)),      # a block a multiprocessor
-    (64, dict(read=16, starts=32, waves=1, sketch_rank=True, final_rerank=0)),
+@pytest.mark.parametrize("dim,blocks,kw", [
+    (64, 2, dict(read=8, starts=16, waves=2, rerank=32, wave_rerank=32)),
+    (98, 2, dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)),             # rows on 8-byte boundaries
+    (98, 4, dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)),
+    (64, 4, dict(read=16, starts=32, waves=2, rerank=64, wave_rerank=64)),
+    (64, 4, dict(read=16, starts=512, waves=0, rerank=32)),                           # nothing but a first round
+    (48, 2, dict(read=16, starts=512, waves=1, sketch_rank=True, final_rerank=40)),   # a block a multiprocessor
+    (64, 4, dict(read=16, starts=32, waves=1, sketch_rank=True, final_rerank=0)),
 ])
-def test_batches_in_halves(dim, kw):
+def test_batches_in_halves(dim, blocks, kw):
     """A batch of more query blocks than the multiprocessors hold goes in two halves on two streams: the answer and
-    the segments of the inspected run, which does not, for arrays on the GPU, in ordinary and in page-locked memory;
-    one query less than the line and whole batches of odd numbers; searches before and after on another stream; what
-    a resident search repeats."""
+    the segments of the inspected run, which does not, for arrays on the GPU, in ordinary and in page-locked memory (those
+    from four million entries on; halves that are staged and halves that are not); one query less than the line and
+    batches of odd numbers; searches before and after on another stream."""
     import torch
     from octex_b200 import synth
-    idx, _ = make_index(dim, copies=6, rows=6000, table_len=32)
-    queries = synth.plumbing(2601, dim, seed=5)
-    for n in (1183, 1184, 1185, 2601):
+    copies, table_len = 40 if kw["waves"] == 0 else 6, 32
+    idx, _ = make_index(dim, copies=copies, rows=6000, blocks=blocks, table_len=table_len)
+    entries = copies * kw["read"] + kw["waves"] * kw["starts"] * table_len
+    queries = synth.plumbing((1 << 22) // entries + 2000, dim, seed=5)
+    line = halves_from(idx, queries, **kw)
+    copied = max(line, ((1 << 22) - 1) // entries + 1)  # and for ordinary memory
+    for n in (line - 1, line, line + 1, copied - 1, copied, copied + 999):
         want, seg = inspected(idx, queries[:n], 10, **kw)
         on_gpu = torch.as_tensor(queries[:n], device="cuda")
         d, i = idx.search(on_gpu, 10, **kw)
+        assert forms(idx)[1] == (n >= line), n
         assert same((d.cpu().numpy(), i.cpu().numpy()), want), n
         assert np.array_equal(idx.fetch("seg", np.int32), seg), n
         assert same(idx.search(queries[:n], 10, **kw), want), n
+        assert forms(idx)[1] == (n >= copied), n
         assert np.array_equal(idx.fetch("seg", np.int32), seg), n
         with torch.cuda.stream(torch.cuda.Stream()):
             d, i = idx.search(on_gpu, 10, **kw)
@@ -432,16 +480,77 @@ def test_batches_in_halves(dim, kw):
     idx.close()
 
 
-def test_halves_and_graphs():
+def test_halves_of_several_threads():
+    """Two threads whose batches go in halves at the same time, on one handle and the one stream it has for second halves,
+    beside a third thread whose stream is under capture; what that captured gives the same answer afterwards."""
+    import threading
+
+    import torch
+    from octex_b200 import synth
+    dim, k, n = 64, 10, 2800
+    idx, _ = make_index(dim, copies=6, blocks=4)
+    kw = dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)
+    queries = torch.as_tensor(synth.plumbing(n, dim, seed=6), device="cuda")
+    whole, _ = inspected(idx, queries.cpu().numpy(), k, **kw)
+    line = halves_from(idx, queries, **kw)
+    idx.search(queries, k, **kw)
+    assert forms(idx)[1] == 1 and n > line + 200
+    failures, finished = [], []
+    began, captured = threading.Barrier(3, timeout=60), threading.Event()
+    ids, dist = torch.empty((n, k), dtype=torch.int64, device="cuda"), torch.empty((n, k), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+
+    def search(seed):
+        rng = np.random.default_rng(seed)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            began.wait()
+            for _ in range(40):
+                a = int(rng.integers(0, n - line))
+                m = int(rng.integers(line, n - a + 1))
+                d, i = (t.cpu().numpy() for t in idx.search(queries[a:a + m], k, **kw))
+                if not same((d, i), (whole[0][a:a + m], whole[1][a:a + m])):
+                    failures.append((seed, a, m))
+        finished.append(seed)
+
+    def capture():
+        side = torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=side, capture_error_mode="thread_local"):
+            began.wait()
+            search_at(idx, queries.data_ptr(), ids.data_ptr(), dist.data_ptr(), n, dim, k, wait=False,
+                      stream=side.cuda_stream, **kw)
+            captured.wait(60)  # the capture stays open until the searches are through
+        finished.append("capture")
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=search, args=(s,)) for s in range(2)]
+    capturing = threading.Thread(target=capture)
+    for t in threads + [capturing]:
+        t.start()
+    for t in threads:
+        t.join()
+    captured.set()
+    capturing.join()
+    assert not failures and len(finished) == 3
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert same((dist.cpu().numpy(), ids.cpu().numpy()), whole)
+    del graph
+    idx.close()
+
+
+@pytest.mark.parametrize("blocks", [2, 4])
+def test_halves_and_graphs(blocks):
     """A search whose stream is captured keeps to it, and the graph gives the answer of the search in halves, also
     while other searches go in halves between its launches; arrays used in place and arrays copied."""
     import torch
     from octex_b200 import synth
     dim, k, n = 64, 10, 2500
-    idx, _ = make_index(dim, copies=6)
+    idx, _ = make_index(dim, copies=6, blocks=blocks)
     kw = dict(read=8, starts=16, waves=1, rerank=32, wave_rerank=32)
     queries = torch.as_tensor(synth.plumbing(n, dim, seed=6))
     want = [t.cpu().numpy() for t in idx.search(queries.cuda(), k, **kw)]
+    assert forms(idx)[1] == 1
     side = torch.cuda.Stream()
     for pinned in (False, True):
         q, ids, dist = queries, torch.empty((n, k), dtype=torch.int64), torch.empty((n, k))
@@ -454,10 +563,12 @@ def test_halves_and_graphs():
         torch.cuda.synchronize()
         call()
         side.synchronize()
+        assert forms(idx)[1] == 1
         assert same((dist.cpu().numpy(), ids.cpu().numpy()), want)
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=side):
             call()
+        assert forms(idx)[1] == 0
         for _ in range(2):
             ids.fill_(-5)
             torch.cuda.synchronize()
@@ -475,16 +586,21 @@ def test_halves_and_graphs():
     idx.close()
 
 
-def test_resident_batches_in_halves():
+@pytest.mark.parametrize("blocks", [2, 4])
+def test_resident_batches_in_halves(blocks):
     """The graph of a large batch holds its halves side by side, as the search before it ran them: replayed, with
     fewer queries than the search had, and again after a search of others."""
     from octex_b200 import synth
-    idx, _ = make_index(64, copies=6)
+    idx, _ = make_index(64, copies=6, blocks=blocks)
     kw = dict(read=8, starts=16, waves=2, rerank=32, wave_rerank=32)
     queries = synth.plumbing(2600, 64, seed=6)
+    captured = 0
     for first in (0, 100):
         want = idx.search(queries[first:first + 2500], 10, **kw)[1]
         for n in (2500, 2500, 1301, 40, 2500):
             idx.search_resident(n, **kw)
+            if n != captured:  # its graph was just made
+                assert forms(idx)[1] == (n >= forms(idx)[0]), n
+            captured = n
             assert np.array_equal(idx.fetch("kept_ids", np.int64, (n, -1))[:, :10], want[:n]), n
     idx.close()
