@@ -192,8 +192,9 @@ __device__ __forceinline__ unsigned long long met(unsigned long long mine, int s
 }
 
 /// src[0, count) and kNoKey up to `width` (a power of two, 64 at least) in ascending order into key [width], another
-/// array: the network of bitonic_sort with 64 keys to a warp, two a lane, so that only steps of 64 places and more go
-/// through shared memory and have barriers (6 of the 45 of 512 keys). All threads of the block call it.
+/// array: the network of bitonic_sort with 64 keys to a warp, two a lane, so that the steps of 32 places and fewer of a
+/// size take one barrier together (512 keys: 10 barriers, where one after every step is 45). All threads of the block
+/// call it.
 __device__ __forceinline__ void sort_keys(const unsigned long long* src, int count, unsigned long long* key, int width)
 {
   const int lane = threadIdx.x & 31, warp0 = (threadIdx.x >> 5) * 64, all = blockDim.x * 2;
@@ -480,9 +481,9 @@ constexpr int kCounted = 128;  // new keys whose places are counted at most (see
 /// The first `want` keys of the ascending list old[0, n) and the m distinct keys add[0, m), none of them in
 /// the list, into dst, ascending; order [m] is scratch. A new key's place is the number of new keys below
 /// it, counted, and of old ones, found by halving; an old key's is its own plus the new ones below it,
-/// halving in their order. One barrier where a sorting network over all of them has 36 (256 keys) to 55
-/// (1 024 keys). Counting is quadratic in the new keys: of more than kCounted the caller has put them into order
-/// already, ascending (sort_keys). us a search with all places counted, and with kCounted of 64, 128 and 256: 1 000
+/// halving in their order. One barrier where a sorting network over all of them, with one after every step, has 36
+/// (256 keys) to 55 (1 024 keys). Counting is quadratic in the new keys: of more than kCounted the caller has put them into order
+/// already, ascending (sort_keys, with barriers of its own). us a search with all places counted, and with kCounted of 64, 128 and 256: 1 000
 /// queries, 512 kept and 512 reranked rows 1 470, 1 427, 1 429 and 1 424; 2 000, 256 and 256 1 550, 1 541, 1 544 and
 /// 1 553; 2 500 ranked by sketch distance into 512 3 265, 3 154, 3 154 and 3 158. All threads of the block call it.
 __device__ __forceinline__ void merge_sorted(const unsigned long long* old, int n, const unsigned long long* add, int m,
