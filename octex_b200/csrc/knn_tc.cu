@@ -36,13 +36,13 @@
 //
 // What bounds it: the MMAs. One of 128 x 128 x 16 with both operands in shared memory takes 101 cycles instead
 // of 64 (128 bytes a cycle would be needed), the norms one more of them, and a tile with nothing looked at 2 200
-// of the 2 800 cycles that it takes (200 001 x 128, K = 64: 11.4 of 14.3 ms; 64 dimensions 8.2 of 11.9); the rest is
+// of the 2 700 cycles that it takes (200 001 x 128, K = 64: 11.4 of 13.8 ms; 64 dimensions 8.2 of 11.3); the rest is
 // what the four warps of a set wait for one another when one of them looks through its improvements.
 // 200 001 x 128, K = 64, ms: 133 with a list update per improvement; 20.5 with buffers in shared memory that the
 // epilogue merges itself and norms it adds; 18.3 with list warps and norms in the MMAs; 15.0 with the groups read
 // again from TMEM (instead of 64 columns kept in registers until it is known which are wanted); 14.2 with the next 32
-// columns on their way while 32 are looked at, 14.5 with the norms last, 14.3 looking through without votes. Two
-// warps per row, a half of the columns each: 18.7.
+// columns on their way while 32 are looked at, 14.5 with the norms last, 14.3 looking through without votes, 13.8 with the
+// ends of the items merged by all warps. Two warps per row, a half of the columns each: 18.7.
 //
 // Roles: warp 0 issues the TMA copies, warps 1 and 2 the MMAs of a set (one lane issues), warp 3 makes the norm
 // operands; eight epilogue warps, four per set, one per quarter of the TMEM lanes; four list warps, a quarter of the rows each.
@@ -822,15 +822,16 @@ __global__ void __launch_bounds__(kKnnThreads, 1)
 
 /// Query rows that stay in shared memory with as many stages as fit behind them, three at least (256 dimensions).
 /// Beyond that they come in again with every tile, in four stages.
-/// Four places for groups: a warp looks through them when there is no room for two more in one of its lanes, and all are noted
-/// at once, so at most kNoted / 4. More hold up what the lists publish, fewer are looked through too often; us a call with
-/// six, four, three and two: 200 001 x 128, K = 64 14 820, 14 560, 14 860 and 16 470, 100 000 x 128, K = 120 5 822, 5 580,
-/// 5 795 and 6 725, 1 000 x 128, K = 64 272, 245, 236 and 232 (248 with lists that the epilogue merged alone). Where query rows
-/// do not stay three leave the room for the fourth stage; us with four places and three stages, three and four, 50 000 rows, K = 10 and 64:
-/// 768 dimensions 4 658 and 4 516, 6 567 and 6 353, 960 5 763 and 5 508, 8 124 and 7 739, 512 3 204 and 3 190, 4 488 and 4 482.
+/// Four places for groups: a warp looks through them when there is no room for two more in one of its lanes, and all are
+/// noted at once, so at most kNoted / 4. More hold up what the lists publish, fewer are looked through too often; us a call
+/// with six, four, three and two: 200 001 x 128, K = 64 14 820, 14 560, 14 860 and 16 470, 100 000 x 128, K = 120 5 822,
+/// 5 580, 5 795 and 6 725, 1 000 x 128, K = 64 272, 245, 236 and 232 (248 with lists that the epilogue merged alone). Where
+/// query rows do not stay three leave the room for the fourth stage; us with four places and three stages and with three and
+/// four, 50 000 rows, K = 10 and 64: 768 dimensions 4 658 and 4 516, 6 567 and 6 353, 960 5 763 and 5 508, 8 124 and 7 739,
+/// 512 3 204 and 3 190, 4 488 and 4 482.
 /// What these take beyond a scan whose epilogue merges alone and adds the norms itself (3 070 at 512 dimensions and K = 10,
-/// 4 420 at 768; 4 610 and 6 350 at K = 64) are the MMAs of the norms; norms in the epilogue of this one 3 560 and 4 910, since
-/// they come out of the shared memory the MMAs wait for. One set that stays instead of two that do not, 264 to 576
+/// 4 420 at 768; 4 610 and 6 350 at K = 64) are the MMAs of the norms; norms in the epilogue of this one 3 560 and 4 910,
+/// since they come out of the shared memory the MMAs wait for. One set that stays instead of two that do not, 264 to 576
 /// dimensions: 3 080 and 4 160 at 512.
 knn_shape choose_shape(int nkb)
 {

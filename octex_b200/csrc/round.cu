@@ -482,9 +482,9 @@ constexpr int kCounted = 128;  // new keys whose places are counted at most (see
 /// the list, into dst, ascending; order [m] is scratch. A new key's place is the number of new keys below
 /// it, counted, and of old ones, found by halving; an old key's is its own plus the new ones below it,
 /// halving in their order. One barrier where a sorting network over all of them, with one after every step, has 36
-/// (256 keys) to 55 (1 024 keys). Counting is quadratic in the new keys: of more than kCounted the caller has put them into order
-/// already, ascending (sort_keys, with barriers of its own). us a search with all places counted, and with kCounted of 64, 128 and 256: 1 000
-/// queries, 512 kept and 512 reranked rows 1 470, 1 427, 1 429 and 1 424; 2 000, 256 and 256 1 550, 1 541, 1 544 and
+/// (256 keys) to 55 (1 024 keys). Counting is quadratic in the new keys: more than kCounted the caller has put into
+/// ascending order (sort_keys, with barriers of its own). us a search with all places counted, and with kCounted of 64,
+/// 128 and 256: 1 000 queries, 512 kept and 512 reranked rows 1 470, 1 427, 1 429 and 1 424; 2 000, 256 and 256 1 550, 1 541, 1 544 and
 /// 1 553; 2 500 ranked by sketch distance into 512 3 265, 3 154, 3 154 and 3 158. All threads of the block call it.
 __device__ __forceinline__ void merge_sorted(const unsigned long long* old, int n, const unsigned long long* add, int m,
                                              unsigned long long* order, int want, unsigned long long* dst)
