@@ -224,13 +224,15 @@ def test_tensor_core_neighbor_scan(n, dim, k):
 @pytest.mark.parametrize("n,dim,k,order", [
     (129, 8, 1, "random"), (257, 64, 32, "random"), (641, 72, 33, "falling"), (1000, 192, 65, "random"),
     (999, 256, 64, "falling"), (900, 264, 122, "random"), (40, 128, 64, "random"), (3001, 128, 64, "ties"),
-    (19101, 16, 64, "falling"), (38001, 128, 10, "ties"), (2100, 520, 40, "falling"), (38001, 264, 33, "ties")])
+    (19101, 16, 64, "falling"), (38001, 128, 10, "ties"), (2100, 520, 40, "falling"), (38001, 264, 33, "ties"),
+    (19001, 64, 40, "falling")])
 def test_tensor_core_scan_is_exact(n, dim, k, order):
     """The tcgen05 scan on whole numbers, where every product and sum is exact: ids and distances as
     float64 has them, equal distances by ascending id. Query rows that stay in shared memory (to 256
     dimensions) and rows that do not (264, 520); lists of one, two and four keys a
     lane; fewer rows than the list is long; one set, two sets and both kinds of item (38001 rows on
-    148 multiprocessors), whose lists are merged by warps of either role; rows that come nearer with every id up to a row's own (each one an
+    148 multiprocessors), a last item of two sets with rows for one (19001), whose lists are merged by warps of either
+    role; rows that come nearer with every id up to a row's own (each one an
     improvement), and many equal rows."""
     import torch
     g = torch.Generator("cuda").manual_seed(n)
